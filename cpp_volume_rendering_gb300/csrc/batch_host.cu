@@ -14,26 +14,29 @@ using namespace cvr::ctxutil;
 struct cvr_batch {
   cvr_ctx* ctx = nullptr;
   int n_jobs = 0;
-  BatchExtJob* d_ext = nullptr;
-  int n_ext = 0;
-  unsigned ext_blocks = 0;
-  int ext_max_table = 0;
+  BatchExtJob* d_ext = nullptr;           // the jobs on SATs, then those on box tables
+  int n_ext = 0, n_box = 0;
+  unsigned ext_blocks = 0, box_blocks = 0;
+  int ext_max_table = 0;                  // longest shadow table of either
   int ext_variant = 0;
   int ext_threads = 128;
   float4* d_tables = nullptr;
+  float* d_cuts = nullptr;
   int n_sur = 0;
   bool sur_tex = false;
-  unsigned int* d_counters = nullptr;  // [0] extinction tiles, [1 + k] surrogate rays of launch k
+  unsigned int* d_counters = nullptr;  // [0] extinction tiles, [1] box-table tiles, [2 + k] surrogate rays of launch k
   unsigned long long* d_stats = nullptr;  // 3 per job, in the caller's job order
   bool ext_compact = false;
   bool ext_aligned = false;  // every job: an aligned shadow table and aligned AO boxes (or AO off)
   std::vector<uint4*> sat32;              // the batch's own compact SATs, one per volume slot used
   std::vector<uint4*> walks;              // their walk tables, one per (slot, walk axis, depth) in use
   std::vector<long long> walk_keys;
+  std::vector<std::unique_ptr<BoxTables>> boxes;  // box tables, one set per (slot, walk axis, interval) in use
+  std::vector<long long> box_keys;
   cudaGraphExec_t graph = nullptr;
   ~cvr_batch() {
     if (graph) cudaGraphExecDestroy(graph);
-    void* bufs[] = {d_ext, d_tables, d_counters, d_stats};
+    void* bufs[] = {d_ext, d_tables, d_cuts, d_counters, d_stats};
     for (void* p : bufs)
       if (p) cudaFree(p);
     for (uint4* p : sat32)
@@ -124,6 +127,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   double slot_vmax[CVR_MAX_VOLUMES] = {};
   bool all_compact = c->compact_sat;
   std::vector<std::vector<float4>> tables;
+  std::vector<std::unique_ptr<ShadowBoxTable>> aligned;  // of the jobs box tables can serve, else null
   std::vector<SurLaunch> sur;  // the surrogate jobs in launches of up to kSurLaunchJobs
   unsigned long long sur_positions = 0;
   const int keep = c->cur_slot;
@@ -149,8 +153,6 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       ext_slot.push_back(j.volume);
       J.f = f;
       J.blocks_x = (unsigned)((j.width + f.tile_w - 1) / f.tile_w);
-      J.first_block = b->ext_blocks;
-      b->ext_blocks += J.blocks_x * (unsigned)((j.height + f.tile_h - 1) / f.tile_h);
       std::vector<float4> t;
       if (table) {
         J.tn = table->n; J.tax = table->axis; J.tiw = table->interval; J.tvmin = table->vmin; J.tvmax = table->vmax;
@@ -160,6 +162,8 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
         b->ext_max_table = std::max(b->ext_max_table, table->n);
       }
       tables.push_back(std::move(t));
+      aligned.emplace_back(table && table->aligned && table->n > 0 && (J.e.ao_aligned || !J.e.apply_occ)
+                               ? new ShadowBoxTable(*table) : nullptr);
       ext.push_back(J);
     } else {
       SurJob J{};
@@ -220,12 +224,62 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
         ext[k].e.sat.inv_scale32 = inv[ext_slot[k]];
       }
       b->ext_compact = true;
+    }
+  }
+  // Box tables for the jobs whose boxes all have integer widths: a batch is
+  // run many times, so they are built whenever they fit (all sets together
+  // within a quarter of the GPU).  The first pass collects every job's widths
+  // in its set, the second takes the jobs whose tables are all there.
+  std::vector<std::unique_ptr<BoxWalk>> walks(ext.size());
+  size_t box_budget = 0, mem_free = 0;
+  if (st == CVR_OK && !ext.empty()) {
+    CK(c, cudaMemGetInfo(&mem_free, &box_budget));
+    box_budget /= 4;
+  }
+  for (int pass = 0; pass < 2 && st == CVR_OK; ++pass) {
+    for (size_t k = 0; k < ext.size() && st == CVR_OK; ++k) {
+      if (!aligned[k]) continue;
+      BatchExtJob& J = ext[k];
+      const ShadowBoxTable& t = *aligned[k];
+      int widths;
+      std::memcpy(&widths, &t.tx[0].w, sizeof widths);
+      const long long key = ((long long)ext_slot[k] * 3 + t.axis) * 1024 + ((widths >> (10 * t.axis)) & 1023);
+      size_t at = std::find(b->box_keys.begin(), b->box_keys.end(), key) - b->box_keys.begin();
+      if (at == b->box_keys.size()) {
+        b->box_keys.push_back(key);
+        b->boxes.emplace_back(new BoxTables());
+      }
+      select_slot(c, ext_slot[k]);
+      const int n[3] = {c->nx + 2, c->ny + 2, c->nz + 2};
+      const bool cm = b->ext_compact;
+      const BoxSource src{cm ? nullptr : c->d_sat, cm ? reinterpret_cast<const unsigned*>(J.e.sat.sat32) : nullptr, 4, 3,
+                          cm ? J.e.sat.inv_scale32 : J.e.sat.inv_scale, {n[0], n[1], n[2]}};
+      std::unique_ptr<BoxWalk> w(new BoxWalk());
+      BoxPlan plan;
+      ExtArgs e = J.e;
+      const unsigned long long gen = 1;  // one source per slot
+      if (!box_plan(*b->boxes[at], gen, n, t, -1.0, &e, w.get(), &plan)) continue;
+      if (pass == 1 && plan.missing > 0) continue;
+      size_t held = 0;
+      for (size_t i = 0; i < b->boxes.size(); ++i)
+        if (i != at) held += b->boxes[i]->ao.cap + b->boxes[i]->sdw.cap;
+      if (held + plan.ao_bytes + plan.sdw_bytes > box_budget) continue;
+      bool used = false;
+      st = box_build(c, *b->boxes[at], src, gen, plan, &e, &used);
+      if (st == CVR_OK && used && pass == 1) {
+        J.e = e;
+        walks[k] = std::move(w);
+      }
+    }
+  }
+  if (st == CVR_OK && b->ext_compact) {
+    {
       // walk tables of these compact tables, one per (slot, walk axis, box
       // depth) that the jobs with an aligned directional table use (a job's
       // table holds its texel offsets after lo and hi when it is aligned)
       for (size_t k = 0; k < ext.size() && st == CVR_OK && c->walk_tables; ++k) {
         BatchExtJob& J = ext[k];
-        if (J.tn <= 0 || tables[k].size() != 3 * (size_t)J.tn) continue;
+        if (walks[k] || J.tn <= 0 || tables[k].size() != 3 * (size_t)J.tn) continue;
         const int slot = ext_slot[k], axis = J.tax, w = (int)std::nearbyint(J.e.interval);
         if (w < 1 || w > 1023) continue;
         const long long key = ((long long)slot * 3 + axis) * 1024 + w;
@@ -240,7 +294,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
           if (e != cudaSuccess) { st = cuda_fail(c, e, "cvr_batch_create: walk table"); break; }
           b->walks.push_back(d);
           b->walk_keys.push_back(key);
-          e = launch_sat_walk(tab[slot], d, sx, sy, sz, axis, w, c->stream);
+          e = launch_sat_walk(J.e.sat.sat32, d, sx, sy, sz, axis, w, c->stream);
           if (e != cudaSuccess) { st = cuda_fail(c, e, "cvr_batch_create: walk table"); break; }
         }
         J.e.walk = WalkView{d, axis, w};
@@ -252,32 +306,68 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   if (!sur.empty() && (!c->mlp || !c->mlp->err)) return fail(c, CVR_ERR_NOT_READY, "cvr_batch_create: no network");
   b->ext_variant = c->variant;
   b->ext_threads = (c->tile_w / 8) * (c->tile_h / 4) * 32;
-  b->n_ext = (int)ext.size();
-  if (b->n_ext) {
-    // shadow tables: one region per job, pointers patched in
-    size_t total = 0;
-    for (auto& t : tables) total += t.size();
-    if (total) {
-      CK(c, cudaMalloc((void**)&b->d_tables, sizeof(float4) * total));
-      size_t off = 0;
+  if (!ext.empty()) {
+    // jobs on SATs first, then those on box tables, each group's tiles numbered from 0
+    std::vector<BatchExtJob> jobs_dev;
+    std::vector<float4> table_dev;
+    std::vector<float> cuts;
+    std::vector<size_t> table_at, cut_at;
+    b->ext_aligned = true;
+    for (int group = 0; group < 2; ++group) {
+      unsigned blocks = 0;
       for (size_t k = 0; k < ext.size(); ++k) {
-        if (tables[k].empty()) continue;
-        CK(c, cudaMemcpy(b->d_tables + off, tables[k].data(), sizeof(float4) * tables[k].size(), cudaMemcpyHostToDevice));
-        ext[k].tlo = b->d_tables + off;
-        ext[k].thi = b->d_tables + off + ext[k].tn;
-        ext[k].ttx = tables[k].size() == 3 * (size_t)ext[k].tn ? b->d_tables + off + 2 * ext[k].tn : nullptr;
-        off += tables[k].size();
+        if ((walks[k] != nullptr) != (group == 1)) continue;
+        BatchExtJob J = ext[k];
+        J.first_block = blocks;
+        blocks += J.blocks_x * (unsigned)((J.f.H + J.f.tile_h - 1) / J.f.tile_h);
+        table_at.push_back(table_dev.size());
+        cut_at.push_back(cuts.size());
+        if (group == 1) {
+          const BoxWalk& w = *walks[k];
+          table_dev.insert(table_dev.end(), w.o, w.o + w.n);
+          cuts.insert(cuts.end(), w.cut, w.cut + w.n);
+          J.bpad_a = w.pad_a; J.bpad_b = w.pad_b; J.bpad_w = w.pad_w; J.bfirst = w.first; J.bper = w.per;
+        } else {
+          if (!J.e.sat.sat32 && !J.e.sat.sat) return fail(c, CVR_ERR_NOT_READY, "cvr_batch_create: a job without a SAT");
+          if (!aligned[k]) b->ext_aligned = false;
+          table_dev.insert(table_dev.end(), tables[k].begin(), tables[k].end());
+        }
+        (group ? b->n_box : b->n_ext) += 1;
+        jobs_dev.push_back(J);
+      }
+      (group ? b->box_blocks : b->ext_blocks) = blocks;
+    }
+    if (!table_dev.empty()) {
+      CK(c, cudaMalloc((void**)&b->d_tables, sizeof(float4) * table_dev.size()));
+      CK(c, cudaMemcpy(b->d_tables, table_dev.data(), sizeof(float4) * table_dev.size(), cudaMemcpyHostToDevice));
+    }
+    if (!cuts.empty()) {
+      CK(c, cudaMalloc((void**)&b->d_cuts, sizeof(float) * cuts.size()));
+      CK(c, cudaMemcpy(b->d_cuts, cuts.data(), sizeof(float) * cuts.size(), cudaMemcpyHostToDevice));
+    }
+    for (size_t k = 0; k < jobs_dev.size(); ++k) {
+      BatchExtJob& J = jobs_dev[k];
+      const float4* base = b->d_tables + table_at[k];
+      if ((int)k >= b->n_ext) {
+        J.bo = base;
+        J.bcut = b->d_cuts + cut_at[k];
+      } else if (J.tn > 0) {
+        J.tlo = base;
+        J.thi = base + J.tn;
+        const size_t next = k + 1 < jobs_dev.size() ? table_at[k + 1] : table_dev.size();
+        J.ttx = next - table_at[k] == 3 * (size_t)J.tn ? base + 2 * J.tn : nullptr;
       }
     }
-    for (const BatchExtJob& J : ext)
-      if (!J.e.sat.sat32 && !J.e.sat.sat) return fail(c, CVR_ERR_NOT_READY, "cvr_batch_create: a job without a SAT");
-    b->ext_aligned = true;
-    for (const BatchExtJob& J : ext)
-      if (!J.ttx || !(J.e.ao_aligned || !J.e.apply_occ)) b->ext_aligned = false;
-    CK(c, cudaMalloc((void**)&b->d_ext, sizeof(BatchExtJob) * ext.size()));
-    CK(c, cudaMemcpy(b->d_ext, ext.data(), sizeof(BatchExtJob) * ext.size(), cudaMemcpyHostToDevice));
+    CK(c, cudaMalloc((void**)&b->d_ext, sizeof(BatchExtJob) * jobs_dev.size()));
+    CK(c, cudaMemcpy(b->d_ext, jobs_dev.data(), sizeof(BatchExtJob) * jobs_dev.size(), cudaMemcpyHostToDevice));
+    // the compact SATs were the box tables' source: they go when no job reads them
+    if (b->n_ext == 0) {
+      CK(c, cudaStreamSynchronize(c->stream));
+      for (uint4* p : b->sat32) cudaFree(p);
+      b->sat32.clear();
+    }
   }
-  const size_t n_counters = 1 + sur.size();
+  const size_t n_counters = 2 + sur.size();
   CK(c, cudaMalloc((void**)&b->d_counters, sizeof(unsigned int) * n_counters));
   // capture: counter and statistics resets, then the persistent launches
   cudaGraph_t g = nullptr;
@@ -287,8 +377,11 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   if (e == cudaSuccess && b->n_ext)
     e = launch_batch_extinction(b->d_ext, b->n_ext, b->ext_blocks, b->d_counters, c->tf_n, b->ext_max_table,
                                 b->ext_threads, b->ext_variant, b->ext_compact, b->ext_aligned, c->stream);
+  if (e == cudaSuccess && b->n_box)
+    e = launch_batch_box(b->d_ext + b->n_ext, b->n_box, b->box_blocks, b->d_counters + 1, c->tf_n, b->ext_max_table,
+                         b->ext_threads, b->ext_variant, c->stream);
   for (size_t k = 0; k < sur.size() && e == cudaSuccess; ++k)
-    e = launch_batch_surrogate(sur[k], c->tf_n, b->sur_tex, b->ext_variant, b->d_counters + 1 + k, c->mlp->err,
+    e = launch_batch_surrogate(sur[k], c->tf_n, b->sur_tex, b->ext_variant, b->d_counters + 2 + k, c->mlp->err,
                                c->stream);
   cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
   if (e != cudaSuccess || e2 != cudaSuccess) {

@@ -288,6 +288,17 @@ cudaError_t launch_sat_build(const void* vox, int dtype, int nx, int ny, int nz,
   return cudaGetLastError();
 }
 
+cudaError_t launch_sat_build32(const void* vox, int dtype, int nx, int ny, int nz, const unsigned* lut, unsigned* out,
+                               cudaStream_t st) {
+  const int R = sat_plane_rows<unsigned>(nx + 2);
+  if (R == 0) return sat_build_lines(vox, dtype, nx, ny, nz, lut, out, st);
+  cudaError_t e = sat_planes(vox, dtype, nx, ny, nz, lut, out, R, st);
+  if (e != cudaSuccess) return e;
+  const long long columns = (long long)(nx + 2) * (ny + 2);
+  k_sat_zscan<unsigned><<<(unsigned)((columns + 255) / 256), 256, 0, st>>>(out, columns, nz + 2);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_sat_build_quads(const void* vox, int dtype, int nx, int ny, int nz, const unsigned* lut,
                                    unsigned* scratch, uint4* out, cudaStream_t st) {
   const int sx = nx + 2, sy = ny + 2, sz = nz + 2;
@@ -396,6 +407,80 @@ cudaError_t launch_sat_walk(const uint4* quads, uint4* out, int sx, int sy, int 
 cudaError_t launch_sat_quads(const unsigned* sat, uint4* out, int sx, int sy, int sz, cudaStream_t st) {
   const long long cells = (long long)sx * sy * sz;
   k_sat_quads<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(sat, out, sx, sy, cells);
+  return cudaGetLastError();
+}
+
+// ------------------------------------------------------------- box tables
+// All tables of a set in one launch: a warp per row segment of 31 cells (lane
+// 31 only supplies the last cell's successor), 8 rows per CTA, kBoxPlanes
+// planes per thread, the sums of the box's rectangle in the planes at its two
+// ends.  Along a walk of interval 2 (the default) a plane's rectangle is the
+// low end of one cell and the high end of the cell two planes before: a ring
+// of two keeps it, four loads a cell instead of eight.
+constexpr int kBoxRow = 31, kBoxRows = 8, kBoxPlanes = 16;
+template <class W>
+__global__ void __launch_bounds__(32 * kBoxRows) k_box_tables(BoxSource src, const __grid_constant__ BoxTableSet set,
+                                                               float* __restrict__ out) {
+  const int ti = blockIdx.z % set.n, c0 = (blockIdx.z / set.n) * kBoxPlanes;
+  const BoxTableDesc& d = set.t[ti];
+  const int lane = threadIdx.x & 31;
+  const int a = blockIdx.x * kBoxRow + lane, b = blockIdx.y * kBoxRows + (threadIdx.x >> 5);
+  if ((int)(blockIdx.x * kBoxRow) >= d.g.na || b >= d.g.nb || c0 >= d.g.nc) return;  // whole warps
+  const size_t strides[3] = {1, (size_t)src.n[0], (size_t)src.n[0] * src.n[1]};
+  size_t lo[2], hi[2];  // element offsets of the box's low and high corner along the fastest and middle axis
+  const int at[2] = {a, b};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int ax = d.axis[i], n = src.n[ax], p = at[i] - d.pad[i];
+    lo[i] = strides[ax] * (size_t)min(max(p, 0), n - 1);
+    hi[i] = strides[ax] * (size_t)min(max(p + d.w[i], 0), n - 1);
+  }
+  const size_t i00 = lo[0] + lo[1], i10 = hi[0] + lo[1], i01 = lo[0] + hi[1], i11 = hi[0] + hi[1];
+  const int nc = src.n[d.axis[2]];
+  const size_t sc = strides[d.axis[2]];
+  auto at_ = [&](size_t i) -> W {
+    if constexpr (sizeof(W) == 8) return (W)__ldg(src.s64 + i);
+    else return __ldg(src.s32 + i * (size_t)src.stride + src.first);
+  };
+  auto rect = [&](int c) -> W {
+    const size_t o = sc * (size_t)min(max(c, 0), nc - 1);
+    return at_(o + i11) - at_(o + i01) - at_(o + i10) + at_(o + i00);
+  };
+  auto value = [&](W v) {
+    if constexpr (sizeof(W) == 8) return ll_to_float((long long)v) * src.scale;
+    else return (float)(int)v * src.scale;
+  };
+  const bool store = lane < kBoxRow && a < d.g.na;
+  float2* dst = reinterpret_cast<float2*>(out) + d.cell + (size_t)b * d.g.na + a;
+  auto put = [&](int c, float v) {
+    const float next = __shfl_down_sync(0xffffffffu, v, 1);
+    if (store) dst[(size_t)c * d.g.nab] = make_float2(v, next);
+  };
+  const int end = min(c0 + kBoxPlanes, d.g.nc), p0 = c0 - d.pad[2];
+  if (d.w[2] == 2) {
+    W r0 = rect(p0), r1 = rect(p0 + 1);
+    for (int c = c0; c < end; ++c) {
+      const W r2 = rect(c - d.pad[2] + 2);
+      put(c, value(r2 - r0));
+      r0 = r1;
+      r1 = r2;
+    }
+  } else {
+    for (int c = c0; c < end; ++c) put(c, value(rect(c - d.pad[2] + d.w[2]) - rect(c - d.pad[2])));
+  }
+}
+
+cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, float* out, cudaStream_t st) {
+  if (set.n == 0) return cudaSuccess;
+  int na = 0, nb = 0, nc = 0;
+  for (int i = 0; i < set.n; ++i) {
+    na = std::max(na, set.t[i].g.na); nb = std::max(nb, set.t[i].g.nb); nc = std::max(nc, set.t[i].g.nc);
+  }
+  const dim3 grid((na + kBoxRow - 1) / kBoxRow, (nb + kBoxRows - 1) / kBoxRows,
+                  ((nc + kBoxPlanes - 1) / kBoxPlanes) * set.n);
+  if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
+  if (src.s32) k_box_tables<unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+  else k_box_tables<unsigned long long><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
   return cudaGetLastError();
 }
 

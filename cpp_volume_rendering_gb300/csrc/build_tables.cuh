@@ -20,6 +20,35 @@ cudaError_t launch_sat_walk(const uint4* quads, uint4* out, int sx, int sy, int 
 // The x-y predecessor-quad layout of a finished plain (sx, sy, sz) table.
 cudaError_t launch_sat_quads(const unsigned* sat, uint4* out, int sx, int sy, int sz, cudaStream_t st);
 
+// The plain 32-bit table (prefix sums of a 32-bit lut modulo 2^32, x fastest)
+// in out: the source of a compact frame's box tables.
+cudaError_t launch_sat_build32(const void* vox, int dtype, int nx, int ny, int nz, const unsigned* lut, unsigned* out,
+                               cudaStream_t st);
+
+// One box table (BoxView): its grid and first cell; per table axis (fastest,
+// middle, slowest) the SAT axis it runs along, the box width and the pad.
+struct BoxTableDesc {
+  BoxGrid g;
+  unsigned cell;
+  int axis[3], w[3], pad[3];
+};
+constexpr int kMaxBoxTables = 96;
+struct BoxTableSet {
+  int n;
+  BoxTableDesc t[kMaxBoxTables];
+};
+// The prefix sums the tables are differences of: the int64 table (s64), or a
+// 32-bit one, element i at s32[i * stride + first] (the plain table: 1, 0; the
+// predecessor quads: 4, 3).  scale: 2^-F of its fixed point.
+struct BoxSource {
+  const long long* s64;
+  const unsigned* s32;
+  int stride, first;
+  float scale;
+  int n[3];  // SAT extents
+};
+cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, float* out, cudaStream_t st);
+
 // Builds every level of P (dims/offsets/grid filled by the caller) into data;
 // levels with a separable form use scratch (scratch_floats floats; see
 // pyramid_scratch_floats), the others the direct 343-tap kernels.

@@ -189,8 +189,53 @@ cvr_status frame_args(cvr_ctx* c, const cvr_camera* cam, const void* params, flo
   return CVR_OK;
 }
 
+static cvr_status upload_lut32(cvr_ctx* c, const std::vector<unsigned>& q);
+
+// The frame's box tables (vmax: the extent its compact table would span, 0:
+// int64 sums): *walk its walk when the frame reads them.
+static cvr_status frame_boxes(cvr_ctx* c, double vmax, const FrameArgs& f, const ShadowBoxTable& t, ExtArgs* a,
+                              const BoxWalk** walk) {
+  const int n[3] = {c->nx + 2, c->ny + 2, c->nz + 2};
+  const size_t cells = (size_t)n[0] * n[1] * n[2];
+  int F = kNoCompactSat;
+  const bool compact = vmax > 0.0 && cells < kCompactMaxCells && compact_fixed_point(c, vmax, &F);
+  if (!compact) F = kNoCompactSat;
+  const unsigned long long gen = box_gen(c->sat_gen, F);
+  if (!c->box_walk) c->box_walk.reset(new BoxWalk());
+  BoxPlan plan;
+  if (!box_plan(c->box, gen, n, t, (double)f.W * f.H, a, c->box_walk.get(), &plan)) return CVR_OK;
+  BoxSource src{nullptr, nullptr, 1, 0, (float)std::ldexp(1.0, -(compact ? F : c->sat_frac_bits)), {n[0], n[1], n[2]}};
+  if (plan.missing > 0 && compact) {
+    if (c->boxsrc_gen != gen) {
+      c->boxsrc_gen = 0;
+      cudaError_t e = ensure(c->d_boxsrc, c->boxsrc_cap, cells * sizeof(unsigned));
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return CVR_OK;
+      }
+      if (e != cudaSuccess) return cuda_fail(c, e, "box table source");
+      std::vector<unsigned> q;
+      compact_values(c->sat_ext, F, &q);
+      cvr_status st = upload_lut32(c, q);
+      if (st != CVR_OK) return st;
+      CK(c, launch_sat_build32(c->d_vol, c->dtype, c->nx, c->ny, c->nz, c->d_lut32, c->d_boxsrc, c->stream));
+      c->boxsrc_gen = gen;
+    }
+    src.s32 = c->d_boxsrc;
+  } else if (plan.missing > 0) {
+    cvr_status st = ensure_sat(c);
+    if (st != CVR_OK) return st;
+    src.s64 = c->d_sat;
+  }
+  bool used = false;
+  cvr_status st = box_build(c, c->box, src, gen, plan, a, &used);
+  if (st == CVR_OK && used) *walk = c->box_walk.get();
+  return st;
+}
+
 cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light, const FrameArgs& f, ExtArgs* eo,
-                    const ShadowBoxTable** table, double* vmax_out) {
+                    const ShadowBoxTable** table, double* vmax_out, const BoxWalk** walk_out) {
+  if (walk_out) *walk_out = nullptr;
   if (!c->sat_ready) return fail(c, CVR_ERR_NOT_READY, "cvr_render: extinction SAT not built");
   if (p->apply_occlusion && (p->ao_n_shells < 1 || p->ao_n_shells > CVR_MAX_AO_SHELLS))
     return fail(c, CVR_ERR_INVALID_ARG, "ao_n_shells must be in [1, 32]");
@@ -241,6 +286,7 @@ cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light,
       cone_extent = std::max(zm * (std::tan(lean + ang) - std::tan(lean - ang)) + msc, iw);
     }
   }
+  double vmax = 0.0;  // 0: no compact table
   if (c->compact_sat && (p->apply_occlusion || p->apply_shadow) && (!p->apply_shadow || *table || cone_extent >= 0.0)) {
     const float3 sc = f.vol.spacing;
     const double sv[3] = {sc.x, sc.y, sc.z};
@@ -248,7 +294,6 @@ cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light,
     // cells a query on a world extent w may span: its taps reach floor(lo) .. floor(hi) + 1,
     // one more for single-precision positions, at most the SAT's n + 1 cells
     auto cells = [&](double w, int ax) { return std::min(std::ceil(w / sv[ax]) + 3.0, (double)n[ax] + 1.0); };
-    double vmax = 0.0;
     if (p->apply_occlusion) {
       float rmax = 0.0f;
       for (int i = 0; i < p->ao_n_shells; ++i) rmax = std::max(rmax, p->ao_radii[i]);
@@ -272,9 +317,22 @@ cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light,
         vmax = std::max(vmax, v);
       }
     }
-    if (vmax_out) {
-      *vmax_out = vmax;  // the caller builds the table (batches own theirs)
-    } else {
+  }
+  if (vmax_out) {
+    *vmax_out = vmax;  // the caller builds the tables (batches own theirs)
+  } else {
+    // a frame whose boxes all have integer widths reads box tables when they
+    // exist or pay for their build
+    if (walk_out && p->apply_shadow && *table && (*table)->n > 0 && (*table)->aligned &&
+        (a.ao_aligned || !p->apply_occlusion) && !f.work) {
+      cvr_status bs = frame_boxes(c, vmax, f, **table, &a, walk_out);
+      if (bs != CVR_OK) return bs;
+      if (*walk_out) {
+        *eo = a;
+        return CVR_OK;
+      }
+    }
+    if (vmax > 0.0) {
       float inv_scale32 = 0.0f;
       cvr_status cs = ensure_compact_sat(c, vmax, &inv_scale32);
       if (cs != CVR_OK) return cs;
@@ -339,22 +397,46 @@ bool compact_plan(const std::vector<double>& ext, double vmax, int* F_out, std::
   const double limit = 2147483647.0;
   int F = maxv > 0.0 ? (int)std::floor(std::log2(limit / (vmax * maxv))) : 0;
   F = std::min(F, 52);
-  q->resize(ext.size());
+  // scaling by a power of two and rounding are monotone: the largest value
+  // of the table is the largest extinction's
   for (;; --F) {
-    const double scale = std::ldexp(1.0, F);
-    double qmax = 0.0;
-    for (size_t i = 0; i < q->size(); ++i) {
-      const double r = std::rint(ext[i] * scale);  // nearbyint's value without its FP-environment save
-      qmax = std::max(qmax, r);
-      (*q)[i] = (unsigned)r;
-    }
+    const double qmax = std::rint(maxv * std::ldexp(1.0, F));
     if (qmax * vmax < limit || F < -64) {
       if (maxv > 0.0 && qmax < 32768.0) return false;
       break;
     }
   }
   *F_out = F;
+  if (q) compact_values(ext, F, q);
   return true;
+}
+
+void compact_values(const std::vector<double>& ext, int F, std::vector<unsigned>* q) {
+  q->resize(ext.size());
+  const double scale = std::ldexp(1.0, F);
+  // rint: nearbyint's value without its FP-environment save
+  for (size_t i = 0; i < q->size(); ++i) (*q)[i] = (unsigned)std::rint(ext[i] * scale);
+}
+
+bool compact_fixed_point(cvr_ctx* c, double vmax, int* F) {
+  if (c->plan_vmax != vmax) {
+    int f = kNoCompactSat;
+    c->plan_F = compact_plan(c->sat_ext, vmax, &f, nullptr) ? f : kNoCompactSat;
+    c->plan_vmax = vmax;
+  }
+  *F = c->plan_F;
+  return c->plan_F != kNoCompactSat;
+}
+
+// Uploads a fixed-point table through the pinned staging region 1 (q may go
+// when the call returns).
+static cvr_status upload_lut32(cvr_ctx* c, const std::vector<unsigned>& q) {
+  CK(c, ensure(c->d_lut32, c->lut32_cap, sizeof(unsigned) * q.size()));
+  void* stage = nullptr;
+  cvr_status st = stage_region(c, 1, &stage);
+  if (st != CVR_OK) return st;
+  std::memcpy(stage, q.data(), sizeof(unsigned) * q.size());
+  return stage_upload(c, 1, c->d_lut32, sizeof(unsigned) * q.size());
 }
 
 // Builds the compact table of the current volume from q into dst, in x-y
@@ -364,12 +446,7 @@ bool compact_plan(const std::vector<double>& ext, double vmax, int* F_out, std::
 // call returns).
 cvr_status build_compact_sat(cvr_ctx* c, const std::vector<unsigned>& q, uint4* dst) {
   const size_t cells = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
-  CK(c, ensure(c->d_lut32, c->lut32_cap, sizeof(unsigned) * q.size()));
-  void* stage = nullptr;
-  cvr_status st = stage_region(c, 1, &stage);
-  if (st != CVR_OK) return st;
-  std::memcpy(stage, q.data(), sizeof(unsigned) * q.size());
-  st = stage_upload(c, 1, c->d_lut32, sizeof(unsigned) * q.size());
+  cvr_status st = upload_lut32(c, q);
   if (st != CVR_OK) return st;
   CK(c, ensure(c->d_satp, c->satp_cap, sizeof(unsigned) * cells));
   cudaError_t e = launch_sat_build_quads(c->d_vol, c->dtype, c->nx, c->ny, c->nz, c->d_lut32, c->d_satp, dst,
@@ -390,8 +467,7 @@ cvr_status ensure_compact_sat(cvr_ctx* c, double vmax, float* inv_scale) {
     return CVR_OK;
   }
   int F;
-  std::vector<unsigned> q;
-  if (!compact_plan(c->sat_ext, vmax, &F, &q)) return CVR_OK;
+  if (!compact_fixed_point(c, vmax, &F)) return CVR_OK;
   if (c->sat32_F != F || !c->d_sat32) {
     const size_t cells = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
     if (cells >= kCompactMaxCells) return CVR_OK;  // 32-bit cell indices: the int64 table
@@ -404,6 +480,8 @@ cvr_status ensure_compact_sat(cvr_ctx* c, double vmax, float* inv_scale) {
       return CVR_OK;
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "compact SAT");
+    std::vector<unsigned> q;
+    compact_values(c->sat_ext, F, &q);
     cvr_status st = build_compact_sat(c, q, c->d_sat32);
     if (st == CVR_ERR_OUT_OF_MEMORY) return CVR_OK;
     if (st != CVR_OK) return st;
@@ -530,7 +608,7 @@ void cvr_destroy(cvr_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_vol, c->d_rgbt, c->d_rgba, c->d_sat, c->d_lut, c->d_pyr, c->d_occ_sec, c->d_sdw_sec,
                   c->d_occ_vec, c->d_sdw_vec, c->d_stats, c->d_out, c->d_flush, c->d_probe, c->d_vbrick, c->d_lcache, c->d_grad, c->d_ms, c->d_msf,
-                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs};
+                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc};
   for (void* p : bufs)
     if (p) cudaFree(p);
   for (int i = 0; i < 4; ++i)
@@ -560,6 +638,10 @@ static cvr_status set_volume_common(cvr_ctx* c, const void* src, bool src_device
   CK(c, cudaSetDevice(c->device));
   size_t bytes = (size_t)w * h * d * (dtype == CVR_U8 ? 1 : 2);
   CK(c, ensure(c->d_vol, c->vol_cap, bytes));
+  if (c->nx != w || c->ny != h || c->nz != d) {  // the pools of another size go back
+    c->box.ao.release();
+    c->box.sdw.release();
+  }
   CK(c, cudaMemcpyAsync(c->d_vol, src, bytes, src_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                         c->stream));
   c->nx = w; c->ny = h; c->nz = d; c->dtype = dtype;
@@ -653,6 +735,9 @@ cvr_status cvr_build_sat(cvr_ctx* c, const double* ext, int n_values) {
   c->sat_ready = true;
   c->sat_pending = true;
   c->sat_ext.assign(ext, ext + n_values);
+  static std::atomic<unsigned long long> builds{0};  // distinct id of every SAT (any context)
+  c->sat_gen = ++builds;
+  c->plan_vmax = -1.0;
   c->sat32_F = kNoCompactSat;
   return CVR_OK;
 }
@@ -865,9 +950,11 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       ExtArgs a{};
       const ShadowBoxTable* table = nullptr;
       double no_compact = 0.0;  // the light cache reads the int64 table: no compact one to build
-      cvr_status es = ext_args(c, p, light, f, &a, &table, c->lc_dims[0] > 0 ? &no_compact : nullptr);
+      const bool cached = c->lc_dims[0] > 0;
+      const BoxWalk* walk = nullptr;
+      cvr_status es = ext_args(c, p, light, f, &a, &table, cached ? &no_compact : nullptr, cached ? nullptr : &walk);
       if (es != CVR_OK) return es;
-      if (c->lc_dims[0] > 0) {  // object-space light cache, then the object-space marcher
+      if (cached) {  // object-space light cache, then the object-space marcher
         if (!c->sdw_table) c->sdw_table.reset(new ShadowBoxTable());
         const size_t cells = (size_t)c->lc_dims[0] * c->lc_dims[1] * c->lc_dims[2];
         CK(c, ensure(c->d_lcache, c->lcache_cap, cells * sizeof(float2)));
@@ -875,6 +962,8 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
         if (e == cudaSuccess)
           e = launch_march_cached(f, c->d_lcache, c->lc_dims, p->apply_occlusion, p->apply_shadow, p->ka, p->kd,
                                   c->stream);
+      } else if (walk) {
+        e = launch_extinction_box(f, a, *walk, c->stream);
       } else {
         if (!c->sdw_table) c->sdw_table.reset(new ShadowBoxTable());
         e = launch_extinction(f, a, table, *c->sdw_table, c->stream);

@@ -97,6 +97,33 @@ constexpr int kQuadCopy = 100;
 // numbers, so larger grids keep the int64 table / the plain layout.
 constexpr size_t kCompactMaxCells = (size_t)1 << 31;
 
+// Box tables of one volume's extinction (BoxView), filled as frames need
+// them: the ambient-occlusion tables of a radii list, and the shadow tables of
+// one walk axis and interval, one per pair of lateral widths seen.  Bounded
+// (kBoxPoolBytes per pool), released with the owner and by a volume of another size.
+constexpr size_t kBoxPoolBytes = (size_t)24 << 30;
+struct BoxPool {
+  float* data = nullptr;
+  size_t cap = 0;                // bytes
+  unsigned long long gen = 0;    // the table source (compact or int64 build) the tables are of
+  std::vector<int> key;          // AO: the widths; shadow: axis, interval, lateral pads
+  std::vector<int> have;         // shadow: the lateral width pairs (wa | wb << 10), in table order
+  ~BoxPool() { release(); }
+  void release() {
+    if (data) cudaFree(data);
+    data = nullptr;
+    cap = 0;
+    gen = 0;
+    key.clear();
+    have.clear();
+  }
+};
+struct BoxTables {
+  BoxPool ao, sdw;
+  double seen = 0.0;             // pixels rendered without the tables they miss (box_tables)
+  unsigned long long seen_gen = 0;
+};
+
 // A resident volume that is not the current one (cvr_select_volume): the
 // volume, its SAT, pyramid and texture copies.  The current volume lives in
 // the cvr_ctx fields of the same names.
@@ -112,6 +139,9 @@ struct VolSlot {
   int sat_frac_bits = 0;
   bool sat_ready = false;
   bool sat_pending = false;
+  unsigned long long sat_gen = 0;
+  double plan_vmax = -1.0;
+  int plan_F = kNoCompactSat;
   std::vector<double> sat_ext;
   uint4* d_sat32 = nullptr;
   size_t sat32_cap = 0;
@@ -182,6 +212,9 @@ struct cvr_ctx {
   int sat_frac_bits = 0;
   bool sat_ready = false;    // cvr_build_sat succeeded for the current volume
   bool sat_pending = false;  // its int64 table is not built yet (ensure_sat)
+  unsigned long long sat_gen = 0;  // distinct id of every cvr_build_sat
+  double plan_vmax = -1.0;         // the query extent compact_plan was last asked for (-1: none since the SAT)
+  int plan_F = kNoCompactSat;      // its answer (kNoCompactSat: keep the int64 table)
   // compact SAT (32-bit prefix sums modulo 2^32 at F32 fractional bits) for
   // frames whose boxes are small enough; the extinction table it is built from
   std::vector<double> sat_ext;
@@ -203,6 +236,13 @@ struct cvr_ctx {
   size_t walk_cap = 0;
   unsigned long long walk_gen = 0;
   int walk_axis = -1, walk_w = 0;
+  // box tables of the frames whose boxes all have integer widths, and the
+  // plain 32-bit table those of compact frames are made from
+  BoxTables box;
+  std::unique_ptr<BoxWalk> box_walk;         // per-frame walk (host staging)
+  unsigned* d_boxsrc = nullptr;
+  size_t boxsrc_cap = 0;
+  unsigned long long boxsrc_gen = 0;         // the SAT and fixed point it holds (box_gen)
   // pyramid, and its x-y quad copy for FP32 taps (built with the first frame that needs it)
   float* d_pyr = nullptr;
   size_t pyr_cap = 0;
@@ -289,6 +329,9 @@ inline void swap_volume(cvr_ctx* c, VolSlot& s) {
   std::swap(c->sat_frac_bits, s.sat_frac_bits);
   std::swap(c->sat_ready, s.sat_ready);
   std::swap(c->sat_pending, s.sat_pending);
+  std::swap(c->sat_gen, s.sat_gen);
+  std::swap(c->plan_vmax, s.plan_vmax);
+  std::swap(c->plan_F, s.plan_F);
   std::swap(c->sat_ext, s.sat_ext);
   std::swap(c->d_sat32, s.d_sat32);
   std::swap(c->sat32_cap, s.sat32_cap);
@@ -429,8 +472,34 @@ cvr_status frame_args(cvr_ctx* c, const cvr_camera* cam, const void* params, flo
 // shadow-box table (context-owned staging, valid until the next call) or null.
 // With vmax_out the compact SAT is left to the caller: *vmax_out = the largest
 // region the frame's queries span (0: the frame cannot use a compact table).
+// With walk_out the frame may read box tables: *walk_out is its walk
+// (context-owned staging) when it does (e->box set), else null.
 cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light, const FrameArgs& f, ExtArgs* e,
-                    const ShadowBoxTable** table, double* vmax_out = nullptr);
+                    const ShadowBoxTable** table, double* vmax_out = nullptr, const BoxWalk** walk_out = nullptr);
+// Box tables of a frame whose boxes all have integer widths (ext_args' *table
+// aligned, AO boxes aligned or off), in two steps.  box_plan lays the frame's
+// tables out in B (W: its walk, e->box: grids and cells) and says whether the
+// frame reads them: not when they exceed the pools or (pixels >= 0) do not
+// pay for their build yet.  box_build then makes the missing ones from src;
+// *used = false when the GPU has no room for them.
+struct BoxPlan {
+  bool ao_new = false, sdw_new = false;  // the pool starts over (its tables are all built again)
+  std::vector<int> ao_key, sdw_key, have;
+  size_t ao_bytes = 0, sdw_bytes = 0, missing = 0;  // missing: cells to build
+  BoxTableSet ao{}, sdw{};                          // the tables to build
+};
+bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable& t, double pixels, ExtArgs* e,
+              BoxWalk* W, BoxPlan* plan);
+cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned long long gen, const BoxPlan& plan,
+                     ExtArgs* e, bool* used);
+// Identifies the sums box tables are made of: a SAT build at a fixed point (F = kNoCompactSat: int64).
+inline unsigned long long box_gen(unsigned long long sat_gen, int F) {
+  return sat_gen * 4096ull + (unsigned long long)(F + 2048);
+}
+// compact_plan's fixed point for the current SAT, remembered per extent.
+bool compact_fixed_point(cvr_ctx* c, double vmax, int* F);
+// The fixed-point extinction table at F (the values compact_plan returns).
+void compact_values(const std::vector<double>& ext, int F, std::vector<unsigned>* q);
 // The compact 32-bit SAT for a frame whose box queries span at most vmax
 // cells, (re)built when its fixed point changes; *inv_scale = 2^-F32, or 0
 // when the frame keeps the int64 table.

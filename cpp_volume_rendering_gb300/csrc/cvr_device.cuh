@@ -225,6 +225,17 @@ struct SatView {
   float3 max_pos;        // MaxSATPosition = grid + spacing*1.5
 };
 
+// floor(u) as an integer, and u - floor(u), for |u| < 2^22: adding 1.5 * 2^23
+// in round-down mode leaves floor(u) in the low mantissa bits.  Three adds at
+// the full FP32 rate, where floorf and the float -> int conversion each run
+// on the quarter-rate special-function unit; the same values (both
+// subtractions are exact).
+__device__ __forceinline__ int cell_of(float u, float& t) {
+  const float r = __fadd_rd(u, 12582912.0f);
+  t = u - (r - 12582912.0f);
+  return __float_as_int(r) - 0x4B400000;
+}
+
 struct BoxAxis {
   int s[4];    // tap sequence a0, a1, b0, b1
   float w[3];  // weights of the consecutive differences: 1-tl, 1, th
@@ -355,7 +366,8 @@ __device__ __forceinline__ float sat_box(const SatView& S, float3 p1, float3 p2)
 }
 
 // A box whose two corners sit at the same fractional texel offset on every
-// axis (integer widths w): low corner texel coordinate u, high corner u + w.
+// axis (integer widths w): low corner texel coordinate u = a + t (a the cell,
+// t in [0, 1)), high corner u + w.
 // With equal fractions t the reference's 1-D functional
 //   (1-t) S[b0] + t S[b1] - (1-t) S[a0] - t S[a1],  b = a + w,
 // is (1-t) (S[a+w] - S[a]) + t (S[a+1+w] - S[a+1]), so the eight trilinear
@@ -365,12 +377,16 @@ __device__ __forceinline__ float sat_box(const SatView& S, float3 p1, float3 p2)
 // 8 conversions (the general query above: 165 and 27).  Coordinates need no
 // clamp: the quad cells are clamped (exact, see SatView::sat32), which equals
 // the reference's clamp of the corner positions.  Compact (quad) table only.
-__device__ __forceinline__ float sat_box_aligned(const SatView& S, float3 u, int wx, int wy, int wz) {
-  const float fx = floorf(u.x), fy = floorf(u.y), fz = floorf(u.z);
-  const float tx = u.x - fx, ty = u.y - fy, tz = u.z - fz;
-  const int ax = int(fx), ay = int(fy), az = int(fz);
-  const unsigned x0 = (unsigned)min(max(ax + 1, 0), S.sx - 1), x1 = (unsigned)min(max(ax + 1 + wx, 0), S.sx - 1);
-  const unsigned y0 = (unsigned)min(max(ay + 1, 0), S.sy - 1), y1 = (unsigned)min(max(ay + 1 + wy, 0), S.sy - 1);
+__device__ __forceinline__ float aligned_weigh(float b00, float b10, float b01, float b11, float e00, float e10,
+                                               float e01, float e11, float3 t) {
+  const float z00 = fmaf(t.z, e00 - b00, b00), z10 = fmaf(t.z, e10 - b10, b10);
+  const float z01 = fmaf(t.z, e01 - b01, b01), z11 = fmaf(t.z, e11 - b11, b11);
+  const float y0v = fmaf(t.y, z01 - z00, z00), y1v = fmaf(t.y, z11 - z10, z10);
+  return fmaf(t.x, y1v - y0v, y0v);
+}
+__device__ __forceinline__ float sat_box_aligned(const SatView& S, int3 a, float3 t, int wx, int wy, int wz) {
+  const unsigned x0 = (unsigned)min(max(a.x + 1, 0), S.sx - 1), x1 = (unsigned)min(max(a.x + 1 + wx, 0), S.sx - 1);
+  const unsigned y0 = (unsigned)min(max(a.y + 1, 0), S.sy - 1), y1 = (unsigned)min(max(a.y + 1 + wy, 0), S.sy - 1);
   const unsigned sx = (unsigned)S.sx;
   // 32-bit cell numbers (the compact table has fewer than 2^31 cells)
   const unsigned c00 = y0 * sx + x0, c01 = y0 * sx + x1, c10 = y1 * sx + x0, c11 = y1 * sx + x1;
@@ -388,20 +404,39 @@ __device__ __forceinline__ float sat_box_aligned(const SatView& S, float3 u, int
   uint4 d0 = make_uint4(0u, 0u, 0u, 0u), d1 = d0;
 #pragma unroll 1
   for (int o = 0; o < 2; ++o) {
-    const uint4 lo = rect(az + o), hi = rect(az + wz + o);
+    const uint4 lo = rect(a.z + o), hi = rect(a.z + wz + o);
     const uint4 dz = make_uint4(hi.x - lo.x, hi.y - lo.y, hi.z - lo.z, hi.w - lo.w);
     if (o == 0) d0 = dz;
     else d1 = dz;
   }
   // sub-box sums (below 2^31 by the compact table's fixed point): z-offset 0 and 1
-  const float b00 = (float)(int)d0.x, b10 = (float)(int)d0.y;
-  const float b01 = (float)(int)d0.z, b11 = (float)(int)d0.w;
-  const float e00 = (float)(int)d1.x, e10 = (float)(int)d1.y;
-  const float e01 = (float)(int)d1.z, e11 = (float)(int)d1.w;
-  const float z00 = fmaf(tz, e00 - b00, b00), z10 = fmaf(tz, e10 - b10, b10);
-  const float z01 = fmaf(tz, e01 - b01, b01), z11 = fmaf(tz, e11 - b11, b11);
-  const float y0v = fmaf(ty, z01 - z00, z00), y1v = fmaf(ty, z11 - z10, z10);
-  return fmaf(tx, y1v - y0v, y0v) * S.inv_scale32;
+  return aligned_weigh((float)(int)d0.x, (float)(int)d0.y, (float)(int)d0.z, (float)(int)d0.w, (float)(int)d1.x,
+                       (float)(int)d1.y, (float)(int)d1.z, (float)(int)d1.w, t) * S.inv_scale32;
+}
+// The same query on the int64 table: exact 64-bit sums of the eight sub-boxes
+// (64 eight-byte loads, 56 differences, 8 conversions).
+__device__ __forceinline__ float sat_box_aligned64(const SatView& S, int3 a, float3 t, int wx, int wy, int wz) {
+  auto clampi = [](int v, int n) { return min(max(v, 0), n - 1); };
+  const int xs[4] = {clampi(a.x, S.sx), clampi(a.x + 1, S.sx), clampi(a.x + wx, S.sx), clampi(a.x + 1 + wx, S.sx)};
+  const size_t rows[4] = {(size_t)clampi(a.y, S.sy) * S.sx, (size_t)clampi(a.y + 1, S.sy) * S.sx,
+                          (size_t)clampi(a.y + wy, S.sy) * S.sx, (size_t)clampi(a.y + 1 + wy, S.sy) * S.sx};
+  const size_t sxy = (size_t)S.sx * (size_t)S.sy;
+  // sum of the width-(wx, wy) rectangle at sub-box offset (i, j) of a plane
+  auto rect = [&](const long long* p, int i, int j) {
+    return __ldg(p + rows[j + 2] + xs[i + 2]) - __ldg(p + rows[j + 2] + xs[i]) - __ldg(p + rows[j] + xs[i + 2]) +
+           __ldg(p + rows[j] + xs[i]);
+  };
+  float v[8];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const long long* lo = S.sat + sxy * (size_t)clampi(a.z + k, S.sz);
+    const long long* hi = S.sat + sxy * (size_t)clampi(a.z + wz + k, S.sz);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) v[4 * k + 2 * j + i] = ll_to_float(rect(hi, i, j) - rect(lo, i, j));
+  }
+  return aligned_weigh(v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], t) * S.inv_scale;
 }
 
 // Walk table of a directional light's shadow cone: the compact table's sums
@@ -435,9 +470,9 @@ struct WalkFetch {
   unsigned q00[8], q10[8], q01[8], q11[8];
 };
 
-__device__ __forceinline__ void walk_fetch(const SatView& S, const WalkView& Wk, float3 u, int wx, int wy, int wz,
+__device__ __forceinline__ void walk_fetch(const SatView& S, const WalkView& Wk, int3 a, int wx, int wy, int wz,
                                            WalkFetch& F) {
-  const int ax = int(floorf(u.x)), ay = int(floorf(u.y)), az = int(floorf(u.z));
+  const int ax = a.x, ay = a.y, az = a.z;
   const unsigned sx = (unsigned)S.sx, sxy = S.sxy;
   const unsigned x0 = (unsigned)min(max(ax + 1, 0), S.sx - 1), x1 = (unsigned)min(max(ax + 1 + wx, 0), S.sx - 1);
   const unsigned y0 = (unsigned)min(max(ay + 1, 0), S.sy - 1), y1 = (unsigned)min(max(ay + 1 + wy, 0), S.sy - 1);
@@ -455,29 +490,61 @@ __device__ __forceinline__ void walk_fetch(const SatView& S, const WalkView& Wk,
   load_oct(Wk.oct + 2u * (pw + pa1 + pb1), F.q11);
 }
 
-__device__ __forceinline__ float walk_sum(const SatView& S, const WalkView& Wk, float3 u, int wx, int wy, int wz,
-                                          const WalkFetch& F) {
-  const float fx = floorf(u.x), fy = floorf(u.y), fz = floorf(u.z);
-  const int aw = Wk.axis == 0 ? int(fx) : (Wk.axis == 1 ? int(fy) : int(fz));
-  if (aw < 0) return sat_box_aligned(S, u, wx, wy, wz);
-  const float tx = u.x - fx, ty = u.y - fy, tz = u.z - fz;
+__device__ __forceinline__ float walk_sum(const SatView& S, const WalkView& Wk, int3 a, float3 t, int wx, int wy,
+                                          int wz, const WalkFetch& F) {
+  const int aw = Wk.axis == 0 ? a.x : (Wk.axis == 1 ? a.y : a.z);
+  if (aw < 0) return sat_box_aligned(S, a, t, wx, wy, wz);
   float b[8];  // sub-box sums (below 2^31 by the compact table's fixed point)
 #pragma unroll
   for (int c = 0; c < 8; ++c) b[c] = (float)(int)(F.q11[c] - F.q01[c] - F.q10[c] + F.q00[c]);
-  // component c = dx + 2 dy + 4 dz: trilinear weights of the fractions, in
-  // sat_box_aligned's order (z, y, x), so both queries give the same bits
-  const float z00 = fmaf(tz, b[4] - b[0], b[0]), z10 = fmaf(tz, b[5] - b[1], b[1]);
-  const float z01 = fmaf(tz, b[6] - b[2], b[2]), z11 = fmaf(tz, b[7] - b[3], b[3]);
-  const float y0v = fmaf(ty, z01 - z00, z00), y1v = fmaf(ty, z11 - z10, z10);
-  return fmaf(tx, y1v - y0v, y0v) * S.inv_scale32;
+  // component c = dx + 2 dy + 4 dz: sat_box_aligned's weights and order, so
+  // both queries give the same bits
+  return aligned_weigh(b[0], b[1], b[2], b[3], b[4], b[5], b[6], b[7], t) * S.inv_scale32;
 }
 
-__device__ __forceinline__ float sat_box_walk(const SatView& S, const WalkView& Wk, float3 u, int wx, int wy,
+__device__ __forceinline__ float sat_box_walk(const SatView& S, const WalkView& Wk, int3 a, float3 t, int wx, int wy,
                                               int wz) {
   WalkFetch F;
-  walk_fetch(S, Wk, u, wx, wy, wz, F);
-  return walk_sum(S, Wk, u, wx, wy, wz, F);
+  walk_fetch(S, Wk, a, wx, wy, wz, F);
+  return walk_sum(S, Wk, a, t, wx, wy, wz, F);
 }
+
+// ---------------------------------------------------------------- box tables
+// Sums of boxes of fixed integer widths w at every integer low corner a,
+//   B(a) = sum of the extinction of the w-box at a (the SAT's sub-box sum),
+// as FP32 (the exact integer sum, converted once), one table per width triple.
+// An equal-fraction query of such a box is the trilinear value of B: eight
+// FP32 values instead of 16 SAT quads (or four walk-table octs) and their
+// integer differences, and the same bits, since those queries weigh the same
+// converted sums in the same order.  A table covers the low corners a = -P-1
+// ... n-1 of each axis (P >= w; n: the SAT's extent): outside them, and in the
+// first and the last of them, every box sum is zero, so a cell number is
+// clamped by one unsigned minimum.  Cell a holds (B(a), B(a + 1)) of the
+// fastest axis, 8 bytes: two rows of two planes are four 8-byte loads.  (One
+// 4-byte value per cell measured 7 % slower frames, quads and octs of 16 and
+// 32 bytes the same frames for two and four times the memory and build.)
+struct BoxGrid {
+  int na, nb, nc;  // cells along the fastest, middle and slowest axis
+  unsigned nab;    // na * nb
+};
+constexpr int kBoxCellFloats = 2;
+struct BoxCorners {
+  float2 v00, v01, v10, v11;  // [slowest][middle], components: the fastest axis
+};
+__device__ __forceinline__ BoxCorners box_corners(const float* __restrict__ tab, unsigned cell, int na, unsigned nab) {
+  const float2* p = reinterpret_cast<const float2*>(tab) + cell;
+  const float2* q = p + nab;
+  return BoxCorners{__ldg(p), __ldg(p + na), __ldg(q), __ldg(q + na)};
+}
+
+#define CVR_MAX_BOX_SHELLS 32
+struct BoxView {
+  const float* ao;   // ambient-occlusion tables (x fastest, z slowest), or nullptr: none
+  const float* sdw;  // shadow tables (the walk axis slowest), or nullptr: none
+  BoxGrid ao_grid[CVR_MAX_BOX_SHELLS];
+  unsigned ao_cell[CVR_MAX_BOX_SHELLS];  // first cell of shell i's table
+  BoxGrid sdw_grid;
+};
 
 // ---------------------------------------------------------------- pyramid
 // Gaussian extinction pyramid, float32 levels concatenated, x fastest.

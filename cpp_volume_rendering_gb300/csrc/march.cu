@@ -135,7 +135,6 @@ cudaError_t launch_batch_extinction(const BatchExtJob* jobs, int n_jobs, unsigne
                                     int tf_n, int max_table, int tile_threads, int variant, bool compact,
                                     bool aligned, cudaStream_t st) {
   const size_t smem = sizeof(float4) * (tf_n + 3 * max_table);
-  aligned = aligned && compact;
   switch (tile_threads) {
     case 64: return launch_batch_nt<64>(jobs, n_jobs, total_blocks, counter, smem, variant, compact, aligned, st);
     case 256: return launch_batch_nt<256>(jobs, n_jobs, total_blocks, counter, smem, variant, compact, aligned, st);
@@ -148,11 +147,12 @@ static cudaError_t launch_extinction_refill(const FrameArgs& f, const ExtArgs& e
                                            const ShadowBoxTable& storage, cudaStream_t st) {
   const RayOrder o = ray_order(f);
   const bool c = e.sat.sat32 != nullptr;
-  const bool a = c && table && table->aligned && (e.ao_aligned || !e.apply_occ);
+  const bool a = table && table->aligned && (e.ao_aligned || !e.apply_occ);
   const ShadowBoxTable& t = table ? *table : storage;
   const int has = table ? 1 : 0;
   const size_t sm = sizeof(float4) * (f.tf_n + (table ? 3 * table->n : 0));
-  if (a) return launch_persistent(k_march_extinction_refill<MINB, true, true>, sm, st, f, e, o, t, has);
+  if (a && c) return launch_persistent(k_march_extinction_refill<MINB, true, true>, sm, st, f, e, o, t, has);
+  if (a) return launch_persistent(k_march_extinction_refill<MINB, false, true>, sm, st, f, e, o, t, has);
   if (c) return launch_persistent(k_march_extinction_refill<MINB, true, false>, sm, st, f, e, o, t, has);
   return launch_persistent(k_march_extinction_refill<MINB, false, false>, sm, st, f, e, o, t, has);
 }

@@ -62,6 +62,8 @@ struct ExtArgs {
   int ao_aligned;
   // the directional shadow's walk table (walk.oct nullptr: none)
   WalkView walk;
+  // box tables (box.sdw or box.ao set: the frame's queries read them)
+  BoxView box;
 };
 
 // Boxes of the SAT shadow cone of a directional light.  The cone direction is
@@ -84,6 +86,14 @@ struct ShadowBoxTable {
   // for the compact table's equal-fraction query.  0: tx is unused.
   int aligned;
   float4 tx[CVR_MAX_SDW_BOXES];
+};
+
+// The boxes of a directional walk for the box-table marcher (ExtBoxShade).
+struct BoxWalk {
+  int n, axis, pad_a, pad_b, pad_w;  // boxes; walk axis; pads of the tables (fastest, middle, walk axis)
+  float first, vmin, vmax, per;
+  float4 o[CVR_MAX_SDW_BOXES];
+  float cut[CVR_MAX_SDW_BOXES];
 };
 
 struct ConeTableDev {
@@ -187,6 +197,12 @@ struct BatchExtJob {
   const float4* ttx;  // the table's texel offsets and widths (ShadowBoxTable::tx), or null
   int tn, tax;
   float tiw, tvmin, tvmax;
+  // the box-table marcher (bo set: every query of the job reads e.box): the
+  // walk's BoxWalk::o and ::cut in global memory (tn boxes) and its constants
+  const float4* bo;
+  const float* bcut;
+  int bpad_a, bpad_b, bpad_w;
+  float bfirst, bper;
   unsigned first_block;  // first batch-wide tile index of the job
   unsigned blocks_x;     // tiles per image row
 };
@@ -219,6 +235,12 @@ cudaError_t launch_iso(const FrameArgs& f, const IsoArgs& a, cudaStream_t st);
 // storage: any table object (the persistent variant's argument when table is null).
 cudaError_t launch_extinction(const FrameArgs& f, const ExtArgs& e, const ShadowBoxTable* table,
                               const ShadowBoxTable& storage, cudaStream_t st);
+// The extinction marcher on box tables (march_box.cu): a frame whose boxes all
+// have integer widths, e.box set.
+cudaError_t launch_extinction_box(const FrameArgs& f, const ExtArgs& e, const BoxWalk& w, cudaStream_t st);
+// The same for a batch's jobs on box tables (BatchExtJob::bo).
+cudaError_t launch_batch_box(const BatchExtJob* jobs, int n_jobs, unsigned total_blocks, unsigned* counter, int tf_n,
+                             int max_table, int tile_threads, int variant, cudaStream_t st);
 // tex_pyramid: the pyramid taps read d.ptex (FP16 level textures).
 cudaError_t launch_dos(const FrameArgs& f, const DosArgs& d, bool tex_pyramid, cudaStream_t st);
 cudaError_t launch_gt(const FrameArgs& f, const GtArgs& g, cudaStream_t st);

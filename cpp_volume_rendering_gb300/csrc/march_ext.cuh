@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(NT, MINB) k_march_extinction(FrameArgs f, ExtA
 
 // Directional light: the shadow boxes come from the per-frame table, staged
 // in shared memory after the transfer function.  A: every box (AO and
-// shadow) has integer texel widths, so every query is the compact table's
-// equal-fraction one (the host selects it; it needs C).
+// shadow) has integer texel widths, so every query is the equal-fraction one
+// (the host selects it).
 template <int NT, int MINB, bool C, bool A>
 __global__ void __launch_bounds__(NT, MINB) k_march_extinction_dir(FrameArgs f, ExtArgs e,
                                                                     const __grid_constant__ ShadowBoxTable t) {
@@ -74,11 +74,35 @@ __global__ void __launch_bounds__(NT, MINB) k_march_extinction_dir(FrameArgs f, 
   march_pixel(f, tf, sh);
 }
 
+// The last job of a batch whose first tile is <= b.
+__device__ __forceinline__ int batch_job_of(const BatchExtJob* __restrict__ jobs, int n_jobs, unsigned b) {
+  int lo = 0, hi = n_jobs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs[mid].first_block <= b) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+__device__ __forceinline__ void copy_job(BatchExtJob* dst, const BatchExtJob* __restrict__ src) {
+  const int* s = reinterpret_cast<const int*>(src);
+  int* d = reinterpret_cast<int*>(dst);
+  for (int i = threadIdx.x; i < (int)(sizeof(BatchExtJob) / sizeof(int)); i += blockDim.x) d[i] = s[i];
+}
+// The thread's pixel of batch tile b of job J.
+__device__ __forceinline__ void batch_pixel(const BatchExtJob& J, unsigned b, int& px, int& py) {
+  const unsigned local = b - J.first_block;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wl = warp_shift(J.f.warp_w);
+  const int warps_x = J.f.tile_w >> wl;
+  px = (int)(local % J.blocks_x) * J.f.tile_w + (warp % warps_x) * (1 << wl) + (lane & ((1 << wl) - 1));
+  py = (int)(local / J.blocks_x) * J.f.tile_h + (warp / warps_x) * (32 >> wl) + (lane >> wl);
+}
+
 // Batched extinction frames: persistent CTAs take tiles of all jobs from one
 // counter; the job descriptor, transfer function and shadow table are staged
 // in shared memory whenever a CTA moves to another job.
 // A: every job has a shadow table and integer box widths (the equal-fraction
-// query; needs C).
+// query).
 template <int NT, int MINB, bool C, bool A>
 __global__ void __launch_bounds__(NT, MINB) k_batch_extinction(const BatchExtJob* __restrict__ jobs, int n_jobs,
                                                                 unsigned total, unsigned* counter) {
@@ -91,24 +115,14 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_extinction(const BatchExtJob
     if (threadIdx.x == 0) {
       const unsigned b = atomicAdd(counter, 1u);
       s_blk = b;
-      if (b < total) {
-        int lo = 0, hi = n_jobs - 1;  // last job whose first tile is <= b
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (jobs[mid].first_block <= b) lo = mid;
-          else hi = mid - 1;
-        }
-        s_job = lo;
-      }
+      if (b < total) s_job = batch_job_of(jobs, n_jobs, b);
     }
     __syncthreads();
     const unsigned b = s_blk;
     if (b >= total) break;
     const int j = s_job;
     if (j != cur) {
-      const int* src = reinterpret_cast<const int*>(jobs + j);
-      int* dst = reinterpret_cast<int*>(&J);
-      for (int i = threadIdx.x; i < (int)(sizeof(BatchExtJob) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+      copy_job(&J, jobs + j);
       __syncthreads();
       for (int i = threadIdx.x; i < J.f.tf_n; i += blockDim.x) sm_bt[i] = J.f.tf[i];
       for (int i = threadIdx.x; i < J.tn; i += blockDim.x) {
@@ -119,11 +133,8 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_extinction(const BatchExtJob
       cur = j;
       __syncthreads();
     }
-    const unsigned local = b - J.first_block;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wl = warp_shift(J.f.warp_w);
-    const int warps_x = J.f.tile_w >> wl;
-    const int px = (int)(local % J.blocks_x) * J.f.tile_w + (warp % warps_x) * (1 << wl) + (lane & ((1 << wl) - 1));
-    const int py = (int)(local / J.blocks_x) * J.f.tile_h + (warp / warps_x) * (32 >> wl) + (lane >> wl);
+    int px, py;
+    batch_pixel(J, b, px, py);
     ExtShadeT<C, A> sh{&J.e};
     if (J.tn > 0) {
       sh.tlo = sm_bt + J.f.tf_n; sh.thi = sm_bt + J.f.tf_n + J.tn; sh.tn = J.tn; sh.tax = J.tax;
@@ -135,23 +146,30 @@ __global__ void __launch_bounds__(NT, MINB) k_batch_extinction(const BatchExtJob
   }
 }
 
+// As many CTAs of a batch kernel as fit on the GPU (at most one per tile).
+template <class K>
+cudaError_t launch_batch_kernel(K kern, int nt, const BatchExtJob* jobs, int n_jobs, unsigned total_blocks,
+                                unsigned* counter, size_t smem, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  if ((e = carve_l1(kern, nt, smem)) != cudaSuccess) return e;
+  int dev = 0, sms = 0, per_sm = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  if ((e = resident_ctas(kern, nt, smem, &per_sm)) != cudaSuccess) return e;
+  unsigned ctas = (unsigned)sms * (unsigned)per_sm;
+  if (ctas > total_blocks) ctas = total_blocks;
+  if (ctas == 0) return cudaSuccess;
+  kern<<<ctas, nt, smem, st>>>(jobs, n_jobs, total_blocks, counter);
+  return cudaGetLastError();
+}
+
 template <int NT, int MINB>
 cudaError_t launch_batch_t(const BatchExtJob* jobs, int n_jobs, unsigned total_blocks, unsigned* counter,
                                   size_t smem, bool compact, bool aligned, cudaStream_t st) {
   auto kern = compact ? (aligned ? k_batch_extinction<NT, MINB, true, true> : k_batch_extinction<NT, MINB, true, false>)
-                      : k_batch_extinction<NT, MINB, false, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  if ((e = carve_l1(kern, NT, smem)) != cudaSuccess) return e;
-  int dev = 0, sms = 0, per_sm = 0;
-  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = resident_ctas(kern, NT, smem, &per_sm)) != cudaSuccess) return e;
-  unsigned ctas = (unsigned)sms * (unsigned)per_sm;
-  if (ctas > total_blocks) ctas = total_blocks;
-  if (ctas == 0) return cudaSuccess;
-  kern<<<ctas, NT, smem, st>>>(jobs, n_jobs, total_blocks, counter);
-  return cudaGetLastError();
+                      : (aligned ? k_batch_extinction<NT, MINB, false, true> : k_batch_extinction<NT, MINB, false, false>);
+  return launch_batch_kernel(kern, NT, jobs, n_jobs, total_blocks, counter, smem, st);
 }
 
 // Register variants as minimum resident CTAs: caps of 128 and 80 registers.
@@ -178,8 +196,8 @@ cudaError_t launch_extinction_t(const FrameArgs& f, const ExtArgs& e, const Shad
   const bool c = e.sat.sat32 != nullptr;
   if (table) {
     size_t sm = sizeof(float4) * (f.tf_n + 3 * table->n);
-    const bool a = c && table->aligned && (e.ao_aligned || !e.apply_occ);
-    auto kern = a ? k_march_extinction_dir<NT, MINB, true, true>
+    const bool a = table->aligned && (e.ao_aligned || !e.apply_occ);
+    auto kern = a ? (c ? k_march_extinction_dir<NT, MINB, true, true> : k_march_extinction_dir<NT, MINB, false, true>)
                   : (c ? k_march_extinction_dir<NT, MINB, true, false> : k_march_extinction_dir<NT, MINB, false, false>);
     const cudaError_t err = carve_l1(kern, NT, sm);
     if (err != cudaSuccess) return err;

@@ -124,12 +124,32 @@ struct PlainShade {
 
 // ====================================================== extinction (rc1pextbsd)
 // COMPACT: the frame's SAT box queries read the 32-bit table (SatView::sat32).
-// ALIGNED (with COMPACT): every AO box and every box of the directional
-// shadow table has integer texel widths, so every query is the equal-fraction
-// one (sat_box_aligned); the kernel then always has a table (ttx set).
+// ALIGNED: every AO box and every box of the directional shadow table has
+// integer texel widths, so every query is the equal-fraction one
+// (sat_box_aligned, sat_box_aligned64); the kernel then always has a table
+// (ttx set).  ExtBoxShade below reads the same frames from box tables.
+
+// SAT texel coordinate of a texture-space position: (tx + spacing) / spacing - 0.5.
+__device__ __forceinline__ float3 sat_texel(const SatView& S, float3 tx) {
+  return f3(fmaf(tx.x, S.inv_spacing.x, 0.5f), fmaf(tx.y, S.inv_spacing.y, 0.5f), fmaf(tx.z, S.inv_spacing.z, 0.5f));
+}
+// Texels between consecutive boxes of an aligned walk: the packed widths' one
+// along the axis (the sample interval), with the walk's sign.
+__device__ __forceinline__ int walk_step(int widths, int axis, float interval) {
+  const int w = (widths >> (10 * axis)) & 1023;
+  return interval < 0.0f ? -w : w;
+}
+
+// Cell and fraction of a directional walk's boxes along its axis: the boxes'
+// low corners are a whole number of texels (dw) apart, so the first box's
+// serve them all.
+struct WalkStart {
+  int cell;
+  float frac;
+};
+
 template <bool COMPACT = false, bool ALIGNED = false>
 struct ExtShadeT {
-  static_assert(COMPACT || !ALIGNED, "the equal-fraction query reads the compact table");
   const ExtArgs* e;
   // Per-frame box table of a directional light (shared memory), or nullptr.
   const float4* tlo = nullptr;
@@ -149,31 +169,31 @@ struct ExtShadeT {
     return sat_box<COMPACT>(S, p1, p2);
   }
 
+  static __device__ __forceinline__ float aligned_box(const SatView& S, int3 a, float3 t, int wx, int wy, int wz) {
+    if constexpr (COMPACT) return sat_box_aligned(S, a, t, wx, wy, wz);
+    else return sat_box_aligned64(S, a, t, wx, wy, wz);
+  }
+
   // ExtinctionAmbientOcclusion (ebs_ray_bbox_marching.comp:112-146), with the
   // shell radii taken from a list (reference: AmbOccRadius * (i + 1)).
   __device__ float ambient_occlusion(float3 tx, const FrameArgs& f) const {
     if constexpr (ALIGNED) {
-      {
-        // the box [tx - r, tx + r] (voxels) starts at texel coordinate
-        // (tx + spacing) / spacing - 0.5 - r = g - r and is 2 r texels wide
-        const SatView& S = e->sat;
-        const float3 g = f3(fmaf(tx.x, S.inv_spacing.x, 0.5f), fmaf(tx.y, S.inv_spacing.y, 0.5f),
-                            fmaf(tx.z, S.inv_spacing.z, 0.5f));
-        float r0 = e->radii[0];
-        int w0 = __float2int_rn(2.0f * r0);
-        float sat0 = sat_box_aligned(S, f3(g.x - r0, g.y - r0, g.z - r0), w0, w0, w0);
-        float t = sat0 * (1.0f / (r0 * r0));
-        float sat_i = sat0;
-        for (int i = 1; i < e->n_shells; ++i) {
-          const float ri = e->radii[i];
-          const int wi = __float2int_rn(2.0f * ri);
-          const float sat_n = sat_box_aligned(S, f3(g.x - ri, g.y - ri, g.z - ri), wi, wi, wi);
-          t = t + (sat_n - sat_i) * (1.0f / (ri * ri));
-          sat_i = sat_n;
-        }
-        const float rk = e->radii[e->n_shells - 1];
-        return expf(-((1.0f / (rk * rk)) * t));
+      // the box [tx - r, tx + r] (voxels) starts at texel coordinate
+      // (tx + spacing) / spacing - 0.5 - r = g - r and is 2 r texels wide
+      const SatView& S = e->sat;
+      const float3 g = sat_texel(S, tx);
+      float t = 0.0f, sat_i = 0.0f;
+      for (int i = 0; i < e->n_shells; ++i) {
+        const float ri = e->radii[i];
+        const int wi = __float2int_rn(2.0f * ri);
+        float3 q;
+        const int3 a = make_int3(cell_of(g.x - ri, q.x), cell_of(g.y - ri, q.y), cell_of(g.z - ri, q.z));
+        const float sat_n = aligned_box(S, a, q, wi, wi, wi);
+        t = i == 0 ? sat_n * (1.0f / (ri * ri)) : t + (sat_n - sat_i) * (1.0f / (ri * ri));
+        sat_i = sat_n;
       }
+      const float rk = e->radii[e->n_shells - 1];
+      return expf(-((1.0f / (rk * rk)) * t));
     }
     float3 sc = f.vol.spacing;
     float r0 = e->radii[0];
@@ -317,22 +337,31 @@ struct ExtShadeT {
     const float pm = tax == 0 ? tx.x : (tax == 1 ? tx.y : tx.z);
     float st = 0.0f;
     if constexpr (ALIGNED) {
-      const float3 g = f3(fmaf(tx.x, S.inv_spacing.x, 0.5f), fmaf(tx.y, S.inv_spacing.y, 0.5f),
-                          fmaf(tx.z, S.inv_spacing.z, 0.5f));
-      {  // every box has integer widths: the equal-fraction query
-        for (int k = 0; k < tn; ++k) {
-          const float nxt = pm + (tlo[k].w + tiw);
-          if (!(nxt > tvmin && nxt < tvmax)) break;
-          const float4 o = ttx[k];
-          const int w = __float_as_int(o.w);
-          const float3 u = f3(g.x + o.x, g.y + o.y, g.z + o.z);
-          const float b = e->walk.oct ? sat_box_walk(S, e->walk, u, w & 1023, (w >> 10) & 1023, w >> 20)
-                                      : sat_box_aligned(S, u, w & 1023, (w >> 10) & 1023, w >> 20);
-          st = fmaf(b, thi[k].w, st);
-          ++aux;
-        }
-        return expf(-st);
+      // every box has integer widths: the equal-fraction query
+      if (tn == 0) return 1.0f;
+      const float3 g = sat_texel(S, tx);
+      const float4 o0 = ttx[0];
+      WalkStart ws;
+      ws.cell = cell_of(tax == 0 ? g.x + o0.x : (tax == 1 ? g.y + o0.y : g.z + o0.z), ws.frac);
+      const int dw = walk_step(__float_as_int(o0.w), tax, tiw);
+      for (int k = 0; k < tn; ++k) {
+        const float nxt = pm + (tlo[k].w + tiw);
+        if (!(nxt > tvmin && nxt < tvmax)) break;
+        const float4 o = ttx[k];
+        const int w = __float_as_int(o.w);
+        float3 q;
+        int3 a = make_int3(cell_of(g.x + o.x, q.x), cell_of(g.y + o.y, q.y), cell_of(g.z + o.z, q.z));
+        const int aw = ws.cell + k * dw;
+        if (tax == 0) { a.x = aw; q.x = ws.frac; }
+        else if (tax == 1) { a.y = aw; q.y = ws.frac; }
+        else { a.z = aw; q.z = ws.frac; }
+        float b;
+        if (COMPACT && e->walk.oct) b = sat_box_walk(S, e->walk, a, q, w & 1023, (w >> 10) & 1023, w >> 20);
+        else b = aligned_box(S, a, q, w & 1023, (w >> 10) & 1023, w >> 20);
+        st = fmaf(b, thi[k].w, st);
+        ++aux;
       }
+      return expf(-st);
     }
     for (int k = 0; k < tn; ++k) {
       const float4 lo = tlo[k];
@@ -377,6 +406,111 @@ struct ExtShadeT {
   }
 };
 using ExtShade = ExtShadeT<false>;
+
+// Extinction shading from box tables (BoxView): the frames of ExtShadeT<.,
+// true>, each box one trilinear lookup of its width's table.  Same images, bit
+// for bit.  so[k] = (texel offset of box k's low corner along the fastest and
+// the middle table axis; weight; first cell of its table plus k boxes' steps
+// along the walk axis, as int bits), scut[k] = the axis offset its
+// CUT_WHEN_AWAY_FROM_VOLUME test adds to the sample.
+struct ExtBoxShade {
+  const ExtArgs* e;
+  const float4* so;
+  const float* scut;
+  int n, axis, pad_a, pad_b, pad_w;  // boxes; walk axis; pads of the tables
+  float first;             // texel offset of the first box's low corner along it
+  float vmin, vmax, per;   // the cut interval, 1 / signed box step (world units)
+  struct Ray {};
+  __device__ __forceinline__ void begin(Ray&, float3) const {}
+
+  __device__ __forceinline__ float ambient_occlusion(float3 g) const {
+    const BoxView& B = e->box;
+    float t = 0.0f, last = 0.0f;
+    for (int i = 0; i < e->n_shells; ++i) {
+      const float r = e->radii[i];
+      const BoxGrid& G = B.ao_grid[i];
+      const int pad = __float2int_rn(2.0f * r) + 1;
+      float3 q;
+      const unsigned x = min((unsigned)(cell_of(g.x - r, q.x) + pad), (unsigned)G.na - 1u);
+      const unsigned y = min((unsigned)(cell_of(g.y - r, q.y) + pad), (unsigned)G.nb - 1u);
+      const unsigned z = min((unsigned)(cell_of(g.z - r, q.z) + pad), (unsigned)G.nc - 1u);
+      const BoxCorners c = box_corners(B.ao, B.ao_cell[i] + x + y * (unsigned)G.na + z * G.nab, G.na, G.nab);
+      const float b = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, q);
+      t = i == 0 ? b * (1.0f / (r * r)) : t + (b - last) * (1.0f / (r * r));
+      last = b;
+    }
+    const float rk = e->radii[e->n_shells - 1];
+    return expf(-((1.0f / (rk * rk)) * t));
+  }
+
+  // Boxes of the walk from a sample at pm along the axis: the index of the
+  // first that fails the cut test.  The test is monotone in k once the first
+  // box passes (the boxes move towards one face), so the index is computed
+  // from the step and corrected by the test itself; a known trip count lets
+  // the loop run with several boxes' loads in flight.
+  __device__ __forceinline__ int boxes(float pm) const {
+    auto in = [&](int k) {
+      const float nxt = pm + scut[k];
+      return nxt > vmin && nxt < vmax;
+    };
+    if (n == 0 || !in(0)) return 0;
+    int k = min(max((int)(((per > 0.0f ? vmax : vmin) - pm - scut[0]) * per) + 1, 1), n);
+    while (k < n && in(k)) ++k;
+    while (k > 1 && !in(k - 1)) --k;
+    return k;
+  }
+
+  // AXIS 2: table axes (x, y, z), 1: (x, z, y), 0: (y, z, x), walk axis last.
+  template <int AXIS>
+  __device__ __forceinline__ float walk(float ga, float gb, float gw, int m) const {
+    const BoxGrid& G = e->box.sdw_grid;
+    const float* __restrict__ tab = e->box.sdw;
+    const int na = G.na;
+    const unsigned nab = G.nab, ma = (unsigned)G.na - 1u, mb = (unsigned)G.nb - 1u;
+    float tw;
+    const unsigned cw = (unsigned)(cell_of(gw + first, tw) + pad_w) * nab;
+    float st = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      const float4 o = so[k];
+      float ta, tb;
+      const unsigned a = min((unsigned)(cell_of(ga + o.x, ta) + pad_a), ma);
+      const unsigned b = min((unsigned)(cell_of(gb + o.y, tb) + pad_b), mb);
+      const BoxCorners c = box_corners(tab, (__float_as_uint(o.w) + cw) + (a + b * (unsigned)na), na, nab);
+      float v;  // corners as (x, y, z) bits, so that the lerp order is z, y, x
+      if constexpr (AXIS == 2)
+        v = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, f3(ta, tb, tw));
+      else if constexpr (AXIS == 1)
+        v = aligned_weigh(c.v00.x, c.v00.y, c.v10.x, c.v10.y, c.v01.x, c.v01.y, c.v11.x, c.v11.y, f3(ta, tw, tb));
+      else
+        v = aligned_weigh(c.v00.x, c.v10.x, c.v00.y, c.v10.y, c.v01.x, c.v11.x, c.v01.y, c.v11.y, f3(tw, ta, tb));
+      st = fmaf(v, o.z, st);
+    }
+    return expf(-st);
+  }
+
+  __device__ __forceinline__ float shadow(float3 tx, float3 g, unsigned& aux) const {
+    const int m = boxes(axis == 0 ? tx.x : (axis == 1 ? tx.y : tx.z));
+    aux += m;
+    if (axis == 2) return walk<2>(g.x, g.y, g.z, m);
+    if (axis == 1) return walk<1>(g.x, g.z, g.y, m);
+    return walk<0>(g.y, g.z, g.x, m);
+  }
+
+  // ShadeSample (ebs_ray_bbox_marching.comp:500-551).
+  __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
+    const float3 g = sat_texel(e->sat, tx);
+    float ka = 0.0f, kd = 0.0f, io = 0.0f, is = 0.0f;
+    if (e->apply_occ) { ka = e->ka; io = ambient_occlusion(g); aux += e->n_shells; }
+    if (e->apply_sdw) { kd = e->kd; is = shadow(tx, g, aux); }
+    if (f.grad.g) return phong_ext(f, src, tx, io, ka, is, kd);
+    const float k = 1.0f / (ka + kd);
+    src.x = k * (src.x * io * ka + src.x * is * kd);
+    src.y = k * (src.y * io * ka + src.y * is * kd);
+    src.z = k * (src.z * io * ka + src.z * is * kd);
+    return src;
+  }
+};
 
 // ==================================================== cone DOS (rc1pdosct)
 // TEX: the pyramid taps through the texture unit (DosArgs::ptex).
