@@ -928,8 +928,10 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
   f.counts = counts;
   fs = grad_args(c, method, light, &f);
   if (fs != CVR_OK) return fs;
-  // the three counters and the ray counter of the persistent marchers
-  CK(c, cudaMemsetAsync(c->d_stats, 0, 4 * sizeof(unsigned long long), c->stream));
+  // the three counters (counted when the caller asks) and the ray counter of
+  // the persistent marchers
+  if (!stats) f.stats = nullptr;
+  if (stats || f.work) CK(c, cudaMemsetAsync(c->d_stats, 0, 4 * sizeof(unsigned long long), c->stream));
   cvr_light dl{};
   if (!light) { light = &dl; }
   cudaError_t e = cudaSuccess;

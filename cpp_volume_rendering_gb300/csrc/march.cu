@@ -13,14 +13,6 @@ CVR_EXTINCTION_EXTERN(64)
 CVR_EXTINCTION_EXTERN(128)
 CVR_EXTINCTION_EXTERN(256)
 
-template <int NT>
-__global__ void __launch_bounds__(NT) k_march_plain(FrameArgs f) {
-  extern __shared__ float4 sm_tf[];
-  const float4* tf = stage_tf(f, sm_tf);
-  __syncthreads();
-  march_pixel(f, tf, PlainShade{});
-}
-
 // MINB: the tuner's register variant, as for the extinction marcher.
 template <int NT, int MINB, bool TEX>
 __global__ void __launch_bounds__(NT, MINB) k_march_dos(DosArgs d, FrameArgs f) {
@@ -33,20 +25,6 @@ __global__ void __launch_bounds__(NT, MINB) k_march_dos(DosArgs d, FrameArgs f) 
   for (int i = threadIdx.x; i < d.sdw.n_sections; i += blockDim.x) sdw[i] = d.sdw_sections[i];
   __syncthreads();
   DosShadeT<TEX> sh{&d, occ, sdw};
-  march_pixel(f, tf, sh);
-}
-
-template <int NT>
-__global__ void __launch_bounds__(NT) k_march_gt(GtArgs g, FrameArgs f) {
-  extern __shared__ float4 sm[];
-  float4* tf = sm;
-  float3* ov = reinterpret_cast<float3*>(sm + f.tf_n);
-  float3* sv = ov + g.n_occ;
-  for (int i = threadIdx.x; i < f.tf_n; i += blockDim.x) tf[i] = f.tf[i];
-  for (int i = threadIdx.x; i < g.n_occ; i += blockDim.x) ov[i] = g.occ_vec[i];
-  for (int i = threadIdx.x; i < g.n_sdw; i += blockDim.x) sv[i] = g.sdw_vec[i];
-  __syncthreads();
-  GtShade sh{&g, tf, f.tf_n, ov, sv};
   march_pixel(f, tf, sh);
 }
 
@@ -103,19 +81,16 @@ template <int MINB>
 __global__ void __launch_bounds__(128, MINB) k_march_gt_refill(GtArgs g, FrameArgs f, RayOrder o) {
   extern __shared__ float4 sm[];
   float4* tf = sm;
-  float3* ov = reinterpret_cast<float3*>(sm + f.tf_n);
-  float3* sv = ov + g.n_occ;
   for (int i = threadIdx.x; i < f.tf_n; i += blockDim.x) tf[i] = f.tf[i];
-  for (int i = threadIdx.x; i < g.n_occ; i += blockDim.x) ov[i] = g.occ_vec[i];
-  for (int i = threadIdx.x; i < g.n_sdw; i += blockDim.x) sv[i] = g.sdw_vec[i];
+  const GtStage gs(f, g, sm + f.tf_n);
   __syncthreads();
-  GtShade sh{&g, tf, f.tf_n, ov, sv};
+  GtShadeT<SampleAny> sh{&g, SampleAny(f.vol), TfAlpha{gs.alpha, f.tf_n}, gs.occ, gs.sdw};
   march_refill(f, tf, sh, f.work, o);
 }
 
 cudaError_t launch_plain(const FrameArgs& f, cudaStream_t st) {
-  size_t sm = sizeof(float4) * f.tf_n;
   if (f.work) {
+    const size_t sm = sizeof(float4) * f.tf_n;
     const RayOrder o = ray_order(f);
     switch (f.variant) {
       case 1: return launch_persistent(k_march_plain_refill<minb128<1>()>, sm, st, f, o);
@@ -123,12 +98,7 @@ cudaError_t launch_plain(const FrameArgs& f, cudaStream_t st) {
       default: return launch_persistent(k_march_plain_refill<1>, sm, st, f, o);
     }
   }
-  switch (threads_of(f)) {
-    case 64: k_march_plain<64><<<grid_of(f), 64, sm, st>>>(f); break;
-    case 256: k_march_plain<256><<<grid_of(f), 256, sm, st>>>(f); break;
-    default: k_march_plain<128><<<grid_of(f), 128, sm, st>>>(f); break;
-  }
-  return cudaGetLastError();
+  return launch_plain_tiles(f, st);
 }
 
 cudaError_t launch_batch_extinction(const BatchExtJob* jobs, int n_jobs, unsigned total_blocks, unsigned* counter,
@@ -221,21 +191,9 @@ cudaError_t launch_dos(const FrameArgs& f, const DosArgs& d, bool tex_pyramid, c
   }
 }
 
-template <int NT>
-static cudaError_t launch_gt_t(const FrameArgs& f, const GtArgs& g, size_t sm, cudaStream_t st) {
-  if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_march_gt<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-  }
-  cudaError_t e = carve_l1(k_march_gt<NT>, NT, sm);
-  if (e != cudaSuccess) return e;
-  k_march_gt<NT><<<grid_of(f), NT, sm, st>>>(g, f);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_gt(const FrameArgs& f, const GtArgs& g, cudaStream_t st) {
-  size_t sm = sizeof(float4) * f.tf_n + sizeof(float3) * (g.n_occ + g.n_sdw);
   if (f.work) {
+    const size_t sm = sizeof(float4) * f.tf_n + GtStage::bytes(f.tf_n, g);
     const RayOrder o = ray_order(f);
     switch (f.variant) {
       case 1: return launch_persistent(k_march_gt_refill<minb128<1>()>, sm, st, g, f, o);
@@ -243,11 +201,7 @@ cudaError_t launch_gt(const FrameArgs& f, const GtArgs& g, cudaStream_t st) {
       default: return launch_persistent(k_march_gt_refill<1>, sm, st, g, f, o);
     }
   }
-  switch (threads_of(f)) {
-    case 64: return launch_gt_t<64>(f, g, sm, st);
-    case 256: return launch_gt_t<256>(f, g, sm, st);
-    default: return launch_gt_t<128>(f, g, sm, st);
-  }
+  return launch_gt_tiles(f, g, st);
 }
 
 }  // namespace cvr

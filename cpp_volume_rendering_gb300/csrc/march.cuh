@@ -226,6 +226,9 @@ cudaError_t launch_march_cached(const FrameArgs& f, const float2* cache, const i
                                 int apply_sdw, float ka, float kd, cudaStream_t st);
 
 cudaError_t launch_plain(const FrameArgs& f, cudaStream_t st);
+// Their tile marchers (march_plain.cu, march_gt.cu).
+cudaError_t launch_plain_tiles(const FrameArgs& f, cudaStream_t st);
+cudaError_t launch_gt_tiles(const FrameArgs& f, const GtArgs& g, cudaStream_t st);
 // The plain marcher with shared-memory brick staging (staged.cu): plain
 // volume layout, FP32 samples only (plain_staging_applies).
 bool plain_staging_applies(const FrameArgs& f);

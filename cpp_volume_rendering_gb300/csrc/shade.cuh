@@ -9,6 +9,7 @@
 #include <cuda_fp16.h>
 
 #include "march.cuh"
+#include "sampler.cuh"
 
 namespace cvr {
 
@@ -664,10 +665,12 @@ using DosShade = DosShadeT<false>;
 
 
 // ================================================= ground truth (rc1pcrtgt)
-struct GtShade {
+// S: the volume sampler; alpha: the transfer function's extinction.
+template <class S>
+struct GtShadeT {
   const GtArgs* g;
-  const float4* tf;
-  int tf_n;
+  S sample;
+  TfAlpha alpha;
   const float3* occ_vec;  // shared-memory copies
   const float3* sdw_vec;
   struct Ray { float3 dir, v_up, v_right; };
@@ -681,22 +684,38 @@ struct GtShade {
 
   // One light ray of ConeOcclusion/ShadowsEvaluationRayCasting
   // (gt_ray_marching.comp:125-159 and 209-242): trapezoidal transmittance.
+  // The samples' positions do not depend on the transmittance, only the ray's
+  // end does, so kAhead samples are fetched together and then taken one by
+  // one until the ray ends: kAhead loads in flight instead of one, for at
+  // most kAhead - 1 samples fetched past the end of a ray.
+  static constexpr int kAhead = 4;
   __device__ float light_ray(float3 tx, float3 w, float dist, const FrameArgs& f, unsigned& aux) const {
     float vt = 1.0f;
     ++aux;
     float s = g->gap;
-    float3 S = f.vol.grid;
-    float st0 = tf_alpha(tf, tf_n, sample_volume(f.vol, tx + w * s));
-    for (int guard = 0; guard < kMaxLightSteps && s < dist; ++guard) {
-      float h = fminf(g->lstep, dist - s);
-      float3 at = tx + w * (s + h);
-      if (at.x < 0.0f || at.x > S.x || at.y < 0.0f || at.y > S.y || at.z < 0.0f || at.z > S.z) break;
-      float st1 = tf_alpha(tf, tf_n, sample_volume(f.vol, at));
-      ++aux;
-      vt *= expf(-((st0 + st1) * 0.5f) * h);
-      if ((1.0f - vt) > 0.99f) break;
-      st0 = st1;
-      s = s + h;
+    const float3 G = f.vol.grid;
+    float st0 = alpha(sample(tx + w * s));
+    for (int guard = 0; guard < kMaxLightSteps && s < dist; guard += kAhead) {
+      float h[kAhead], st[kAhead];
+      bool in[kAhead];
+      float sj = s;
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        h[j] = fminf(g->lstep, dist - sj);
+        const float3 at = tx + w * (sj + h[j]);
+        in[j] = sj < dist && !(at.x < 0.0f || at.x > G.x || at.y < 0.0f || at.y > G.y || at.z < 0.0f || at.z > G.z);
+        st[j] = alpha(sample(at));
+        sj = sj + h[j];
+      }
+#pragma unroll
+      for (int j = 0; j < kAhead; ++j) {
+        if (!in[j]) return vt;
+        ++aux;
+        vt *= expf(-((st0 + st[j]) * 0.5f) * h[j]);
+        if ((1.0f - vt) > 0.99f) return vt;
+        st0 = st[j];
+      }
+      s = sj;
     }
     return vt;
   }
@@ -767,6 +786,7 @@ __device__ __forceinline__ void pixel_of(const FrameArgs& f, int& px, int& py) {
 }
 
 __device__ __forceinline__ void add_stats(const FrameArgs& f, unsigned int n, unsigned int shaded, unsigned int aux) {
+  if (!f.stats) return;  // nobody asked: no shuffles, no atomics on three addresses
   unsigned long long a = n, b = shaded, c = aux;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -774,7 +794,7 @@ __device__ __forceinline__ void add_stats(const FrameArgs& f, unsigned int n, un
     b += __shfl_down_sync(0xffffffffu, b, o);
     c += __shfl_down_sync(0xffffffffu, c, o);
   }
-  if ((threadIdx.x & 31) == 0 && f.stats) {
+  if ((threadIdx.x & 31) == 0) {
     atomicAdd(f.stats + 0, a);
     atomicAdd(f.stats + 1, b);
     atomicAdd(f.stats + 2, c);
@@ -784,8 +804,9 @@ __device__ __forceinline__ void add_stats(const FrameArgs& f, unsigned int n, un
 // The a5 loop (ray_marching_1p.comp:170-247): h = min(StepSize, D - s),
 // sample at s + h/2, skip transparent samples, alpha = 1 - exp(-sigma h),
 // front-to-back composite, stop once alpha > 0.99.
-template <class Shade>
-__device__ __forceinline__ void march_ray(const FrameArgs& f, const float4* tf, const Shade& sh, int px, int py) {
+template <class S, class Tf, class Shade>
+__device__ __forceinline__ void march_ray_with(const FrameArgs& f, const S& sample, const Tf& tf, const Shade& sh,
+                                               int px, int py) {
   bool inside = px < f.W && py < f.H;
   unsigned int n = 0, shaded = 0, aux = 0;
   if (inside) {
@@ -803,8 +824,7 @@ __device__ __forceinline__ void march_ray(const FrameArgs& f, const float4* tf, 
       for (float s = 0.0f; s < D && n < max_iter;) {
         float h = fminf(f.step, D - s);
         float3 p = tex0 + dir * (s + h * 0.5f);
-        float density = sample_volume(f.vol, p);
-        float4 src = tf_lookup(tf, f.tf_n, density);
+        float4 src = tf(sample(p));
         ++n;
         if (src.w > 0.0f) {
           ++shaded;
@@ -823,6 +843,18 @@ __device__ __forceinline__ void march_ray(const FrameArgs& f, const float4* tf, 
     if (f.counts) f.counts[o] = n;
   }
   add_stats(f, n, shaded, aux);
+}
+
+// The transfer function as staged by stage_tf.
+struct TfStaged {
+  const float4* e;
+  int n;
+  __device__ __forceinline__ float4 operator()(float density) const { return tf_lookup(e, n, density); }
+};
+
+template <class Shade>
+__device__ __forceinline__ void march_ray(const FrameArgs& f, const float4* tf, const Shade& sh, int px, int py) {
+  march_ray_with(f, SampleAny(f.vol), TfStaged{tf, f.tf_n}, sh, px, py);
 }
 
 // One CTA-tile pixel per thread (pixel_of).
@@ -980,6 +1012,21 @@ inline RayOrder ray_order(const FrameArgs& f) {
   o.total = (unsigned)(2 * R + 1) * (unsigned)(2 * R + 1) * 32u;  // frames <= 32768^2: below 2^32
   return o;
 }
+
+// Kernel vectors of the ground truth, staged after its extinction table.
+struct GtStage {
+  float2* alpha;
+  float3 *occ, *sdw;
+  __device__ __forceinline__ GtStage(const FrameArgs& f, const GtArgs& g, void* smem)
+      : alpha(static_cast<float2*>(smem)), occ(reinterpret_cast<float3*>(alpha + f.tf_n + 1)), sdw(occ + g.n_occ) {
+    stage_tf_alpha(f.tf, f.tf_n, alpha);
+    for (int i = threadIdx.x; i < g.n_occ; i += blockDim.x) occ[i] = g.occ_vec[i];
+    for (int i = threadIdx.x; i < g.n_sdw; i += blockDim.x) sdw[i] = g.sdw_vec[i];
+  }
+  static size_t bytes(int tf_n, const GtArgs& g) {
+    return sizeof(float2) * ((size_t)tf_n + 1) + sizeof(float3) * ((size_t)g.n_occ + g.n_sdw);
+  }
+};
 
 // Loads the RGBt table into shared memory (n <= tf_smem_cap) and returns it.
 __device__ __forceinline__ const float4* stage_tf(const FrameArgs& f, float4* smem) {

@@ -80,17 +80,14 @@ __global__ void __launch_bounds__(128) k_sur_label(const float4* __restrict__ pt
   float4* tf = sm_lab;
   float4* occ_tab = tf + f.tf_n;
   float4* sdw_tab = occ_tab + (want_dos ? d.occ.n_sections : 0);
-  float3* ov = reinterpret_cast<float3*>(sdw_tab + (want_dos ? d.sdw.n_sections : 0));
-  float3* sv = ov + (want_gt ? g.n_occ : 0);
+  float2* gt_smem = reinterpret_cast<float2*>(sdw_tab + (want_dos ? d.sdw.n_sections : 0));
   for (int i = threadIdx.x; i < f.tf_n; i += blockDim.x) tf[i] = f.tf[i];
   if (want_dos) {
     for (int i = threadIdx.x; i < d.occ.n_sections; i += blockDim.x) occ_tab[i] = d.occ_sections[i];
     for (int i = threadIdx.x; i < d.sdw.n_sections; i += blockDim.x) sdw_tab[i] = d.sdw_sections[i];
   }
-  if (want_gt) {
-    for (int i = threadIdx.x; i < g.n_occ; i += blockDim.x) ov[i] = g.occ_vec[i];
-    for (int i = threadIdx.x; i < g.n_sdw; i += blockDim.x) sv[i] = g.sdw_vec[i];
-  }
+  if (!want_gt) g.n_occ = g.n_sdw = 0;
+  const GtStage gs(f, g, gt_smem);
   __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -102,8 +99,8 @@ __global__ void __launch_bounds__(128) k_sur_label(const float4* __restrict__ pt
   }
   unsigned aux = 0;
   if (want_gt) {
-    GtShade sh{&g, tf, f.tf_n, ov, sv};
-    GtShade::Ray r;
+    GtShadeT<SampleAny> sh{&g, SampleAny(f.vol), TfAlpha{gs.alpha, f.tf_n}, gs.occ, gs.sdw};
+    GtShadeT<SampleAny>::Ray r;
     sh.begin(r, dir);
     t_out[2 * (size_t)i] = sh.occlusion(tx, r, f, aux);
     t_out[2 * (size_t)i + 1] = sh.shadow(tx, f, aux);
@@ -130,7 +127,7 @@ cudaError_t launch_sur_label(const float4* pts, int n, const FrameArgs& f, const
   const int want_gt = g && t_out ? 1 : 0, want_dos = d && dos_out ? 1 : 0;
   size_t sm = sizeof(float4) * f.tf_n;
   if (want_dos) sm += sizeof(float4) * (dd.occ.n_sections + dd.sdw.n_sections);
-  if (want_gt) sm += sizeof(float3) * (gg.n_occ + gg.n_sdw);
+  sm += GtStage::bytes(f.tf_n, want_gt ? gg : GtArgs{});
   auto kern = tex ? k_sur_label<true> : k_sur_label<false>;
   if (sm > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
