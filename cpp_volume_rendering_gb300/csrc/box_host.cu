@@ -20,6 +20,8 @@ namespace {
 // once the pixels rendered without them would have paid for them.
 constexpr double kPixelsPerCell = 4.0e-4;
 
+constexpr size_t kCellBytes = sizeof(float) * kBoxCellFloats;
+
 int texel_width(const ShadowBoxTable& t, int k, int axis) {
   int packed;
   std::memcpy(&packed, &t.tx[k].w, sizeof packed);
@@ -38,7 +40,8 @@ BoxTableDesc table_desc(const int n[3], const int ax[3], const int w[3], const i
   d.g.na = n[ax[0]] + pad[0];
   d.g.nb = n[ax[1]] + pad[1] + 1;
   d.g.nc = n[ax[2]] + pad[2] + 1;
-  d.g.nab = (unsigned)d.g.na * (unsigned)d.g.nb;
+  d.g.row = (int)padded_row((unsigned)d.g.na, (int)kCellBytes);
+  d.g.nab = padded_plane((unsigned)d.g.row * (unsigned)d.g.nb, (int)kCellBytes);
   return d;
 }
 size_t cells_of(const BoxGrid& g) { return (size_t)g.nab * (size_t)g.nc; }
@@ -48,7 +51,6 @@ BoxGrid lookup_grid(BoxGrid g) {
   --g.nc;
   return g;
 }
-constexpr size_t kCellBytes = sizeof(float) * kBoxCellFloats;
 
 }  // namespace
 

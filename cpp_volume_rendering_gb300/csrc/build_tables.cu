@@ -319,45 +319,45 @@ cudaError_t launch_sat_build_quads(const void* vox, int dtype, int nx, int ny, i
 // x-y quads of the volume: cell (x, y, z) = the voxels at (x, y), (x', y),
 // (x, y'), (x', y') of plane z, with the successors clamped to the volume.
 template <class T, class Q>
-__global__ void k_quad_volume(const T* __restrict__ v, Q* __restrict__ out, int nx, int ny, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int x = (int)(i % nx), y = (int)((i / nx) % ny);
-  const long long dx = x + 1 < nx ? 1 : 0, dy = y + 1 < ny ? nx : 0;
-  Q q;
-  q.x = v[i]; q.y = v[i + dx]; q.z = v[i + dy]; q.w = v[i + dy + dx];
-  out[i] = q;
+__global__ void __launch_bounds__(128) k_quads(const T* __restrict__ v, Q* __restrict__ out, int nx, int ny, int nz,
+                                               unsigned qrow, unsigned qplane) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= nx) return;
+  const int dx = x + 1 < nx ? 1 : 0;
+  // rows and planes beyond the grid's limits are strided over
+  for (int z = blockIdx.z; z < nz; z += gridDim.z)
+    for (int y = blockIdx.y; y < ny; y += gridDim.y) {
+      const T* p = v + ((size_t)z * ny + y) * (size_t)nx + x;
+      const T* r = p + (y + 1 < ny ? nx : 0);
+      Q q;
+      q.x = p[0]; q.y = p[dx]; q.z = r[0]; q.w = r[dx];
+      out[(size_t)z * qplane + (size_t)y * qrow + x] = q;
+    }
 }
 
-cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, int ny, int nz, cudaStream_t st) {
-  const long long n = (long long)nx * ny * nz;
-  const unsigned blocks = (unsigned)((n + 255) / 256);
-  if (dtype == 1)
-    k_quad_volume<uint8_t, uchar4><<<blocks, 256, 0, st>>>(static_cast<const uint8_t*>(src), static_cast<uchar4*>(dst),
-                                                           nx, ny, n);
-  else
-    k_quad_volume<uint16_t, ushort4><<<blocks, 256, 0, st>>>(static_cast<const uint16_t*>(src),
-                                                             static_cast<ushort4*>(dst), nx, ny, n);
+template <class T, class Q>
+static cudaError_t launch_quads(const T* v, Q* out, int nx, int ny, int nz, unsigned qrow, unsigned qplane,
+                                cudaStream_t st) {
+  const dim3 grid((nx + 127) / 128, std::min(ny, 65535), std::min(nz, 65535));
+  k_quads<T, Q><<<grid, 128, 0, st>>>(v, out, nx, ny, nz, qrow, qplane);
   return cudaGetLastError();
+}
+
+cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, int ny, int nz, unsigned qrow,
+                               unsigned qplane, cudaStream_t st) {
+  if (dtype == 1)
+    return launch_quads(static_cast<const uint8_t*>(src), static_cast<uchar4*>(dst), nx, ny, nz, qrow, qplane, st);
+  return launch_quads(static_cast<const uint16_t*>(src), static_cast<ushort4*>(dst), nx, ny, nz, qrow, qplane, st);
 }
 
 // x-y quads of every pyramid level (successors clamped within the level).
-__global__ void k_quad_pyramid(const float* __restrict__ src, float4* __restrict__ dst, int dx, int dy,
-                               long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int x = (int)(i % dx), y = (int)((i / dx) % dy);
-  const long long ox = x + 1 < dx ? 1 : 0, oy = y + 1 < dy ? dx : 0;
-  dst[i] = make_float4(src[i], src[i + ox], src[i + oy], src[i + oy + ox]);
-}
-
 cudaError_t launch_pyramid_quads(const PyramidView& P, const float* data, float4* dst, cudaStream_t st) {
   for (int l = 0; l < P.n_levels; ++l) {
-    const long long n = (long long)P.dims[l][0] * P.dims[l][1] * P.dims[l][2];
-    k_quad_pyramid<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(data + P.offset[l], dst + P.offset[l], P.dims[l][0],
-                                                                P.dims[l][1], n);
+    const cudaError_t e = launch_quads(data + P.offset[l], dst + P.qoff[l], P.dims[l][0], P.dims[l][1], P.dims[l][2],
+                                       P.quad_row(l), P.quad_plane(l), st);
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 // x-y predecessor quads of a table: out[(x, y, z)] = s at (x-1, y-1),
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(32 * kBoxRows) k_box_tables(BoxSource src, con
     else return (float)(int)v * src.scale;
   };
   const bool store = lane < kBoxRow && a < d.g.na;
-  float2* dst = reinterpret_cast<float2*>(out) + d.cell + (size_t)b * d.g.na + a;
+  float2* dst = reinterpret_cast<float2*>(out) + d.cell + (size_t)b * d.g.row + a;
   auto put = [&](int c, float v) {
     const float next = __shfl_down_sync(0xffffffffu, v, 1);
     if (store) dst[(size_t)c * d.g.nab] = make_float2(v, next);

@@ -60,10 +60,13 @@ long long pyramid_scratch_floats(const VolumeView& vol, const PyramidView& P, fl
 
 // Grid-stride fill of a device buffer (used to flush L2 between timed frames).
 cudaError_t launch_fill(void* p, size_t bytes, unsigned int v, cudaStream_t st);
-// The x-y quad copy of every pyramid level (float4 per value, same offsets).
+// The x-y quad copy of every pyramid level (float4 per value, at P.qoff with
+// pitches quad_row, quad_plane).
 cudaError_t launch_pyramid_quads(const PyramidView& P, const float* data, float4* dst, cudaStream_t st);
-// The x-y quad copy of a plain volume (uchar4 / ushort4 per voxel).
-cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, int ny, int nz, cudaStream_t st);
+// The x-y quad copy of a plain volume (uchar4 / ushort4 per voxel), rows of
+// qrow and planes of qplane cells.
+cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, int ny, int nz, unsigned qrow,
+                               unsigned qplane, cudaStream_t st);
 // Bricked copy of a plain volume (bricks of 2^bs voxels per edge); the copy
 // holds brick_elements(...) elements.
 long long brick_elements(int nx, int ny, int nz, int bs);

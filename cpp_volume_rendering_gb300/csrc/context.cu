@@ -122,11 +122,15 @@ namespace ctxutil {
 cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex) {
   VolumeView v = volume_view(c);
   // the quad copy is indexed with 32-bit cell numbers
-  if (c->quads && (size_t)c->nx * c->ny * c->nz < kCompactMaxCells) {
+  const int qbytes = c->dtype == CVR_U8 ? 4 : 8;
+  const size_t qrow = padded_row((unsigned)c->nx, qbytes);
+  const size_t qplane = qrow * c->ny < kCompactMaxCells ? padded_plane((unsigned)(qrow * c->ny), qbytes) : kCompactMaxCells;
+  if (c->quads && qplane * c->nz < kCompactMaxCells) {
+    v.qrow = (unsigned)qrow;
+    v.qplane = (unsigned)qplane;
     if (c->vbrick_bs != kQuadCopy) {
-      const size_t n = (size_t)c->nx * c->ny * c->nz;
-      CK(c, ensure(c->d_vbrick, c->vbrick_cap, n * 4 * (c->dtype == CVR_U8 ? 1 : 2)));
-      CK(c, launch_quad_volume(c->d_vol, c->d_vbrick, c->dtype, c->nx, c->ny, c->nz, c->stream));
+      CK(c, ensure(c->d_vbrick, c->vbrick_cap, qplane * c->nz * qbytes));
+      CK(c, launch_quad_volume(c->d_vol, c->d_vbrick, c->dtype, c->nx, c->ny, c->nz, v.qrow, v.qplane, c->stream));
       c->vbrick_bs = kQuadCopy;
     }
     v.voxels = c->d_vbrick;
@@ -502,9 +506,16 @@ cvr_status pyramid_view(cvr_ctx* c, PyramidView* out) {
     *out = P;
     return CVR_OK;
   }
+  size_t n = 0;
+  for (int l = 0; l < P.n_levels; ++l) {
+    P.qoff[l] = (unsigned)n;
+    n += (size_t)P.quad_plane(l) * P.dims[l][2];  // dims <= 4096: a plane is below 2^25 cells
+    if (n >= kCompactMaxCells) {  // 32-bit cell numbers: the plain levels
+      *out = P;
+      return CVR_OK;
+    }
+  }
   if (!c->pyrq_ready) {
-    const int L = c->pyr.n_levels - 1;
-    const size_t n = (size_t)c->pyr.offset[L] + (size_t)c->pyr.dims[L][0] * c->pyr.dims[L][1] * c->pyr.dims[L][2];
     // without room for the copy the taps read the plain levels
     cudaError_t e = ensure(c->d_pyrq, c->pyrq_cap, n * sizeof(float4));
     if (e == cudaErrorMemoryAllocation) {
@@ -784,7 +795,7 @@ cvr_status cvr_build_ext_pyramid(cvr_ctx* c, const cvr_pyramid_params* p) {
   long long off = 0;
   for (int l = 0; l < levels; ++l) {
     for (int a = 0; a < 3; ++a) P.dims[l][a] = std::max(1, p->base_dims[a] >> l);
-    P.offset[l] = off;
+    P.offset[l] = (unsigned)std::min<long long>(off, 0xffffffffLL);  // >= 2^31 in all: rejected below
     off += (long long)P.dims[l][0] * P.dims[l][1] * P.dims[l][2];
   }
   if (off >= (1LL << 31))

@@ -418,6 +418,7 @@ inline VolumeView volume_view(const cvr_ctx* c) {
   v.inv_grid = f3(1.0f / v.grid.x, 1.0f / v.grid.y, 1.0f / v.grid.z);
   v.bs = 0;
   v.quad = 0;
+  v.qrow = v.qplane = 0;
   v.stride[0] = 1;
   v.stride[1] = c->nx;
   v.stride[2] = (long long)c->nx * c->ny;

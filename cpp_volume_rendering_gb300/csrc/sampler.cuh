@@ -51,9 +51,8 @@ struct SampleQuads {
     const int x = min(cell_of(texel_of(p.x, v.inv_spacing.x), tx), v.nx - 1);
     const int y = min(cell_of(texel_of(p.y, v.inv_spacing.y), ty), v.ny - 1);
     const int z = min(cell_of(texel_of(p.z, v.inv_spacing.z), tz), v.nz - 1);
-    const unsigned plane = (unsigned)v.nx * (unsigned)v.ny;
-    const Q* q = static_cast<const Q*>(v.voxels) + ((unsigned)x + (unsigned)v.nx * (unsigned)y + plane * (unsigned)z);
-    const Q a = __ldg(q), b = __ldg(q + (z < v.nz - 1 ? plane : 0u));
+    const Q* q = static_cast<const Q*>(v.voxels) + ((unsigned)x + v.qrow * (unsigned)y + v.qplane * (unsigned)z);
+    const Q a = __ldg(q), b = __ldg(q + (z < v.nz - 1 ? v.qplane : 0u));
     return trilinear(a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, tx, ty, tz) * v.norm;
   }
 };

@@ -435,7 +435,7 @@ struct ExtBoxShade {
       const unsigned x = min((unsigned)(cell_of(g.x - r, q.x) + pad), (unsigned)G.na - 1u);
       const unsigned y = min((unsigned)(cell_of(g.y - r, q.y) + pad), (unsigned)G.nb - 1u);
       const unsigned z = min((unsigned)(cell_of(g.z - r, q.z) + pad), (unsigned)G.nc - 1u);
-      const BoxCorners c = box_corners(B.ao, B.ao_cell[i] + x + y * (unsigned)G.na + z * G.nab, G.na, G.nab);
+      const BoxCorners c = box_corners(B.ao, B.ao_cell[i] + x + y * (unsigned)G.row + z * G.nab, G.row, G.nab);
       const float b = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, q);
       t = i == 0 ? b * (1.0f / (r * r)) : t + (b - last) * (1.0f / (r * r));
       last = b;
@@ -466,7 +466,7 @@ struct ExtBoxShade {
   __device__ __forceinline__ float walk(float ga, float gb, float gw, int m) const {
     const BoxGrid& G = e->box.sdw_grid;
     const float* __restrict__ tab = e->box.sdw;
-    const int na = G.na;
+    const int row = G.row;
     const unsigned nab = G.nab, ma = (unsigned)G.na - 1u, mb = (unsigned)G.nb - 1u;
     float tw;
     const unsigned cw = (unsigned)(cell_of(gw + first, tw) + pad_w) * nab;
@@ -477,7 +477,7 @@ struct ExtBoxShade {
       float ta, tb;
       const unsigned a = min((unsigned)(cell_of(ga + o.x, ta) + pad_a), ma);
       const unsigned b = min((unsigned)(cell_of(gb + o.y, tb) + pad_b), mb);
-      const BoxCorners c = box_corners(tab, (__float_as_uint(o.w) + cw) + (a + b * (unsigned)na), na, nab);
+      const BoxCorners c = box_corners(tab, (__float_as_uint(o.w) + cw) + (a + b * (unsigned)row), row, nab);
       float v;  // corners as (x, y, z) bits, so that the lerp order is z, y, x
       if constexpr (AXIS == 2)
         v = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, f3(ta, tb, tw));
