@@ -11,7 +11,7 @@ __global__ void __launch_bounds__(NT) k_march_plain(const __grid_constant__ Fram
   __syncthreads();
   int px, py;
   pixel_of(f, px, py);
-  march_ray_with(f, S(f.vol), TfTable{sm_tf, f.tf_n}, PlainShade{}, px, py);
+  march_ray_pairs(f, S(f.vol), TfTable{sm_tf, f.tf_n}, PlainShade{}, px, py);
 }
 
 template <int NT>

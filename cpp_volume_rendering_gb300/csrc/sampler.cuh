@@ -10,6 +10,7 @@
 #pragma once
 
 #include "march.cuh"
+#include "pack2.cuh"
 
 namespace cvr {
 
@@ -18,6 +19,7 @@ struct SampleAny {
   const VolumeView& v;
   __device__ __forceinline__ explicit SampleAny(const VolumeView& view) : v(view) {}
   __device__ __forceinline__ float operator()(float3 p) const { return sample_volume(v, p); }
+  __device__ __forceinline__ f2 two(const pos2& p) const { return mk2((*this)(pos_lo(p)), (*this)(pos_hi(p))); }
 };
 
 // The texture unit's copy.
@@ -27,6 +29,7 @@ struct SampleTex {
   __device__ __forceinline__ float operator()(float3 p) const {
     return tex3D<float>(v.tex, p.x * v.inv_grid.x, p.y * v.inv_grid.y, p.z * v.inv_grid.z);
   }
+  __device__ __forceinline__ f2 two(const pos2& p) const { return mk2((*this)(pos_lo(p)), (*this)(pos_hi(p))); }
 };
 
 // Texel coordinate of one axis raised to 0: below the first texel centre both
@@ -39,6 +42,19 @@ __device__ __forceinline__ float trilinear(float c000, float c100, float c010, f
   const float c01 = fmaf(tx, c101 - c001, c001), c11 = fmaf(tx, c111 - c011, c011);
   const float c0 = fmaf(ty, c10 - c00, c00), c1 = fmaf(ty, c11 - c01, c01);
   return fmaf(tz, c1 - c0, c0);
+}
+
+// Cells and fractions of two positions along one axis (raised to 0, at most n - 1).
+__device__ __forceinline__ int2 texel_cells2(f2 p, float inv_spacing, int n, f2& t) {
+  const float2 u = un2(fma2(p, dup2(inv_spacing), dup2(-0.5f)));
+  const int2 c = cell_of2(mk2(fmaxf(u.x, 0.0f), fmaxf(u.y, 0.0f)), t);
+  return make_int2(min(c.x, n - 1), min(c.y, n - 1));
+}
+__device__ __forceinline__ f2 trilinear2(f2 c000, f2 c100, f2 c010, f2 c110, f2 c001, f2 c101, f2 c011, f2 c111,
+                                         f2 tx, f2 ty, f2 tz) {
+  const f2 c0 = lerp2(ty, lerp2(tx, c000, c100), lerp2(tx, c010, c110));
+  const f2 c1 = lerp2(ty, lerp2(tx, c001, c101), lerp2(tx, c011, c111));
+  return lerp2(tz, c0, c1);
 }
 
 // The x-y quad copy (VolumeView::quad): two loads, planes z0 and z0 + 1.
@@ -54,6 +70,18 @@ struct SampleQuads {
     const Q* q = static_cast<const Q*>(v.voxels) + ((unsigned)x + v.qrow * (unsigned)y + v.qplane * (unsigned)z);
     const Q a = __ldg(q), b = __ldg(q + (z < v.nz - 1 ? v.qplane : 0u));
     return trilinear(a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, tx, ty, tz) * v.norm;
+  }
+  __device__ __forceinline__ f2 two(const pos2& p) const {
+    f2 tx, ty, tz;
+    const int2 x = texel_cells2(p.x, v.inv_spacing.x, v.nx, tx), y = texel_cells2(p.y, v.inv_spacing.y, v.ny, ty),
+               z = texel_cells2(p.z, v.inv_spacing.z, v.nz, tz);
+    const Q* base = static_cast<const Q*>(v.voxels);
+    const Q* q = base + ((unsigned)x.x + v.qrow * (unsigned)y.x + v.qplane * (unsigned)z.x);
+    const Q* r = base + ((unsigned)x.y + v.qrow * (unsigned)y.y + v.qplane * (unsigned)z.y);
+    const Q a = __ldg(q), b = __ldg(q + (z.x < v.nz - 1 ? v.qplane : 0u));
+    const Q c = __ldg(r), d = __ldg(r + (z.y < v.nz - 1 ? v.qplane : 0u));
+    return mul2(trilinear2(mk2(a.x, c.x), mk2(a.y, c.y), mk2(a.z, c.z), mk2(a.w, c.w), mk2(b.x, d.x), mk2(b.y, d.y),
+                           mk2(b.z, d.z), mk2(b.w, d.w), tx, ty, tz), dup2(v.norm));
   }
 };
 
@@ -76,6 +104,29 @@ struct SamplePlain {
     return trilinear(__ldg(q), __ldg(q + dx), __ldg(r), __ldg(r + dx), __ldg(s), __ldg(s + dx), __ldg(t), __ldg(t + dx),
                      tx, ty, tz) * v.norm;
   }
+  __device__ __forceinline__ f2 two(const pos2& p) const {
+    f2 tx, ty, tz;
+    const int2 x = texel_cells2(p.x, v.inv_spacing.x, v.nx, tx), y = texel_cells2(p.y, v.inv_spacing.y, v.ny, ty),
+               z = texel_cells2(p.z, v.inv_spacing.z, v.nz, tz);
+    const unsigned nx = (unsigned)v.nx, plane = nx * (unsigned)v.ny;
+    const T* base = static_cast<const T*>(v.voxels);
+    T g[2][8];
+    auto gather = [&](int X, int Y, int Z, T* o) {
+      const T* q = base + ((unsigned)X + nx * (unsigned)Y + plane * (unsigned)Z);
+      const unsigned dx = X < v.nx - 1 ? 1u : 0u, dy = Y < v.ny - 1 ? nx : 0u, dz = Z < v.nz - 1 ? plane : 0u;
+      const T* r = q + dy;
+      const T* s = q + dz;
+      const T* t = r + dz;
+      o[0] = __ldg(q); o[1] = __ldg(q + dx); o[2] = __ldg(r); o[3] = __ldg(r + dx);
+      o[4] = __ldg(s); o[5] = __ldg(s + dx); o[6] = __ldg(t); o[7] = __ldg(t + dx);
+    };
+    gather(x.x, y.x, z.x, g[0]);
+    gather(x.y, y.y, z.y, g[1]);
+    f2 c[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) c[k] = mk2(g[0][k], g[1][k]);
+    return mul2(trilinear2(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], tx, ty, tz), dup2(v.norm));
+  }
 };
 
 // Calls fn with the sampler type of a volume view.
@@ -91,6 +142,11 @@ cudaError_t with_sampler(const VolumeView& v, F fn) {
 }
 
 // ---------------------------------------------------------------- transfer function
+// Entry and fraction of two densities.
+__device__ __forceinline__ uint2 tf_cells2(f2 density, int n, f2& t) {
+  const int2 c = cell_of2(fma2(density, dup2((float)n), dup2(-0.5f)), t);
+  return make_uint2(min((unsigned)(c.x + 1), (unsigned)n), min((unsigned)(c.y + 1), (unsigned)n));
+}
 // texture(TexTransferFunc, density) from a table of entries and differences:
 // entry k holds tf[k - 1] and tf[k] - tf[k - 1] (0 past either end, where
 // both taps are the edge entry), so a lookup is one index, one clamp and one
@@ -104,6 +160,18 @@ struct TfTable {
     const float4 a = e[2 * i], d = e[2 * i + 1];
     return make_float4(fmaf(t, d.x, a.x), fmaf(t, d.y, a.y), fmaf(t, d.z, a.z), fmaf(t, d.w, a.w));
   }
+  __device__ __forceinline__ void two(f2 density, float4& s0, float4& s1) const {
+    f2 t;
+    const uint2 i = tf_cells2(density, n, t);
+    const float2 f = un2(t);
+    s0 = mix(i.x, f.x);
+    s1 = mix(i.y, f.y);
+  }
+  __device__ __forceinline__ float4 mix(unsigned i, float t) const {
+    const float4 a = e[2 * i], d = e[2 * i + 1];
+    const float2 lo = un2(fma2(dup2(t), mk2(d.x, d.y), mk2(a.x, a.y))), hi = un2(fma2(dup2(t), mk2(d.z, d.w), mk2(a.z, a.w)));
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
 };
 // The extinction channel alone: 8 bytes per entry.
 struct TfAlpha {
@@ -114,6 +182,12 @@ struct TfAlpha {
     const unsigned i = min((unsigned)(cell_of(fmaf(density, (float)n, -0.5f), t) + 1), (unsigned)n);
     const float2 a = e[i];
     return fmaf(t, a.y, a.x);
+  }
+  __device__ __forceinline__ f2 two(f2 density) const {
+    f2 t;
+    const uint2 i = tf_cells2(density, n, t);
+    const float2 a = e[i.x], b = e[i.y];
+    return fma2(t, mk2(a.y, b.y), mk2(a.x, b.x));
   }
 };
 // Filled by the whole CTA (a barrier before the first lookup is the caller's).

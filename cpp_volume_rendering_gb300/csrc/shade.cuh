@@ -700,12 +700,19 @@ struct GtShadeT {
       bool in[kAhead];
       float sj = s;
 #pragma unroll
-      for (int j = 0; j < kAhead; ++j) {
+      for (int j = 0; j < kAhead; j += 2) {
         h[j] = fminf(g->lstep, dist - sj);
-        const float3 at = tx + w * (sj + h[j]);
-        in[j] = sj < dist && !(at.x < 0.0f || at.x > G.x || at.y < 0.0f || at.y > G.y || at.z < 0.0f || at.z > G.z);
-        st[j] = alpha(sample(at));
-        sj = sj + h[j];
+        const float e0 = sj + h[j];
+        h[j + 1] = fminf(g->lstep, dist - e0);
+        const float e1 = e0 + h[j + 1];
+        const pos2 at = along2(tx, w, mk2(e0, e1));
+        const float2 x = un2(at.x), y = un2(at.y), z = un2(at.z);
+        in[j] = sj < dist && !(x.x < 0.0f || x.x > G.x || y.x < 0.0f || y.x > G.y || z.x < 0.0f || z.x > G.z);
+        in[j + 1] = e0 < dist && !(x.y < 0.0f || x.y > G.x || y.y < 0.0f || y.y > G.y || z.y < 0.0f || z.y > G.z);
+        const float2 a = un2(alpha.two(sample.two(at)));
+        st[j] = a.x;
+        st[j + 1] = a.y;
+        sj = e1;
       }
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
@@ -851,6 +858,59 @@ struct TfStaged {
   int n;
   __device__ __forceinline__ float4 operator()(float density) const { return tf_lookup(e, n, density); }
 };
+
+// The same loop two samples at a time, their positions, cells and lerps in
+// packed pairs (their positions do not depend on the compositing): for the
+// marchers whose step is mostly the sample itself.
+template <class S, class Shade>
+__device__ __forceinline__ void march_ray_pairs(const FrameArgs& f, const S& sample, const TfTable& tf,
+                                                const Shade& sh, int px, int py) {
+  const bool inside = px < f.W && py < f.H;
+  unsigned int n = 0, shaded = 0, aux = 0;
+  if (inside) {
+    const float3 dir = primary_dir(f.cam, px, py, f.W, f.H);
+    float tnear, tfar;
+    float4 dst = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (ray_aabb(f.cam.eye, dir, f.vol.grid, tnear, tfar)) {
+      typename Shade::Ray ray;
+      sh.begin(ray, dir);
+      const float D = fabsf(tfar - tnear);
+      const float3 tex0 = f.cam.eye + dir * tnear + f.vol.grid * 0.5f;
+      const unsigned max_iter = (unsigned)fminf(D / f.step, 1.0e9f) + 4u;
+      // one step; false when it ends the ray
+      auto take = [&](float4 src, float3 p, float h) {
+        ++n;
+        if (src.w > 0.0f) {
+          ++shaded;
+          src = sh.shade(src, p, ray, f, aux);
+          src.w = 1.0f - expf(-src.w * h);
+          src.x *= src.w; src.y *= src.w; src.z *= src.w;
+          const float r = 1.0f - dst.w;
+          dst.x += r * src.x; dst.y += r * src.y; dst.z += r * src.z; dst.w += r * src.w;
+          if (dst.w > 0.99f) return false;
+        }
+        return true;
+      };
+      for (float s = 0.0f; s < D && n < max_iter;) {
+        const float h0 = fminf(f.step, D - s);
+        const float s1 = s + h0;
+        const float h1 = fminf(f.step, D - s1);
+        const pos2 p = along2(tex0, dir, mk2(s + h0 * 0.5f, s1 + h1 * 0.5f));
+        float4 src0, src1;
+        tf.two(sample.two(p), src0, src1);
+        if (!take(src0, pos_lo(p), h0)) break;
+        s = s1;
+        if (!(s < D && n < max_iter)) break;
+        if (!take(src1, pos_hi(p), h1)) break;
+        s = s + h1;
+      }
+    }
+    const size_t o = (size_t)py * f.W + px;
+    f.out[o] = dst;
+    if (f.counts) f.counts[o] = n;
+  }
+  add_stats(f, n, shaded, aux);
+}
 
 template <class Shade>
 __device__ __forceinline__ void march_ray(const FrameArgs& f, const float4* tf, const Shade& sh, int px, int py) {
