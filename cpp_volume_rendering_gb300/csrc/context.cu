@@ -570,6 +570,42 @@ cvr_status ensure_sat(cvr_ctx* c) {
   return CVR_OK;
 }
 
+// Renders a frame with deferred shading: light(d) launches the light pass over
+// a band's records.  *done = false leaves the frame to the direct marcher (a
+// ray with more steps than the lists hold, or no room for them).
+template <class Light>
+static cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t, bool ext, Light light,
+                                   bool* done) {
+  *done = false;
+  DeferredPlan p;
+  // from very far away a ray's length is mostly rounding: the direct marcher
+  const double diag2 = (double)dot3(f.vol.grid, f.vol.grid), eye2 = (double)dot3(f.cam.eye, f.cam.eye);
+  if (f.work || !(eye2 <= 1.0e4 * diag2) || !deferred_plan(f, &p)) return cudaSuccess;
+  const size_t head = 256, chunk_bytes = (p.warps * p.chunks * sizeof(unsigned) + 255) / 256 * 256;
+  cudaError_t e = ensure(c->d_defer, c->defer_cap, head + chunk_bytes + p.records * (sizeof(float4) + sizeof(float2)));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  if (e != cudaSuccess) return e;
+  char* base = static_cast<char*>(c->d_defer);
+  Deferred d;
+  d.counter = reinterpret_cast<unsigned*>(base);
+  d.chunk = reinterpret_cast<unsigned*>(base + head);
+  d.rec = reinterpret_cast<float4*>(base + head + chunk_bytes);
+  d.light = reinterpret_cast<float2*>(d.rec + p.records);
+  d.chunks = p.chunks;
+  for (unsigned b = 0; b < p.bands && e == cudaSuccess; ++b) {
+    d.y0 = b * p.rows;
+    e = cudaMemsetAsync(d.counter, 0, 2 * sizeof(unsigned), c->stream);
+    if (e == cudaSuccess) e = launch_collect(f, d, p.rows, c->stream);
+    if (e == cudaSuccess) e = light(d);
+    if (e == cudaSuccess) e = launch_resolve(f, d, p.rows, t, ext, c->stream);
+  }
+  *done = e == cudaSuccess;
+  return e;
+}
+
 }  // namespace ctxutil
 }  // namespace cvr
 
@@ -619,7 +655,7 @@ void cvr_destroy(cvr_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_vol, c->d_rgbt, c->d_rgba, c->d_sat, c->d_lut, c->d_pyr, c->d_occ_sec, c->d_sdw_sec,
                   c->d_occ_vec, c->d_sdw_vec, c->d_stats, c->d_out, c->d_flush, c->d_probe, c->d_vbrick, c->d_lcache, c->d_grad, c->d_ms, c->d_msf,
-                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc};
+                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc, c->d_defer};
   for (void* p : bufs)
     if (p) cudaFree(p);
   for (int i = 0; i < 4; ++i)
@@ -1036,7 +1072,10 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       a.light_pos = make3(light->position); a.light_fwd = make3(light->forward);
       a.light_up = make3(light->up); a.light_right = make3(light->right);
       a.ka = p->ka; a.kd = p->kd;
-      e = launch_gt(f, a, c->stream);
+      bool done = false;
+      e = render_deferred(c, f, light_terms(a.apply_occ, a.apply_sdw, a.ka, a.kd), false,
+                          [&](const Deferred& d) { return launch_light_gt(f, a, d, c->stream); }, &done);
+      if (e == cudaSuccess && !done) e = launch_gt(f, a, c->stream);
       break;
     }
     case CVR_METHOD_ISO: {

@@ -13,6 +13,7 @@
 
 #include "../../include/cvr.h"
 #include "build_tables.cuh"
+#include "deferred.cuh"
 #include "march.cuh"
 #include "surrogate.cuh"
 
@@ -243,6 +244,9 @@ struct cvr_ctx {
   unsigned* d_boxsrc = nullptr;
   size_t boxsrc_cap = 0;
   unsigned long long boxsrc_gen = 0;         // the SAT and fixed point it holds (box_gen)
+  // deferred shading's lists (deferred.cuh), bounded by deferred_plan
+  void* d_defer = nullptr;
+  size_t defer_cap = 0;
   // pyramid, and its x-y quad copy for FP32 taps (built with the first frame that needs it)
   float* d_pyr = nullptr;
   size_t pyr_cap = 0;

@@ -1,0 +1,214 @@
+// deferred.cu — the two marching passes of deferred shading.
+#include "deferred.cuh"
+#include "march_ext.cuh"
+
+namespace cvr {
+
+namespace {
+
+constexpr size_t kDeferredRecords = (size_t)64 << 20;  // 24 bytes each: at most 1.5 GiB per context
+constexpr unsigned kMaxBands = 512;
+
+__device__ __forceinline__ void band_pixel(const FrameArgs& f, const Deferred& d, int& px, int& py, unsigned& warp) {
+  pixel_of(f, px, py);
+  py += (int)d.y0 * f.tile_h;
+  warp = (blockIdx.y * gridDim.x + blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+}
+
+// The primary ray of a pixel; false: it misses the box or lies outside the image.
+struct Primary {
+  float3 dir, tex0;
+  float D;
+  unsigned max_iter;
+};
+__device__ __forceinline__ bool primary_ray(const FrameArgs& f, int px, int py, Primary& r) {
+  r = Primary{f3(0.0f, 0.0f, 0.0f), f3(0.0f, 0.0f, 0.0f), 0.0f, 0u};
+  if (px >= f.W || py >= f.H) return false;
+  r.dir = primary_dir(f.cam, px, py, f.W, f.H);
+  float tnear, tfar;
+  if (!ray_aabb(f.cam.eye, r.dir, f.vol.grid, tnear, tfar)) return false;
+  r.D = fabsf(tfar - tnear);
+  r.tex0 = f.cam.eye + r.dir * tnear + f.vol.grid * 0.5f;
+  r.max_iter = (unsigned)fminf(r.D / f.step, 1.0e9f) + 4u;
+  return true;
+}
+
+template <int NT, class S>
+__global__ void __launch_bounds__(NT) k_collect(const __grid_constant__ FrameArgs f, const __grid_constant__ Deferred d) {
+  extern __shared__ float2 sm_alpha[];
+  stage_tf_alpha(f.tf, f.tf_n, sm_alpha);
+  __syncthreads();
+  const TfAlpha tf{sm_alpha, f.tf_n};
+  const S sample(f.vol);
+  int px, py;
+  unsigned warp;
+  band_pixel(f, d, px, py, warp);
+  const int lane = threadIdx.x & 31;
+  unsigned* chunk = d.chunk + (size_t)warp * d.chunks;
+  Primary r;
+  bool live = primary_ray(f, px, py, r) && r.D > 0.0f;
+  const int pixel = py * f.W + px;
+  float s = 0.0f, opacity = 0.0f;
+  unsigned n = 0;
+  unsigned filled = 0, base = 0, next = 0;  // records of the warp; first slot of its current and of its next chunk
+  while (__any_sync(0xffffffffu, live)) {
+    bool shaded = false;
+    float3 p = f3(0.0f, 0.0f, 0.0f);
+    if (live) {
+      const float h = fminf(f.step, r.D - s);
+      p = r.tex0 + r.dir * (s + h * 0.5f);
+      float a = tf(sample(p));
+      ++n;
+      if (a > 0.0f) {
+        shaded = true;
+        a = 1.0f - expf(-a * h);
+        const float left = 1.0f - opacity;
+        opacity += left * a;
+        if (opacity > 0.99f) live = false;
+      }
+      s = s + h;
+      live = live && s < r.D && n < r.max_iter;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, shaded);
+    if (m == 0) continue;
+    const unsigned take = (unsigned)__popc(m), slot = filled % kRecChunk;
+    if (filled + take > d.chunks * kRecChunk) break;  // deferred_plan's bound holds; never past the lists
+    // a step may end one chunk and begin the next
+    const bool first = slot == 0, over = slot != 0 && slot + take > kRecChunk;
+    if (first || over) {
+      if (lane == 0) next = atomicAdd(d.counter, kRecChunk);
+      next = __shfl_sync(0xffffffffu, next, 0);
+      if (lane == 0) chunk[(filled + take - 1) / kRecChunk] = next;
+      if (first) base = next;
+    }
+    if (shaded) {
+      const unsigned i = slot + (unsigned)__popc(m & ((1u << lane) - 1u));
+      d.rec[i < kRecChunk ? base + i : next + (i - kRecChunk)] = make_float4(p.x, p.y, p.z, __int_as_float(pixel));
+    }
+    if (over) base = next;
+    filled += take;
+  }
+  // the unused slots of the last chunk
+  if (filled % kRecChunk)
+    for (unsigned i = filled % kRecChunk + lane; i < kRecChunk; i += 32) d.rec[base + i].w = __int_as_float(-1);
+}
+
+template <int NT, class S>
+__global__ void __launch_bounds__(NT) k_resolve(const __grid_constant__ FrameArgs f, const __grid_constant__ Deferred d,
+                                                LightTerms t, int ext) {
+  extern __shared__ float4 sm_tf[];
+  stage_tf_table(f.tf, f.tf_n, sm_tf);
+  __syncthreads();
+  const TfTable tf{sm_tf, f.tf_n};
+  const S sample(f.vol);
+  int px, py;
+  unsigned warp;
+  band_pixel(f, d, px, py, warp);
+  const int lane = threadIdx.x & 31;
+  const unsigned* chunk = d.chunk + (size_t)warp * d.chunks;
+  Primary r;
+  bool live = primary_ray(f, px, py, r) && r.D > 0.0f;
+  float4 dst = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float s = 0.0f;
+  unsigned n = 0, n_shaded = 0, filled = 0;
+  while (__any_sync(0xffffffffu, live)) {
+    bool shaded = false;
+    float h = 0.0f;
+    float3 p = f3(0.0f, 0.0f, 0.0f);
+    float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (live) {
+      h = fminf(f.step, r.D - s);
+      p = r.tex0 + r.dir * (s + h * 0.5f);
+      src = tf(sample(p));
+      ++n;
+      shaded = src.w > 0.0f;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, shaded);
+    if (filled + (unsigned)__popc(m) > d.chunks * kRecChunk) break;  // as collect
+    if (shaded) {
+      ++n_shaded;
+      const unsigned i = filled + (unsigned)__popc(m & ((1u << lane) - 1u));
+      const float2 l = d.light[chunk[i / kRecChunk] + i % kRecChunk];
+      src = ext ? t.apply<true>(f, src, p, l) : t.apply<false>(f, src, p, l);
+      src.w = 1.0f - expf(-src.w * h);
+      src.x *= src.w; src.y *= src.w; src.z *= src.w;
+      const float left = 1.0f - dst.w;
+      dst.x += left * src.x; dst.y += left * src.y; dst.z += left * src.z; dst.w += left * src.w;
+      if (dst.w > 0.99f) live = false;
+    }
+    filled += (unsigned)__popc(m);
+    s = s + h;
+    live = live && s < r.D && n < r.max_iter;
+  }
+  if (px < f.W && py < f.H) {
+    const size_t o = (size_t)py * f.W + px;
+    f.out[o] = dst;
+    if (f.counts) f.counts[o] = n;
+  }
+  add_stats(f, n, n_shaded, 0u);
+}
+
+dim3 band_grid(const FrameArgs& f, const Deferred& d, unsigned rows) {
+  const unsigned all = (unsigned)((f.H + f.tile_h - 1) / f.tile_h);
+  return dim3((unsigned)((f.W + f.tile_w - 1) / f.tile_w), std::min(rows, all - d.y0));
+}
+
+template <class F>
+cudaError_t with_threads(const FrameArgs& f, F fn) {
+  switch (threads_of(f)) {
+    case 64: return fn(std::integral_constant<int, 64>());
+    case 256: return fn(std::integral_constant<int, 256>());
+    default: return fn(std::integral_constant<int, 128>());
+  }
+}
+
+}  // namespace
+
+bool deferred_plan(const FrameArgs& f, DeferredPlan* p) {
+  // steps of the longest ray of any camera: the diagonal, and the four the
+  // marchers' own bound allows past it
+  const double diag = std::sqrt((double)dot3(f.vol.grid, f.vol.grid));
+  const double steps = diag * 1.0001 / (double)f.step + 8.0;
+  const double chunks = std::ceil(steps * 32.0 / kRecChunk) + 1.0;
+  const size_t row_warps = (size_t)((f.W + f.tile_w - 1) / f.tile_w) * (size_t)(threads_of(f) / 32);
+  const size_t all = (size_t)((f.H + f.tile_h - 1) / f.tile_h);
+  if (!(chunks * kRecChunk * (double)row_warps <= (double)kDeferredRecords)) return false;
+  if ((size_t)f.W * f.H > 0x7fffffff) return false;
+  p->chunks = (unsigned)chunks;
+  const size_t row = row_warps * p->chunks * kRecChunk;
+  p->rows = (unsigned)std::min(all, kDeferredRecords / row);
+  p->bands = (unsigned)((all + p->rows - 1) / p->rows);
+  p->records = row * p->rows;
+  p->warps = row_warps * p->rows;
+  return p->bands <= kMaxBands;
+}
+
+cudaError_t launch_collect(const FrameArgs& f, const Deferred& d, unsigned rows, cudaStream_t st) {
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    return with_threads(f, [&](auto nt) {
+      constexpr int NT = decltype(nt)::value;
+      k_collect<NT, S><<<band_grid(f, d, rows), NT, sizeof(float2) * ((size_t)f.tf_n + 1), st>>>(f, d);
+      return cudaGetLastError();
+    });
+  });
+}
+
+cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows, const LightTerms& t, bool ext,
+                           cudaStream_t st) {
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    return with_threads(f, [&](auto nt) {
+      constexpr int NT = decltype(nt)::value;
+      const size_t sm = tf_table_bytes(f.tf_n);
+      auto kern = k_resolve<NT, S>;
+      cudaError_t e = cudaSuccess;
+      if (sm > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (e != cudaSuccess) return e;
+      kern<<<band_grid(f, d, rows), NT, sm, st>>>(f, d, t, ext ? 1 : 0);
+      return cudaGetLastError();
+    });
+  });
+}
+
+}  // namespace cvr

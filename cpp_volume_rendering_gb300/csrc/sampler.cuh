@@ -20,6 +20,8 @@ struct SampleAny {
   __device__ __forceinline__ explicit SampleAny(const VolumeView& view) : v(view) {}
   __device__ __forceinline__ float operator()(float3 p) const { return sample_volume(v, p); }
   __device__ __forceinline__ f2 two(const pos2& p) const { return mk2((*this)(pos_lo(p)), (*this)(pos_hi(p))); }
+  __device__ __forceinline__ f2 two_inside(const pos2& p) const { return two(p); }
+  static constexpr bool kInside = false;
 };
 
 // The texture unit's copy.
@@ -30,6 +32,8 @@ struct SampleTex {
     return tex3D<float>(v.tex, p.x * v.inv_grid.x, p.y * v.inv_grid.y, p.z * v.inv_grid.z);
   }
   __device__ __forceinline__ f2 two(const pos2& p) const { return mk2((*this)(pos_lo(p)), (*this)(pos_hi(p))); }
+  __device__ __forceinline__ f2 two_inside(const pos2& p) const { return two(p); }
+  static constexpr bool kInside = false;
 };
 
 // Texel coordinate of one axis raised to 0: below the first texel centre both
@@ -55,6 +59,49 @@ __device__ __forceinline__ f2 trilinear2(f2 c000, f2 c100, f2 c010, f2 c110, f2 
   const f2 c0 = lerp2(ty, lerp2(tx, c000, c100), lerp2(tx, c010, c110));
   const f2 c1 = lerp2(ty, lerp2(tx, c001, c101), lerp2(tx, c011, c111));
   return lerp2(tz, c0, c1);
+}
+
+// The part [ta, tb] of the line o + d t whose positions are at least 0.51
+// voxels inside the box on every axis: there a sample's cell needs no clamp
+// and both its planes exist (0.01 voxels are far more than the roundings of
+// t and of the position, for axes of up to 8192 voxels; larger ones, and
+// lines with a NaN, get an empty part).
+__device__ __forceinline__ void inside_part(const VolumeView& v, float3 o, float3 d, float& ta, float& tb) {
+  const float3 m = v.spacing * 0.51f;
+  const float3 inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+  const float3 t0 = (m - o) * inv, t1 = (v.grid - m - o) * inv;
+  const float3 lo = fmin3(t0, t1), hi = fmax3(t0, t1);
+  ta = fmaxf(fmaxf(lo.x, lo.y), lo.z);
+  tb = fminf(fminf(hi.x, hi.y), hi.z);
+  const float sum = d.x + d.y + d.z + o.x + o.y + o.z;
+  if (!(sum - sum == 0.0f) || v.nx > 8192 || v.ny > 8192 || v.nz > 8192) tb = -1.0f, ta = 0.0f;
+}
+
+// Voxel values as FP32 plus 2^23: the integer below 2^16 placed in the
+// mantissa of 8388608.0f by one byte permute.  Differences of two such values
+// are exact, so a lerp subtracts them as they are and unbiases one end.
+struct biased8 {
+  unsigned w;
+  template <int K>
+  __device__ __forceinline__ float at() const { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650u + K)); }
+};
+struct biased16 {
+  uint2 w;
+  template <int K>
+  __device__ __forceinline__ float at() const {
+    return __uint_as_float(__byte_perm(K < 2 ? w.x : w.y, 0x4B000000u, (K & 1) ? 0x7632u : 0x7610u));
+  }
+};
+// lerp of biased ends: fmaf(t, b - a, a - 2^23).
+__device__ __forceinline__ f2 lerp_biased2(f2 t, f2 a, f2 b) { return fma2(t, sub2(b, a), sub2(a, dup2(8388608.0f))); }
+
+// Cells (plus 0x4B400000) and fractions of two positions inside the box along one axis.
+__device__ __forceinline__ uint2 inside_cells2(f2 p, float inv_spacing, f2& t) {
+  const f2 u = fma2(p, dup2(inv_spacing), dup2(-0.5f)), magic = dup2(12582912.0f);
+  const f2 r = add_rd2(u, magic);
+  t = sub2(u, sub2(r, magic));
+  const float2 b = un2(r);
+  return make_uint2(__float_as_uint(b.x), __float_as_uint(b.y));
 }
 
 // The x-y quad copy (VolumeView::quad): two loads, planes z0 and z0 + 1.
@@ -83,6 +130,27 @@ struct SampleQuads {
     return mul2(trilinear2(mk2(a.x, c.x), mk2(a.y, c.y), mk2(a.z, c.z), mk2(a.w, c.w), mk2(b.x, d.x), mk2(b.y, d.y),
                            mk2(b.z, d.z), mk2(b.w, d.w), tx, ty, tz), dup2(v.norm));
   }
+  // two() for positions inside_part holds: no raise, no clamp, no last plane.
+  static constexpr bool kInside = true;
+  __device__ __forceinline__ f2 two_inside(const pos2& p) const {
+    using B = typename std::conditional<sizeof(Q) == 4, biased8, biased16>::type;
+    f2 tx, ty, tz;
+    const uint2 x = inside_cells2(p.x, v.inv_spacing.x, tx), y = inside_cells2(p.y, v.inv_spacing.y, ty),
+                z = inside_cells2(p.z, v.inv_spacing.z, tz);
+    // cells carry the bias: 32-bit arithmetic takes it off the sum
+    const unsigned bias = 0u - 0x4B400000u * (1u + v.qrow + v.qplane);
+    const B* base = static_cast<const B*>(v.voxels);
+    const B* q = base + (x.x + bias + v.qrow * y.x + v.qplane * z.x);
+    const B* r = base + (x.y + bias + v.qrow * y.y + v.qplane * z.y);
+    const B a = load(q), b = load(q + v.qplane), c = load(r), d = load(r + v.qplane);
+    const f2 c00 = lerp_biased2(tx, mk2(a.template at<0>(), c.template at<0>()), mk2(a.template at<1>(), c.template at<1>()));
+    const f2 c10 = lerp_biased2(tx, mk2(a.template at<2>(), c.template at<2>()), mk2(a.template at<3>(), c.template at<3>()));
+    const f2 c01 = lerp_biased2(tx, mk2(b.template at<0>(), d.template at<0>()), mk2(b.template at<1>(), d.template at<1>()));
+    const f2 c11 = lerp_biased2(tx, mk2(b.template at<2>(), d.template at<2>()), mk2(b.template at<3>(), d.template at<3>()));
+    return mul2(lerp2(tz, lerp2(ty, c00, c10), lerp2(ty, c01, c11)), dup2(v.norm));
+  }
+  static __device__ __forceinline__ biased8 load(const biased8* p) { return biased8{__ldg(&p->w)}; }
+  static __device__ __forceinline__ biased16 load(const biased16* p) { return biased16{__ldg(&p->w)}; }
 };
 
 // The plain x-fastest array: eight loads.
@@ -126,6 +194,20 @@ struct SamplePlain {
 #pragma unroll
     for (int k = 0; k < 8; ++k) c[k] = mk2(g[0][k], g[1][k]);
     return mul2(trilinear2(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], tx, ty, tz), dup2(v.norm));
+  }
+  static constexpr bool kInside = true;
+  __device__ __forceinline__ f2 two_inside(const pos2& p) const {
+    f2 tx, ty, tz;
+    const uint2 x = inside_cells2(p.x, v.inv_spacing.x, tx), y = inside_cells2(p.y, v.inv_spacing.y, ty),
+                z = inside_cells2(p.z, v.inv_spacing.z, tz);
+    const unsigned nx = (unsigned)v.nx, plane = nx * (unsigned)v.ny;
+    const unsigned bias = 0u - 0x4B400000u * (1u + nx + plane);
+    const T* base = static_cast<const T*>(v.voxels);
+    const T* q = base + (x.x + bias + nx * y.x + plane * z.x);
+    const T* r = base + (x.y + bias + nx * y.y + plane * z.y);
+    auto pair = [&](unsigned o) { return mk2((float)__ldg(q + o), (float)__ldg(r + o)); };
+    return mul2(trilinear2(pair(0u), pair(1u), pair(nx), pair(nx + 1u), pair(plane), pair(plane + 1u), pair(plane + nx),
+                           pair(plane + nx + 1u), tx, ty, tz), dup2(v.norm));
   }
 };
 

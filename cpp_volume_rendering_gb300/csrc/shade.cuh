@@ -112,6 +112,25 @@ __device__ __forceinline__ float4 phong_cone(const FrameArgs& f, float4 L, float
   return L;
 }
 
+// The weights of ShadeSample's occlusion and shadow terms and the colour of a
+// sample from its (occlusion, shadow); EXT: the extinction renderer's gradient
+// branch, else the cone's and the ground truth's.
+struct LightTerms {
+  float ka, kd;
+  template <bool EXT>
+  __device__ __forceinline__ float4 apply(const FrameArgs& f, float4 src, float3 tx, float2 l) const {
+    if (f.grad.g) return EXT ? phong_ext(f, src, tx, l.x, ka, l.y, kd) : phong_cone(f, src, tx, l.x, ka, l.y, kd);
+    const float k = 1.0f / (ka + kd);
+    src.x = k * (src.x * l.x * ka + src.x * l.y * kd);
+    src.y = k * (src.y * l.x * ka + src.y * l.y * kd);
+    src.z = k * (src.z * l.x * ka + src.z * l.y * kd);
+    return src;
+  }
+};
+__host__ __device__ __forceinline__ LightTerms light_terms(int occ, int sdw, float ka, float kd) {
+  return LightTerms{occ ? ka : 0.0f, sdw ? kd : 0.0f};
+}
+
 // ============================================================ plain (rc1pass)
 struct PlainShade {
   struct Ray {};
@@ -389,21 +408,19 @@ struct ExtShadeT {
     return expf(-st);
   }
 
-  // ShadeSample (ebs_ray_bbox_marching.comp:500-551).
-  __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
-    float ka = 0.0f, kd = 0.0f, io = 0.0f, is = 0.0f;
-    if (e->apply_occ) { ka = e->ka; io = ambient_occlusion(tx, f); aux += e->n_shells; }
+  // ShadeSample (ebs_ray_bbox_marching.comp:500-551): the light terms, and
+  // the colour from them.
+  __device__ __forceinline__ float2 light(float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
+    float io = 0.0f, is = 0.0f;
+    if (e->apply_occ) { io = ambient_occlusion(tx, f); aux += e->n_shells; }
     if (e->apply_sdw) {
-      kd = e->kd;
       if constexpr (ALIGNED) is = shadow_table(tx, f, aux);
       else is = tlo ? shadow_table(tx, f, aux) : shadow(tx, f, aux);
     }
-    if (f.grad.g) return phong_ext(f, src, tx, io, ka, is, kd);
-    float k = 1.0f / (ka + kd);
-    src.x = k * (src.x * io * ka + src.x * is * kd);
-    src.y = k * (src.y * io * ka + src.y * is * kd);
-    src.z = k * (src.z * io * ka + src.z * is * kd);
-    return src;
+    return make_float2(io, is);
+  }
+  __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
+    return light_terms(e->apply_occ, e->apply_sdw, e->ka, e->kd).apply<true>(f, src, tx, light(tx, r, f, aux));
   }
 };
 using ExtShade = ExtShadeT<false>;
@@ -499,17 +516,15 @@ struct ExtBoxShade {
   }
 
   // ShadeSample (ebs_ray_bbox_marching.comp:500-551).
-  __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
+  __device__ __forceinline__ float2 light(float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
     const float3 g = sat_texel(e->sat, tx);
-    float ka = 0.0f, kd = 0.0f, io = 0.0f, is = 0.0f;
-    if (e->apply_occ) { ka = e->ka; io = ambient_occlusion(g); aux += e->n_shells; }
-    if (e->apply_sdw) { kd = e->kd; is = shadow(tx, g, aux); }
-    if (f.grad.g) return phong_ext(f, src, tx, io, ka, is, kd);
-    const float k = 1.0f / (ka + kd);
-    src.x = k * (src.x * io * ka + src.x * is * kd);
-    src.y = k * (src.y * io * ka + src.y * is * kd);
-    src.z = k * (src.z * io * ka + src.z * is * kd);
-    return src;
+    float io = 0.0f, is = 0.0f;
+    if (e->apply_occ) { io = ambient_occlusion(g); aux += e->n_shells; }
+    if (e->apply_sdw) is = shadow(tx, g, aux);
+    return make_float2(io, is);
+  }
+  __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
+    return light_terms(e->apply_occ, e->apply_sdw, e->ka, e->kd).apply<true>(f, src, tx, light(tx, r, f, aux));
   }
 };
 
@@ -649,16 +664,14 @@ struct DosShadeT {
   }
 
   // ShadeSample (ray_bbox_marching.comp:607-656).
+  __device__ __forceinline__ float2 light(float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
+    float io = 0.0f, is = 0.0f;
+    if (d->apply_occ) io = occlusion(tx, r, f, aux);
+    if (d->apply_sdw) is = shadow(tx, f, aux);
+    return make_float2(io, is);
+  }
   __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
-    float ka = 0.0f, kd = 0.0f, io = 0.0f, is = 0.0f;
-    if (d->apply_occ) { ka = d->ka; io = occlusion(tx, r, f, aux); }
-    if (d->apply_sdw) { kd = d->kd; is = shadow(tx, f, aux); }
-    if (f.grad.g) return phong_cone(f, src, tx, io, ka, is, kd);
-    float kk = 1.0f / (ka + kd);
-    src.x = kk * (src.x * io * ka + src.x * is * kd);
-    src.y = kk * (src.y * io * ka + src.y * is * kd);
-    src.z = kk * (src.z * io * ka + src.z * is * kd);
-    return src;
+    return light_terms(d->apply_occ, d->apply_sdw, d->ka, d->kd).apply<false>(f, src, tx, light(tx, r, f, aux));
   }
 };
 using DosShade = DosShadeT<false>;
@@ -693,26 +706,39 @@ struct GtShadeT {
     float vt = 1.0f;
     ++aux;
     float s = g->gap;
-    const float3 G = f.vol.grid;
+    const float3 B = f.vol.grid;
     float st0 = alpha(sample(tx + w * s));
+    float ta = 0.0f, tb = -1.0f;  // the samples that need no box test and no clamp
+    if constexpr (S::kInside) inside_part(f.vol, tx, w, ta, tb);
     for (int guard = 0; guard < kMaxLightSteps && s < dist; guard += kAhead) {
-      float h[kAhead], st[kAhead];
+      float h[kAhead], at[kAhead], st[kAhead];
       bool in[kAhead];
       float sj = s;
 #pragma unroll
-      for (int j = 0; j < kAhead; j += 2) {
+      for (int j = 0; j < kAhead; ++j) {
         h[j] = fminf(g->lstep, dist - sj);
-        const float e0 = sj + h[j];
-        h[j + 1] = fminf(g->lstep, dist - e0);
-        const float e1 = e0 + h[j + 1];
-        const pos2 at = along2(tx, w, mk2(e0, e1));
-        const float2 x = un2(at.x), y = un2(at.y), z = un2(at.z);
-        in[j] = sj < dist && !(x.x < 0.0f || x.x > G.x || y.x < 0.0f || y.x > G.y || z.x < 0.0f || z.x > G.z);
-        in[j + 1] = e0 < dist && !(x.y < 0.0f || x.y > G.x || y.y < 0.0f || y.y > G.y || z.y < 0.0f || z.y > G.z);
-        const float2 a = un2(alpha.two(sample.two(at)));
-        st[j] = a.x;
-        st[j + 1] = a.y;
-        sj = e1;
+        in[j] = sj < dist;
+        sj = sj + h[j];
+        at[j] = sj;
+      }
+      if (S::kInside && at[0] >= ta && at[kAhead - 1] <= tb) {
+#pragma unroll
+        for (int j = 0; j < kAhead; j += 2) {
+          const float2 a = un2(alpha.two(sample.two_inside(along2(tx, w, mk2(at[j], at[j + 1])))));
+          st[j] = a.x;
+          st[j + 1] = a.y;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kAhead; j += 2) {
+          const pos2 p = along2(tx, w, mk2(at[j], at[j + 1]));
+          const float2 x = un2(p.x), y = un2(p.y), z = un2(p.z);
+          in[j] = in[j] && !(x.x < 0.0f || x.x > B.x || y.x < 0.0f || y.x > B.y || z.x < 0.0f || z.x > B.z);
+          in[j + 1] = in[j + 1] && !(x.y < 0.0f || x.y > B.x || y.y < 0.0f || y.y > B.y || z.y < 0.0f || z.y > B.z);
+          const float2 a = un2(alpha.two(sample.two(p)));
+          st[j] = a.x;
+          st[j + 1] = a.y;
+        }
       }
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
@@ -768,16 +794,14 @@ struct GtShadeT {
   }
 
   // ShadeSample (gt_ray_marching.comp:254-303).
+  __device__ __forceinline__ float2 light(float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
+    float io = 0.0f, is = 0.0f;
+    if (g->apply_occ) io = occlusion(tx, r, f, aux);
+    if (g->apply_sdw) is = shadow(tx, f, aux);
+    return make_float2(io, is);
+  }
   __device__ __forceinline__ float4 shade(float4 src, float3 tx, const Ray& r, const FrameArgs& f, unsigned& aux) const {
-    float ka = 0.0f, kd = 0.0f, io = 0.0f, is = 0.0f;
-    if (g->apply_occ) { ka = g->ka; io = occlusion(tx, r, f, aux); }
-    if (g->apply_sdw) { kd = g->kd; is = shadow(tx, f, aux); }
-    if (f.grad.g) return phong_cone(f, src, tx, io, ka, is, kd);
-    float kk = 1.0f / (ka + kd);
-    src.x = kk * (src.x * io * ka + src.x * is * kd);
-    src.y = kk * (src.y * io * ka + src.y * is * kd);
-    src.z = kk * (src.z * io * ka + src.z * is * kd);
-    return src;
+    return light_terms(g->apply_occ, g->apply_sdw, g->ka, g->kd).apply<false>(f, src, tx, light(tx, r, f, aux));
   }
 };
 
