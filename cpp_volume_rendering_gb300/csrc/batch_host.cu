@@ -1,6 +1,7 @@
 // batch_host.cu — resident volume slots and batched rendering: a fixed list
-// of frames over the resident volumes, one persistent launch per method,
-// captured with the resets of its counters in one CUDA graph.
+// of frames over the resident volumes, captured in one CUDA graph: the
+// extinction jobs in persistent launches, the surrogate jobs as deferred
+// frames on lanes beside them.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -10,6 +11,10 @@
 #include "ctx.cuh"
 
 using namespace cvr::ctxutil;
+
+// Lanes of the surrogate jobs in a batch's graph: a frame's collect and resolve
+// passes leave most of the GPU idle, so they run beside another lane's.
+constexpr int kSurLanes = 3;
 
 struct cvr_batch {
   cvr_ctx* ctx = nullptr;
@@ -22,9 +27,8 @@ struct cvr_batch {
   int ext_threads = 128;
   float4* d_tables = nullptr;
   float* d_cuts = nullptr;
-  int n_sur = 0;
-  bool sur_tex = false;
-  unsigned int* d_counters = nullptr;  // [0] extinction tiles, [1] box-table tiles, [2 + k] surrogate rays of launch k
+  void* lists[kSurLanes] = {};            // deferred shading's lists, one set per lane
+  unsigned int* d_counters = nullptr;  // [0] extinction tiles, [1] box-table tiles, [2 + k] rays of surrogate job k (direct marcher)
   unsigned long long* d_stats = nullptr;  // 3 per job, in the caller's job order
   bool ext_compact = false;
   bool ext_aligned = false;  // every job: an aligned shadow table and aligned AO boxes (or AO off)
@@ -38,6 +42,8 @@ struct cvr_batch {
     if (graph) cudaGraphExecDestroy(graph);
     void* bufs[] = {d_ext, d_tables, d_cuts, d_counters, d_stats};
     for (void* p : bufs)
+      if (p) cudaFree(p);
+    for (void* p : lists)
       if (p) cudaFree(p);
     for (uint4* p : sat32)
       if (p) cudaFree(p);
@@ -128,8 +134,14 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   bool all_compact = c->compact_sat;
   std::vector<std::vector<float4>> tables;
   std::vector<std::unique_ptr<ShadowBoxTable>> aligned;  // of the jobs box tables can serve, else null
-  std::vector<SurLaunch> sur;  // the surrogate jobs in launches of up to kSurLaunchJobs
-  unsigned long long sur_positions = 0;
+  struct SurFrameJob {
+    FrameArgs f;
+    SurArgs a;
+    DeferredPlan plan;
+    size_t bytes;  // of its lists; 0: the direct marcher
+    bool tex;
+  };
+  std::vector<SurFrameJob> sur;
   const int keep = c->cur_slot;
   cvr_status st = CVR_OK;
   for (int oi = 0; oi < n_jobs && st == CVR_OK; ++oi) {
@@ -166,33 +178,12 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
                                ? new ShadowBoxTable(*table) : nullptr);
       ext.push_back(J);
     } else {
-      SurJob J{};
-      bool tex = false;
-      st = sur_job_args(c, static_cast<const cvr_gt_params*>(j.params), &j.light, &J.a, &tex);
+      SurFrameJob J{};
+      st = sur_job_args(c, static_cast<const cvr_gt_params*>(j.params), &j.light, &J.a, &J.tex);
       if (st != CVR_OK) break;
-      if (!sur.empty() && tex != b->sur_tex) { st = fail(c, CVR_ERR_INVALID_ARG, "cvr_batch_create: mixed sampling"); break; }
-      b->sur_tex = tex;
       J.f = f;
-      const SurSpiral o = sur_spiral(f);
-      J.cx = o.cx;
-      J.cy = o.cy;
-      J.tiles_x = (j.width + 7) / 8;
-      J.tiles_y = (j.height + 3) / 4;
-      if (sur.empty() || sur.back().n_jobs == kSurLaunchJobs) {
-        sur.emplace_back();
-        std::memset(&sur.back(), 0, sizeof(SurLaunch));
-        sur_positions = 0;
-      }
-      SurLaunch& L = sur.back();
-      J.first_tile = (unsigned)sur_positions;
-      sur_positions += o.positions;
-      if (sur_positions * 32ull > 0xFFFFFFF0ull) {
-        st = fail(c, CVR_ERR_UNSUPPORTED, "cvr_batch_create: more than 2^32 surrogate rays in one launch");
-        break;
-      }
-      L.total = (unsigned)(sur_positions * 32ull);
-      L.jobs[L.n_jobs++] = J;
-      ++b->n_sur;
+      J.bytes = deferred_bytes(f, &J.plan);
+      sur.push_back(J);
     }
   }
   // Compact SATs owned by the batch (a later frame may rebuild the context's
@@ -369,20 +360,66 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   }
   const size_t n_counters = 2 + sur.size();
   CK(c, cudaMalloc((void**)&b->d_counters, sizeof(unsigned int) * n_counters));
-  // capture: counter and statistics resets, then the persistent launches
+  // the lanes' lists, each as large as its largest job needs (a lane without
+  // room leaves its jobs to the direct marcher)
+  const int lanes = (int)std::min<size_t>(sur.size(), kSurLanes);
+  for (int l = 0; l < lanes; ++l) {
+    size_t bytes = 0;
+    for (size_t k = l; k < sur.size(); k += lanes) bytes = std::max(bytes, sur[k].bytes);
+    if (bytes == 0) continue;
+    const cudaError_t me = cudaMalloc(&b->lists[l], bytes);
+    if (me == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      for (size_t k = l; k < sur.size(); k += lanes) sur[k].bytes = 0;
+    } else if (me != cudaSuccess) {
+      return cuda_fail(c, me, "cvr_batch_create: sample lists");
+    }
+  }
+  // capture: counter and statistics resets, then the extinction launches
+  // beside the lanes of surrogate frames
+  struct Lanes {
+    cudaStream_t s[kSurLanes] = {};
+    cudaEvent_t fork = nullptr, join[kSurLanes] = {};
+    ~Lanes() {
+      for (cudaStream_t x : s)
+        if (x) cudaStreamDestroy(x);
+      for (cudaEvent_t x : join)
+        if (x) cudaEventDestroy(x);
+      if (fork) cudaEventDestroy(fork);
+    }
+  } lane;
+  if (lanes > 0) CK(c, cudaEventCreateWithFlags(&lane.fork, cudaEventDisableTiming));
+  for (int l = 0; l < lanes; ++l) {
+    CK(c, cudaStreamCreateWithFlags(&lane.s[l], cudaStreamNonBlocking));
+    CK(c, cudaEventCreateWithFlags(&lane.join[l], cudaEventDisableTiming));
+  }
   cudaGraph_t g = nullptr;
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
   cudaError_t e = cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned int) * n_counters, c->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(b->d_stats, 0, sizeof(unsigned long long) * 3 * n_jobs, c->stream);
+  if (e == cudaSuccess && lanes > 0) e = cudaEventRecord(lane.fork, c->stream);
+  for (int l = 0; l < lanes && e == cudaSuccess; ++l) {
+    cudaStream_t ls = lane.s[l];
+    e = cudaStreamWaitEvent(ls, lane.fork, 0);
+    for (size_t k = l; k < sur.size() && e == cudaSuccess; k += lanes) {
+      const SurFrameJob& J = sur[k];
+      if (J.bytes > 0)
+        e = launch_deferred(b->lists[l], J.plan, J.f, light_terms(J.a.apply_occ, J.a.apply_sdw, J.a.ka, J.a.kd), false,
+                            (unsigned)kSurPyramidTaps,
+                            [&](const Deferred& d) { return launch_light_sur(J.f, J.a, J.tex, d, c->mlp->err, ls); },
+                            ls);
+      else
+        e = launch_surrogate(J.f, J.a, J.tex, sur_spiral(J.f), b->d_counters + 2 + k, c->mlp->err, ls);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(lane.join[l], ls);
+  }
   if (e == cudaSuccess && b->n_ext)
     e = launch_batch_extinction(b->d_ext, b->n_ext, b->ext_blocks, b->d_counters, c->tf_n, b->ext_max_table,
                                 b->ext_threads, b->ext_variant, b->ext_compact, b->ext_aligned, c->stream);
   if (e == cudaSuccess && b->n_box)
     e = launch_batch_box(b->d_ext + b->n_ext, b->n_box, b->box_blocks, b->d_counters + 1, c->tf_n, b->ext_max_table,
                          b->ext_threads, b->ext_variant, c->stream);
-  for (size_t k = 0; k < sur.size() && e == cudaSuccess; ++k)
-    e = launch_batch_surrogate(sur[k], c->tf_n, b->sur_tex, b->ext_variant, b->d_counters + 2 + k, c->mlp->err,
-                               c->stream);
+  for (int l = 0; l < lanes && e == cudaSuccess; ++l) e = cudaStreamWaitEvent(c->stream, lane.join[l], 0);
   cudaError_t e2 = cudaStreamEndCapture(c->stream, &g);
   if (e != cudaSuccess || e2 != cudaSuccess) {
     if (g) cudaGraphDestroy(g);

@@ -319,8 +319,8 @@ cudaError_t launch_sat_build_quads(const void* vox, int dtype, int nx, int ny, i
 // x-y quads of the volume: cell (x, y, z) = the voxels at (x, y), (x', y),
 // (x, y'), (x', y') of plane z, with the successors clamped to the volume.
 template <class T, class Q>
-__global__ void __launch_bounds__(128) k_quads(const T* __restrict__ v, Q* __restrict__ out, int nx, int ny, int nz,
-                                               unsigned qrow, unsigned qplane) {
+__global__ void __launch_bounds__(128) k_quad_volume(const T* __restrict__ v, Q* __restrict__ out, int nx, int ny,
+                                                     int nz, unsigned qrow, unsigned qplane) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= nx) return;
   const int dx = x + 1 < nx ? 1 : 0;
@@ -339,7 +339,7 @@ template <class T, class Q>
 static cudaError_t launch_quads(const T* v, Q* out, int nx, int ny, int nz, unsigned qrow, unsigned qplane,
                                 cudaStream_t st) {
   const dim3 grid((nx + 127) / 128, std::min(ny, 65535), std::min(nz, 65535));
-  k_quads<T, Q><<<grid, 128, 0, st>>>(v, out, nx, ny, nz, qrow, qplane);
+  k_quad_volume<T, Q><<<grid, 128, 0, st>>>(v, out, nx, ny, nz, qrow, qplane);
   return cudaGetLastError();
 }
 
@@ -350,14 +350,26 @@ cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, in
   return launch_quads(static_cast<const uint16_t*>(src), static_cast<ushort4*>(dst), nx, ny, nz, qrow, qplane, st);
 }
 
-// x-y quads of every pyramid level (successors clamped within the level).
+// The bordered x-y quads of every pyramid level (PyramidView::quads) in one
+// launch: blockIdx.z runs over the planes of all levels.
+__global__ void __launch_bounds__(128) k_quad_pyramid(const __grid_constant__ PyramidView P, const float* __restrict__ v,
+                                                      float4* __restrict__ out) {
+  int l = 0, z = blockIdx.z;
+  while (z >= P.dims[l][2] + 2) z -= P.dims[l++][2] + 2;
+  const int nx = P.dims[l][0], ny = P.dims[l][1], nz = P.dims[l][2];
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+  if (x > nx || y > ny) return;
+  const float* p = v + P.offset[l] + (size_t)min(max(z - 1, 0), nz - 1) * nx * ny;
+  const int x0 = max(x - 1, 0), x1 = min(x, nx - 1), y0 = max(y - 1, 0) * nx, y1 = min(y, ny - 1) * nx;
+  out[(size_t)P.qoff[l] + (size_t)z * P.quad_plane(l) + (size_t)y * P.quad_row(l) + x] =
+      make_float4(p[y0 + x0], p[y1 + x0], p[y0 + x1], p[y1 + x1]);
+}
+
 cudaError_t launch_pyramid_quads(const PyramidView& P, const float* data, float4* dst, cudaStream_t st) {
-  for (int l = 0; l < P.n_levels; ++l) {
-    const cudaError_t e = launch_quads(data + P.offset[l], dst + P.qoff[l], P.dims[l][0], P.dims[l][1], P.dims[l][2],
-                                       P.quad_row(l), P.quad_plane(l), st);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  int planes = 0;
+  for (int l = 0; l < P.n_levels; ++l) planes += P.dims[l][2] + 2;
+  k_quad_pyramid<<<dim3(P.dims[0][0] / 128 + 1, P.dims[0][1] + 1, planes), 128, 0, st>>>(P, data, dst);
+  return cudaGetLastError();
 }
 
 // x-y predecessor quads of a table: out[(x, y, z)] = s at (x-1, y-1),

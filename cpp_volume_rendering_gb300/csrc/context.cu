@@ -119,17 +119,37 @@ bool build_shadow_table(const cvr_ext_params* p, const float fwd[3], float3 spac
 namespace cvr {
 namespace ctxutil {
 
-cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex) {
+// Whether the marchers of a plain-layout volume read an x-y quad copy all the
+// same.  The copy costs about 2 ps a voxel; a sample from it saves 4 ps against
+// the plain array's eight loads, and a frame takes about a voxel edge of them
+// per pixel.  pixels: of this frame (0: asks for a copy that exists).
+static bool quads_pay(cvr_ctx* c, double pixels) {
+  if (c->brick_bs > 0 || c->staging) return false;
+  const double voxels = (double)c->nx * c->ny * c->nz;
+  if (voxels * 4.0 * (c->dtype == CVR_U8 ? 1 : 2) > (double)kAutoCopyBytes) return false;
+  if (c->vbrick_bs == kQuadCopy) return true;
+  c->quad_seen += pixels;
+  return 2.0 * c->quad_seen * std::max(c->nx, std::max(c->ny, c->nz)) >= voxels;
+}
+
+cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, double pixels) {
   VolumeView v = volume_view(c);
   // the quad copy is indexed with 32-bit cell numbers
   const int qbytes = c->dtype == CVR_U8 ? 4 : 8;
   const size_t qrow = padded_row((unsigned)c->nx, qbytes);
   const size_t qplane = qrow * c->ny < kCompactMaxCells ? padded_plane((unsigned)(qrow * c->ny), qbytes) : kCompactMaxCells;
-  if (c->quads && qplane * c->nz < kCompactMaxCells) {
+  const bool tex = allow_tex && (c->sampling & CVR_SAMPLING_TEX_VOLUME);
+  if ((c->quads || (!tex && quads_pay(c, pixels))) && qplane * c->nz < kCompactMaxCells) {
     v.qrow = (unsigned)qrow;
     v.qplane = (unsigned)qplane;
     if (c->vbrick_bs != kQuadCopy) {
-      CK(c, ensure(c->d_vbrick, c->vbrick_cap, qplane * c->nz * qbytes));
+      cudaError_t qe = ensure(c->d_vbrick, c->vbrick_cap, qplane * c->nz * qbytes);
+      if (qe == cudaErrorMemoryAllocation && !c->quads) {  // not asked for: the plain array serves
+        cudaGetLastError();
+        *out = volume_view(c);
+        return CVR_OK;
+      }
+      CK(c, qe);
       CK(c, launch_quad_volume(c->d_vol, c->d_vbrick, c->dtype, c->nx, c->ny, c->nz, v.qrow, v.qplane, c->stream));
       c->vbrick_bs = kQuadCopy;
     }
@@ -150,7 +170,7 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex) {
     v.stride[1] = bx * v.stride[0];
     v.stride[2] = by * v.stride[1];
   }
-  if (allow_tex && (c->sampling & CVR_SAMPLING_TEX_VOLUME)) {
+  if (tex) {
     cvr_status st = ensure_volume_texture(c);
     if (st != CVR_OK) return st;
     v.tex = c->tex.vol.tex;
@@ -168,7 +188,7 @@ cvr_status frame_args(cvr_ctx* c, const cvr_camera* cam, const void* params, flo
   if (!finite3(cam->eye) || !finite3(cam->center) || !finite3(cam->up))
     return fail(c, CVR_ERR_INVALID_ARG, "cvr_render: non-finite camera");
   FrameArgs f;
-  cvr_status vs = render_volume_view(c, &f.vol);
+  cvr_status vs = render_volume_view(c, &f.vol, true, (double)w * h);
   if (vs != CVR_OK) return vs;
   f.cam = camera_view(cam, w, h);
   f.tf = c->d_rgbt;
@@ -502,15 +522,13 @@ cvr_status pyramid_view(cvr_ctx* c, PyramidView* out) {
   PyramidView P = c->pyr;
   P.data = c->d_pyr;
   P.quads = nullptr;
-  if (!c->quads) {  // the plain layout
-    *out = P;
-    return CVR_OK;
-  }
   size_t n = 0;
   for (int l = 0; l < P.n_levels; ++l) {
     P.qoff[l] = (unsigned)n;
-    n += (size_t)P.quad_plane(l) * P.dims[l][2];  // dims <= 4096: a plane is below 2^25 cells
-    if (n >= kCompactMaxCells) {  // 32-bit cell numbers: the plain levels
+    n += (size_t)P.quad_plane(l) * (P.dims[l][2] + 2);  // dims <= 4096: a plane is below 2^25 cells
+    // 32-bit cell numbers, and without the quad layout a copy of at most
+    // kAutoCopyBytes: else the plain levels
+    if (n >= kCompactMaxCells || (!c->quads && n * sizeof(float4) > kAutoCopyBytes)) {
       *out = P;
       return CVR_OK;
     }
@@ -568,42 +586,6 @@ cvr_status ensure_sat(cvr_ctx* c) {
   CK(c, launch_sat_build(c->d_vol, c->dtype, c->nx, c->ny, c->nz, c->d_lut, c->d_sat, c->stream));
   c->sat_pending = false;
   return CVR_OK;
-}
-
-// Renders a frame with deferred shading: light(d) launches the light pass over
-// a band's records.  *done = false leaves the frame to the direct marcher (a
-// ray with more steps than the lists hold, or no room for them).
-template <class Light>
-static cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t, bool ext, Light light,
-                                   bool* done) {
-  *done = false;
-  DeferredPlan p;
-  // from very far away a ray's length is mostly rounding: the direct marcher
-  const double diag2 = (double)dot3(f.vol.grid, f.vol.grid), eye2 = (double)dot3(f.cam.eye, f.cam.eye);
-  if (f.work || !(eye2 <= 1.0e4 * diag2) || !deferred_plan(f, &p)) return cudaSuccess;
-  const size_t head = 256, chunk_bytes = (p.warps * p.chunks * sizeof(unsigned) + 255) / 256 * 256;
-  cudaError_t e = ensure(c->d_defer, c->defer_cap, head + chunk_bytes + p.records * (sizeof(float4) + sizeof(float2)));
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    return cudaSuccess;
-  }
-  if (e != cudaSuccess) return e;
-  char* base = static_cast<char*>(c->d_defer);
-  Deferred d;
-  d.counter = reinterpret_cast<unsigned*>(base);
-  d.chunk = reinterpret_cast<unsigned*>(base + head);
-  d.rec = reinterpret_cast<float4*>(base + head + chunk_bytes);
-  d.light = reinterpret_cast<float2*>(d.rec + p.records);
-  d.chunks = p.chunks;
-  for (unsigned b = 0; b < p.bands && e == cudaSuccess; ++b) {
-    d.y0 = b * p.rows;
-    e = cudaMemsetAsync(d.counter, 0, 2 * sizeof(unsigned), c->stream);
-    if (e == cudaSuccess) e = launch_collect(f, d, p.rows, c->stream);
-    if (e == cudaSuccess) e = light(d);
-    if (e == cudaSuccess) e = launch_resolve(f, d, p.rows, t, ext, c->stream);
-  }
-  *done = e == cudaSuccess;
-  return e;
 }
 
 }  // namespace ctxutil
@@ -702,6 +684,7 @@ static cvr_status set_volume_common(cvr_ctx* c, const void* src, bool src_device
   c->tex.vol_valid = false;
   c->tex.pyr_valid = false;
   c->vbrick_bs = -1;
+  c->quad_seen = 0.0;
   c->grad_ready = false;  // rebuilt with the slot's gradient model on the next shaded frame
   c->tex.grad_valid = false;
   return CVR_OK;
@@ -884,7 +867,8 @@ cvr_status cvr_download_pyramid_level(cvr_ctx* c, int level, float* host) {
   return CVR_OK;
 }
 
-static cvr_status upload_cone(cvr_ctx* c, const cvr_cone_table* t, float4** d, ConeTableDev* out) {
+static cvr_status upload_cone(cvr_ctx* c, const cvr_cone_table* t, float4** d, ConeTableDev* out,
+                              std::vector<float4>* host) {
   if (t->n_sections < 0 || t->n_sections > CVR_MAX_CONE_SECTIONS)
     return fail(c, CVR_ERR_INVALID_ARG, "cone table: bad section count");
   int n1 = t->integration_samples[0], n3 = t->integration_samples[1], n7 = t->integration_samples[2];
@@ -894,6 +878,8 @@ static cvr_status upload_cone(cvr_ctx* c, const cvr_cone_table* t, float4** d, C
   size_t bytes = sizeof(float4) * std::max(1, t->n_sections);
   CK(c, cudaMalloc((void**)d, bytes));
   if (t->n_sections) CK(c, cudaMemcpy(*d, t->sections, sizeof(float4) * t->n_sections, cudaMemcpyHostToDevice));
+  host->resize(t->n_sections);
+  std::memcpy(host->data(), t->sections, sizeof(float4) * t->n_sections);
   out->n_sections = t->n_sections;
   out->n1 = n1; out->n3 = n3; out->n7 = n7;
   for (int i = 0; i < 10; ++i) out->axes[i] = make3(t->axes[i]);
@@ -906,9 +892,9 @@ static cvr_status upload_cone(cvr_ctx* c, const cvr_cone_table* t, float4** d, C
 cvr_status cvr_set_cone_tables(cvr_ctx* c, const cvr_cone_table* occ, const cvr_cone_table* sdw) {
   if (!c || !occ || !sdw) return fail(c, CVR_ERR_INVALID_ARG, "cvr_set_cone_tables: bad arguments");
   CK(c, cudaSetDevice(c->device));
-  cvr_status s = upload_cone(c, occ, &c->d_occ_sec, &c->occ);
+  cvr_status s = upload_cone(c, occ, &c->d_occ_sec, &c->occ, &c->occ_host);
   if (s != CVR_OK) return s;
-  s = upload_cone(c, sdw, &c->d_sdw_sec, &c->sdw);
+  s = upload_cone(c, sdw, &c->d_sdw_sec, &c->sdw, &c->sdw_host);
   if (s != CVR_OK) return s;
   c->cone_ready = true;
   return CVR_OK;
@@ -1051,7 +1037,10 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
           for (int l = 0; l < c->tex.n_pyr; ++l) a.ptex[l] = c->tex.pyr[l].tex;
           tex = true;
         }
-        e = launch_dos(f, a, tex, c->stream);
+        bool done = false;
+        e = render_deferred(c, f, light_terms(a.apply_occ, a.apply_sdw, a.ka, a.kd), false, 0u,
+                            [&](const Deferred& d) { return launch_light_dos(f, a, c->occ_host.data(), c->sdw_host.data(), tex, d, c->stream); }, &done);
+        if (e == cudaSuccess && !done) e = launch_dos(f, a, tex, c->stream);
       }
       break;
     }
@@ -1073,7 +1062,7 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       a.light_up = make3(light->up); a.light_right = make3(light->right);
       a.ka = p->ka; a.kd = p->kd;
       bool done = false;
-      e = render_deferred(c, f, light_terms(a.apply_occ, a.apply_sdw, a.ka, a.kd), false,
+      e = render_deferred(c, f, light_terms(a.apply_occ, a.apply_sdw, a.ka, a.kd), false, 0u,
                           [&](const Deferred& d) { return launch_light_gt(f, a, d, c->stream); }, &done);
       if (e == cudaSuccess && !done) e = launch_gt(f, a, c->stream);
       break;

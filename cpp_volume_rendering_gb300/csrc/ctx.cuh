@@ -125,6 +125,9 @@ struct BoxTables {
   unsigned long long seen_gen = 0;
 };
 
+// Largest quad copy made without cvr_set_volume_layout asking for the quads.
+constexpr size_t kAutoCopyBytes = (size_t)2 << 30;
+
 // A resident volume that is not the current one (cvr_select_volume): the
 // volume, its SAT, pyramid and texture copies.  The current volume lives in
 // the cvr_ctx fields of the same names.
@@ -162,6 +165,7 @@ struct VolSlot {
   void* d_vbrick = nullptr;
   size_t vbrick_cap = 0;
   int vbrick_bs = -1;
+  double quad_seen = 0.0;
   uint2* d_grad = nullptr;
   size_t grad_cap = 0;
   bool grad_ready = false;
@@ -259,6 +263,7 @@ struct cvr_ctx {
   float4* d_occ_sec = nullptr;
   float4* d_sdw_sec = nullptr;
   ConeTableDev occ{}, sdw{};
+  std::vector<float4> occ_host, sdw_host;    // their sections
   bool cone_ready = false;
   // GT kernel vectors
   float3* d_occ_vec = nullptr;
@@ -296,6 +301,7 @@ struct cvr_ctx {
   bool quads = false;                        // tuning: the x-y quad layout (takes precedence)
   void* d_vbrick = nullptr;
   size_t vbrick_cap = 0;
+  double quad_seen = 0.0;                    // pixels of the volume's frames without a quad copy (quads_pay)
   int vbrick_bs = -1;                        // layout of d_vbrick's contents (-1: stale, kQuadCopy: quads)
   // object-space light cache (cvr_set_light_cache): 0 = off
   int lc_dims[3] = {0, 0, 0};
@@ -355,6 +361,7 @@ inline void swap_volume(cvr_ctx* c, VolSlot& s) {
   std::swap(c->d_vbrick, s.d_vbrick);
   std::swap(c->vbrick_cap, s.vbrick_cap);
   std::swap(c->vbrick_bs, s.vbrick_bs);
+  std::swap(c->quad_seen, s.quad_seen);
   std::swap(c->d_grad, s.d_grad);
   std::swap(c->grad_cap, s.grad_cap);
   std::swap(c->grad_ready, s.grad_ready);
@@ -406,6 +413,57 @@ cudaError_t ensure(T*& p, size_t& cap, size_t bytes) {
   cap = 0;
   cudaError_t e = cudaMalloc((void**)&p, bytes);
   if (e == cudaSuccess) cap = bytes;
+  return e;
+}
+
+// Deferred shading of one frame: its bands and the lists they need.
+// deferred_bytes: 0 leaves the frame to the direct marcher (the ray-refill
+// variant, a ray with more steps than the lists hold, or a camera so far away
+// that a ray's length is mostly rounding).
+inline size_t deferred_bytes(const FrameArgs& f, DeferredPlan* p) {
+  const double diag2 = (double)dot3(f.vol.grid, f.vol.grid), eye2 = (double)dot3(f.cam.eye, f.cam.eye);
+  if (f.work || !(eye2 <= 1.0e4 * diag2) || !deferred_plan(f, p)) return 0;
+  return 256 + (p->warps * p->chunks * sizeof(unsigned) + 255) / 256 * 256 + p->records * (sizeof(float4) + sizeof(float2));
+}
+// The launches of a frame over lists in mem (deferred_bytes of it): light(d)
+// launches the light pass over a band's records; taps: secondary lookups it
+// makes per sample and does not count.
+template <class Light>
+cudaError_t launch_deferred(void* mem, const DeferredPlan& p, const FrameArgs& f, const LightTerms& t, bool ext,
+                            unsigned taps, Light light, cudaStream_t st) {
+  char* base = static_cast<char*>(mem);
+  Deferred d;
+  d.counter = reinterpret_cast<unsigned*>(base);
+  d.chunk = reinterpret_cast<unsigned*>(base + 256);
+  d.rec = reinterpret_cast<float4*>(base + 256 + (p.warps * p.chunks * sizeof(unsigned) + 255) / 256 * 256);
+  d.light = reinterpret_cast<float2*>(d.rec + p.records);
+  d.chunks = p.chunks;
+  cudaError_t e = cudaSuccess;
+  for (unsigned b = 0; b < p.bands && e == cudaSuccess; ++b) {
+    d.y0 = b * p.rows;
+    e = cudaMemsetAsync(d.counter, 0, 2 * sizeof(unsigned), st);
+    if (e == cudaSuccess) e = launch_collect(f, d, p.rows, st);
+    if (e == cudaSuccess) e = light(d);
+    if (e == cudaSuccess) e = launch_resolve(f, d, p.rows, t, ext, taps, st);
+  }
+  return e;
+}
+// On the context's stream and lists; *done = false: the direct marcher's frame
+// (also when there is no room for the lists).
+template <class Light>
+cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t, bool ext, unsigned taps, Light light,
+                            bool* done) {
+  *done = false;
+  DeferredPlan p;
+  const size_t bytes = deferred_bytes(f, &p);
+  if (bytes == 0) return cudaSuccess;
+  cudaError_t e = ensure(c->d_defer, c->defer_cap, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return cudaSuccess;
+  }
+  if (e == cudaSuccess) e = launch_deferred(c->d_defer, p, f, t, ext, taps, light, c->stream);
+  *done = e == cudaSuccess;
   return e;
 }
 
@@ -468,7 +526,9 @@ cudaError_t launch_multiscale(int mode, int kern, float4* src, int gw, int gh, f
 size_t multiscale_scratch(int mode, int kern, int gw, int gh, int w, int h);
 // The volume as the marchers read it: the plain layout, or the bricked copy
 // of the context's brick size (made on first use after the volume changed).
-cvr_status render_volume_view(cvr_ctx* c, VolumeView* v, bool allow_tex = true);
+// pixels: of the frame that will read it (a plain-layout volume gets a quad
+// copy once its frames repay it).
+cvr_status render_volume_view(cvr_ctx* c, VolumeView* v, bool allow_tex = true, double pixels = 0.0);
 // Frame arguments of a render of the current volume (validated; f.step from
 // the params struct's leading step_size, f.counts null, f.stats the context's).
 cvr_status frame_args(cvr_ctx* c, const cvr_camera* cam, const void* params, float* out, int w, int h,

@@ -569,9 +569,12 @@ struct BoxView {
 #define CVR_MAX_LEVELS 16
 struct PyramidView {
   const float* data;
-  // x-y quads of every level (cell (x, y, z) = the values at (x, y), (x', y),
-  // (x, y'), (x', y') of its level, successors clamped), or nullptr; level l
-  // starts at cell qoff[l], with pitches quad_row(l) and quad_plane(l)
+  // x-y quads of every level, with a border: cell (x + 1, y + 1, z + 1), x
+  // from -1 to the extent less one (z to the extent), holds the values at
+  // (x, y), (x, y'), (x', y), (x', y') of plane z, every coordinate clamped to
+  // the level, so a coordinate inside the volume needs no clamp (the two ends
+  // of the x lerp are register pairs); or nullptr.  Level l starts at cell
+  // qoff[l], with pitches quad_row(l) and quad_plane(l).
   const float4* quads;
   unsigned qoff[CVR_MAX_LEVELS];
   int n_levels;
@@ -580,10 +583,10 @@ struct PyramidView {
   float3 grid;         // VolumeScaledSizes
   float3 inv_grid;
   __host__ __device__ __forceinline__ unsigned quad_row(int l) const {
-    return padded_row((unsigned)dims[l][0], sizeof(float4));
+    return padded_row((unsigned)dims[l][0] + 1u, sizeof(float4));
   }
   __host__ __device__ __forceinline__ unsigned quad_plane(int l) const {
-    return padded_plane(quad_row(l) * (unsigned)dims[l][1], sizeof(float4));
+    return padded_plane(quad_row(l) * ((unsigned)dims[l][1] + 1u), sizeof(float4));
   }
 };
 
@@ -598,12 +601,12 @@ __device__ __forceinline__ float pyr_sample_level(const PyramidView& P, int l, f
     // quad's (both taps read the edge value there, as without the raise).
     const Tap qx = axis_tap(fmaxf(fmaf(tex_pos.x * P.inv_grid.x, float(d[0]), -0.5f), 0.0f), d[0]);
     const Tap qy = axis_tap(fmaxf(fmaf(tex_pos.y * P.inv_grid.y, float(d[1]), -0.5f), 0.0f), d[1]);
-    const unsigned cell = P.qoff[l] + (unsigned)qx.i0 + P.quad_row(l) * (unsigned)qy.i0;
     const unsigned plane = P.quad_plane(l);
+    const unsigned cell = P.qoff[l] + (unsigned)(qx.i0 + 1) + P.quad_row(l) * (unsigned)(qy.i0 + 1) + plane;
     const float4 a = __ldg(P.quads + (cell + plane * (unsigned)tz.i0));
     const float4 e = __ldg(P.quads + (cell + plane * (unsigned)tz.i1));
-    const float c00 = fmaf(qx.t, a.y - a.x, a.x), c10 = fmaf(qx.t, a.w - a.z, a.z);
-    const float c01 = fmaf(qx.t, e.y - e.x, e.x), c11 = fmaf(qx.t, e.w - e.z, e.z);
+    const float c00 = fmaf(qx.t, a.z - a.x, a.x), c10 = fmaf(qx.t, a.w - a.y, a.y);
+    const float c01 = fmaf(qx.t, e.z - e.x, e.x), c11 = fmaf(qx.t, e.w - e.y, e.y);
     const float c0 = fmaf(qy.t, c10 - c00, c00), c1 = fmaf(qy.t, c11 - c01, c01);
     return fmaf(tz.t, c1 - c0, c0);
   }

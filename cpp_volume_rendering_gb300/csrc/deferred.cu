@@ -33,6 +33,33 @@ __device__ __forceinline__ bool primary_ray(const FrameArgs& f, int px, int py, 
   return true;
 }
 
+// The next kAhead steps of a ray: lengths, positions and densities, fetched
+// together (a small frame is one chain of loads per ray: with one sample in
+// flight the two passes of a 256^2 frame took 0.9 ms).  A ray at its end gets
+// steps past it, which the passes do not take.
+constexpr int kAhead = 4;
+struct Steps {
+  float h[kAhead], end[kAhead];  // length, ray parameter after the step
+  pos2 p[kAhead / 2];
+  float density[kAhead];
+  __device__ __forceinline__ float3 at(int j) const { return j & 1 ? pos_hi(p[j / 2]) : pos_lo(p[j / 2]); }
+};
+template <class S>
+__device__ __forceinline__ void fetch_steps(const S& sample, const Primary& r, float step, float s, Steps& o) {
+#pragma unroll
+  for (int j = 0; j < kAhead; j += 2) {
+    o.h[j] = fminf(step, r.D - s);
+    o.end[j] = s + o.h[j];
+    o.h[j + 1] = fminf(step, r.D - o.end[j]);
+    o.end[j + 1] = o.end[j] + o.h[j + 1];
+    o.p[j / 2] = along2(r.tex0, r.dir, mk2(s + o.h[j] * 0.5f, o.end[j] + o.h[j + 1] * 0.5f));
+    const float2 d = un2(sample.two(o.p[j / 2]));
+    o.density[j] = d.x;
+    o.density[j + 1] = d.y;
+    s = o.end[j + 1];
+  }
+}
+
 template <int NT, class S>
 __global__ void __launch_bounds__(NT) k_collect(const __grid_constant__ FrameArgs f, const __grid_constant__ Deferred d) {
   extern __shared__ float2 sm_alpha[];
@@ -51,42 +78,47 @@ __global__ void __launch_bounds__(NT) k_collect(const __grid_constant__ FrameArg
   float s = 0.0f, opacity = 0.0f;
   unsigned n = 0;
   unsigned filled = 0, base = 0, next = 0;  // records of the warp; first slot of its current and of its next chunk
-  while (__any_sync(0xffffffffu, live)) {
-    bool shaded = false;
-    float3 p = f3(0.0f, 0.0f, 0.0f);
-    if (live) {
-      const float h = fminf(f.step, r.D - s);
-      p = r.tex0 + r.dir * (s + h * 0.5f);
-      float a = tf(sample(p));
-      ++n;
-      if (a > 0.0f) {
-        shaded = true;
-        a = 1.0f - expf(-a * h);
-        const float left = 1.0f - opacity;
-        opacity += left * a;
-        if (opacity > 0.99f) live = false;
+  bool room = true;  // deferred_plan's bound holds; never past the lists
+  while (room && __any_sync(0xffffffffu, live)) {
+    Steps st;
+    fetch_steps(sample, r, f.step, s, st);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      bool shaded = false;
+      if (live) {
+        float a = tf(st.density[j]);
+        ++n;
+        if (a > 0.0f) {
+          shaded = true;
+          a = 1.0f - expf(-a * st.h[j]);
+          const float left = 1.0f - opacity;
+          opacity += left * a;
+          if (opacity > 0.99f) live = false;
+        }
+        s = st.end[j];
+        live = live && s < r.D && n < r.max_iter;
       }
-      s = s + h;
-      live = live && s < r.D && n < r.max_iter;
+      const unsigned m = __ballot_sync(0xffffffffu, shaded);
+      const unsigned take = (unsigned)__popc(m), slot = filled % kRecChunk;
+      if (m == 0 || !room) continue;
+      room = filled + take <= d.chunks * kRecChunk;
+      if (!room) continue;
+      // a step may end one chunk and begin the next
+      const bool first = slot == 0, over = slot != 0 && slot + take > kRecChunk;
+      if (first || over) {
+        if (lane == 0) next = atomicAdd(d.counter, kRecChunk);
+        next = __shfl_sync(0xffffffffu, next, 0);
+        if (lane == 0) chunk[(filled + take - 1) / kRecChunk] = next;
+        if (first) base = next;
+      }
+      if (shaded) {
+        const unsigned i = slot + (unsigned)__popc(m & ((1u << lane) - 1u));
+        const float3 p = st.at(j);
+        d.rec[i < kRecChunk ? base + i : next + (i - kRecChunk)] = make_float4(p.x, p.y, p.z, __int_as_float(pixel));
+      }
+      if (over) base = next;
+      filled += take;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, shaded);
-    if (m == 0) continue;
-    const unsigned take = (unsigned)__popc(m), slot = filled % kRecChunk;
-    if (filled + take > d.chunks * kRecChunk) break;  // deferred_plan's bound holds; never past the lists
-    // a step may end one chunk and begin the next
-    const bool first = slot == 0, over = slot != 0 && slot + take > kRecChunk;
-    if (first || over) {
-      if (lane == 0) next = atomicAdd(d.counter, kRecChunk);
-      next = __shfl_sync(0xffffffffu, next, 0);
-      if (lane == 0) chunk[(filled + take - 1) / kRecChunk] = next;
-      if (first) base = next;
-    }
-    if (shaded) {
-      const unsigned i = slot + (unsigned)__popc(m & ((1u << lane) - 1u));
-      d.rec[i < kRecChunk ? base + i : next + (i - kRecChunk)] = make_float4(p.x, p.y, p.z, __int_as_float(pixel));
-    }
-    if (over) base = next;
-    filled += take;
   }
   // the unused slots of the last chunk
   if (filled % kRecChunk)
@@ -95,7 +127,7 @@ __global__ void __launch_bounds__(NT) k_collect(const __grid_constant__ FrameArg
 
 template <int NT, class S>
 __global__ void __launch_bounds__(NT) k_resolve(const __grid_constant__ FrameArgs f, const __grid_constant__ Deferred d,
-                                                LightTerms t, int ext) {
+                                                LightTerms t, int ext, unsigned taps) {
   extern __shared__ float4 sm_tf[];
   stage_tf_table(f.tf, f.tf_n, sm_tf);
   __syncthreads();
@@ -111,41 +143,44 @@ __global__ void __launch_bounds__(NT) k_resolve(const __grid_constant__ FrameArg
   float4 dst = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float s = 0.0f;
   unsigned n = 0, n_shaded = 0, filled = 0;
-  while (__any_sync(0xffffffffu, live)) {
-    bool shaded = false;
-    float h = 0.0f;
-    float3 p = f3(0.0f, 0.0f, 0.0f);
-    float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (live) {
-      h = fminf(f.step, r.D - s);
-      p = r.tex0 + r.dir * (s + h * 0.5f);
-      src = tf(sample(p));
-      ++n;
-      shaded = src.w > 0.0f;
+  bool room = true;  // as collect
+  while (room && __any_sync(0xffffffffu, live)) {
+    Steps st;
+    fetch_steps(sample, r, f.step, s, st);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (live) {
+        src = tf(st.density[j]);
+        ++n;
+      }
+      const bool shaded = src.w > 0.0f;
+      const unsigned m = __ballot_sync(0xffffffffu, shaded);
+      room = room && filled + (unsigned)__popc(m) <= d.chunks * kRecChunk;
+      if (shaded && room) {
+        ++n_shaded;
+        const unsigned i = filled + (unsigned)__popc(m & ((1u << lane) - 1u));
+        const float2 l = d.light[chunk[i / kRecChunk] + i % kRecChunk];
+        src = ext ? t.apply<true>(f, src, st.at(j), l) : t.apply<false>(f, src, st.at(j), l);
+        src.w = 1.0f - expf(-src.w * st.h[j]);
+        src.x *= src.w; src.y *= src.w; src.z *= src.w;
+        const float left = 1.0f - dst.w;
+        dst.x += left * src.x; dst.y += left * src.y; dst.z += left * src.z; dst.w += left * src.w;
+        if (dst.w > 0.99f) live = false;
+      }
+      filled += (unsigned)__popc(m);
+      if (live) {
+        s = st.end[j];
+        live = s < r.D && n < r.max_iter;
+      }
     }
-    const unsigned m = __ballot_sync(0xffffffffu, shaded);
-    if (filled + (unsigned)__popc(m) > d.chunks * kRecChunk) break;  // as collect
-    if (shaded) {
-      ++n_shaded;
-      const unsigned i = filled + (unsigned)__popc(m & ((1u << lane) - 1u));
-      const float2 l = d.light[chunk[i / kRecChunk] + i % kRecChunk];
-      src = ext ? t.apply<true>(f, src, p, l) : t.apply<false>(f, src, p, l);
-      src.w = 1.0f - expf(-src.w * h);
-      src.x *= src.w; src.y *= src.w; src.z *= src.w;
-      const float left = 1.0f - dst.w;
-      dst.x += left * src.x; dst.y += left * src.y; dst.z += left * src.z; dst.w += left * src.w;
-      if (dst.w > 0.99f) live = false;
-    }
-    filled += (unsigned)__popc(m);
-    s = s + h;
-    live = live && s < r.D && n < r.max_iter;
   }
   if (px < f.W && py < f.H) {
     const size_t o = (size_t)py * f.W + px;
     f.out[o] = dst;
     if (f.counts) f.counts[o] = n;
   }
-  add_stats(f, n, n_shaded, 0u);
+  add_stats(f, n, n_shaded, n_shaded * taps);
 }
 
 dim3 band_grid(const FrameArgs& f, const Deferred& d, unsigned rows) {
@@ -195,7 +230,7 @@ cudaError_t launch_collect(const FrameArgs& f, const Deferred& d, unsigned rows,
 }
 
 cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows, const LightTerms& t, bool ext,
-                           cudaStream_t st) {
+                           unsigned taps, cudaStream_t st) {
   return with_sampler(f.vol, [&](auto* s) {
     using S = std::remove_pointer_t<decltype(s)>;
     return with_threads(f, [&](auto nt) {
@@ -205,7 +240,7 @@ cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows,
       cudaError_t e = cudaSuccess;
       if (sm > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
       if (e != cudaSuccess) return e;
-      kern<<<band_grid(f, d, rows), NT, sm, st>>>(f, d, t, ext ? 1 : 0);
+      kern<<<band_grid(f, d, rows), NT, sm, st>>>(f, d, t, ext ? 1 : 0, taps);
       return cudaGetLastError();
     });
   });

@@ -48,12 +48,21 @@ __device__ __forceinline__ void light_samples(const FrameArgs& f, const Deferred
     at = __shfl_sync(0xffffffffu, at, 0);
     if (at >= total) break;
     for (unsigned i = at + lane; i < at + kLightGrab; i += 32) {
+      // an unused slot takes the pixel and the place of a neutral sample, so
+      // that the warp stays whole through the light terms
       const float4 r = d.rec[i];
       const int pixel = __float_as_int(r.w);
-      if (pixel < 0) continue;
+      const bool used = pixel >= 0;
+      const int at_pixel = used ? pixel : 0;
+      const float3 p = used ? f3(r.x, r.y, r.z) : f.vol.grid * 0.5f;
       typename Shade::Ray ray;
-      sh.begin(ray, primary_dir(f.cam, pixel % f.W, pixel / f.W, f.W, f.H));
-      d.light[i] = sh.light(f3(r.x, r.y, r.z), ray, f, aux);
+      sh.begin(ray, primary_dir(f.cam, at_pixel % f.W, at_pixel / f.W, f.W, f.H));
+      unsigned a = 0;
+      const float2 l = sh.light(p, ray, f, a);
+      if (used) {
+        d.light[i] = l;
+        aux += a;
+      }
     }
   }
   if (f.stats) {
@@ -71,10 +80,14 @@ struct DeferredPlan {
 };
 bool deferred_plan(const FrameArgs& f, DeferredPlan* p);
 cudaError_t launch_collect(const FrameArgs& f, const Deferred& d, unsigned rows, cudaStream_t st);
-// ext: the extinction renderer's gradient branch.
+// ext: the extinction renderer's gradient branch; taps: secondary lookups per
+// shaded sample to count (0: the light pass counts its own).
 cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows, const LightTerms& t, bool ext,
-                           cudaStream_t st);
+                           unsigned taps, cudaStream_t st);
 
+// occ, sdw: host copies of the section tables.
+cudaError_t launch_light_dos(const FrameArgs& f, const DosArgs& a, const float4* occ, const float4* sdw, bool tex,
+                             const Deferred& d, cudaStream_t st);
 cudaError_t launch_light_gt(const FrameArgs& f, const GtArgs& g, const Deferred& d, cudaStream_t st);
 
 }  // namespace cvr

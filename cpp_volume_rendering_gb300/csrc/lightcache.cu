@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(128) k_cache_dos(FrameArgs f, DosArgs d, Cache
   if (i >= n) return;
   const int x = (int)(i % cd.d[0]), y = (int)((i / cd.d[0]) % cd.d[1]), z = (int)(i / ((long long)cd.d[0] * cd.d[1]));
   const float3 tx = cache_cell_pos(f, cd.d, x, y, z);
-  DosShade ds{&d, occ, sdw};
+  DosShade ds{&d, occ, sdw, TapsFp32{&d}};
   unsigned aux = 0;
   float io = 1.0f, is = 1.0f;
   if (d.apply_occ) {

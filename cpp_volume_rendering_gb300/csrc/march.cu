@@ -24,7 +24,8 @@ __global__ void __launch_bounds__(NT, MINB) k_march_dos(DosArgs d, FrameArgs f) 
   for (int i = threadIdx.x; i < d.occ.n_sections; i += blockDim.x) occ[i] = d.occ_sections[i];
   for (int i = threadIdx.x; i < d.sdw.n_sections; i += blockDim.x) sdw[i] = d.sdw_sections[i];
   __syncthreads();
-  DosShadeT<TEX> sh{&d, occ, sdw};
+  using Taps = typename std::conditional<TEX, TapsTex, TapsFp32>::type;
+  DosShadeT<Taps> sh{&d, occ, sdw, Taps{&d}};
   march_pixel(f, tf, sh);
 }
 
@@ -73,7 +74,8 @@ __global__ void __launch_bounds__(128, MINB) k_march_dos_refill(DosArgs d, Frame
   for (int i = threadIdx.x; i < d.occ.n_sections; i += blockDim.x) occ[i] = d.occ_sections[i];
   for (int i = threadIdx.x; i < d.sdw.n_sections; i += blockDim.x) sdw[i] = d.sdw_sections[i];
   __syncthreads();
-  DosShadeT<TEX> sh{&d, occ, sdw};
+  using Taps = typename std::conditional<TEX, TapsTex, TapsFp32>::type;
+  DosShadeT<Taps> sh{&d, occ, sdw, Taps{&d}};
   march_refill(f, tf, sh, f.work, o);
 }
 

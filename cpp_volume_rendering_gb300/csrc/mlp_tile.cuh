@@ -47,7 +47,7 @@ __device__ __forceinline__ void store_chunk(uint8_t* tile, int r, int c, uint32_
 // Hidden layer epilogue: TMEM columns col..col+63 of this thread's row, plus
 // bias, ReLU, to BF16 row r of tile; 16 columns at a time.
 __device__ __forceinline__ void epilogue_relu64(uint32_t tmem, int col, const float* bias, uint8_t* tile, int r) {
-  const uint32_t lane = (uint32_t)(threadIdx.x & ~31);
+  const uint32_t lane = (uint32_t)(r & ~31);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     float v[16];
@@ -76,9 +76,21 @@ __device__ __forceinline__ void issue_k64(uint32_t d, const uint8_t* a, const ui
              kb > 0);
 }
 
+// The 128 threads that share a tile: the whole CTA, or one of several groups
+// of it with named barrier 'bar' (1..15).
+struct TileCta {
+  __device__ __forceinline__ int tid() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct TileGroup {
+  int bar;
+  __device__ __forceinline__ int tid() const { return (int)(threadIdx.x & 127u); }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, 128;" ::"r"(bar) : "memory"); }
+};
+
 // Runs one commit/wait round trip: the issuing thread has queued MMAs.
-__device__ __forceinline__ bool complete(uint64_t* bar, uint32_t& phase) {
-  if (threadIdx.x == 0) commit(bar);
+__device__ __forceinline__ bool complete(uint64_t* bar, uint32_t& phase, bool issuer = threadIdx.x == 0) {
+  if (issuer) commit(bar);
   bool ok = mbar_wait(bar, phase, kPolls);
   phase ^= 1u;
   fence_after_sync();
@@ -91,41 +103,44 @@ __device__ __forceinline__ void ld_row64(uint32_t tmem, int col, float* v) {
   for (int c = 0; c < 4; ++c) tmem_ld16(taddr(tmem, lane, (uint32_t)(col + 16 * c)), v + 16 * c);
 }
 
-__device__ __forceinline__ void sync_tiles() {
+template <class Tile = TileCta>
+__device__ __forceinline__ void sync_tiles(const Tile& t = Tile()) {
   fence_before_sync();
   fence_async_smem();
-  __syncthreads();
+  t.sync();
 }
 
 // Forward of the 128-point tile whose input rows are in s.x; returns this
-// thread's two outputs.  Must be called by all 128 threads.  Every layer
-// accumulates into TMEM columns 0..63 (a layer's result is read out before
-// the next is issued), and the hidden activations go to s.h, which may be
-// the same buffer as s.x (the input is dead once layer 1 has completed).
-__device__ __forceinline__ bool mlp_forward_tile(MlpSmem& s, float y[2]) {
+// thread's two outputs.  Must be called by all 128 threads of the tile.  Every
+// layer accumulates into TMEM columns 0..63 (a layer's result is read out
+// before the next is issued), and the hidden activations go to s.h, which may
+// be the same buffer as s.x (the input is dead once layer 1 has completed).
+template <class Tile = TileCta>
+__device__ __forceinline__ bool mlp_forward_tile(MlpSmem& s, float y[2], const Tile& t = Tile()) {
   const float* bias = reinterpret_cast<const float*>(s.w + kPkBias);
+  const int tid = t.tid();
   bool ok = true;
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     fence_after_sync();
     issue_k64(s.tmem, s.x, s.w + kPkW1, idesc_bf16(128, 64));
   }
-  ok &= complete(s.bar, s.phase);
-  epilogue_relu64(s.tmem, 0, bias, s.h, threadIdx.x);
-  sync_tiles();
-  if (threadIdx.x == 0) {
+  ok &= complete(s.bar, s.phase, tid == 0);
+  epilogue_relu64(s.tmem, 0, bias, s.h, tid);
+  sync_tiles(t);
+  if (tid == 0) {
     fence_after_sync();
     issue_k64(s.tmem, s.h, s.w + kPkW2, idesc_bf16(128, 64));
   }
-  ok &= complete(s.bar, s.phase);
-  epilogue_relu64(s.tmem, 0, bias + 64, s.h, threadIdx.x);
-  sync_tiles();
-  if (threadIdx.x == 0) {
+  ok &= complete(s.bar, s.phase, tid == 0);
+  epilogue_relu64(s.tmem, 0, bias + 64, s.h, tid);
+  sync_tiles(t);
+  if (tid == 0) {
     fence_after_sync();
     issue_k64(s.tmem, s.h, s.w + kPkW3, idesc_bf16(128, 16));
   }
-  ok &= complete(s.bar, s.phase);
+  ok &= complete(s.bar, s.phase, tid == 0);
   float o[16];
-  tmem_ld16(taddr(s.tmem, (uint32_t)(threadIdx.x & ~31), 0), o);
+  tmem_ld16(taddr(s.tmem, (uint32_t)(tid & ~31), 0), o);
   y[0] = o[0] + bias[128];
   y[1] = o[1] + bias[129];
   fence_before_sync();
@@ -135,10 +150,10 @@ __device__ __forceinline__ bool mlp_forward_tile(MlpSmem& s, float y[2]) {
 // Shared set-up of an MLP CTA: TMEM allocation, mbarrier, the first 'bytes'
 // of the weight image (kPkBytes, or kPkFwdBytes for the forward pass only).
 __device__ __forceinline__ void mlp_cta_begin(uint8_t* w, const uint8_t* packed, uint64_t* bar, uint32_t* tslot,
-                                              uint32_t tmem_cols = 128, uint32_t bytes = kPkBytes) {
+                                              uint32_t tmem_cols = 128, uint32_t bytes = kPkBytes, int bars = 1) {
   if (threadIdx.x < 32) tmem_alloc(tslot, tmem_cols);
   if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
+    for (int i = 0; i < bars; ++i) mbar_init(bar + i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const uint4* src = reinterpret_cast<const uint4*>(packed);

@@ -529,37 +529,23 @@ struct ExtBoxShade {
 };
 
 // ==================================================== cone DOS (rc1pdosct)
-// TEX: the pyramid taps through the texture unit (DosArgs::ptex).
-template <bool TEX = false>
-struct DosShadeT {
+// Pyramid taps of the cones at a section's lod: by FP32 lookups, through the
+// texture unit, or from the quad copy with the section's levels laid out.
+struct TapsFp32 {
   const DosArgs* d;
-  const float4* occ_tab;  // shared-memory copies of the section tables
-  const float4* sdw_tab;
-  struct Ray { float3 v_up, v_right; };
+  using Section = float;
+  __device__ __forceinline__ Section section(const float4* s, int i) const { return s[i].y; }
+  __device__ __forceinline__ float operator()(Section lod, float3 p) const { return pyr_sample(d->pyr, lod, p); }
+};
 
-  // main(), ray_bbox_marching.comp:682-684.
-  __device__ __forceinline__ void begin(Ray& r, float3 dir) const {
-    r.v_right = normalize3(cross3(dir, f3(0.0f, 1.0f, 0.0f)));
-    r.v_up = normalize3(cross3(-dir, r.v_right));
-  }
-
-  // GetGaussianExtinction with CONSIDER_BORDERS (ray_bbox_marching.comp:92-112).
-  __device__ __forceinline__ float gauss_ext(float3 p, float level, const FrameArgs& f) const {
-    float rg = TEX ? pyr_sample_tex(level, p) : pyr_sample(d->pyr, level, p);
-    float3 S = f.vol.grid;
-    if (p.x < 0.0f || p.x > S.x || p.y < 0.0f || p.y > S.y || p.z < 0.0f || p.z > S.z) {
-      float sg = exp2f(level);
-      float3 c = clamp3(p, f3(0.0f, 0.0f, 0.0f), S) - p;
-      float dist = c.x * c.x + c.y * c.y + c.z * c.z;
-      rg = rg * expf(-(dist) / (2.0f * sg * sg));
-    }
-    return rg;
-  }
-
-  // pyr_sample's GL_LINEAR_MIPMAP_LINEAR lookup on the level textures: hardware
-  // trilinear within a level (normalised coordinates, all levels span the
-  // grid), linear between the two levels of a fractional lod.
-  __device__ __forceinline__ float pyr_sample_tex(float lod, float3 p) const {
+// pyr_sample's GL_LINEAR_MIPMAP_LINEAR lookup on the level textures: hardware
+// trilinear within a level (normalised coordinates, all levels span the
+// grid), linear between the two levels of a fractional lod.
+struct TapsTex {
+  const DosArgs* d;
+  using Section = float;
+  __device__ __forceinline__ Section section(const float4* s, int i) const { return s[i].y; }
+  __device__ __forceinline__ float operator()(Section lod, float3 p) const {
     const PyramidView& P = d->pyr;
     lod = fminf(fmaxf(lod, 0.0f), float(P.n_levels - 1));
     const float fl = floorf(lod);
@@ -570,6 +556,93 @@ struct DosShadeT {
     if (t == 0.0f) return a;
     const float b = tex3D<float>(d->ptex[min(l0 + 1, P.n_levels - 1)], u, v, w);
     return fmaf(t, b - a, a);
+  }
+};
+
+// A section's two levels for TapsQuads: extents as floats (and less one), the
+// levels' first cells and pitches, the lod's fraction.
+struct QuadSection {
+  float4 x, y, z;    // d0, d1, d0 - 1, d1 - 1
+  uint4 cell;        // first cell 0, 1; row 0, 1
+  uint2 plane;
+  float t;
+  float pad;
+};
+// One lookup of both levels: their coordinates and cells as packed pairs, a
+// coordinate clamped to [0, d - 1] as a float (both taps are the edge value
+// beyond it).  pyr_sample's values, bit for bit.
+struct TapsQuads {
+  const float4* quads;
+  const float4* first;           // the section tables this view's sections are numbered from
+  const QuadSection* sections;
+  float3 inv_grid;
+  using Section = const QuadSection*;
+  __device__ __forceinline__ Section section(const float4* s, int i) const { return sections + (s - first) + i; }
+  static __device__ __forceinline__ uint2 cells(float q, float4 d, f2& t) {
+    const float2 u = un2(fma2(dup2(q), mk2(d.x, d.y), dup2(-0.5f)));
+    const int2 c = cell_of2(mk2(fminf(fmaxf(u.x, 0.0f), d.z), fminf(fmaxf(u.y, 0.0f), d.w)), t);
+    return make_uint2((unsigned)(c.x + 1), (unsigned)(c.y + 1));  // past the border cell
+  }
+  static __device__ __forceinline__ float level(float4 a, float4 e, float tx, float ty, float tz) {
+    const f2 t = dup2(tx);
+    const float2 c0 = un2(lerp2(t, mk2(a.x, a.y), mk2(a.z, a.w))), c1 = un2(lerp2(t, mk2(e.x, e.y), mk2(e.z, e.w)));
+    const float z0 = fmaf(ty, c0.y - c0.x, c0.x), z1 = fmaf(ty, c1.y - c1.x, c1.x);
+    return fmaf(tz, z1 - z0, z0);
+  }
+  __device__ __forceinline__ float operator()(Section s, float3 p) const {
+    f2 tx, ty, tz;
+    const uint2 x = cells(p.x * inv_grid.x, s->x, tx), y = cells(p.y * inv_grid.y, s->y, ty),
+                z = cells(p.z * inv_grid.z, s->z, tz);
+    const float2 fx = un2(tx), fy = un2(ty), fz = un2(tz);
+    const uint4 o = s->cell;
+    const uint2 pl = s->plane;
+    const float4* q = quads + (o.x + x.x + o.z * y.x + pl.x * z.x);
+    const float4 a = __ldg(q), b = __ldg(q + pl.x);
+    if (s->t == 0.0f) return level(a, b, fx.x, fy.x, fz.x);
+    const float4* r = quads + (o.y + x.y + o.w * y.y + pl.y * z.y);
+    const float4 c = __ldg(r), e = __ldg(r + pl.y);
+    const float v0 = level(a, b, fx.x, fy.x, fz.x);
+    return fmaf(s->t, level(c, e, fx.y, fy.y, fz.y) - v0, v0);
+  }
+};
+// The QuadSection of a lod.
+__device__ __forceinline__ QuadSection quad_section(const PyramidView& P, float lod) {
+  lod = fminf(fmaxf(lod, 0.0f), float(P.n_levels - 1));
+  const float fl = floorf(lod);
+  const int a = int(fl), b = min(a + 1, P.n_levels - 1);
+  auto axis = [&](int k) {
+    const float da = (float)P.dims[a][k], db = (float)P.dims[b][k];
+    return make_float4(da, db, da - 1.0f, db - 1.0f);
+  };
+  return QuadSection{axis(0), axis(1), axis(2), make_uint4(P.qoff[a], P.qoff[b], P.quad_row(a), P.quad_row(b)),
+                     make_uint2(P.quad_plane(a), P.quad_plane(b)), lod - fl, 0.0f};
+}
+
+template <class Taps>
+struct DosShadeT {
+  const DosArgs* d;
+  const float4* occ_tab;  // shared-memory copies of the section tables
+  const float4* sdw_tab;
+  Taps taps;
+  struct Ray { float3 v_up, v_right; };
+
+  // main(), ray_bbox_marching.comp:682-684.
+  __device__ __forceinline__ void begin(Ray& r, float3 dir) const {
+    r.v_right = normalize3(cross3(dir, f3(0.0f, 1.0f, 0.0f)));
+    r.v_up = normalize3(cross3(-dir, r.v_right));
+  }
+
+  // GetGaussianExtinction with CONSIDER_BORDERS (ray_bbox_marching.comp:92-112).
+  __device__ __forceinline__ float gauss_ext(float3 p, typename Taps::Section sec, float level, const FrameArgs& f) const {
+    float rg = taps(sec, p);
+    float3 S = f.vol.grid;
+    if (p.x < 0.0f || p.x > S.x || p.y < 0.0f || p.y > S.y || p.z < 0.0f || p.z > S.z) {
+      float sg = exp2f(level);
+      float3 c = clamp3(p, f3(0.0f, 0.0f, 0.0f), S) - p;
+      float dist = c.x * c.x + c.y * c.y + c.z * c.z;
+      rg = rg * expf(-(dist) / (2.0f * sg * sg));
+    }
+    return rg;
   }
 
   // Cone1/3/7Ray{Occlusion,Shadow} (ray_bbox_marching.comp:124-322, 345-531):
@@ -583,7 +656,7 @@ struct DosShadeT {
     // Cone1Ray*: one sample per section.
     for (int i = 0; i < T.n1; ++i) {
       float4 s = tab[i];
-      float tau = gauss_ext(pos + k * track, s.y, f);
+      float tau = gauss_ext(pos + k * track, taps.section(tab, i), s.y, f);
       float amptau = tau * s.w;
       rays[0] += (last[0] + amptau) * s.z * T.ui_weight;
       last[0] = amptau;
@@ -599,9 +672,10 @@ struct DosShadeT {
       for (int r = 0; r < 3; ++r) vk[r] = k * T.axes[r].z + u * T.axes[r].y + v * T.axes[r].x;
       for (int i = 0; i < T.n3; ++i) {
         float4 s = tab[T.n1 + i];
+        const typename Taps::Section sec = taps.section(tab, T.n1 + i);
 #pragma unroll
         for (int r = 0; r < 3; ++r) {
-          float tau = gauss_ext(pos + vk[r] * track, s.y, f);
+          float tau = gauss_ext(pos + vk[r] * track, sec, s.y, f);
           float amptau = tau * s.w;
           rays[r] += (last[r] + amptau) * s.z * T.ui_weight;
           last[r] = amptau;
@@ -627,9 +701,10 @@ struct DosShadeT {
     int step0 = T.n1 + T.n3;
     for (int i = 0; i < T.n7; ++i) {
       float4 s = tab[step0 + i];
+      const typename Taps::Section sec = taps.section(tab, step0 + i);
 #pragma unroll
       for (int r = 0; r < 7; ++r) {
-        float tau = gauss_ext(pos + vk[r] * track, s.y, f);
+        float tau = gauss_ext(pos + vk[r] * track, sec, s.y, f);
         float amptau = tau * s.w;
         rays[r] += (last[r] + amptau) * s.z * T.ui_weight;
         last[r] = amptau;
@@ -674,7 +749,7 @@ struct DosShadeT {
     return light_terms(d->apply_occ, d->apply_sdw, d->ka, d->kd).apply<false>(f, src, tx, light(tx, r, f, aux));
   }
 };
-using DosShade = DosShadeT<false>;
+using DosShade = DosShadeT<TapsFp32>;
 
 
 // ================================================= ground truth (rc1pcrtgt)

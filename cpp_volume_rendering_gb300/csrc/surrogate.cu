@@ -1,6 +1,7 @@
 // surrogate.cu — shading-point collection, feature/target labelling and the
 // surrogate-shaded marcher (network inference fused into the ray loop).
 #include "mlp_tile.cuh"
+#include "tile_sink.cuh"
 #include "shade.cuh"
 #include "surrogate.cuh"
 
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(128) k_sur_label(const float4* __restrict__ pt
     // behind the point gives the same axis.
     FrameArgs fl = f;
     fl.cam.eye = (tx - f.vol.grid * 0.5f) - dir;
-    DosShade ds{&d, occ_tab, sdw_tab};
+    DosShade ds{&d, occ_tab, sdw_tab, TapsFp32{&d}};
     DosShade::Ray r;
     ds.begin(r, dir);
     dos_out[2 * (size_t)i] = ds.occlusion(tx, r, fl, aux);
@@ -144,85 +145,18 @@ struct SurRay {
   float4 dst;
   unsigned n, max_iter;
   int px, py;
-  int job;
 };
 
-// Where a marcher thread's rays come from.  SingleSource: one frame, tiles
-// in the square spiral around (cx, cy) (positions outside the image are
-// skipped: px = -1).  BatchSource: the jobs of one batch launch, each a run
-// of spiral positions of one counter (jobs ordered by first position), each
-// in the square spiral around its own centre tile.
-struct SingleSource {
-  const FrameArgs& f0;
-  const SurArgs& a0;
-  int cx, cy, tiles_x, tiles_y;
-  unsigned total;
-  __device__ __forceinline__ const FrameArgs& f(int) const { return f0; }
-  __device__ __forceinline__ const SurArgs& a(int) const { return a0; }
-  __device__ __forceinline__ void locate(unsigned idx, SurRay& r) const {
-    int dx, dy;
-    spiral_tile(idx >> 5, dx, dy);
-    const int tx = cx + dx, ty = cy + dy, within = (int)(idx & 31u);
-    r.job = 0;
-    if (tx < 0 || ty < 0 || tx >= tiles_x || ty >= tiles_y) { r.px = -1; r.py = -1; return; }
-    r.px = tx * 8 + (within & 7);
-    r.py = ty * 4 + (within >> 3);
-  }
-};
-
-struct BatchSource {
-  const SurJob* jobs;
-  int n_jobs;
-  unsigned total;
-  __device__ __forceinline__ const FrameArgs& f(int j) const { return jobs[j].f; }
-  __device__ __forceinline__ const SurArgs& a(int j) const { return jobs[j].a; }
-  __device__ __forceinline__ bool holds(int j, unsigned tile) const {
-    return jobs[j].first_tile <= tile && (j + 1 == n_jobs || jobs[j + 1].first_tile > tile);
-  }
-  // r.job on entry: the job of the thread's previous ray.  Rays are taken in
-  // increasing order, so the position is almost always in that job or the
-  // next; else a binary search for the last job whose first position is <= tile.
-  __device__ __forceinline__ void locate(unsigned idx, SurRay& r) const {
-    const unsigned tile = idx >> 5;
-    int j = r.job < 0 || r.job >= n_jobs ? 0 : r.job;
-    if (!holds(j, tile)) {
-      if (j + 1 < n_jobs && holds(j + 1, tile)) {
-        ++j;
-      } else {
-        int lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (jobs[mid].first_tile <= tile) lo = mid;
-          else hi = mid - 1;
-        }
-        j = lo;
-      }
-    }
-    const SurJob& J = jobs[j];
-    int dx, dy;
-    spiral_tile(tile - J.first_tile, dx, dy);
-    const int tx = J.cx + dx, ty = J.cy + dy, within = (int)(idx & 31u);
-    r.job = j;
-    if (tx < 0 || ty < 0 || tx >= J.tiles_x || ty >= J.tiles_y) { r.px = -1; r.py = -1; return; }
-    r.px = tx * 8 + (within & 7);
-    r.py = ty * 4 + (within >> 3);
-  }
-};
-
-// Step counts of the rays a thread finished, flushed to the job's counters
-// when the thread moves to another job and at the end.
-struct SurCounts {
-  int job = -1;
-  unsigned n = 0, shaded = 0;
-  __device__ __forceinline__ void flush(unsigned long long* stats) {
-    if (job >= 0 && stats && (n | shaded)) {
-      atomicAdd(stats + 0, (unsigned long long)n);
-      atomicAdd(stats + 1, (unsigned long long)shaded);
-      atomicAdd(stats + 2, (unsigned long long)shaded * (unsigned long long)kSurPyramidTaps);
-    }
-    n = shaded = 0;
-  }
-};
+// Where a marcher thread's rays come from: tiles in the square spiral around
+// (cx, cy) (positions outside the image are skipped: px = -1).
+__device__ __forceinline__ void locate_ray(unsigned idx, int cx, int cy, int tiles_x, int tiles_y, SurRay& r) {
+  int dx, dy;
+  spiral_tile(idx >> 5, dx, dy);
+  const int tx = cx + dx, ty = cy + dy, within = (int)(idx & 31u);
+  if (tx < 0 || ty < 0 || tx >= tiles_x || ty >= tiles_y) { r.px = -1; r.py = -1; return; }
+  r.px = tx * 8 + (within & 7);
+  r.py = ty * 4 + (within >> 3);
+}
 
 // sur_shade's light terms through the ground truth's gradient branch
 // (gt_ray_marching.comp:277-295) when gradient shading is on.
@@ -240,49 +174,33 @@ __device__ __forceinline__ void sur_finish(const FrameArgs& f, const SurRay& r) 
   if (f.counts) f.counts[o] = r.n;
 }
 
-// Packs features pairwise to BF16 and stores each 8-feature chunk of this
-// thread's row of the input tile as soon as it is complete.
-struct TileSink {
-  uint8_t* tile;
-  int row;
-  uint32_t w[4];
-  float lo;
-  __device__ __forceinline__ void operator()(int k, float v) {
-    if (k & 1) {
-      w[(k >> 1) & 3] = pack_bf16(lo, v);
-      if ((k & 7) == 7) store_chunk(tile, row, k >> 3, w[0], w[1], w[2], w[3]);
-    } else {
-      lo = v;
-    }
-  }
-};
-
 constexpr uint32_t kSurTmemCols = 64;
 
-// The marcher body for either source.  tf_src / tf_n: the transfer function
-// (shared by all jobs), packed: the network image.
-template <bool TEX, bool BATCH, class Src>
-__device__ __forceinline__ void sur_march(const Src& src_rays, const float4* tf_src, int tf_n, const uint8_t* packed,
-                                          unsigned int* work, int* err) {
+// The direct marcher: frames whose rays have too many steps to defer, and the
+// ray-refill variant (deferred frames: light_sur.cu).
+template <bool TEX, int MINB>
+__global__ void __launch_bounds__(128, MINB) k_march_surrogate(const __grid_constant__ FrameArgs f,
+                                                               const __grid_constant__ SurArgs a, int cx, int cy,
+                                                               unsigned total, unsigned int* work, int* err) {
   extern __shared__ __align__(1024) uint8_t sm_sur[];
   uint8_t* w = sm_sur;
   uint8_t* xt = w + kPkFwdBytes;  // input tile, then the hidden activations of the same tile
   float4* tf = reinterpret_cast<float4*>(xt + kRowTile);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(tf + tf_n);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(tf + f.tf_n);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + 1);
-  mlp_cta_begin(w, packed, bar, tslot, kSurTmemCols, kPkFwdBytes);
-  for (int i = threadIdx.x; i < tf_n; i += blockDim.x) tf[i] = tf_src[i];
+  mlp_cta_begin(w, a.packed, bar, tslot, kSurTmemCols, kPkFwdBytes);
+  for (int i = threadIdx.x; i < f.tf_n; i += blockDim.x) tf[i] = f.tf[i];
   fence_async_smem();
   __syncthreads();
   MlpSmem ms{w, xt, xt, bar, *tslot, 0u};
 
-  const unsigned total = src_rays.total;
+  const int tiles_x = (f.W + 7) >> 3, tiles_y = (f.H + 3) >> 2;
   SurRay ray{};
   bool has_ray = false, pending = false, no_work = false;
   float4 src = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float3 p = f3(0.0f, 0.0f, 0.0f);
   float h = 0.0f;
-  SurCounts cnt;
+  unsigned n = 0, shaded = 0;
   while (true) {
     // Advance this thread's ray to its next shaded sample, taking new rays
     // as rays end, until a sample is pending or no rays are left.
@@ -290,13 +208,8 @@ __device__ __forceinline__ void sur_march(const Src& src_rays, const float4* tf_
       if (!has_ray) {
         unsigned idx = take_ray(work);
         if (idx >= total) { no_work = true; break; }
-        src_rays.locate(idx, ray);
-        const FrameArgs& f = src_rays.f(ray.job);
+        locate_ray(idx, cx, cy, tiles_x, tiles_y, ray);
         if (ray.px < 0 || ray.px >= f.W || ray.py >= f.H) continue;
-        if (ray.job != cnt.job) {
-          if (BATCH) cnt.flush(src_rays.f(cnt.job < 0 ? 0 : cnt.job).stats);
-          cnt.job = ray.job;
-        }
         ray.dir = primary_dir(f.cam, ray.px, ray.py, f.W, f.H);
         ray.dst = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         ray.n = 0;
@@ -311,21 +224,18 @@ __device__ __forceinline__ void sur_march(const Src& src_rays, const float4* tf_
         ray.max_iter = (unsigned)fminf(ray.D / f.step, 1.0e9f) + 4u;
         has_ray = true;
       }
-      {
-        const FrameArgs& f = src_rays.f(ray.job);
-        while (ray.s < ray.D && ray.n < ray.max_iter) {
-          h = fminf(f.step, ray.D - ray.s);
-          p = ray.tex0 + ray.dir * (ray.s + h * 0.5f);
-          src = tf_lookup(tf, tf_n, sample_volume(f.vol, p));
-          ++ray.n;
-          if (src.w > 0.0f) { pending = true; break; }
-          ray.s = ray.s + h;
-        }
-        if (!pending) {
-          sur_finish(f, ray);
-          cnt.n += ray.n;
-          has_ray = false;
-        }
+      while (ray.s < ray.D && ray.n < ray.max_iter) {
+        h = fminf(f.step, ray.D - ray.s);
+        p = ray.tex0 + ray.dir * (ray.s + h * 0.5f);
+        src = tf_lookup(tf, f.tf_n, sample_volume(f.vol, p));
+        ++ray.n;
+        if (src.w > 0.0f) { pending = true; break; }
+        ray.s = ray.s + h;
+      }
+      if (!pending) {
+        sur_finish(f, ray);
+        n += ray.n;
+        has_ray = false;
       }
     }
     if (!__syncthreads_or(pending)) break;
@@ -335,7 +245,7 @@ __device__ __forceinline__ void sur_march(const Src& src_rays, const float4* tf_
     // which halves the partial-warp stores of every chunk.
     if (pending) {
       TileSink out{xt, (int)threadIdx.x};
-      sur_features<TEX>(src_rays.a(ray.job), src_rays.f(ray.job).vol, tf, tf_n, p, ray.dir, out);
+      sur_features<TEX>(a, f.vol, tf, f.tf_n, p, ray.dir, out);
     }
     // K padding (inputs 48..63): the previous round's hidden layers wrote there
     store_chunk(xt, threadIdx.x, 6, 0u, 0u, 0u, 0u);
@@ -348,48 +258,24 @@ __device__ __forceinline__ void sur_march(const Src& src_rays, const float4* tf_
       break;
     }
     if (pending) {
-      ++cnt.shaded;
+      ++shaded;
       pending = false;
-      const FrameArgs& fj = src_rays.f(ray.job);
-      src = fj.grad.g ? sur_phong(src_rays.a(ray.job), fj, src, p, y[0], y[1])
-                      : sur_shade(src_rays.a(ray.job), src, y[0], y[1]);
+      src = f.grad.g ? sur_phong(a, f, src, p, y[0], y[1]) : sur_shade(a, src, y[0], y[1]);
       src.w = 1.0f - expf(-src.w * h);
       src.x *= src.w; src.y *= src.w; src.z *= src.w;
       float r = 1.0f - ray.dst.w;
       ray.dst.x += r * src.x; ray.dst.y += r * src.y; ray.dst.z += r * src.z; ray.dst.w += r * src.w;
       if (ray.dst.w > 0.99f) {
-        sur_finish(src_rays.f(ray.job), ray);
-        cnt.n += ray.n;
+        sur_finish(f, ray);
+        n += ray.n;
         has_ray = false;
       } else {
         ray.s = ray.s + h;
       }
     }
   }
-  if (BATCH) {
-    cnt.flush(src_rays.f(cnt.job < 0 ? 0 : cnt.job).stats);
-  } else {
-    add_stats(src_rays.f(0), cnt.n, cnt.shaded, cnt.shaded * (unsigned)kSurPyramidTaps);
-  }
+  add_stats(f, n, shaded, shaded * (unsigned)kSurPyramidTaps);
   mlp_cta_end(ms.tmem, kSurTmemCols);
-}
-
-// MINB: resident CTAs per SM the register budget is cut for (5: at most 96
-// registers; 4: at most 128).  The single-frame marcher runs at 5 for every
-// variant (measured faster than 4 at the 4-CTA variant); the batch marcher,
-// which keeps its job's descriptor fields live, takes 4 where 5 would spill.
-template <bool TEX, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_march_surrogate(FrameArgs f, SurArgs a, int cx, int cy, unsigned total,
-                                                               unsigned int* work, int* err) {
-  SingleSource s{f, a, cx, cy, (f.W + 7) >> 3, (f.H + 3) >> 2, total};
-  sur_march<TEX, false>(s, f.tf, f.tf_n, a.packed, work, err);
-}
-
-template <bool TEX, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_batch_surrogate(const __grid_constant__ SurLaunch L, unsigned int* work,
-                                                               int* err) {
-  BatchSource s{L.jobs, L.n_jobs, L.total};
-  sur_march<TEX, true>(s, L.jobs[0].f.tf, L.jobs[0].f.tf_n, L.jobs[0].a.packed, work, err);
 }
 
 // Persistent grid.  CTAs per SM: at most 4 for variant 0, the most that fit
@@ -420,20 +306,6 @@ static cudaError_t surrogate_grid(K kern, size_t smem, unsigned rays, int varian
   if (n > groups) n = groups;
   *ctas = n < 1 ? 1u : (unsigned)n;
   return cudaSuccess;
-}
-
-cudaError_t launch_batch_surrogate(const SurLaunch& L, int tf_n, bool tex, int variant, unsigned int* work, int* err,
-                                   cudaStream_t st) {
-  const size_t smem = kPkFwdBytes + kRowTile + sizeof(float4) * tf_n + 16;
-  // texture-unit features: 124 registers without spills at MINB 4 (at 5 they
-  // spill and the launch ran at 0.7x the single frames), so every variant takes 4
-  const bool wide = variant == 1 || variant == 3;
-  auto kern = tex ? k_batch_surrogate<true, 4> : (wide ? k_batch_surrogate<false, 5> : k_batch_surrogate<false, 4>);
-  unsigned ctas = 0;
-  cudaError_t e = surrogate_grid(kern, smem, L.total, variant, &ctas);
-  if (e != cudaSuccess) return e;
-  kern<<<ctas, 128, smem, st>>>(L, work, err);
-  return cudaGetLastError();
 }
 
 SurSpiral sur_spiral(const FrameArgs& f) {

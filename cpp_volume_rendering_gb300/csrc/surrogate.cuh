@@ -205,17 +205,6 @@ cudaError_t launch_sur_label(const float4* pts, int n, const FrameArgs& f, const
                              const GtArgs* g, const DosArgs* d, float* x_out, float* t_out, float* dos_out,
                              cudaStream_t st);
 
-// One job of a batch of surrogate frames (device table entry).  f.stats points
-// at the job's three counters; f.tf / f.tf_n and a.packed of a launch's first
-// job serve all its jobs (one transfer function and network per batch).
-struct SurJob {
-  FrameArgs f;
-  SurArgs a;
-  unsigned first_tile;  // batch-wide index of the job's first spiral position
-  int cx, cy;           // the job's spiral centre tile
-  int tiles_x, tiles_y;
-};
-
 // Ray order of a surrogate frame: 8x4-pixel tiles in the square spiral around
 // the tile of the projected volume centre (long rays first, neighbouring
 // tiles together); positions = the tiles of the spiral's bounding square
@@ -226,22 +215,10 @@ struct SurSpiral {
 };
 SurSpiral sur_spiral(const FrameArgs& f);
 
-// One persistent launch of a batch's surrogate jobs: up to kSurLaunchJobs
-// jobs whose descriptors are the launch's parameters (the constant bank, read
-// as the single-frame marcher reads its own), ordered by first_tile (relative
-// to the launch), each job's rays in its spiral order; total = 32 x the
-// spiral positions of its jobs.
-constexpr int kSurLaunchJobs = 32;
-struct SurLaunch {
-  int n_jobs;
-  unsigned total;
-  SurJob jobs[kSurLaunchJobs];
-};
-static_assert(sizeof(SurLaunch) <= 32000, "kernel parameters are limited to 32764 bytes");
-
-// Rays taken from *work (zeroed before the launch).
-cudaError_t launch_batch_surrogate(const SurLaunch& L, int tf_n, bool tex, int variant, unsigned int* work, int* err,
-                                   cudaStream_t st);
+struct Deferred;
+// The light terms of a frame's collected samples (deferred.cuh).
+cudaError_t launch_light_sur(const FrameArgs& f, const SurArgs& a, bool tex, const Deferred& d, int* err,
+                             cudaStream_t st);
 
 // The surrogate-shaded marcher: persistent CTAs take rays from *work (zeroed
 // before the launch) in 8x4-pixel tiles in the frame's spiral order; every

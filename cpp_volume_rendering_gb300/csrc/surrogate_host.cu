@@ -209,6 +209,11 @@ cvr_status render_surrogate(cvr_ctx* c, const FrameArgs& f, const cvr_gt_params*
   bool tex = false;
   cvr_status st = sur_job_args(c, p, light, &a, &tex);
   if (st != CVR_OK) return st;
+  bool done = false;
+  CK(c, render_deferred(c, f, light_terms(a.apply_occ, a.apply_sdw, a.ka, a.kd), false, (unsigned)kSurPyramidTaps,
+                        [&](const Deferred& d) { return launch_light_sur(f, a, tex, d, c->mlp->err, c->stream); },
+                        &done));
+  if (done) return CVR_OK;
   CK(c, cudaMemsetAsync(c->sur->counter, 0, sizeof(unsigned int), c->stream));
   CK(c, launch_surrogate(f, a, tex, sur_spiral(f), c->sur->counter, c->mlp->err, c->stream));
   return CVR_OK;

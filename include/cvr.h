@@ -306,7 +306,10 @@ int cvr_get_brick_size(cvr_ctx* ctx);
  * where each cell holds the 2 x 2 values of its x-y neighbourhood (4 x the
  * volume's bytes, 16 bytes per pyramid value), so a trilinear sample is two
  * loads instead of eight; results are bit-identical to the plain layout.
- * It takes precedence over bricks; the autotuner tries it with them. */
+ * It takes precedence over bricks; the autotuner tries it with them.
+ * CVR_LAYOUT_PLAIN (the default) asks for no copy: with neither bricks nor
+ * staging the marchers still keep one of at most 2 GiB once a volume's frames
+ * repay it, and read the plain array until then and beyond that size. */
 /* Warp shape of the marchers' pixel tiles (no reference counterpart): 4, 8
  * (default) or 16 pixels per warp row (warps of 4x8, 8x4 or 16x2 pixels),
  * used where the tile holds whole warps of that shape (8x4 otherwise); same
@@ -318,8 +321,10 @@ int cvr_get_warp_shape(cvr_ctx* ctx);
  * threads whose lanes each advance their own ray to its next shaded sample,
  * shade together, and take the next ray of the frame (8x4-pixel tiles in a
  * spiral around the projected volume centre) when theirs ends; a warp leaves
- * when a ballot finds no lane with a ray.  Same images; the tile shape does
- * not apply.  The autotuner tries it at every register variant. */
+ * when a ballot finds no lane with a ray.  Without it cone, ground-truth and
+ * surrogate frames collect their shaded samples in lists (at most 1.5 GiB a
+ * context) and evaluate their light terms in a pass of its own; with it every
+ * ray evaluates its own.  Same images; the tile shape does not apply.  The autotuner tries it at every register variant. */
 cvr_status cvr_set_ray_refill(cvr_ctx* ctx, int enable);
 int cvr_get_ray_refill(const cvr_ctx* ctx);
 /* Shared-memory brick staging for CVR_METHOD_PLAIN (no reference counterpart;
@@ -492,12 +497,13 @@ cvr_status cvr_get_blinn_phong(cvr_ctx* ctx, cvr_blinn_phong* out);
 /* ---- batched rendering ------------------------------------------------------
  * No reference counterpart (the reference renders one view per Redraw()).
  * A batch is a fixed list of frames over the resident volumes, views and
- * lights, rendered by persistent launches (CVR_METHOD_EXTINCTION: one over
- * all its jobs; CVR_METHOD_SURROGATE: one per 32 jobs, their descriptors the
- * launch's parameters; other methods are rejected) whose CTAs take ray tiles
- * of their jobs from one work counter per launch, longest jobs first.  The
- * launches, with the resets of their counters, are captured in one CUDA
- * graph at creation; cvr_batch_run replays it.  Every image equals the image
+ * lights (CVR_METHOD_EXTINCTION: persistent launches over all their jobs,
+ * whose CTAs take ray tiles from one work counter per launch, longest jobs
+ * first; CVR_METHOD_SURROGATE: each job's passes on one of three lanes beside
+ * them; other methods are rejected).  The launches, with the resets of their
+ * counters, are captured in one CUDA graph at creation; cvr_batch_run replays
+ * it.  A batch holds its jobs' tables and at most 1.5 GiB of sample lists a
+ * lane.  Every image equals the image
  * of the same job rendered alone by cvr_render with the context's tuning at
  * creation.  Jobs keep pointers to their output buffers; the volumes, tables
  * and network they use must not change while the batch exists (re-create it). */
