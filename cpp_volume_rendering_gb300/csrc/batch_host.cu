@@ -249,7 +249,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       BoxPlan plan;
       ExtArgs e = J.e;
       const unsigned long long gen = 1;  // one source per slot
-      if (!box_plan(*b->boxes[at], gen, n, t, -1.0, &e, w.get(), &plan)) continue;
+      if (!box_plan(*b->boxes[at], gen, n, &t, -1.0, &e, w.get(), &plan)) continue;
       if (pass == 1 && plan.missing > 0) continue;
       size_t held = 0;
       for (size_t i = 0; i < b->boxes.size(); ++i)

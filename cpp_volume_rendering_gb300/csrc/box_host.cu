@@ -52,31 +52,10 @@ BoxGrid lookup_grid(BoxGrid g) {
   return g;
 }
 
-}  // namespace
-
-bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable& t, double pixels, ExtArgs* e,
-              BoxWalk* W, BoxPlan* P) {
-  // ambient occlusion: one table per shell, each with its own pad
-  if (e->apply_occ) {
-    const int xyz[3] = {0, 1, 2};
-    size_t cell = 0;
-    for (int i = 0; i < e->n_shells; ++i) {
-      const int w = (int)std::nearbyint(2.0f * e->radii[i]);
-      const int ww[3] = {w, w, w}, pad[3] = {w + 1, w + 1, w + 1};
-      BoxTableDesc d = table_desc(n, xyz, ww, pad);
-      d.cell = (unsigned)cell;
-      cell += cells_of(d.g);
-      if (cell * kCellBytes > kBoxPoolBytes) return false;
-      e->box.ao_cell[i] = d.cell;
-      e->box.ao_grid[i] = lookup_grid(d.g);
-      P->ao.t[P->ao.n++] = d;
-      P->ao_key.push_back(w);
-    }
-    P->ao_bytes = cell * kCellBytes;
-    P->ao_new = !(B.ao.data && B.ao.gen == gen && B.ao.key == P->ao_key);
-    if (P->ao_new) P->missing += cell;
-    else P->ao.n = 0;
-  }
+// The shadow tables of box_plan, and the frame's walk over them.
+bool shadow_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable& t, BoxWalk* W, ExtArgs* e,
+                 BoxPlan* P) {
+  const BoxPool& pool = B.sdw;
   // shadow: one table per pair of lateral widths, the walk axis slowest
   const int axis = t.axis;
   const int ax[3] = {axis == 0 ? 1 : 0, axis == 2 ? 1 : 2, axis};
@@ -93,45 +72,37 @@ bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const Shadow
   }
   // pads in steps of eight: a light that moves a little keeps the pool's grid
   for (int i = 0; i < 2; ++i) pad[i] = (pad[i] + 7) / 8 * 8 + 1;
-  const bool kin = B.sdw.data && B.sdw.gen == gen && B.sdw.key.size() == 4 && B.sdw.key[0] == axis && B.sdw.key[1] == ww;
+  const bool kin = pool.data && pool.gen == gen && pool.key.size() == 4 && pool.key[0] == axis && pool.key[1] == ww;
   if (kin) {
-    pad[0] = std::max(pad[0], B.sdw.key[2]);
-    pad[1] = std::max(pad[1], B.sdw.key[3]);
+    pad[0] = std::max(pad[0], pool.key[2]);
+    pad[1] = std::max(pad[1], pool.key[3]);
   }
-  const bool same = kin && B.sdw.key[2] == pad[0] && B.sdw.key[3] == pad[1];
+  const bool same = kin && pool.key[2] == pad[0] && pool.key[3] == pad[1];
   const int none[3] = {0, 0, 0};
   const BoxTableDesc grid = table_desc(n, ax, none, pad);
   const size_t cells = cells_of(grid.g);
+  P->shadow = true;
   P->sdw_key = {axis, ww, pad[0], pad[1]};
-  if (kin) P->have = B.sdw.have;
+  if (kin) P->have = pool.have;
   const size_t had = P->have.size();
   for (int p : need)
     if (std::find(P->have.begin(), P->have.end(), p) == P->have.end()) P->have.push_back(p);
   auto fits = [&]() { return P->have.size() <= (size_t)kMaxBoxTables && P->have.size() * cells * kCellBytes <= kBoxPoolBytes; };
   P->sdw_new = !same;
-  if (!fits() || P->have.size() * cells * kCellBytes > B.sdw.cap) {
+  if (!fits() || P->have.size() * cells * kCellBytes > pool.cap) {
     P->sdw_new = true;          // the pool grows: its tables are built again
     if (!fits()) P->have = need;  // without the widths of earlier lights
     if (!fits()) return false;
   }
   // room for a few more widths (a moving light's), as far as the bound goes
   const size_t room = std::min((P->have.size() + 3) / 4 * 4, kBoxPoolBytes / (cells * kCellBytes));
-  P->sdw_bytes = P->sdw_new ? std::max(room, P->have.size()) * cells * kCellBytes : B.sdw.cap;
+  P->sdw_bytes = P->sdw_new ? std::max(room, P->have.size()) * cells * kCellBytes : pool.cap;
   for (size_t i = P->sdw_new ? 0 : had; i < P->have.size(); ++i) {
     const int w[3] = {P->have[i] & 1023, P->have[i] >> 10, ww};
     BoxTableDesc d = table_desc(n, ax, w, pad);
     d.cell = (unsigned)(i * cells);
     P->sdw.t[P->sdw.n++] = d;
     P->missing += cells;
-  }
-  if (P->missing > 0 && pixels >= 0.0) {
-    if (B.seen_gen != gen) {
-      B.seen_gen = gen;
-      B.seen = 0.0;
-    }
-    B.seen += pixels;
-    if ((double)P->missing * kPixelsPerCell > B.seen) return false;
-    B.seen = 0.0;
   }
   // the walk
   e->box.sdw_grid = lookup_grid(grid.g);
@@ -155,6 +126,44 @@ bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const Shadow
   }
   W->pad_a = pad[0];
   W->pad_b = pad[1];
+  return true;
+}
+
+}  // namespace
+
+bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable* table, double pixels,
+              ExtArgs* e, BoxWalk* W, BoxPlan* P) {
+  // ambient occlusion: one table per shell, each with its own pad
+  if (e->apply_occ) {
+    const int xyz[3] = {0, 1, 2};
+    size_t cell = 0;
+    for (int i = 0; i < e->n_shells; ++i) {
+      const int w = (int)std::nearbyint(2.0f * e->radii[i]);
+      const int ww[3] = {w, w, w}, pad[3] = {w + 1, w + 1, w + 1};
+      BoxTableDesc d = table_desc(n, xyz, ww, pad);
+      d.cell = (unsigned)cell;
+      cell += cells_of(d.g);
+      if (cell * kCellBytes > kBoxPoolBytes) return false;
+      e->box.ao_cell[i] = d.cell;
+      e->box.ao_grid[i] = lookup_grid(d.g);
+      P->ao.t[P->ao.n++] = d;
+      P->ao_key.push_back(w);
+    }
+    P->ao_bytes = cell * kCellBytes;
+    P->ao_new = !(B.ao.data && B.ao.gen == gen && B.ao.key == P->ao_key);
+    if (P->ao_new) P->missing += cell;
+    else P->ao.n = 0;
+  }
+  if (table && !shadow_plan(B, gen, n, *table, W, e, P)) return false;
+  if (P->missing > 0 && pixels >= 0.0) {
+    if (B.seen_gen != gen) {
+      B.seen_gen = gen;
+      B.seen = 0.0;
+    }
+    B.seen += pixels;
+    if ((double)P->missing * kPixelsPerCell > B.seen) return false;
+    B.seen = 0.0;
+  }
   return true;
 }
 
@@ -187,7 +196,7 @@ cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned lo
       B.ao.key = P.ao_key;
     }
   }
-  if (err == cudaSuccess) {
+  if (err == cudaSuccess && P.shadow) {
     err = build(B.sdw, P.sdw_new, P.sdw_bytes, P.sdw);
     if (err == cudaSuccess) {
       B.sdw.gen = gen;
@@ -200,8 +209,8 @@ cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned lo
     return CVR_OK;
   }
   if (err != cudaSuccess) return cuda_fail(c, err, "box tables");
-  e->box.ao = B.ao.data;
-  e->box.sdw = B.sdw.data;
+  e->box.ao = e->apply_occ ? B.ao.data : nullptr;
+  e->box.sdw = P.shadow ? B.sdw.data : nullptr;
   *used = true;
   return CVR_OK;
 }

@@ -548,12 +548,14 @@ cvr_status ext_args(cvr_ctx* c, const cvr_ext_params* p, const cvr_light* light,
 // pay for their build yet.  box_build then makes the missing ones from src;
 // *used = false when the GPU has no room for them.
 struct BoxPlan {
+  bool shadow = false;                   // the frame's shadow boxes read tables too
   bool ao_new = false, sdw_new = false;  // the pool starts over (its tables are all built again)
   std::vector<int> ao_key, sdw_key, have;
   size_t ao_bytes = 0, sdw_bytes = 0, missing = 0;  // missing: cells to build
   BoxTableSet ao{}, sdw{};                          // the tables to build
 };
-bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable& t, double pixels, ExtArgs* e,
+// t null: the occlusion tables alone.
+bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const ShadowBoxTable* t, double pixels, ExtArgs* e,
               BoxWalk* W, BoxPlan* plan);
 cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned long long gen, const BoxPlan& plan,
                      ExtArgs* e, bool* used);

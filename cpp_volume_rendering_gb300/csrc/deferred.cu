@@ -6,7 +6,7 @@ namespace cvr {
 
 namespace {
 
-constexpr size_t kDeferredRecords = (size_t)64 << 20;  // 24 bytes each: at most 1.5 GiB per context
+constexpr size_t kDeferredRecords = (size_t)192 << 20;  // 24 bytes each: at most 4.5 GiB per context
 constexpr unsigned kMaxBands = 512;
 
 __device__ __forceinline__ void band_pixel(const FrameArgs& f, const Deferred& d, int& px, int& py, unsigned& warp) {

@@ -34,6 +34,7 @@ struct Deferred {
   unsigned y0;        // first tile row of the band
 };
 constexpr unsigned kRecChunk = 256;
+constexpr unsigned kBoxBands = 4;    // most bands of a deferred box-table frame
 constexpr unsigned kLightGrab = 64;  // records a warp takes at a time
 
 // The light terms of every record, by persistent warps.
@@ -88,6 +89,10 @@ cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows,
 // occ, sdw: host copies of the section tables.
 cudaError_t launch_light_dos(const FrameArgs& f, const DosArgs& a, const float4* occ, const float4* sdw, bool tex,
                              const Deferred& d, cudaStream_t st);
+// table, storage as launch_extinction.
+cudaError_t launch_light_ext(const FrameArgs& f, const ExtArgs& e, const ShadowBoxTable* table,
+                             const ShadowBoxTable& storage, const Deferred& d, cudaStream_t st);
+cudaError_t launch_light_box(const FrameArgs& f, const ExtArgs& e, const BoxWalk& w, const Deferred& d, cudaStream_t st);
 cudaError_t launch_light_gt(const FrameArgs& f, const GtArgs& g, const Deferred& d, cudaStream_t st);
 
 }  // namespace cvr

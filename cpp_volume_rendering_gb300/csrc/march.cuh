@@ -53,7 +53,8 @@ struct ExtArgs {
   int apply_occ, apply_sdw;
   int n_shells;
   float radii[32];
-  float cone_angle, interval, initial, ui_weight, max_dist;
+  float cone_cos, cone_sin, interval, initial, ui_weight, max_dist;
+  int whole_interval;  // interval is a whole number of texels
   int shadow_type;
   float3 light_pos, light_fwd;
   float ka, kd;

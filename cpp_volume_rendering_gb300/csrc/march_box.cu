@@ -4,14 +4,6 @@
 
 namespace cvr {
 
-// The walk's offsets and cut tests, staged after the transfer function.
-__device__ __forceinline__ void stage_walk(float4* so, float* scut, const float4* o, const float* cut, int n) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    so[i] = o[i];
-    scut[i] = cut[i];
-  }
-}
-
 static size_t box_smem(int tf_n, int n) { return sizeof(float4) * tf_n + (sizeof(float4) + sizeof(float)) * n; }
 
 template <int NT, int MINB>

@@ -98,6 +98,14 @@ __device__ __forceinline__ void batch_pixel(const BatchExtJob& J, unsigned b, in
   py = (int)(local / J.blocks_x) * J.f.tile_h + (warp / warps_x) * (32 >> wl) + (lane >> wl);
 }
 
+// The walk's offsets and cut tests, staged in shared memory.
+__device__ __forceinline__ void stage_walk(float4* so, float* scut, const float4* o, const float* cut, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    so[i] = o[i];
+    scut[i] = cut[i];
+  }
+}
+
 // Batched extinction frames: persistent CTAs take tiles of all jobs from one
 // counter; the job descriptor, transfer function and shadow table are staged
 // in shared memory whenever a CTA moves to another job.

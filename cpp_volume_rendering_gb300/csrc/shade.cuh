@@ -168,6 +168,27 @@ struct WalkStart {
   float frac;
 };
 
+// ExtinctionAmbientOcclusion from the box tables; g: the sample's SAT texel coordinate.
+__device__ __forceinline__ float box_occlusion(const ExtArgs& e, float3 g) {
+  const BoxView& B = e.box;
+  float t = 0.0f, last = 0.0f;
+  for (int i = 0; i < e.n_shells; ++i) {
+    const float r = e.radii[i];
+    const BoxGrid& G = B.ao_grid[i];
+    const int pad = __float2int_rn(2.0f * r) + 1;
+    float3 q;
+    const unsigned x = min((unsigned)(cell_of(g.x - r, q.x) + pad), (unsigned)G.na - 1u);
+    const unsigned y = min((unsigned)(cell_of(g.y - r, q.y) + pad), (unsigned)G.nb - 1u);
+    const unsigned z = min((unsigned)(cell_of(g.z - r, q.z) + pad), (unsigned)G.nc - 1u);
+    const BoxCorners c = box_corners(B.ao, B.ao_cell[i] + x + y * (unsigned)G.row + z * G.nab, G.row, G.nab);
+    const float b = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, q);
+    t = i == 0 ? b * (1.0f / (r * r)) : t + (b - last) * (1.0f / (r * r));
+    last = b;
+  }
+  const float rk = e.radii[e.n_shells - 1];
+  return expf(-((1.0f / (rk * rk)) * t));
+}
+
 template <bool COMPACT = false, bool ALIGNED = false>
 struct ExtShadeT {
   const ExtArgs* e;
@@ -197,11 +218,12 @@ struct ExtShadeT {
   // ExtinctionAmbientOcclusion (ebs_ray_bbox_marching.comp:112-146), with the
   // shell radii taken from a list (reference: AmbOccRadius * (i + 1)).
   __device__ float ambient_occlusion(float3 tx, const FrameArgs& f) const {
-    if constexpr (ALIGNED) {
+    if (ALIGNED || e->ao_aligned) {
+      const float3 g = sat_texel(e->sat, tx);
+      if (!ALIGNED && e->box.ao) return box_occlusion(*e, g);
       // the box [tx - r, tx + r] (voxels) starts at texel coordinate
       // (tx + spacing) / spacing - 0.5 - r = g - r and is 2 r texels wide
       const SatView& S = e->sat;
-      const float3 g = sat_texel(S, tx);
       float t = 0.0f, sat_i = 0.0f;
       for (int i = 0; i < e->n_shells; ++i) {
         const float ri = e->radii[i];
@@ -241,110 +263,74 @@ struct ExtShadeT {
     return (sat_box<COMPACT>(S, p1, p2) / volq) * e->ui_weight;
   }
 
-  // ConeZAxis (ebs_ray_bbox_marching.comp:190-270).
-  __device__ float cone_z(float3 pos, float3 c, const FrameArgs& f, unsigned& aux) const {
-    float3 sc = f.vol.spacing;
-    float st = 0.0f;
-    float signal = c.z < 0.0f ? -1.0f : 1.0f;
-    float3 proj_y = normalize3(f3(0.0f, c.y, c.z));
-    float3 proj_x = normalize3(f3(c.x, 0.0f, c.z));
-    float p_cs = cosf(e->cone_angle), p_sn = sinf(e->cone_angle);
-    float n_cs = cosf(-e->cone_angle), n_sn = sinf(-e->cone_angle);
-    float3 pj_x1 = normalize3(f3(proj_x.x * n_cs - proj_x.z * n_sn, 0.0f, proj_x.x * n_sn + proj_x.z * n_cs));
-    float3 pj_x2 = normalize3(f3(proj_x.x * p_cs - proj_x.z * p_sn, 0.0f, proj_x.x * p_sn + proj_x.z * p_cs));
-    float3 pj_y1 = normalize3(f3(0.0f, proj_y.y * n_cs - proj_y.z * n_sn, proj_y.y * n_sn + proj_y.z * n_cs));
-    float3 pj_y2 = normalize3(f3(0.0f, proj_y.y * p_cs - proj_y.z * p_sn, proj_y.y * p_sn + proj_y.z * p_cs));
-    float interval = e->interval * signal * sc.z;
-    float zp = e->initial * signal * sc.z;
-    float vmin = sc.z * 0.5f, vmax = f.vol.grid.z - sc.z * 0.5f;
-    for (int guard = 0; guard < kMaxConeBoxes && (zp / c.z) < e->max_dist &&
-                        (pos.z + (zp + interval) > vmin && pos.z + (zp + interval) < vmax); ++guard) {
-      float zm = fabsf(zp + interval * 0.5f);
-      float px1 = pj_x1.x * (zm / fabsf(pj_x1.z)), px2 = pj_x2.x * (zm / fabsf(pj_x2.z));
-      float py1 = pj_y1.y * (zm / fabsf(pj_y1.z)), py2 = pj_y2.y * (zm / fabsf(pj_y2.z));
-      float x1 = fminf(px1, px2), x2 = fmaxf(px1, px2);
-      float y1 = fminf(py1, py2), y2 = fmaxf(py1, py2);
-      float xd = fabsf(x2 - x1), yd = fabsf(y2 - y1);
-      float xs = (ceilf(xd / sc.x) - (xd / sc.x)) * 0.5f;
-      float ys = (ceilf(yd / sc.y) - (yd / sc.y)) * 0.5f;
-      x1 = x1 - xs * sc.x; x2 = x2 + xs * sc.x;
-      y1 = y1 - ys * sc.y; y2 = y2 + ys * sc.y;
-      float z1 = fminf(zp, zp + interval), z2 = fmaxf(zp, zp + interval);
-      st += shadow_box(pos + f3(x1, y1, z1), pos + f3(x2, y2, z2), f);
-      ++aux;
-      zp = zp + interval;
+  // ConeZAxis / ConeYAxis / ConeXAxis (ebs_ray_bbox_marching.comp:190-430):
+  // the walk of a cone c along its dominant axis.  The cone's edges in the
+  // planes of the walk axis m and a lateral axis are straight lines through
+  // the sample, so their slopes are formed once and a box's lateral extent is
+  // [lo, hi] times its depth, rounded up to whole voxels about its middle.
+  // With a whole interval every width is whole: the equal-fraction query, the
+  // walk axis stepping whole cells.  Products that meet a sum are fused or
+  // rounded explicitly, so that every kernel that inlines this rounds alike.
+  template <int AXIS>
+  __device__ float cone_walk(float3 pos, float3 c, const FrameArgs& f, unsigned& aux) const {
+    const SatView& S = e->sat;
+    const float3 sc = f.vol.spacing;
+    auto pick = [](float3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); };
+    constexpr int A = AXIS == 0 ? 1 : 0, B = AXIS == 2 ? 1 : 2;
+    const float cm = pick(c, AXIS), scm = pick(sc, AXIS), pm = pick(pos, AXIS);
+    // edge slopes in texels of the lateral axis per world unit of depth
+    float lo[2], hi[2];
+#pragma unroll
+    for (int l = 0; l < 2; ++l) {
+      const float ca = pick(c, l == 0 ? A : B), inv = pick(S.inv_spacing, l == 0 ? A : B);
+      const float as = __fmul_rn(ca, e->cone_sin), ms = __fmul_rn(cm, e->cone_sin);
+      const float s1 = fmaf(ca, e->cone_cos, ms) / fabsf(fmaf(cm, e->cone_cos, -as));
+      const float s2 = fmaf(ca, e->cone_cos, -ms) / fabsf(fmaf(cm, e->cone_cos, as));
+      lo[l] = fminf(s1, s2) * inv;
+      hi[l] = fmaxf(s1, s2) * inv;
     }
-    return st;
-  }
-
-  // ConeYAxis (ebs_ray_bbox_marching.comp:272-350).
-  __device__ float cone_y(float3 pos, float3 c, const FrameArgs& f, unsigned& aux) const {
-    float3 sc = f.vol.spacing;
+    const float signal = cm < 0.0f ? -1.0f : 1.0f;
+    const float interval = e->interval * signal * scm;
+    float mp = e->initial * signal * scm;
+    const float vmin = scm * 0.5f, vmax = pick(f.vol.grid, AXIS) - scm * 0.5f;
+    const float inv_c = 1.0f / cm;
+    const float3 g = sat_texel(S, pos);
+    float tw;
+    int aw = cell_of(fmaf(fminf(mp, mp + interval), pick(S.inv_spacing, AXIS), pick(g, AXIS)), tw);
+    const int ww = __float2int_rn(e->interval), dw = cm < 0.0f ? -ww : ww;
     float st = 0.0f;
-    float signal = c.y < 0.0f ? -1.0f : 1.0f;
-    float3 proj_x = normalize3(f3(c.x, c.y, 0.0f));
-    float3 proj_z = normalize3(f3(0.0f, c.y, c.z));
-    float p_cs = cosf(e->cone_angle), p_sn = sinf(e->cone_angle);
-    float n_cs = cosf(-e->cone_angle), n_sn = sinf(-e->cone_angle);
-    float3 pj_x1 = normalize3(f3(proj_x.x * n_cs - proj_x.y * n_sn, proj_x.x * n_sn + proj_x.y * n_cs, 0.0f));
-    float3 pj_x2 = normalize3(f3(proj_x.x * p_cs - proj_x.y * p_sn, proj_x.x * p_sn + proj_x.y * p_cs, 0.0f));
-    float3 pj_z1 = normalize3(f3(0.0f, proj_z.z * n_sn + proj_z.y * n_cs, proj_z.z * n_cs - proj_z.y * n_sn));
-    float3 pj_z2 = normalize3(f3(0.0f, proj_z.z * p_sn + proj_z.y * p_cs, proj_z.z * p_cs - proj_z.y * p_sn));
-    float interval = e->interval * signal * sc.y;
-    float yp = e->initial * signal * sc.y;
-    float vmin = sc.y * 0.5f, vmax = f.vol.grid.y - sc.y * 0.5f;
-    for (int guard = 0; guard < kMaxConeBoxes && (yp / c.y) < e->max_dist &&
-                        (pos.y + (yp + interval) > vmin && pos.y + (yp + interval) < vmax); ++guard) {
-      float ym = fabsf(yp + interval * 0.5f);
-      float px1 = pj_x1.x * (ym / fabsf(pj_x1.y)), px2 = pj_x2.x * (ym / fabsf(pj_x2.y));
-      float pz1 = pj_z1.z * (ym / fabsf(pj_z1.y)), pz2 = pj_z2.z * (ym / fabsf(pj_z2.y));
-      float x1 = fminf(px1, px2), x2 = fmaxf(px1, px2);
-      float z1 = fminf(pz1, pz2), z2 = fmaxf(pz1, pz2);
-      float xd = fabsf(x2 - x1), zd = fabsf(z2 - z1);
-      float xs = (ceilf(xd / sc.x) - (xd / sc.x)) * 0.5f;
-      float zs = (ceilf(zd / sc.z) - (zd / sc.z)) * 0.5f;
-      x1 = x1 - xs * sc.x; x2 = x2 + xs * sc.x;
-      z1 = z1 - zs * sc.z; z2 = z2 + zs * sc.z;
-      float y1 = fminf(yp, yp + interval), y2 = fmaxf(yp, yp + interval);
-      st += shadow_box(pos + f3(x1, y1, z1), pos + f3(x2, y2, z2), f);
+    for (int guard = 0; guard < kMaxConeBoxes && mp * inv_c < e->max_dist &&
+                        (pm + (mp + interval) > vmin && pm + (mp + interval) < vmax); ++guard) {
+      const float zm = fabsf(mp + interval * 0.5f);
+      // widths rounded up (ceil by a round-up add), low corners about the middle
+      float w[2], u[2];
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const float a = __fmul_rn(lo[l], zm), b = __fmul_rn(hi[l], zm);
+        w[l] = __fadd_ru(b - a, 12582912.0f) - 12582912.0f;
+        u[l] = 0.5f * ((a + b) - w[l]);
+      }
+      if (e->whole_interval) {
+        float ta, tb;
+        const int ia = cell_of(pick(g, A) + u[0], ta), ib = cell_of(pick(g, B) + u[1], tb);
+        const int wa = __float2int_rn(w[0]), wb = __float2int_rn(w[1]);
+        int3 at, wd;
+        float3 q;
+        if constexpr (AXIS == 2) { at = make_int3(ia, ib, aw); wd = make_int3(wa, wb, ww); q = f3(ta, tb, tw); }
+        else if constexpr (AXIS == 1) { at = make_int3(ia, aw, ib); wd = make_int3(wa, ww, wb); q = f3(ta, tw, tb); }
+        else { at = make_int3(aw, ia, ib); wd = make_int3(ww, wa, wb); q = f3(tw, ta, tb); }
+        st = fmaf(aligned_box(S, at, q, wd.x, wd.y, wd.z) / (w[0] * w[1] * e->interval), e->ui_weight, st);
+      } else {
+        const float a0 = u[0] * pick(sc, A), b0 = u[1] * pick(sc, B);
+        const float a1 = a0 + w[0] * pick(sc, A), b1 = b0 + w[1] * pick(sc, B);
+        const float m0 = fminf(mp, mp + interval), m1 = fmaxf(mp, mp + interval);
+        if constexpr (AXIS == 2) st += shadow_box(pos + f3(a0, b0, m0), pos + f3(a1, b1, m1), f);
+        else if constexpr (AXIS == 1) st += shadow_box(pos + f3(a0, m0, b0), pos + f3(a1, m1, b1), f);
+        else st += shadow_box(pos + f3(m0, a0, b0), pos + f3(m1, a1, b1), f);
+      }
       ++aux;
-      yp = yp + interval;
-    }
-    return st;
-  }
-
-  // ConeXAxis (ebs_ray_bbox_marching.comp:352-430).
-  __device__ float cone_x(float3 pos, float3 c, const FrameArgs& f, unsigned& aux) const {
-    float3 sc = f.vol.spacing;
-    float st = 0.0f;
-    float signal = c.x < 0.0f ? -1.0f : 1.0f;
-    float3 proj_y = normalize3(f3(c.x, c.y, 0.0f));
-    float3 proj_z = normalize3(f3(c.x, 0.0f, c.z));
-    float p_cs = cosf(e->cone_angle), p_sn = sinf(e->cone_angle);
-    float n_cs = cosf(-e->cone_angle), n_sn = sinf(-e->cone_angle);
-    float3 pj_y1 = normalize3(f3(proj_y.y * n_sn + proj_y.x * n_cs, proj_y.y * n_cs - proj_y.x * n_sn, 0.0f));
-    float3 pj_y2 = normalize3(f3(proj_y.y * p_sn + proj_y.x * p_cs, proj_y.y * p_cs - proj_y.x * p_sn, 0.0f));
-    float3 pj_z1 = normalize3(f3(proj_z.z * n_sn + proj_z.x * n_cs, 0.0f, proj_z.z * n_cs - proj_z.x * n_sn));
-    float3 pj_z2 = normalize3(f3(proj_z.z * p_sn + proj_z.x * p_cs, 0.0f, proj_z.z * p_cs - proj_z.x * p_sn));
-    float interval = e->interval * signal * sc.x;
-    float xp = e->initial * signal * sc.x;
-    float vmin = sc.x * 0.5f, vmax = f.vol.grid.x - sc.x * 0.5f;
-    for (int guard = 0; guard < kMaxConeBoxes && (xp / c.x) < e->max_dist &&
-                        (pos.x + (xp + interval) > vmin && pos.x + (xp + interval) < vmax); ++guard) {
-      float xm = fabsf(xp + interval * 0.5f);
-      float py1 = pj_y1.y * (xm / fabsf(pj_y1.x)), py2 = pj_y2.y * (xm / fabsf(pj_y2.x));
-      float pz1 = pj_z1.z * (xm / fabsf(pj_z1.x)), pz2 = pj_z2.z * (xm / fabsf(pj_z2.x));
-      float y1 = fminf(py1, py2), y2 = fmaxf(py1, py2);
-      float z1 = fminf(pz1, pz2), z2 = fmaxf(pz1, pz2);
-      float yd = fabsf(y2 - y1), zd = fabsf(z2 - z1);
-      float ys = (ceilf(yd / sc.y) - (yd / sc.y)) * 0.5f;
-      float zs = (ceilf(zd / sc.z) - (zd / sc.z)) * 0.5f;
-      y1 = y1 - ys * sc.y; y2 = y2 + ys * sc.y;
-      z1 = z1 - zs * sc.z; z2 = z2 + zs * sc.z;
-      float x1 = fminf(xp, xp + interval), x2 = fmaxf(xp, xp + interval);
-      st += shadow_box(pos + f3(x1, y1, z1), pos + f3(x2, y2, z2), f);
-      ++aux;
-      xp = xp + interval;
+      mp = mp + interval;
+      aw += dw;
     }
     return st;
   }
@@ -402,9 +388,9 @@ struct ExtShadeT {
     float3 c = (e->shadow_type == 0) ? normalize3(e->light_pos - realpos) : normalize3(e->light_fwd);
     float3 a = abs3(c);
     float st;
-    if (a.z > a.x && a.z > a.y) st = cone_z(tx, c, f, aux);
-    else if (a.y > a.x) st = cone_y(tx, c, f, aux);
-    else st = cone_x(tx, c, f, aux);
+    if (a.z > a.x && a.z > a.y) st = cone_walk<2>(tx, c, f, aux);
+    else if (a.y > a.x) st = cone_walk<1>(tx, c, f, aux);
+    else st = cone_walk<0>(tx, c, f, aux);
     return expf(-st);
   }
 
@@ -440,26 +426,6 @@ struct ExtBoxShade {
   float vmin, vmax, per;   // the cut interval, 1 / signed box step (world units)
   struct Ray {};
   __device__ __forceinline__ void begin(Ray&, float3) const {}
-
-  __device__ __forceinline__ float ambient_occlusion(float3 g) const {
-    const BoxView& B = e->box;
-    float t = 0.0f, last = 0.0f;
-    for (int i = 0; i < e->n_shells; ++i) {
-      const float r = e->radii[i];
-      const BoxGrid& G = B.ao_grid[i];
-      const int pad = __float2int_rn(2.0f * r) + 1;
-      float3 q;
-      const unsigned x = min((unsigned)(cell_of(g.x - r, q.x) + pad), (unsigned)G.na - 1u);
-      const unsigned y = min((unsigned)(cell_of(g.y - r, q.y) + pad), (unsigned)G.nb - 1u);
-      const unsigned z = min((unsigned)(cell_of(g.z - r, q.z) + pad), (unsigned)G.nc - 1u);
-      const BoxCorners c = box_corners(B.ao, B.ao_cell[i] + x + y * (unsigned)G.row + z * G.nab, G.row, G.nab);
-      const float b = aligned_weigh(c.v00.x, c.v00.y, c.v01.x, c.v01.y, c.v10.x, c.v10.y, c.v11.x, c.v11.y, q);
-      t = i == 0 ? b * (1.0f / (r * r)) : t + (b - last) * (1.0f / (r * r));
-      last = b;
-    }
-    const float rk = e->radii[e->n_shells - 1];
-    return expf(-((1.0f / (rk * rk)) * t));
-  }
 
   // Boxes of the walk from a sample at pm along the axis: the index of the
   // first that fails the cut test.  The test is monotone in k once the first
@@ -519,7 +485,7 @@ struct ExtBoxShade {
   __device__ __forceinline__ float2 light(float3 tx, const Ray&, const FrameArgs& f, unsigned& aux) const {
     const float3 g = sat_texel(e->sat, tx);
     float io = 0.0f, is = 0.0f;
-    if (e->apply_occ) { io = ambient_occlusion(g); aux += e->n_shells; }
+    if (e->apply_occ) { io = box_occlusion(*e, g); aux += e->n_shells; }
     if (e->apply_sdw) is = shadow(tx, g, aux);
     return make_float2(io, is);
   }

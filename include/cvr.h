@@ -321,8 +321,8 @@ int cvr_get_warp_shape(cvr_ctx* ctx);
  * threads whose lanes each advance their own ray to its next shaded sample,
  * shade together, and take the next ray of the frame (8x4-pixel tiles in a
  * spiral around the projected volume centre) when theirs ends; a warp leaves
- * when a ballot finds no lane with a ray.  Without it cone, ground-truth and
- * surrogate frames collect their shaded samples in lists (at most 1.5 GiB a
+ * when a ballot finds no lane with a ray.  Without it cone, ground-truth,
+ * surrogate and most extinction frames collect their shaded samples in lists (at most 4.5 GiB a
  * context) and evaluate their light terms in a pass of its own; with it every
  * ray evaluates its own.  Same images; the tile shape does not apply.  The autotuner tries it at every register variant. */
 cvr_status cvr_set_ray_refill(cvr_ctx* ctx, int enable);
@@ -502,7 +502,7 @@ cvr_status cvr_get_blinn_phong(cvr_ctx* ctx, cvr_blinn_phong* out);
  * first; CVR_METHOD_SURROGATE: each job's passes on one of three lanes beside
  * them; other methods are rejected).  The launches, with the resets of their
  * counters, are captured in one CUDA graph at creation; cvr_batch_run replays
- * it.  A batch holds its jobs' tables and at most 1.5 GiB of sample lists a
+ * it.  A batch holds its jobs' tables and at most 4.5 GiB of sample lists a
  * lane.  Every image equals the image
  * of the same job rendered alone by cvr_render with the context's tuning at
  * creation.  Jobs keep pointers to their output buffers; the volumes, tables
