@@ -10,8 +10,11 @@ namespace cvr {
 // a crossing (prev <= iso < d or prev >= iso > d) is placed at the linear
 // root inside the interval, shaded with the constant colour (ShadeBlinnPhong
 // when gradient shading is on) and composited front to back until alpha > 0.99.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_march_iso(FrameArgs f, IsoArgs a) {
+// A step's length depends on the density before it, so the steps of a ray are
+// a chain: specialised on the volume's storage, each is as short as it gets.
+template <int NT, class S>
+__global__ void __launch_bounds__(NT) k_march_iso(const __grid_constant__ FrameArgs f, IsoArgs a) {
+  const S sample(f.vol);
   int px, py;
   pixel_of(f, px, py);
   const bool inside = px < f.W && py < f.H;
@@ -23,13 +26,13 @@ __global__ void __launch_bounds__(NT) k_march_iso(FrameArgs f, IsoArgs a) {
     if (ray_aabb(f.cam.eye, dir, f.vol.grid, tnear, tfar)) {
       const float D = fabsf(tfar - tnear);
       const float3 tex0 = f.cam.eye + dir * tnear + f.vol.grid * 0.5f;
-      float prev = sample_volume(f.vol, tex0);
+      float prev = sample(tex0);
       // bound on the step count (never reached for validated step sizes)
       const unsigned max_iter = (unsigned)fminf(D / a.step_small, 1.0e9f) + 4u;
       for (float s = 0.0f; s < D && n < max_iter;) {
         const float step = fabsf(prev - a.iso) < a.step_range ? a.step_small : a.step_large;
         const float h = fminf(step, D - s);
-        const float d = sample_volume(f.vol, tex0 + dir * (s + h));
+        const float d = sample(tex0 + dir * (s + h));
         ++n;
         if ((prev <= a.iso && a.iso < d) || (prev >= a.iso && a.iso > d)) {
           ++hits;
@@ -53,14 +56,22 @@ __global__ void __launch_bounds__(NT) k_march_iso(FrameArgs f, IsoArgs a) {
   add_stats(f, n, hits, 0u);
 }
 
-cudaError_t launch_iso(const FrameArgs& f, const IsoArgs& a, cudaStream_t st) {
+template <int NT>
+static cudaError_t launch_iso_nt(const FrameArgs& f, const IsoArgs& a, cudaStream_t st) {
   const dim3 grid((f.W + f.tile_w - 1) / f.tile_w, (f.H + f.tile_h - 1) / f.tile_h, 1);
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    k_march_iso<NT, S><<<grid, NT, 0, st>>>(f, a);
+    return cudaGetLastError();
+  });
+}
+
+cudaError_t launch_iso(const FrameArgs& f, const IsoArgs& a, cudaStream_t st) {
   switch ((f.tile_w / 8) * (f.tile_h / 4) * 32) {
-    case 64: k_march_iso<64><<<grid, 64, 0, st>>>(f, a); break;
-    case 256: k_march_iso<256><<<grid, 256, 0, st>>>(f, a); break;
-    default: k_march_iso<128><<<grid, 128, 0, st>>>(f, a); break;
+    case 64: return launch_iso_nt<64>(f, a, st);
+    case 256: return launch_iso_nt<256>(f, a, st);
+    default: return launch_iso_nt<128>(f, a, st);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace cvr

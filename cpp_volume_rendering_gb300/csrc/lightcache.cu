@@ -76,79 +76,65 @@ __global__ void __launch_bounds__(128) k_cache_dos(FrameArgs f, DosArgs d, Cache
 }
 
 // texture(TexVolumeLightCache, tx_pos / VolumeScaledSizes).rg: trilinear,
-// texel centres, clamp-to-edge.
+// texel centres, clamp-to-edge.  At most 2^30 cells: 32-bit cell numbers.
 __device__ __forceinline__ float2 cache_lookup(const float2* __restrict__ c, const CacheDims& cd, float3 tx,
                                                float3 inv_grid) {
-  Tap a = axis_tap(fmaf(tx.x * inv_grid.x, float(cd.d[0]), -0.5f), cd.d[0]);
-  Tap b = axis_tap(fmaf(tx.y * inv_grid.y, float(cd.d[1]), -0.5f), cd.d[1]);
-  Tap g = axis_tap(fmaf(tx.z * inv_grid.z, float(cd.d[2]), -0.5f), cd.d[2]);
-  auto at = [&](int x, int y, int z) {
-    return __ldg(c + (size_t)x + (size_t)cd.d[0] * ((size_t)y + (size_t)cd.d[1] * z));
+  // a coordinate clamped to [0, n - 1]: beyond it both taps are the edge cell
+  auto cell = [](float p, int n, float& t, unsigned& step) {
+    const int i = min(cell_of(fmaxf(fmaf(p, float(n), -0.5f), 0.0f), t), n - 1);
+    step = i < n - 1 ? 1u : 0u;
+    return (unsigned)i;
   };
-  float2 c000 = at(a.i0, b.i0, g.i0), c100 = at(a.i1, b.i0, g.i0), c010 = at(a.i0, b.i1, g.i0),
-         c110 = at(a.i1, b.i1, g.i0), c001 = at(a.i0, b.i0, g.i1), c101 = at(a.i1, b.i0, g.i1),
-         c011 = at(a.i0, b.i1, g.i1), c111 = at(a.i1, b.i1, g.i1);
-  auto lerp2 = [](float t, float2 p, float2 q) { return make_float2(fmaf(t, q.x - p.x, p.x), fmaf(t, q.y - p.y, p.y)); };
-  float2 c00 = lerp2(a.t, c000, c100), c10 = lerp2(a.t, c010, c110), c01 = lerp2(a.t, c001, c101),
-         c11 = lerp2(a.t, c011, c111);
-  float2 c0 = lerp2(b.t, c00, c10), c1 = lerp2(b.t, c01, c11);
-  return lerp2(g.t, c0, c1);
+  float a, b, g;
+  unsigned dx, dy, dz;
+  const unsigned x = cell(tx.x * inv_grid.x, cd.d[0], a, dx), y = cell(tx.y * inv_grid.y, cd.d[1], b, dy),
+                 z = cell(tx.z * inv_grid.z, cd.d[2], g, dz);
+  const unsigned row = (unsigned)cd.d[0], plane = row * (unsigned)cd.d[1];
+  dy *= row;
+  dz *= plane;
+  const float2* q = c + (x + row * y + plane * z);
+  const float2 *r = q + dy, *s = q + dz, *u = r + dz;
+  auto pair = [](const float2* p) { const float2 v = __ldg(p); return mk2(v.x, v.y); };
+  const f2 ta = dup2(a), tb = dup2(b);
+  const f2 c0 = lerp2(tb, lerp2(ta, pair(q), pair(q + dx)), lerp2(ta, pair(r), pair(r + dx)));
+  const f2 c1 = lerp2(tb, lerp2(ta, pair(s), pair(s + dx)), lerp2(ta, pair(u), pair(u + dx)));
+  return un2(lerp2(dup2(g), c0, c1));
 }
 
 // obj_ray_marching.comp main() + ShadeSample (both branches): the a5
 // loop, but a sample is composited only when occlusion or shadow is on (the
 // reference's `src.a > 0.0 && Shade`), its light terms read from the cache.
-__global__ void __launch_bounds__(128) k_march_cached(FrameArgs f, CacheDims cd, const float2* __restrict__ cache,
-                                                      int apply_occ, int apply_sdw, float ka_in, float kd_in) {
+// The two samples of a step of the loop are fetched together, as are their
+// cache lookups' volume cells (march_ray_pairs).
+struct CachedShade {
+  CacheDims cd;
+  const float2* cache;
+  int apply_occ, apply_sdw;
+  LightTerms terms;
+  float3 inv_grid;
+  struct Ray {};
+  __device__ __forceinline__ void begin(Ray&, float3) const {}
+  // the reference's `src.a > 0.0 && Shade`: nothing is composited with both terms off
+  __device__ __forceinline__ bool shades() const { return apply_occ || apply_sdw; }
+  __device__ __forceinline__ float4 shade(float4 src, float3 p, const Ray&, const FrameArgs& f, unsigned& aux) const {
+    const float2 l = cache_lookup(cache, cd, p, inv_grid);
+    ++aux;
+    return terms.apply<true>(f, src, p, make_float2(apply_occ ? l.x : 0.0f, apply_sdw ? l.y : 0.0f));
+  }
+};
+
+template <class S>
+__global__ void __launch_bounds__(128) k_march_cached(const __grid_constant__ FrameArgs f, CacheDims cd,
+                                                      const float2* __restrict__ cache, int apply_occ, int apply_sdw,
+                                                      float ka, float kd) {
   extern __shared__ float4 sm_mc[];
-  const float4* tf = stage_tf(f, sm_mc);
+  stage_tf_table(f.tf, f.tf_n, sm_mc);
   __syncthreads();
   int px, py;
   pixel_of(f, px, py);
-  const bool inside = px < f.W && py < f.H;
-  unsigned n = 0, shaded = 0;
-  if (inside) {
-    const float3 dir = primary_dir(f.cam, px, py, f.W, f.H);
-    float4 dst = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float tnear, tfar;
-    if (ray_aabb(f.cam.eye, dir, f.vol.grid, tnear, tfar)) {
-      const bool shade = apply_occ || apply_sdw;
-      const float ka = apply_occ ? ka_in : 0.0f, kd = apply_sdw ? kd_in : 0.0f;
-      const float kk = 1.0f / (ka + kd);
-      const float3 inv_grid = f3(1.0f / f.vol.grid.x, 1.0f / f.vol.grid.y, 1.0f / f.vol.grid.z);
-      const float D = fabsf(tfar - tnear);
-      const float3 tex0 = f.cam.eye + dir * tnear + f.vol.grid * 0.5f;
-      const unsigned max_iter = (unsigned)fminf(D / f.step, 1.0e9f) + 4u;
-      for (float s = 0.0f; s < D && n < max_iter;) {
-        const float h = fminf(f.step, D - s);
-        const float3 p = tex0 + dir * (s + h * 0.5f);
-        float4 src = tf_lookup(tf, f.tf_n, sample_volume(f.vol, p));
-        ++n;
-        if (src.w > 0.0f && shade) {
-          ++shaded;
-          const float2 IaIs = cache_lookup(cache, cd, p, inv_grid);
-          const float io = apply_occ ? IaIs.x : 0.0f, is = apply_sdw ? IaIs.y : 0.0f;
-          if (f.grad.g) {
-            src = phong_ext(f, src, p, io, ka, is, kd);
-          } else {
-            src.x = kk * (src.x * io * ka + src.x * is * kd);
-            src.y = kk * (src.y * io * ka + src.y * is * kd);
-            src.z = kk * (src.z * io * ka + src.z * is * kd);
-          }
-          src.w = 1.0f - expf(-src.w * h);
-          src.x *= src.w; src.y *= src.w; src.z *= src.w;
-          const float r = 1.0f - dst.w;
-          dst.x += r * src.x; dst.y += r * src.y; dst.z += r * src.z; dst.w += r * src.w;
-          if (dst.w > 0.99f) break;
-        }
-        s = s + h;
-      }
-    }
-    const size_t o = (size_t)py * f.W + px;
-    f.out[o] = dst;
-    if (f.counts) f.counts[o] = n;
-  }
-  add_stats(f, n, shaded, shaded);
+  const float3 inv_grid = f3(1.0f / f.vol.grid.x, 1.0f / f.vol.grid.y, 1.0f / f.vol.grid.z);
+  const CachedShade sh{cd, cache, apply_occ, apply_sdw, light_terms(apply_occ, apply_sdw, ka, kd), inv_grid};
+  march_ray_pairs(f, S(f.vol), TfTable{sm_mc, f.tf_n}, sh, px, py);
 }
 
 cudaError_t launch_cache_extinction(const FrameArgs& f, const ExtArgs& e, const ShadowBoxTable* t,
@@ -179,9 +165,17 @@ cudaError_t launch_march_cached(const FrameArgs& f, const float2* cache, const i
   FrameArgs g = f;
   g.tile_w = 16;  // 128-thread CTAs of 8x4-pixel warps
   g.tile_h = 8;
-  dim3 grid((f.W + 15) / 16, (f.H + 7) / 8, 1);
-  k_march_cached<<<grid, 128, sizeof(float4) * f.tf_n, st>>>(g, cd, cache, apply_occ, apply_sdw, ka, kd);
-  return cudaGetLastError();
+  const dim3 grid((f.W + 15) / 16, (f.H + 7) / 8, 1);
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    const size_t sm = tf_table_bytes(f.tf_n);
+    auto kern = k_march_cached<S>;
+    cudaError_t e = cudaSuccess;
+    if (sm > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, 128, sm, st>>>(g, cd, cache, apply_occ, apply_sdw, ka, kd);
+    return cudaGetLastError();
+  });
 }
 
 }  // namespace cvr

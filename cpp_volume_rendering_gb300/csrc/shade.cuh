@@ -133,6 +133,7 @@ __host__ __device__ __forceinline__ LightTerms light_terms(int occ, int sdw, flo
 
 // ============================================================ plain (rc1pass)
 struct PlainShade {
+  __device__ __forceinline__ bool shades() const { return true; }
   struct Ray {};
   __device__ __forceinline__ void begin(Ray&, float3) const {}
   // ShadeSample is the identity unless gradient shading is on
@@ -945,7 +946,7 @@ __device__ __forceinline__ void march_ray_pairs(const FrameArgs& f, const S& sam
       // one step; false when it ends the ray
       auto take = [&](float4 src, float3 p, float h) {
         ++n;
-        if (src.w > 0.0f) {
+        if (src.w > 0.0f && sh.shades()) {
           ++shaded;
           src = sh.shade(src, p, ray, f, aux);
           src.w = 1.0f - expf(-src.w * h);
