@@ -19,6 +19,8 @@ constexpr int kMlpK = 64;  // input width padded to a multiple of 16
 constexpr int kMlpParams = 64 * 48 + 64 + 64 * 64 + 64 + 2 * 64 + 2;  // 7426
 constexpr int kOffW1 = 0, kOffB1 = 64 * 48, kOffW2 = kOffB1 + 64, kOffB2 = kOffW2 + 64 * 64, kOffW3 = kOffB2 + 64,
               kOffB3 = kOffW3 + 2 * 64;
+// Floats of one tile's gradient partials: every parameter, the loss, padded to 16 bytes.
+constexpr int kMlpPitch = (kMlpParams + 1 + 3) & ~3;
 
 // Packed image byte offsets (all multiples of 128).  The forward operands
 // and the biases come first, so a forward-only CTA copies kPkFwdBytes.
@@ -44,14 +46,18 @@ struct MlpSmem {
 
 cudaError_t launch_mlp_pack(const float* params, uint8_t* packed, cudaStream_t st);
 cudaError_t launch_mlp_infer(const uint8_t* packed, const float* x, int n, float* y, int* err, cudaStream_t st);
-// Forward + backward of a batch; per-CTA gradient partials (ceil(n/128) x kMlpParams).
+// Forward + backward of a batch; per-CTA gradient partials (ceil(n/128) x
+// kMlpPitch).  step (may be null) is incremented.  behind: the launch may start
+// while the kernel in front of it runs (and waits for it before its weights).
 cudaError_t launch_mlp_train_tiles(const uint8_t* packed, const float* x, const float* t, const int* idx, int n,
-                                   float inv_count, float* partials, float* loss_sum, int* err, cudaStream_t st);
-// Sums the partials and applies one Adam step to params (m, v moments); the
-// step number is *step_dev + 1 (step_dev may be null: step 1).  lr <= 0 only
-// reduces the gradient into grad_out.
-cudaError_t launch_mlp_adam(float* params, float* m, float* v, const float* partials, int n_parts, float lr,
-                            float beta1, float beta2, float eps, const int* step_dev, float* grad_out,
-                            cudaStream_t st);
+                                   float inv_count, float* partials, int* step, int* err, bool behind,
+                                   cudaStream_t st);
+// Sums the partials and applies one Adam step to params (m, v moments) and to
+// their packed image; adds the batch's loss to loss_acc.  The step number is
+// *step_dev (step_dev may be null: step 1; packed and loss_acc may be null).
+// lr <= 0 only reduces the gradient into grad_out.
+cudaError_t launch_mlp_adam(float* params, float* m, float* v, uint8_t* packed, float* loss_acc, const float* partials,
+                            int n_parts, float lr, float beta1, float beta2, float eps, const int* step_dev,
+                            float* grad_out, bool behind, cudaStream_t st);
 
 }  // namespace cvr

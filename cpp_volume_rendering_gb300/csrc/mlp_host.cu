@@ -68,23 +68,16 @@ cudaError_t grow(T*& p, size_t& cap, size_t n) {
   return e;
 }
 
-// Bumps the Adam step counter after an update (single thread).
-__global__ void k_step_inc(int* step) { *step += 1; }
-__global__ void k_add_loss(float* acc, const float* grad) { *acc += grad[kMlpParams]; }
-
-// One Adam step on the batch of 'count' points starting at idx[offset].
+// One Adam step on the batch of 'count' points starting at idx[offset]: two
+// launches, each but the epoch's first able to start while the one in front of
+// it runs.
 cvr_status enqueue_step(cvr_ctx* c, int offset, int count, float lr) {
   MlpState& s = *c->mlp;
   int tiles = (count + 127) / 128;
-  CK(c, launch_mlp_train_tiles(s.packed, s.x, s.t, s.idx + offset, count, 1.0f / (float)count, s.partials, nullptr,
-                               s.err, c->stream));
-  // step counter: read as step + 1 inside the update
-  CK(c, launch_mlp_adam(s.params, s.m, s.v, s.partials, tiles, lr, 0.9f, 0.999f, 1e-8f, s.step, s.grad, c->stream));
-  k_add_loss<<<1, 1, 0, c->stream>>>(s.loss_acc, s.grad);
-  CK(c, cudaGetLastError());
-  k_step_inc<<<1, 1, 0, c->stream>>>(s.step);
-  CK(c, cudaGetLastError());
-  CK(c, launch_mlp_pack(s.params, s.packed, c->stream));
+  CK(c, launch_mlp_train_tiles(s.packed, s.x, s.t, s.idx + offset, count, 1.0f / (float)count, s.partials, s.step,
+                               s.err, offset > 0, c->stream));
+  CK(c, launch_mlp_adam(s.params, s.m, s.v, s.packed, s.loss_acc, s.partials, tiles, lr, 0.9f, 0.999f, 1e-8f, s.step,
+                        s.grad, true, c->stream));
   return CVR_OK;
 }
 
@@ -175,14 +168,14 @@ cvr_status cvr_mlp_gradients(cvr_ctx* c, const float* x, const float* t, int n, 
   cudaError_t e = cudaMalloc((void**)&dx, sizeof(float) * 48 * (size_t)n);
   if (e == cudaSuccess) e = cudaMalloc((void**)&dt, sizeof(float) * 2 * (size_t)n);
   if (e == cudaSuccess) e = cudaMalloc((void**)&di, sizeof(int) * (size_t)n);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&parts, sizeof(float) * (kMlpParams + 1) * (size_t)tiles);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&parts, sizeof(float) * kMlpPitch * (size_t)tiles);
   std::vector<int> id(n);
   std::iota(id.begin(), id.end(), 0);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, sizeof(float) * 48 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dt, t, sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(di, id.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = launch_mlp_train_tiles(s.packed, dx, dt, di, n, 1.0f / (float)n, parts, nullptr, s.err, c->stream);
-  if (e == cudaSuccess) e = launch_mlp_adam(s.params, s.m, s.v, parts, tiles, 0.0f, 0.9f, 0.999f, 1e-8f, nullptr, s.grad, c->stream);
+  if (e == cudaSuccess) e = launch_mlp_train_tiles(s.packed, dx, dt, di, n, 1.0f / (float)n, parts, nullptr, s.err, false, c->stream);
+  if (e == cudaSuccess) e = launch_mlp_adam(s.params, s.m, s.v, nullptr, nullptr, parts, tiles, 0.0f, 0.9f, 0.999f, 1e-8f, nullptr, s.grad, false, c->stream);
   std::vector<float> g(kMlpParams + 1);
   if (e == cudaSuccess) e = cudaMemcpyAsync(g.data(), s.grad, sizeof(float) * (kMlpParams + 1), cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -252,7 +245,7 @@ cvr_status cvr_mlp_train(cvr_ctx* c, int epochs, int batch, float lr, uint64_t s
   const int n = s.n;
   const int n_batches = (n + batch - 1) / batch;
   CK(c, grow(s.idx, s.idx_cap, (size_t)n));
-  CK(c, grow(s.partials, s.partials_cap, (size_t)(batch / 128) * (kMlpParams + 1)));
+  CK(c, grow(s.partials, s.partials_cap, (size_t)(batch / 128) * kMlpPitch));
   // (Re)capture the epoch when the batch structure or the rate changed.
   if (!s.epoch_graph || s.graph_batch != batch || s.graph_n != n || s.graph_lr != lr) {
     if (s.epoch_graph) {

@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kMaxPoints = CVR_MLP_NOALLOC_MAX_POINTS;
 constexpr int kMaxTiles = kMaxPoints / 128;
-constexpr size_t kPartFloats = (size_t)kMaxTiles * (kMlpParams + 1);  // per-tile partials
+constexpr size_t kPartFloats = (size_t)kMaxTiles * kMlpPitch;  // per-tile partials
 constexpr size_t kRedFloats = ((kMlpParams + 1 + 63) / 64) * 64;      // reduced gradient + loss
 constexpr size_t kScratchBytes = (kPartFloats + kRedFloats) * sizeof(float) + (size_t)kMaxPoints * sizeof(int);
 
@@ -83,8 +83,10 @@ cvr_status cvr_mlp_gradients_noalloc(cvr_ctx* c, const float* x_dev, const float
   const int* idx = reinterpret_cast<const int*>(reduced + kRedFloats);
   MlpState& s = *c->mlp;
   const int tiles = (n + 127) / 128;
-  CK(c, launch_mlp_train_tiles(s.packed, x_dev, t_dev, idx, n, 1.0f / (float)n, partials, nullptr, s.err, c->stream));
-  CK(c, launch_mlp_adam(s.params, s.m, s.v, partials, tiles, 0.0f, 0.9f, 0.999f, 1e-8f, nullptr, reduced, c->stream));
+  CK(c, launch_mlp_train_tiles(s.packed, x_dev, t_dev, idx, n, 1.0f / (float)n, partials, nullptr, s.err, false,
+                               c->stream));
+  CK(c, launch_mlp_adam(s.params, s.m, s.v, nullptr, nullptr, partials, tiles, 0.0f, 0.9f, 0.999f, 1e-8f, nullptr, reduced,
+                        false, c->stream));
   CK(c, cudaMemcpyAsync(grad_dev, reduced, sizeof(float) * kMlpParams, cudaMemcpyDeviceToDevice, c->stream));
   if (loss_dev)
     CK(c, cudaMemcpyAsync(loss_dev, reduced + kMlpParams, sizeof(float), cudaMemcpyDeviceToDevice, c->stream));

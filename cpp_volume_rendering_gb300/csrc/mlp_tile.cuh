@@ -14,9 +14,10 @@ constexpr uint32_t kPolls = 1u << 22;  // bound of every mbarrier wait
 
 // Tile geometry (bytes): row tiles of K = 64 (lbo 128, sbo 1024), K = 16 row
 // tiles (lbo 128, sbo 256), and the transposed K = 128 tiles of the weight
-// gradients (lbo 144 so that column-wise 16-bit stores are bank-conflict free).
+// gradients (lbo 160 so that stores of two columns of two rows by lane pairs,
+// and 16-byte loads along a row, are bank-conflict free).
 constexpr uint32_t kRowSbo = 1024, kRow16Sbo = 256;
-constexpr uint32_t kTLbo = 144, kTSbo = 16 * 144;
+constexpr uint32_t kTLbo = 160, kTSbo = 16 * kTLbo;
 constexpr uint32_t kRowTile = 128 * 128;      // 128 x 64 bf16
 constexpr uint32_t kRow16Tile = 16 * 256;     // 128 x 16 bf16
 constexpr uint32_t kTTile = 16 * kTSbo;       // 128 x 128 bf16 (transposed layout)
@@ -63,12 +64,6 @@ __device__ __forceinline__ void epilogue_relu64(uint32_t tmem, int col, const fl
   }
 }
 
-// Column m (rows r0 .. r0+n-1) of a transposed K = 128 tile.
-__device__ __forceinline__ void store_col(uint8_t* tile, int m, int r0, const float* v, int n) {
-  for (int r = 0; r < n; ++r)
-    *reinterpret_cast<uint16_t*>(tile + tile_off(r0 + r, m, kTLbo, kTSbo)) = to_bf16(v[r]);
-}
-
 __device__ __forceinline__ void issue_k64(uint32_t d, const uint8_t* a, const uint8_t* b, uint32_t idesc) {
 #pragma unroll
   for (int kb = 0; kb < 4; ++kb)
@@ -95,12 +90,6 @@ __device__ __forceinline__ bool complete(uint64_t* bar, uint32_t& phase, bool is
   phase ^= 1u;
   fence_after_sync();
   return ok;
-}
-
-__device__ __forceinline__ void ld_row64(uint32_t tmem, int col, float* v) {
-  const uint32_t lane = (uint32_t)(threadIdx.x & ~31);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) tmem_ld16(taddr(tmem, lane, (uint32_t)(col + 16 * c)), v + 16 * c);
 }
 
 template <class Tile = TileCta>
