@@ -42,7 +42,7 @@ template <class Shade>
 __device__ __forceinline__ void light_samples(const FrameArgs& f, const Deferred& d, const Shade& sh) {
   const unsigned total = *d.counter;
   const int lane = threadIdx.x & 31;
-  unsigned aux = 0;
+  unsigned long long aux = 0;
   for (;;) {
     unsigned at = 0;
     if (lane == 0) at = atomicAdd(d.counter + 1, kLightGrab);
@@ -69,7 +69,7 @@ __device__ __forceinline__ void light_samples(const FrameArgs& f, const Deferred
   if (f.stats) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) aux += __shfl_down_sync(0xffffffffu, aux, o);
-    if (lane == 0) atomicAdd(f.stats + 2, (unsigned long long)aux);
+    if (lane == 0) atomicAdd(f.stats + 2, aux);
   }
 }
 
