@@ -38,6 +38,9 @@ struct MlpState {
   int n = 0;
   int* idx = nullptr;        // epoch permutation
   size_t idx_cap = 0;
+  int* order = nullptr;      // pinned: the permutations of two epochs (up to kPinnedOrder points) and their losses
+  size_t order_cap = 0;
+  cudaEvent_t epoch_done[2] = {};
   float* io_x = nullptr;     // staging of host batches (forward / gradients)
   float* io_y = nullptr;
   size_t io_cap = 0;
@@ -50,6 +53,9 @@ struct MlpState {
     for (void* p : bufs)
       if (p) cudaFree(p);
     if (epoch_graph) cudaGraphExecDestroy(epoch_graph);
+    if (order) cudaFreeHost(order);
+    for (cudaEvent_t e : epoch_done)
+      if (e) cudaEventDestroy(e);
   }
 };
 

