@@ -6,6 +6,7 @@
 //    (ExtinctionCoefficientVolume::GenerateExtinctionCoefficientVolumeAnySize,
 //    extcoefvolumegenerator.cpp:230-408, gen_extcoefvol_anysize*.comp, backtotau.comp).
 #include "build_tables.cuh"
+#include "sampler.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -351,24 +352,31 @@ cudaError_t launch_quad_volume(const void* src, void* dst, int dtype, int nx, in
 }
 
 // The bordered x-y quads of every pyramid level (PyramidView::quads) in one
-// launch: blockIdx.z runs over the planes of all levels.
-__global__ void __launch_bounds__(128) k_quad_pyramid(const __grid_constant__ PyramidView P, const float* __restrict__ v,
+// launch: blockIdx.y runs over the planes of all levels, a warp takes a row.
+// Bound by its 16-byte stores: 128^3 and its levels 36 -> 11 us (CTAs of 128
+// cells left the last of 129 to a CTA of its own).
+__global__ void __launch_bounds__(256) k_quad_pyramid(const __grid_constant__ PyramidView P, const float* __restrict__ v,
                                                       float4* __restrict__ out) {
-  int l = 0, z = blockIdx.z;
+  int l = 0, z = blockIdx.y;
   while (z >= P.dims[l][2] + 2) z -= P.dims[l++][2] + 2;
   const int nx = P.dims[l][0], ny = P.dims[l][1], nz = P.dims[l][2];
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-  if (x > nx || y > ny) return;
   const float* p = v + P.offset[l] + (size_t)min(max(z - 1, 0), nz - 1) * nx * ny;
-  const int x0 = max(x - 1, 0), x1 = min(x, nx - 1), y0 = max(y - 1, 0) * nx, y1 = min(y, ny - 1) * nx;
-  out[(size_t)P.qoff[l] + (size_t)z * P.quad_plane(l) + (size_t)y * P.quad_row(l) + x] =
-      make_float4(p[y0 + x0], p[y1 + x0], p[y0 + x1], p[y1 + x1]);
+  float4* o = out + (size_t)P.qoff[l] + (size_t)z * P.quad_plane(l);
+  for (int y = blockIdx.x * 8 + (threadIdx.x >> 5); y <= ny; y += gridDim.x * 8) {
+    const float *lo = p + max(y - 1, 0) * nx, *hi = p + min(y, ny - 1) * nx;
+    float4* row = o + (size_t)y * P.quad_row(l);
+#pragma unroll 4
+    for (int x = threadIdx.x & 31; x <= nx; x += 32) {
+      const int x0 = max(x - 1, 0), x1 = min(x, nx - 1);
+      row[x] = make_float4(__ldg(lo + x0), __ldg(hi + x0), __ldg(lo + x1), __ldg(hi + x1));
+    }
+  }
 }
 
 cudaError_t launch_pyramid_quads(const PyramidView& P, const float* data, float4* dst, cudaStream_t st) {
   int planes = 0;
   for (int l = 0; l < P.n_levels; ++l) planes += P.dims[l][2] + 2;
-  k_quad_pyramid<<<dim3(P.dims[0][0] / 128 + 1, P.dims[0][1] + 1, planes), 128, 0, st>>>(P, data, dst);
+  k_quad_pyramid<<<dim3((P.dims[0][1] + 8) / 8, planes), 256, 0, st>>>(P, data, dst);
   return cudaGetLastError();
 }
 
@@ -522,8 +530,18 @@ __device__ __forceinline__ bool in_grid(float3 p, float3 g) {
   return !(p.x < 0.0f || p.y < 0.0f || p.z < 0.0f || p.x > g.x || p.y > g.y || p.z > g.z);
 }
 
+// A level's cell: its opacity (what the next level reads) and its extinction
+// (backtotau.comp: -log(1 - opacity)).  tau == nullptr: op is converted later.
+struct PyrOut {
+  float *op, *tau;
+  __device__ __forceinline__ void put(size_t i, float o) const {
+    op[i] = o;
+    if (tau) tau[i] = -1.0f * logf(1.0f - o);
+  }
+};
+
 __global__ void k_pyr_base(VolumeView vol, const float4* __restrict__ tf_rgba, int tf_n, int bx, int by, int bz,
-                           float s0, float* __restrict__ out) {
+                           float s0, PyrOut out) {
   __shared__ float sm_w[343];
   extern __shared__ float4 sm_tf[];
   for (int i = threadIdx.x; i < tf_n; i += blockDim.x) sm_tf[i] = tf_rgba[i];
@@ -546,12 +564,12 @@ __global__ void k_pyr_base(VolumeView vol, const float4* __restrict__ tf_rgba, i
       }
     }
   }
-  out[idx] = sum_wc / sum_w;
+  out.put(idx, sum_wc / sum_w);
 }
 
 // gen_extcoefvol_anysize_mmlevel.comp: level l from level l-1 with sigma
 // Si = S0 * 2^l, sampling level l-1 trilinearly (textureLod at an integer lod).
-__global__ void k_pyr_level(PyramidView P, int l, float si, float* __restrict__ out) {
+__global__ void k_pyr_level(PyramidView P, int l, float si, PyrOut out) {
   __shared__ float sm_w[343];
   const float sum_w = stage_gauss(si, sm_w);
   const int* d = P.dims[l];
@@ -573,185 +591,417 @@ __global__ void k_pyr_level(PyramidView P, int l, float si, float* __restrict__ 
       }
     }
   }
-  out[idx] = sum_wc / sum_w;
+  out.put(idx, sum_wc / sum_w);
 }
 
-// backtotau.comp: opacity -> extinction, -log(1 - opacity), every level.
+// Opacity -> extinction of every level, in place: only where there was no room
+// for the opacities beside the extinctions.
 __global__ void k_pyr_backtotau(float* data, long long n) {
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) data[i] = -1.0f * logf(1.0f - data[i]);
 }
 
-// ---- separable form of the two level builders
-// Where a level's cells and taps fall on one lattice of input texel
-// coordinates with a constant fraction on every axis -- m input texels per
-// output cell and t per tap step, both whole numbers (the reference's base
-// 128^3 of a 256^3 volume with S0 = 1 voxel; every level from the one below it
-// when the dimensions halve) -- the Gaussian weights factor per axis
-// (exp(-|k|^2 / 2) = product of exp(-k_a^2 / 2)), so a level is one pass that
-// takes every lattice sample once (the TF opacity of the trilinear volume for
-// the base, the trilinear level below for the others; 0 outside the box, as
-// in_grid) and three 7-tap passes, instead of 343 samples per cell.  Cell i,
-// tap k reads lattice point i m + (k + 3) t, at texel coordinate j0 + q + f.
-struct PyrAxis {
-  int m, t;   // texels per cell, per tap step
-  int j0, g;  // lattice start (integer part) and size
-  int n_out;  // cells
-  float f;    // the constant fraction
-};
+// ---- the level builders without 343 samples per cell
+// The Gaussian weights factor per axis (exp(-|k|^2 / 2) = product of
+// exp(-k_a^2 / 2)) and so does the mask of the box (in_grid), so only what
+// stands between the taps and the sum decides what can be shared:
+//  - levels from the level below: trilinear sampling is linear and factors per
+//    axis too, whatever the sizes, so a level is three passes of dense weights
+//    (k_pyr_level_tile);
+//  - the base: the transfer function stands between, so every tap's value is
+//    needed.  With taps one voxel apart a cell's 343 taps have one fraction per
+//    axis and lie in an 8^3 window of voxels, interpolated axis by axis
+//    (k_pyr_base_window); with half as many cells as voxels on every axis (the
+//    reference's 128^3 base of a 256^3 volume) the taps of all cells are one
+//    lattice, whose points are taken once (k_pyr_base_half).
+// Other tap spacings, and windows that shared memory cannot hold, take the
+// direct kernels above.
 struct PyrWeights { float w[7]; };
 
-static bool pyr_axis(int n_in, int n_out, double tap_texels, PyrAxis* a) {
-  if (n_out < 1 || n_in % n_out) return false;
-  const double t = std::nearbyint(tap_texels);
-  if (!(t >= 1.0) || std::fabs(tap_texels - t) > 1e-9 * t) return false;
-  a->m = n_in / n_out;
-  a->t = (int)t;
-  const double c0 = 0.5 * a->m - 0.5;  // texel coordinate of cell 0, tap 0
-  a->f = (float)(c0 - std::floor(c0));
-  a->j0 = (int)std::floor(c0) - 3 * a->t;
-  a->g = (n_out - 1) * a->m + 6 * a->t + 1;
-  a->n_out = n_out;
-  return a->g <= 65535;  // a grid dimension of the lattice and pass launches
+// The centre of cell i in texels of the input, exact before the one rounding
+// of its fraction.  I: holds 2 n_out n_in.
+template <class I>
+__device__ __forceinline__ int cell_centre(int i, int n_in, int n_out, float& frac) {
+  const I num = (I)(2 * i + 1) * n_in - n_out, den = (I)2 * n_out;
+  I q = num / den, r = num - q * den;
+  if (r < 0) r += den, --q;
+  frac = (float)r / (float)den;
+  return (int)q;
+}
+// Texel coordinate i + f in [-0.5, n - 0.5]: inside the box.
+__device__ __forceinline__ bool in_axis(int i, float f, int n) {
+  return (i >= 0 || (i == -1 && f >= 0.5f)) && (i <= n - 2 || (i == n - 1 && f <= 0.5f));
 }
 
-// The plan of level l (l = 0: from the volume): false when it has no separable form.
-static bool pyr_plan(const VolumeView& vol, const PyramidView& P, int l, float s0, PyrAxis ax[3]) {
+// The opacity of a mean of voxels v in [0, 2^bits): tf_alpha of v * norm, the
+// scale folded into the table's (scale = norm * n).  v lies between its voxels
+// to FP32 rounding, so the entry is in the table without a clamp.
+__device__ __forceinline__ float alpha_of(const float2* e, float v, float scale) {
+  float t;
+  const float2 a = e[cell_of(fmaf(v, scale, -0.5f), t) + 1];
+  return fmaf(t, a.y, a.x);
+}
+
+// Base of half the volume's size, S0 = one voxel.  A CTA takes 16 x 16 columns
+// of kHalfZ cells and streams the lattice planes of its window along z: voxels
+// of two planes added in registers, the 37 x 37 points of a plane (each the
+// mean of 8 voxels, exact in FP32) through the transfer function once, 7-tap
+// passes along x and y in shared memory, along z in four running sums per
+// thread.  Bound by issue (the points of a tile overlap its neighbours' by a
+// third) and shared memory.  256^3 -> 128^3: 78 us; 204 as one lattice in memory
+// and three passes.
+constexpr int kHalfT = 16, kHalfL = 2 * kHalfT + 5, kHalfV = kHalfL + 1, kHalfZ = 16;
+template <class T>
+__global__ void __launch_bounds__(256, 4) k_pyr_base_half(const T* __restrict__ vox, int nx, int ny, int nz, float norm,
+                                                       const float4* __restrict__ tf_rgba, int tf_n, PyrWeights w,
+                                                       int bx, int by, int bz, PyrOut out) {
+  constexpr int kV = (kHalfV * kHalfV + 255) / 256, kL = (kHalfL * kHalfL + 255) / 256;
+  constexpr int kX = (kHalfL * kHalfT + 255) / 256;
+  __shared__ float V[kHalfV * kHalfV], A[kHalfL * kHalfL], X[kHalfL * kHalfT];
+  extern __shared__ float2 sm_alpha[];
+  stage_tf_alpha(tf_rgba, tf_n, sm_alpha);
+  const int tid = threadIdx.x;
+  // lattice point q of an axis is the middle of texels q - 3 and q - 2; inside the box: 2 <= q <= n + 2
+  const int qx0 = blockIdx.x * 2 * kHalfT, qy0 = blockIdx.y * 2 * kHalfT, oz0 = blockIdx.z * kHalfZ;
+  unsigned off[kV], inside = 0u;
+#pragma unroll
+  for (int s = 0; s < kV; ++s) {
+    const int i = min(tid + 256 * s, kHalfV * kHalfV - 1);
+    const int x = min(max(qx0 - 3 + i % kHalfV, 0), nx - 1), y = min(max(qy0 - 3 + i / kHalfV, 0), ny - 1);
+    off[s] = (unsigned)x + (unsigned)nx * (unsigned)y;
+  }
+#pragma unroll
+  for (int s = 0; s < kL; ++s) {
+    const int i = tid + 256 * s, x = qx0 + i % kHalfL, y = qy0 + i / kHalfL;
+    if (x >= 2 && x <= nx + 2 && y >= 2 && y <= ny + 2) inside |= 1u << s;
+  }
+  const float scale = 0.125f * norm * (float)tf_n;
+  const size_t plane = (size_t)nx * ny;
+  const int planes = 2 * min(kHalfZ, bz - oz0) + 5;
+  const int ox = blockIdx.x * kHalfT + (tid & 15), oy = blockIdx.y * kHalfT + (tid >> 4);
+  float prev[kV], r0 = 0.0f, r1 = 0.0f, r2 = 0.0f, r3 = 0.0f;
+  const T* pl = vox + plane * (size_t)min(max(2 * oz0 - 3, 0), nz - 1);
+#pragma unroll
+  for (int s = 0; s < kV; ++s) prev[s] = (float)__ldg(pl + off[s]);
+  __syncthreads();
+  for (int p = 0; p < planes; ++p) {
+    const int qz = 2 * oz0 + p;
+    pl = vox + plane * (size_t)min(max(qz - 2, 0), nz - 1);
+#pragma unroll
+    for (int s = 0; s < kV; ++s) {
+      const float cur = (float)__ldg(pl + off[s]);
+      if (tid + 256 * s < kHalfV * kHalfV) V[tid + 256 * s] = prev[s] + cur;
+      prev[s] = cur;
+    }
+    float g = 0.0f;
+    __syncthreads();
+    if (qz >= 2 && qz <= nz + 2) {  // the same for the whole CTA
+#pragma unroll
+      for (int s = 0; s < kL; ++s) {
+        const int i = tid + 256 * s;
+        if (i < kHalfL * kHalfL) {
+          const float* v = V + (i + i / kHalfL);
+          A[i] = (inside >> s) & 1u ? alpha_of(sm_alpha, (v[0] + v[1]) + (v[kHalfV] + v[kHalfV + 1]), scale) : 0.0f;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int s = 0; s < kX; ++s) {
+        const int i = tid + 256 * s;
+        if (i < kHalfL * kHalfT) {
+          const float* a = A + (i >> 4) * kHalfL + 2 * (i & 15);
+          float acc = 0.0f;
+#pragma unroll
+          for (int k = 0; k < 7; ++k) acc = fmaf(w.w[k], a[k], acc);
+          X[i] = acc;
+        }
+      }
+      __syncthreads();
+      const float* c = X + 2 * (tid >> 4) * kHalfT + (tid & 15);
+#pragma unroll
+      for (int k = 0; k < 7; ++k) g = fmaf(w.w[k], c[k * kHalfT], g);
+    }
+    if (p & 1) {
+      r0 = fmaf(w.w[1], g, r0);
+      r1 = fmaf(w.w[3], g, r1);
+      r2 = fmaf(w.w[5], g, r2);
+    } else {
+      r3 = fmaf(w.w[6], g, r2);
+      r2 = fmaf(w.w[4], g, r1);
+      r1 = fmaf(w.w[2], g, r0);
+      r0 = w.w[0] * g;
+      if (p >= 6 && ox < bx && oy < by) out.put(((size_t)(oz0 + p / 2 - 3) * by + oy) * bx + ox, r3);
+    }
+  }
+}
+
+// Base of any size with taps one voxel apart: one thread per cell walks the
+// eight voxel planes of its window, holding the 7 x 7 in-plane interpolations
+// of the plane before.  Bound by issue: 343 transfer-function lookups and 1183
+// lerps per cell instead of 343 trilinear samples of eight voxels; three CTAs
+// per SM hold the 7 x 7 values in registers (two: 595 us, four: 470).
+// 203 x 171 x 230 -> 101 x 85 x 115: 450 us; 1130 with the direct kernel.
+template <class T>
+__global__ void __launch_bounds__(128, 3) k_pyr_base_window(const T* __restrict__ vox, int nx, int ny, int nz, float norm,
+                                                         const float4* __restrict__ tf_rgba, int tf_n, PyrWeights w,
+                                                         int bx, int by, int bz, PyrOut out) {
+  extern __shared__ float2 sm_alpha[];
+  stage_tf_alpha(tf_rgba, tf_n, sm_alpha);
+  __syncthreads();
+  const float scale = norm * (float)tf_n;
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (long long)bx * by * bz) return;
+  const unsigned row = (unsigned)(idx / bx);
+  const int x = (int)(idx - (long long)row * bx), y = (int)(row % (unsigned)by), z = (int)(row / (unsigned)by);
+  float fx, fy, fz;
+  const int cx = cell_centre<long long>(x, nx, bx, fx), cy = cell_centre<long long>(y, ny, by, fy),
+            cz = cell_centre<long long>(z, nz, bz, fz);
+  float wx[7], wy[7];
+  unsigned xo[8], yo[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k < 7) {
+      wx[k] = in_axis(cx + k - 3, fx, nx) ? w.w[k] : 0.0f;
+      wy[k] = in_axis(cy + k - 3, fy, ny) ? w.w[k] : 0.0f;
+    }
+    xo[k] = (unsigned)min(max(cx + k - 3, 0), nx - 1);
+    yo[k] = (unsigned)min(max(cy + k - 3, 0), ny - 1) * (unsigned)nx;
+  }
+  float prev[7][7], sum = 0.0f;
+  for (int kz = 0; kz < 8; ++kz) {
+    const T* pl = vox + (size_t)nx * ny * (size_t)min(max(cz + kz - 3, 0), nz - 1);
+    const float wz = kz > 0 && in_axis(cz + kz - 4, fz, nz) ? w.w[max(kz - 1, 0)] : 0.0f;
+    float before[7], acc = 0.0f;
+#pragma unroll
+    for (int ky = 0; ky < 8; ++ky) {
+      float t[8], line = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t[k] = (float)__ldg(pl + (yo[ky] + xo[k]));
+#pragma unroll
+      for (int k = 0; k < 7; ++k) {
+        const float r = fmaf(fx, t[k + 1] - t[k], t[k]);
+        if (ky > 0) {
+          const float q = fmaf(fy, r - before[k], before[k]);
+          if (kz > 0) line = fmaf(wx[k], alpha_of(sm_alpha, fmaf(fz, q - prev[ky - 1][k], prev[ky - 1][k]), scale), line);
+          prev[ky - 1][k] = q;
+        }
+        before[k] = r;
+      }
+      if (ky > 0) acc = fmaf(wy[ky - 1], line, acc);
+    }
+    sum = fmaf(wz, acc, sum);
+  }
+  out.put(idx, sum);
+}
+
+// A level from the one below, all three passes in one CTA of T^3 cells: the
+// window of the input in shared memory, then along each axis a dense dot
+// product per cell, whose weights (7 taps of two texels each, folded to the
+// span they cover) the CTA works out first.  Latency-bound at these sizes
+// (64^3 cells are 512 CTAs, 8^3 one), so what counts is one launch per level
+// instead of four (lattices) or 343 samples in a row per thread (other sizes):
+// levels 1-4 of a 256^3 volume 112 -> 76 us, of a 203 x 171 x 230 one 416 -> 54
+// (cold caches, serialised).
+struct LevelAxis {
+  int n_in, n_out, span, win;  // span: texels of a cell's taps; win: of a tile's (upper bound)
+  float t;                     // texels per tap step
+};
+struct LevelAxes { LevelAxis a[3]; };
+
+template <int kLevelT>
+__global__ void __launch_bounds__(kLevelT * 64) k_pyr_level_tile(const float* __restrict__ in, LevelAxes L,
+                                                                 PyrWeights w, PyrOut out) {
+  constexpr int kThreads = kLevelT * 64, kLanes = 4 * kLevelT;  // lanes per row of the window's load
+  extern __shared__ float sm_level[];
+  __shared__ int start[3][kLevelT], first[3], extent[3];
+  const int tid = threadIdx.x;
+  const int cell0[3] = {(int)blockIdx.x * kLevelT, (int)blockIdx.y * kLevelT, (int)blockIdx.z * kLevelT};
+  const int pitch = L.a[0].win | 1;
+  float* win = sm_level;                                                // [z][y][pitch]
+  float* X = win + (size_t)L.a[2].win * L.a[1].win * pitch;             // [z][y][T]
+  float* Y = X + (size_t)L.a[2].win * L.a[1].win * kLevelT;             // [z][T][T]
+  float* wt = Y + (size_t)L.a[2].win * kLevelT * kLevelT;               // axis: [T][span]
+  if (tid < 3 * kLevelT) {
+    const int ax = tid / kLevelT, c = tid % kLevelT;
+    const LevelAxis A = ax == 0 ? L.a[0] : (ax == 1 ? L.a[1] : L.a[2]);
+    float* d = wt + kLevelT * ((ax > 0 ? L.a[0].span : 0) + (ax > 1 ? L.a[1].span : 0)) + c * A.span;
+    const int last = min(kLevelT, A.n_out - cell0[ax]) - 1;  // cells past the level repeat the last one
+    float f, f0, f1;
+    const int i = cell_centre<int>(cell0[ax] + min(c, last), A.n_in, A.n_out, f);
+    const int lo = i + (int)floorf(fmaf(-3.0f, A.t, f));
+    const int i0 = cell_centre<int>(cell0[ax], A.n_in, A.n_out, f0) + (int)floorf(fmaf(-3.0f, A.t, f0));
+    const int i1 = cell_centre<int>(cell0[ax] + last, A.n_in, A.n_out, f1) + (int)floorf(fmaf(-3.0f, A.t, f1));
+    for (int j = 0; j < A.span; ++j) d[j] = 0.0f;
+    for (int k = 0; k < 7; ++k) {
+      const float u = fmaf((float)(k - 3), A.t, f), fl = floorf(u);
+      float g = u - fl;
+      int j = i + (int)fl - lo;
+      if (!in_axis(i + (int)fl, g, A.n_in)) continue;
+      if (j > A.span - 2) g += (float)(j - (A.span - 2)), j = A.span - 2;  // a coordinate rounded up to a whole texel
+      d[j] += w.w[k] * (1.0f - g);
+      d[j + 1] += w.w[k] * g;
+    }
+    start[ax][c] = min(lo - i0, A.win - A.span);
+    if (c == 0) first[ax] = i0, extent[ax] = min(i1 - i0 + A.span, A.win);
+  }
+  __syncthreads();
+  const int ex = extent[0], ey = extent[1], ez = extent[2];
+  {
+    const int nx = L.a[0].n_in, ny = L.a[1].n_in, nz = L.a[2].n_in;
+#pragma unroll 8
+    for (int r = tid / kLanes; r < ey * ez; r += kThreads / kLanes) {
+      const int y = r % ey, z = r / ey;
+      const float* src = in + ((size_t)min(max(first[2] + z, 0), nz - 1) * ny + min(max(first[1] + y, 0), ny - 1)) * nx;
+      float* dst = win + ((size_t)z * ey + y) * pitch;
+      const int x = tid % kLanes;
+      if (x < ex) dst[x] = __ldg(src + min(max(first[0] + x, 0), nx - 1));
+      for (int u = x + kLanes; u < ex; u += kLanes) dst[u] = __ldg(src + min(max(first[0] + u, 0), nx - 1));
+    }
+  }
+  __syncthreads();
+  const int cx = tid % kLevelT, cy = tid / kLevelT % kLevelT;
+  {
+    const float* d = wt + cx * L.a[0].span;
+#pragma unroll 4
+    for (int r = tid / kLevelT; r < ey * ez; r += kThreads / kLevelT) {
+      const float* v = win + (size_t)r * pitch + start[0][cx];
+      float acc = 0.0f;
+      for (int j = 0; j < L.a[0].span; ++j) acc = fmaf(d[j], v[j], acc);
+      X[r * kLevelT + cx] = acc;
+    }
+  }
+  __syncthreads();
+  {
+    const float* d = wt + kLevelT * L.a[0].span + cy * L.a[1].span;
+    for (int z = tid / (kLevelT * kLevelT); z < ez; z += kThreads / (kLevelT * kLevelT)) {
+      const float* v = X + (size_t)(z * ey + start[1][cy]) * kLevelT + cx;
+      float acc = 0.0f;
+      for (int j = 0; j < L.a[1].span; ++j) acc = fmaf(d[j], v[j * kLevelT], acc);
+      Y[(z * kLevelT + cy) * kLevelT + cx] = acc;
+    }
+  }
+  __syncthreads();
+  const int cz = tid / (kLevelT * kLevelT), x = cell0[0] + cx, y = cell0[1] + cy, z = cell0[2] + cz;
+  if (cz >= kLevelT || x >= L.a[0].n_out || y >= L.a[1].n_out || z >= L.a[2].n_out) return;
+  const float* d = wt + kLevelT * (L.a[0].span + L.a[1].span) + cz * L.a[2].span;
+  const float* v = Y + (start[2][cz] * kLevelT + cy) * kLevelT + cx;
+  float acc = 0.0f;
+  for (int j = 0; j < L.a[2].span; ++j) acc = fmaf(d[j], v[j * kLevelT * kLevelT], acc);
+  out.put(((size_t)z * L.a[1].n_out + y) * L.a[0].n_out + x, acc);
+}
+
+// Texels per tap step of level l (0: from the volume) along axis a.
+static double pyr_tap_step(const VolumeView& vol, const PyramidView& P, int l, float s0, int a) {
   const int in[3] = {l == 0 ? vol.nx : P.dims[l - 1][0], l == 0 ? vol.ny : P.dims[l - 1][1],
                      l == 0 ? vol.nz : P.dims[l - 1][2]};
   const double grid[3] = {P.grid.x, P.grid.y, P.grid.z};
-  const double sigma = (double)s0 * std::ldexp(1.0, l);
-  for (int a = 0; a < 3; ++a)
-    if (!pyr_axis(in[a], P.dims[l][a], sigma * in[a] / grid[a], &ax[a])) return false;
-  return true;
+  return (double)s0 * std::ldexp(1.0, l) * in[a] / grid[a];
 }
 
-static long long pyr_scratch(const PyrAxis ax[3]) {
-  return (long long)ax[0].g * ax[1].g * ax[2].g + (long long)ax[0].n_out * ax[1].g * ax[2].g +
-         (long long)ax[0].n_out * ax[1].n_out * ax[2].g;
+// The tile plan of level l >= 1; returns its shared memory, 0 if a tap span is
+// out of proportion (such a window never fits).
+static size_t pyr_level_plan(const VolumeView& vol, const PyramidView& P, int l, float s0, int tile, LevelAxes* L) {
+  for (int a = 0; a < 3; ++a) {
+    LevelAxis& A = L->a[a];
+    const double t = pyr_tap_step(vol, P, l, s0, a);
+    if (!(t < 64.0)) return 0;
+    A.n_in = P.dims[l - 1][a];
+    A.n_out = P.dims[l][a];
+    A.t = (float)t;
+    A.span = (int)std::ceil(6.0 * t - 1e-6) + 2;
+    A.win = (int)std::ceil((double)(std::min(tile, A.n_out) - 1) * A.n_in / A.n_out) + 1 + A.span;
+  }
+  const size_t yz = (size_t)L->a[1].win * L->a[2].win;
+  return sizeof(float) * (yz * (L->a[0].win | 1) + yz * tile + (size_t)L->a[2].win * tile * tile +
+                          (size_t)tile * (L->a[0].span + L->a[1].span + L->a[2].span));
 }
 
-long long pyramid_scratch_floats(const VolumeView& vol, const PyramidView& P, float s0) {
-  long long need = 0;
-  PyrAxis ax[3];
-  for (int l = 0; l < P.n_levels; ++l)
-    if (pyr_plan(vol, P, l, s0, ax)) need = std::max(need, pyr_scratch(ax));
-  return need;
+template <class T>
+static cudaError_t launch_pyr_base(const VolumeView& v, const float4* tf_rgba, int tf_n, const int* d, bool half,
+                                   const PyrWeights& w, const PyrOut& out, cudaStream_t st) {
+  const T* vox = static_cast<const T*>(v.voxels);
+  const size_t sm = sizeof(float2) * ((size_t)tf_n + 1);
+  auto raise = [&](auto kern) {
+    return sm > 30 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) : cudaSuccess;
+  };
+  if (half) {
+    cudaError_t e = raise(k_pyr_base_half<T>);
+    if (e != cudaSuccess) return e;
+    const dim3 grid((d[0] + kHalfT - 1) / kHalfT, (d[1] + kHalfT - 1) / kHalfT, (d[2] + kHalfZ - 1) / kHalfZ);
+    k_pyr_base_half<T><<<grid, 256, sm, st>>>(vox, v.nx, v.ny, v.nz, v.norm, tf_rgba, tf_n, w, d[0], d[1], d[2], out);
+  } else {
+    cudaError_t e = raise(k_pyr_base_window<T>);
+    if (e != cudaSuccess) return e;
+    const long long n = (long long)d[0] * d[1] * d[2];
+    k_pyr_base_window<T><<<(unsigned)((n + 127) / 128), 128, sm, st>>>(vox, v.nx, v.ny, v.nz, v.norm, tf_rgba, tf_n, w,
+                                                                      d[0], d[1], d[2], out);
+  }
+  return cudaGetLastError();
 }
 
-// Lattice point (qx, qy, qz) of a launch whose grid is (x blocks, g_y, g_z).
-__device__ __forceinline__ bool pyr_lattice_point(const PyrAxis* A, const int n_in[3], int qx, int qy, int qz,
-                                                  float3& u) {
-  u = f3((float)(A[0].j0 + qx) + A[0].f, (float)(A[1].j0 + qy) + A[1].f, (float)(A[2].j0 + qz) + A[2].f);
-  // inside the box [0, S]: texel coordinates in [-0.5, n - 0.5]
-  return u.x >= -0.5f && u.y >= -0.5f && u.z >= -0.5f && u.x <= (float)n_in[0] - 0.5f &&
-         u.y <= (float)n_in[1] - 0.5f && u.z <= (float)n_in[2] - 0.5f;
-}
-
-struct PyrAxes { PyrAxis a[3]; };
-
-// The lattice and pass kernels run on (x blocks, y, z) grids: no division of
-// a flat index per element.
-__global__ void k_pyr_lattice_base(VolumeView vol, const float4* __restrict__ tf_rgba, int tf_n, PyrAxes A,
-                                   float* __restrict__ G) {
-  extern __shared__ float4 sm_tf[];
-  for (int i = threadIdx.x; i < tf_n; i += blockDim.x) sm_tf[i] = tf_rgba[i];
-  __syncthreads();
-  const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y, qz = blockIdx.z;
-  if (qx >= A.a[0].g) return;
-  const size_t idx = ((size_t)qz * A.a[1].g + qy) * A.a[0].g + qx;
-  const int n_in[3] = {vol.nx, vol.ny, vol.nz};
-  float3 u;
-  const bool inside = pyr_lattice_point(A.a, n_in, qx, qy, qz, u);
-  const float3 p = f3((u.x + 0.5f) * vol.spacing.x, (u.y + 0.5f) * vol.spacing.y, (u.z + 0.5f) * vol.spacing.z);
-  G[idx] = inside ? tf_alpha(sm_tf, tf_n, sample_volume(vol, p)) : 0.0f;
-}
-
-__global__ void k_pyr_lattice_level(PyramidView P, int l_in, PyrAxes A, float* __restrict__ G) {
-  const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y, qz = blockIdx.z;
-  if (qx >= A.a[0].g) return;
-  const size_t idx = ((size_t)qz * A.a[1].g + qy) * A.a[0].g + qx;
-  const int* n_in = P.dims[l_in];
-  float3 u;
-  const bool inside = pyr_lattice_point(A.a, n_in, qx, qy, qz, u);
-  const float3 p = f3((u.x + 0.5f) * (P.grid.x / (float)n_in[0]), (u.y + 0.5f) * (P.grid.y / (float)n_in[1]),
-                      (u.z + 0.5f) * (P.grid.z / (float)n_in[2]));
-  G[idx] = inside ? pyr_sample_level(P, l_in, p) : 0.0f;
-}
-
-// One 7-tap pass along axis ax of an (nx, ny, nz) array: out has n_out cells
-// along that axis, out[i] = sum_k w[k] in[i m + (k + 3) t].  Grid: (x blocks
-// of the output's x extent, its y extent, its z extent).
-__global__ void k_pyr_pass(const float* __restrict__ in, int nx, int ny, int nz, int ax, PyrAxis a, PyrWeights w,
-                           float* __restrict__ out) {
-  const int ox = ax == 0 ? a.n_out : nx, oy = ax == 1 ? a.n_out : ny;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
-  if (x >= ox) return;
-  const size_t idx = ((size_t)z * oy + y) * ox + x;
-  const int i = ax == 0 ? x : (ax == 1 ? y : z);
-  const long long stride = ax == 0 ? 1 : (ax == 1 ? (long long)nx : (long long)nx * ny);
-  const long long base = (ax == 0 ? 0 : x) + (ax == 1 ? 0 : (long long)y * nx) + (ax == 2 ? 0 : (long long)z * nx * ny);
-  float acc = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 7; ++k) acc = fmaf(w.w[k], __ldg(in + base + (long long)(i * a.m + k * a.t) * stride), acc);
-  out[idx] = acc;
-}
-
-static cudaError_t pyr_separable(const PyrAxis A[3], float* G, float* T1, float* T2, float* out, cudaStream_t st) {
+cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain, const float4* tf_rgba, int tf_n,
+                                 float s0, PyramidView& P, float* data, float* opacity, cudaStream_t st) {
+  const int threads = 128;
+  const int* d0 = P.dims[0];
+  float* op = opacity ? opacity : data;
+  auto out = [&](int l) { return PyrOut{op + P.offset[l], opacity ? data + P.offset[l] : nullptr}; };
   PyrWeights w;
   double sum = 0.0;
   for (int k = -3; k <= 3; ++k) sum += std::exp(-0.5 * k * k);
   for (int k = -3; k <= 3; ++k) w.w[k + 3] = (float)(std::exp(-0.5 * k * k) / sum);
-  const unsigned bx_n = (unsigned)(A[0].n_out + 127) / 128;  // every pass's output has n_out along x
-  k_pyr_pass<<<dim3(bx_n, A[1].g, A[2].g), 128, 0, st>>>(G, A[0].g, A[1].g, A[2].g, 0, A[0], w, T1);
-  k_pyr_pass<<<dim3(bx_n, A[1].n_out, A[2].g), 128, 0, st>>>(T1, A[0].n_out, A[1].g, A[2].g, 1, A[1], w, T2);
-  k_pyr_pass<<<dim3(bx_n, A[1].n_out, A[2].n_out), 128, 0, st>>>(T2, A[0].n_out, A[1].n_out, A[2].g, 2, A[2], w, out);
-  return cudaGetLastError();
-}
 
-cudaError_t launch_pyramid_build(const VolumeView& vol, const float4* tf_rgba, int tf_n, float s0,
-                                 PyramidView& P, float* data, float* scratch, long long scratch_floats,
-                                 cudaStream_t st) {
-  const int threads = 128;
-  long long n0 = (long long)P.dims[0][0] * P.dims[0][1] * P.dims[0][2];
-  size_t sm = sizeof(float4) * tf_n;
-  if (sm > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_pyr_base, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_pyr_lattice_base, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return e;
-  }
-  PyrAxes A;
-  if (scratch && pyr_plan(vol, P, 0, s0, A.a) && pyr_scratch(A.a) <= scratch_floats) {
-    const long long g = (long long)A.a[0].g * A.a[1].g * A.a[2].g;
-    float* T1 = scratch + g;
-    float* T2 = T1 + (long long)A.a[0].n_out * A.a[1].g * A.a[2].g;
-    k_pyr_lattice_base<<<dim3((A.a[0].g + 127) / 128, A.a[1].g, A.a[2].g), 128, sm, st>>>(vol, tf_rgba, tf_n, A,
-                                                                                          scratch);
-    cudaError_t e = pyr_separable(A.a, scratch, T1, T2, data + P.offset[0], st);
-    if (e != cudaSuccess) return e;
+  // a step of one voxel to FP32 accuracy: the taps of a cell share their fractions
+  bool window = (size_t)plain.nx * plain.ny < ((size_t)1 << 31);
+  for (int a = 0; a < 3; ++a) window = window && std::fabs(pyr_tap_step(plain, P, 0, s0, a) - 1.0) <= 1e-6;
+  cudaError_t e = cudaSuccess;
+  if (window) {
+    const bool half = plain.nx == 2 * d0[0] && plain.ny == 2 * d0[1] && plain.nz == 2 * d0[2];
+    e = plain.dtype == 1 ? launch_pyr_base<uint8_t>(plain, tf_rgba, tf_n, d0, half, w, out(0), st)
+                         : launch_pyr_base<uint16_t>(plain, tf_rgba, tf_n, d0, half, w, out(0), st);
   } else {
-    k_pyr_base<<<(unsigned)((n0 + threads - 1) / threads), threads, sm, st>>>(
-        vol, tf_rgba, tf_n, P.dims[0][0], P.dims[0][1], P.dims[0][2], s0, data + P.offset[0]);
+    const size_t sm = sizeof(float4) * tf_n;
+    if (sm > 48 * 1024) e = cudaFuncSetAttribute(k_pyr_base, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    const long long n0 = (long long)d0[0] * d0[1] * d0[2];
+    k_pyr_base<<<(unsigned)((n0 + threads - 1) / threads), threads, sm, st>>>(vol, tf_rgba, tf_n, d0[0], d0[1], d0[2],
+                                                                              s0, out(0));
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return e;
+  P.data = op;
+  // windows of up to 160 KB: taps of up to three texels apart
+  constexpr size_t kLevelSmem = 160 * 1024;
+  e = cudaFuncSetAttribute(k_pyr_level_tile<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_pyr_level_tile<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmem);
+  if (e != cudaSuccess) return e;
+  for (int l = 1; l < P.n_levels; ++l) {
+    LevelAxes L;
+    const int* d = P.dims[l];
+    // 8^3 cells read 2.6 times their texels, 4^3 cells 5.4 times: the smaller
+    // tile where the larger leaves SMs idle (32^3: 21 -> 12 us
+    // as 512 CTAs; 64^3 would take 52 instead of 41)
+    auto tiles = [&](int t) { return dim3((d[0] + t - 1) / t, (d[1] + t - 1) / t, (d[2] + t - 1) / t); };
+    const dim3 g8 = tiles(8);
+    const int tile = (long long)g8.x * g8.y * g8.z < 152 ? 4 : 8;
+    const size_t sm = pyr_level_plan(vol, P, l, s0, tile, &L);
+    if (sm > 0 && sm <= kLevelSmem) {
+      const float* below = op + P.offset[l - 1];
+      if (tile == 8) k_pyr_level_tile<8><<<g8, 512, sm, st>>>(below, L, w, out(l));
+      else k_pyr_level_tile<4><<<tiles(4), 256, sm, st>>>(below, L, w, out(l));
+    } else {
+      const long long nl = (long long)d[0] * d[1] * d[2];
+      const float si = s0 * powf(2.0f, float(l));
+      k_pyr_level<<<(unsigned)((nl + threads - 1) / threads), threads, 0, st>>>(P, l, si, out(l));
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   P.data = data;
-  for (int l = 1; l < P.n_levels; ++l) {
-    long long nl = (long long)P.dims[l][0] * P.dims[l][1] * P.dims[l][2];
-    float si = s0 * powf(2.0f, float(l));
-    if (scratch && pyr_plan(vol, P, l, s0, A.a) && pyr_scratch(A.a) <= scratch_floats) {
-      const long long g = (long long)A.a[0].g * A.a[1].g * A.a[2].g;
-      float* T1 = scratch + g;
-      float* T2 = T1 + (long long)A.a[0].n_out * A.a[1].g * A.a[2].g;
-      k_pyr_lattice_level<<<dim3((A.a[0].g + 127) / 128, A.a[1].g, A.a[2].g), 128, 0, st>>>(P, l - 1, A, scratch);
-      cudaError_t e = pyr_separable(A.a, scratch, T1, T2, data + P.offset[l], st);
-      if (e != cudaSuccess) return e;
-    } else {
-      k_pyr_level<<<(unsigned)((nl + threads - 1) / threads), threads, 0, st>>>(P, l, si, data + P.offset[l]);
-    }
+  if (!opacity) {
+    const int top = P.n_levels - 1;
+    const long long total = P.offset[top] + (long long)P.dims[top][0] * P.dims[top][1] * P.dims[top][2];
+    k_pyr_backtotau<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(data, total);
   }
-  long long total = P.offset[P.n_levels - 1] +
-                    (long long)P.dims[P.n_levels - 1][0] * P.dims[P.n_levels - 1][1] * P.dims[P.n_levels - 1][2];
-  k_pyr_backtotau<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(data, total);
   return cudaGetLastError();
 }
 

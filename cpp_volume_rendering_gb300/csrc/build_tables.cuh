@@ -49,14 +49,12 @@ struct BoxSource {
 };
 cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, float* out, cudaStream_t st);
 
-// Builds every level of P (dims/offsets/grid filled by the caller) into data;
-// levels with a separable form use scratch (scratch_floats floats; see
-// pyramid_scratch_floats), the others the direct 343-tap kernels.
-cudaError_t launch_pyramid_build(const VolumeView& vol, const float4* tf_rgba, int tf_n, float s0,
-                                 PyramidView& P, float* data, float* scratch, long long scratch_floats,
-                                 cudaStream_t st);
-// Floats of scratch the separable levels of P need (0: none is separable).
-long long pyramid_scratch_floats(const VolumeView& vol, const PyramidView& P, float s0);
+// Builds every level of P (dims/offsets/grid filled by the caller) into data,
+// their opacities into opacity (as many floats; nullptr: none to spare, and the
+// extinctions are converted in place at the end).  vol: the marchers' storage
+// of the volume, plain: the x-fastest array.
+cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain, const float4* tf_rgba, int tf_n,
+                                 float s0, PyramidView& P, float* data, float* opacity, cudaStream_t st);
 
 // Grid-stride fill of a device buffer (used to flush L2 between timed frames).
 cudaError_t launch_fill(void* p, size_t bytes, unsigned int v, cudaStream_t st);
