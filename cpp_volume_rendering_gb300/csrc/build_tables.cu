@@ -443,7 +443,11 @@ cudaError_t launch_sat_quads(const unsigned* sat, uint4* out, int sx, int sy, in
 // low end of one cell and the high end of the cell two planes before: a ring
 // of two keeps it, four loads a cell instead of eight.
 constexpr int kBoxRow = 31, kBoxRows = 8, kBoxPlanes = 16;
-template <class W>
+// I: the type of an element's number, 32-bit where the sums have fewer than
+// 2^32 elements: a cell is then 4 loads and some 30 instructions, and the tables
+// are bound by their stores (200 x 180 x 222, shadow tables of 1.4 GB: 393 us,
+// 546 with 64-bit numbers, bound by issue).
+template <class W, class I>
 __global__ void __launch_bounds__(32 * kBoxRows) k_box_tables(BoxSource src, const __grid_constant__ BoxTableSet set,
                                                                float* __restrict__ out) {
   const int ti = blockIdx.z % set.n, c0 = (blockIdx.z / set.n) * kBoxPlanes;
@@ -451,47 +455,53 @@ __global__ void __launch_bounds__(32 * kBoxRows) k_box_tables(BoxSource src, con
   const int lane = threadIdx.x & 31;
   const int a = blockIdx.x * kBoxRow + lane, b = blockIdx.y * kBoxRows + (threadIdx.x >> 5);
   if ((int)(blockIdx.x * kBoxRow) >= d.g.na || b >= d.g.nb || c0 >= d.g.nc) return;  // whole warps
-  const size_t strides[3] = {1, (size_t)src.n[0], (size_t)src.n[0] * src.n[1]};
-  size_t lo[2], hi[2];  // element offsets of the box's low and high corner along the fastest and middle axis
+  const I each = sizeof(W) == 8 ? (I)1 : (I)src.stride;
+  const I strides[3] = {each, each * (I)src.n[0], each * (I)src.n[0] * (I)src.n[1]};
+  I lo[2], hi[2];  // element numbers of the box's low and high corner along the fastest and middle axis
   const int at[2] = {a, b};
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int ax = d.axis[i], n = src.n[ax], p = at[i] - d.pad[i];
-    lo[i] = strides[ax] * (size_t)min(max(p, 0), n - 1);
-    hi[i] = strides[ax] * (size_t)min(max(p + d.w[i], 0), n - 1);
+    lo[i] = strides[ax] * (I)min(max(p, 0), n - 1);
+    hi[i] = strides[ax] * (I)min(max(p + d.w[i], 0), n - 1);
   }
-  const size_t i00 = lo[0] + lo[1], i10 = hi[0] + lo[1], i01 = lo[0] + hi[1], i11 = hi[0] + hi[1];
+  const I i00 = lo[0] + lo[1], i10 = hi[0] + lo[1], i01 = lo[0] + hi[1], i11 = hi[0] + hi[1];
   const int nc = src.n[d.axis[2]];
-  const size_t sc = strides[d.axis[2]];
-  auto at_ = [&](size_t i) -> W {
-    if constexpr (sizeof(W) == 8) return (W)__ldg(src.s64 + i);
-    else return __ldg(src.s32 + i * (size_t)src.stride + src.first);
-  };
+  const I sc = strides[d.axis[2]];
+  const W* base;
+  if constexpr (sizeof(W) == 8) base = reinterpret_cast<const W*>(src.s64);
+  else base = src.s32 + src.first;
   auto rect = [&](int c) -> W {
-    const size_t o = sc * (size_t)min(max(c, 0), nc - 1);
-    return at_(o + i11) - at_(o + i01) - at_(o + i10) + at_(o + i00);
+    const I o = sc * (I)min(max(c, 0), nc - 1);
+    return __ldg(base + (o + i11)) - __ldg(base + (o + i01)) - __ldg(base + (o + i10)) + __ldg(base + (o + i00));
   };
   auto value = [&](W v) {
     if constexpr (sizeof(W) == 8) return ll_to_float((long long)v) * src.scale;
     else return (float)(int)v * src.scale;
   };
   const bool store = lane < kBoxRow && a < d.g.na;
-  float2* dst = reinterpret_cast<float2*>(out) + d.cell + (size_t)b * d.g.row + a;
-  auto put = [&](int c, float v) {
+  const size_t plane = d.g.nab;
+  float2* dst = reinterpret_cast<float2*>(out) + d.cell + (size_t)b * d.g.row + a + (size_t)c0 * plane;
+  auto put = [&](float v) {
     const float next = __shfl_down_sync(0xffffffffu, v, 1);
-    if (store) dst[(size_t)c * d.g.nab] = make_float2(v, next);
+    if (store) *dst = make_float2(v, next);
+    dst += plane;
   };
-  const int end = min(c0 + kBoxPlanes, d.g.nc), p0 = c0 - d.pad[2];
+  const int end = min(c0 + kBoxPlanes, d.g.nc) - d.pad[2];
+  int c = c0 - d.pad[2];
   if (d.w[2] == 2) {
-    W r0 = rect(p0), r1 = rect(p0 + 1);
-    for (int c = c0; c < end; ++c) {
-      const W r2 = rect(c - d.pad[2] + 2);
-      put(c, value(r2 - r0));
+    W r0 = rect(c), r1 = rect(c + 1);
+#pragma unroll 4
+    for (; c < end; ++c) {
+      const W r2 = rect(c + 2);
+      put(value(r2 - r0));
       r0 = r1;
       r1 = r2;
     }
   } else {
-    for (int c = c0; c < end; ++c) put(c, value(rect(c - d.pad[2] + d.w[2]) - rect(c - d.pad[2])));
+    const int w = d.w[2];
+#pragma unroll 2
+    for (; c < end; ++c) put(value(rect(c + w) - rect(c)));
   }
 }
 
@@ -504,8 +514,15 @@ cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, floa
   const dim3 grid((na + kBoxRow - 1) / kBoxRow, (nb + kBoxRows - 1) / kBoxRows,
                   ((nc + kBoxPlanes - 1) / kBoxPlanes) * set.n);
   if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-  if (src.s32) k_box_tables<unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
-  else k_box_tables<unsigned long long><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+  const size_t cells = (size_t)src.n[0] * src.n[1] * src.n[2];
+  const bool small = cells * (src.s32 ? src.stride : 1) < ((size_t)1 << 32);
+  if (src.s32) {
+    if (small) k_box_tables<unsigned, unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+    else k_box_tables<unsigned, size_t><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+  } else {
+    if (small) k_box_tables<unsigned long long, unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+    else k_box_tables<unsigned long long, size_t><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+  }
   return cudaGetLastError();
 }
 
