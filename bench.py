@@ -12,12 +12,10 @@ and a directional SAT cone shadow, step 0.5 voxel.  A step is one frame.
            volume is copied from pinned host memory (cvr_set_volume), the SAT
            is rebuilt (cvr_build_sat) and the frame is rendered and read back
            (cvr_render_host) — the Init() + Redraw() + readback sequence.
-  roofline: the marcher is bound by the L1 load path (its volume and SAT
-           quads are cache-resident): the bytes its 16-byte gathers request
-           per launch / kernel time, against the L1 hit bandwidth of the same
-           load instruction measured in this run (cvr_measure_l1_bandwidth);
-           its DRAM traffic (ncu) against the measured HBM copy bandwidth is
-           reported beside it.
+  roofline: the bytes the marcher's loads request per launch / kernel time,
+           against the L1 hit bandwidth of coalesced 16-byte loads measured
+           in this run (cvr_measure_l1_bandwidth); its DRAM traffic (ncu)
+           against the measured HBM copy bandwidth is reported beside it.
   cpu_baseline: the FP32 CPU oracle (a restatement of the reference shaders)
            on all host cores over a band of rows of the same frame.
 
@@ -189,18 +187,15 @@ def algorithmic_bytes(wl, st, abi):
     return st.samples * 8 * bvox + st.aux_fetches * per_aux + wl.width * wl.height * 16
 
 
-def l1_request_bytes(wl, st, abi, walk):
+def l1_request_bytes(wl, st, abi, tables):
     """Bytes the extinction marcher's loads request from L1 per frame: the
-    volume's trilinear footprint per primary step, 16 sixteen-byte quads per
-    AO box, per shadow box 16 quads or, from a walk table, 4 thirty-two-byte
-    octs, and the image.  Other methods: their algorithmic bytes."""
+    volume's trilinear footprint per primary step, per AO and shadow box 4
+    eight-byte pairs of its box table or, without tables, 16 sixteen-byte
+    quads, and the image.  Other methods: their algorithmic bytes."""
     if wl.method != abi.EXTINCTION:
         return algorithmic_bytes(wl, st, abi)
     bvox = 1 if wl.dtype == abi.CVR_U8 else 2
-    p = wl.params
-    ao = st.shaded_samples * (p.ao_n_shells if p.apply_occlusion else 0)
-    shadow = st.aux_fetches - ao
-    return (st.samples * 8 * bvox + ao * 256 + shadow * (128 if walk else 256) + wl.width * wl.height * 16)
+    return st.samples * 8 * bvox + st.aux_fetches * (32 if tables else 256) + wl.width * wl.height * 16
 
 
 def cpu_baseline(wl, target_s=12.0, threads=None):
@@ -595,9 +590,8 @@ def tables_section(ctx, lib, wl, log=print):
     out["pyramid"] = {"volume": list(wc.dims), "base": list(wc.pyramid["base_dims"]),
                       "levels": wc.pyramid["n_levels"], "gpu_ms": min(pyr_ms.values()),
                       "gpu_ms_by_layout": pyr_ms,
-                      "note": "the 7x7x7 Gaussian of gen_extcoefvol_anysize / _mmlevel per level as one lattice "
-                              "pass (the trilinear samples the 343 taps share) and three 7-tap passes, then the "
-                              "opacity -> extinction pass"}
+                      "note": "the 7x7x7 Gaussian of gen_extcoefvol_anysize / _mmlevel, one kernel per level: the "
+                              "base's trilinear samples once per lattice point, 7-tap passes in shared memory"}
     log(f"tables: SAT {m:.3f} ms GPU vs {cpu_s * 1000:.0f} ms CPU, pyramid {out['pyramid']['gpu_ms']:.3f} ms")
     return out
 
@@ -822,8 +816,8 @@ def batch_section(ctx, lib, args, log=print):
                        "quads": lib.cvr_get_volume_layout(ctx.h), "warp_w": lib.cvr_get_warp_shape(ctx.h),
                        "refill": lib.cvr_get_ray_refill(ctx.h), "staging": lib.cvr_get_brick_staging(ctx.h)},
             "prepare_s": t_prep,
-            "launch": "one CUDA graph: 2 memsets + the persistent extinction launch + persistent surrogate launches "
-                      "of up to 32 jobs each (their descriptors as kernel parameters)"}
+            "launch": "one CUDA graph: persistent extinction launches (jobs on box tables, jobs on the SAT) and the "
+                      "surrogate jobs as collect / light / resolve passes on side streams"}
 
 
 def run_ours(args):
@@ -890,7 +884,7 @@ def run_ours(args):
     # roofline of the dominant kernel (the marcher is the only launch per frame)
     alg = algorithmic_bytes(wl, st, abi)
     walk = bool(lib.cvr_get_walk_tables(ctx.h)) and wl.method == abi.EXTINCTION and wl.params.shadow_type == 1
-    req = l1_request_bytes(wl, st, abi, walk)
+    req = l1_request_bytes(wl, st, abi, wl.method == abi.EXTINCTION and wl.params.shadow_type == 1)
     med_ms = statistics.median(times)
     achieved = req / (med_ms / 1000.0) / 1e9
     peak_hbm, peak_src = measured_peak_hbm()
@@ -900,8 +894,8 @@ def run_ours(args):
                 "peak_source": "measured in this run: cvr_measure_l1_bandwidth (coalesced 16-byte L1 hits)",
                 "bytes_per_launch": req, "kernel_ms": round(med_ms, 4),
                 "effective_gather_gbs": round(alg / (med_ms / 1000.0) / 1e9, 1),
-                "note": "achieved = bytes the marcher's loads request from L1 per launch (walk-table shadow boxes: "
-                        "4 x 32 B) / CUDA-event time; effective_gather_gbs counts the reference's 64 SAT texels "
+                "note": "achieved = bytes the marcher's loads request from L1 per launch (box tables: 4 x 8 B per "
+                        "box) / CUDA-event time; effective_gather_gbs counts the reference's 64 SAT texels "
                         "of 4 B per box query"}
     if traffic:
         roofline["hbm"] = {"achieved": round(traffic / (med_ms / 1000.0) / 1e9, 2), "peak": peak_hbm,
@@ -955,8 +949,7 @@ def run_ours(args):
         emit_here = rank == 0
         # the headline frame at its tuned configuration against the alternatives:
         # the persistent ray refill switched the other way, and (extinction) the
-        # directional shadow's boxes through the equal-fraction query instead of
-        # the walk table
+        # walk table off, which frames with box tables do not read
         hv = {"workload": WORKLOAD_DESC[args.workload], "tuned_ms": med_ms, "tuning": tuning}
         was = lib.cvr_get_ray_refill(ctx.h)
         abi.check(lib.cvr_set_ray_refill(ctx.h, 1 - was), ctx.h)

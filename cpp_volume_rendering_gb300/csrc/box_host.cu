@@ -12,8 +12,8 @@ namespace ctxutil {
 namespace {
 
 // Pixels a frame (or the frames so far that went without) must have per cell
-// to build.  Building costs 3.5 ps a cell (27 tables of a 256^3 volume, 526 M
-// cells: 1.9 ms with their source); the tables save 9 ns a pixel against the
+// to build.  Building costs 2 to 3.5 ps a cell (shadow tables of a 200 x 180 x
+// 222 volume, 190 M cells: 0.39 ms, and their source); the tables save 9 ns a pixel against the
 // compact table and its walk table (1024^2 frame 13.7 -> 4.3 ms) and 53 ns
 // against the int64 table (61 -> 5.5 ms).  At 4e-4 pixels a cell the frame
 // itself repays the build; smaller frames add up, and the tables are built

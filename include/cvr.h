@@ -351,14 +351,17 @@ int cvr_get_volume_layout(cvr_ctx* ctx);
  * int64 table; batches build their own.  0 disables it. */
 cvr_status cvr_set_compact_sat(cvr_ctx* ctx, int enable);
 int cvr_get_compact_sat(cvr_ctx* ctx);
-/* Walk tables (no reference counterpart; default on): a frame on the compact
- * SAT whose directional-shadow boxes all have integer widths (the sample
- * interval along the walk axis, ceil-rounded cross-sections) reads a second
- * table for its shadow queries: the compact sums differenced along the walk
- * axis by the interval, 32 bytes per cell (8 x the volume's cells x 4 bytes),
- * built on the first frame that needs it and kept until the SAT, the walk
- * axis or the interval changes.  A shadow box is then four 32-byte loads
- * instead of sixteen 16-byte ones; same images.  0 disables it. */
+/* Walk tables (no reference counterpart; default on).  Extinction frames whose
+ * boxes all have integer widths (ambient-occlusion radii in half voxels; for
+ * directional light the sample interval along the walk axis, ceil-rounded
+ * cross-sections) read them from box tables: per distinct box the sum at
+ * every cell, 8 bytes each, at most 24 GiB for the shadow and 24 GiB for the
+ * occlusion of a volume, built by the first frames whose pixels repay it and
+ * kept until the SAT, the walk axis or the interval changes.  Directional
+ * frames on the compact SAT that do not repay them, or whose tables find no
+ * room, read a walk table for their shadow: the compact sums differenced
+ * along the walk axis by the interval, 32 bytes per cell.  Same images.  0
+ * disables the walk table. */
 cvr_status cvr_set_walk_tables(cvr_ctx* ctx, int enable);
 int cvr_get_walk_tables(const cvr_ctx* ctx);
 
