@@ -994,17 +994,26 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
   cvr_light dl{};
   if (!light) { light = &dl; }
   cudaError_t e = cudaSuccess;
-  // the lists of a frame shaded in a pass of its own, outside the frame's time
-  // (256^2 through 128^3: 0.4 ms of allocation beside 0.7 ms of kernels)
+  c->deferred_frame = false;
+  // the lists of a frame shaded in a pass of its own, and the code of its
+  // kernels, outside the frame's time (256^2 through 128^3: 0.4 ms of
+  // allocation and 0.9 ms of loading beside 0.75 ms of kernels)
   const float step = deferred_step(c, method, params, params_size);
   if (step > 0.0f) {
     f.step = step;
     DeferredPlan plan;
     if (const size_t bytes = deferred_bytes(f, &plan)) {
       e = ensure(c->d_defer, c->defer_cap, bytes);
-      if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // the direct marcher needs none
-      else if (e != cudaSuccess) return cuda_fail(c, e, "render lists");
-      e = cudaSuccess;
+      if (e == cudaErrorMemoryAllocation) {  // the direct marcher needs none
+        cudaGetLastError();
+        e = cudaSuccess;
+      } else if (e == cudaSuccess && stats) {
+        e = load_deferred(f);
+        if (e == cudaSuccess && method == CVR_METHOD_GROUND_TRUTH) e = load_light_gt(f);
+        if (e == cudaSuccess && method == CVR_METHOD_SURROGATE)
+          e = load_light_sur((c->sampling & CVR_SAMPLING_TEX_FEATURES) != 0);
+      }
+      if (e != cudaSuccess) return cuda_fail(c, e, "render lists");
     }
   }
   if (stats) CK(c, cudaEventRecord(c->ev[2], c->stream));
@@ -1357,7 +1366,8 @@ cvr_status cvr_autotune(cvr_ctx* c, int method, const cvr_camera* cam, const cvr
     for (int t = 0; t < 6; ++t)
       for (int wi = 0; wi < 3; ++wi)
         if (warp_fits(tiles[t][0], tiles[t][1], warps[wi])) trial(t, bvar, wi, bb);
-    for (int v = 0; v < n_variants; ++v) trial(bt, v, bw, bb);
+    // the passes of a deferred frame have one register budget each
+    for (int v = 0; v < (c->deferred_frame ? 1 : n_variants); ++v) trial(bt, v, bw, bb);
     for (int k = 0; k < 5; ++k) trial(bt, bvar, bw, k);
     if (before[0] == bt && before[1] == bvar && before[2] == bw && before[3] == bb) break;
   }

@@ -311,6 +311,7 @@ struct cvr_ctx {
   int vbrick_bs = -1;                        // layout of d_vbrick's contents (-1: stale, kQuadCopy: quads)
   // object-space light cache (cvr_set_light_cache): 0 = off
   int lc_dims[3] = {0, 0, 0};
+  bool deferred_frame = false;  // the last frame was shaded in a pass of its own
   float2* d_lcache = nullptr;
   size_t lcache_cap = 0;
   // per-voxel gradient of the current volume (cvr_build_gradient) and the
@@ -459,7 +460,7 @@ cudaError_t launch_deferred(void* mem, const DeferredPlan& p, const FrameArgs& f
 template <class Light>
 cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t, bool ext, unsigned taps, Light light,
                             bool* done) {
-  *done = false;
+  *done = c->deferred_frame = false;
   DeferredPlan p;
   const size_t bytes = deferred_bytes(f, &p);
   if (bytes == 0) return cudaSuccess;
@@ -469,7 +470,7 @@ cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t,
     return cudaSuccess;
   }
   if (e == cudaSuccess) e = launch_deferred(c->d_defer, p, f, t, ext, taps, light, c->stream);
-  *done = e == cudaSuccess;
+  *done = c->deferred_frame = e == cudaSuccess;
   return e;
 }
 

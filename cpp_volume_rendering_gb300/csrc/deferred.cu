@@ -246,4 +246,16 @@ cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows,
   });
 }
 
+cudaError_t load_deferred(const FrameArgs& f) {
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    return with_threads(f, [&](auto nt) {
+      constexpr int NT = decltype(nt)::value;
+      cudaFuncAttributes a;
+      const cudaError_t e = cudaFuncGetAttributes(&a, k_collect<NT, S>);
+      return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_resolve<NT, S>);
+    });
+  });
+}
+
 }  // namespace cvr

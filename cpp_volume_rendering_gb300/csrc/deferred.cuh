@@ -81,6 +81,10 @@ struct DeferredPlan {
 };
 bool deferred_plan(const FrameArgs& f, DeferredPlan* p);
 cudaError_t launch_collect(const FrameArgs& f, const Deferred& d, unsigned rows, cudaStream_t st);
+// A kernel's code is loaded at its first use (0.1 to 0.4 ms each): loaded ahead
+// of a frame that is timed.
+cudaError_t load_deferred(const FrameArgs& f);
+cudaError_t load_light_gt(const FrameArgs& f);
 // ext: the extinction renderer's gradient branch; taps: secondary lookups per
 // shaded sample to count (0: the light pass counts its own).
 cudaError_t launch_resolve(const FrameArgs& f, const Deferred& d, unsigned rows, const LightTerms& t, bool ext,

@@ -92,4 +92,9 @@ cudaError_t launch_light_sur(const FrameArgs& f, const SurArgs& a, bool tex, con
   return tex ? launch_light_sur_t<true>(f, a, d, err, st) : launch_light_sur_t<false>(f, a, d, err, st);
 }
 
+cudaError_t load_light_sur(bool tex) {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, tex ? k_light_sur<true, kSurGroups> : k_light_sur<false, kSurGroups>);
+}
+
 }  // namespace cvr

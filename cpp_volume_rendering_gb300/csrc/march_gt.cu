@@ -35,9 +35,10 @@ static cudaError_t launch_gt_nt(const FrameArgs& f, const GtArgs& g, cudaStream_
 }
 
 // The light terms of a frame's collected samples (deferred.cuh): the frame's
-// whole time (256^3 quads -> 512^2, 14.8 G light steps: 45.4 ms of 45.8; the
-// direct marcher 72.6, 148.7 with one clamped sample in flight).  Bound by
-// instruction issue; 6 CTAs a SM (80 registers) 45.4 ms, 5 45.9, 4 47.8.
+// whole time (256^3 quads -> 512^2, 14.8 G light steps: 37.3 ms of 37.7; with
+// an exponential a step 45.4 of 45.8, the direct marcher then 72.6, 148.7 with
+// one clamped sample in flight).  Bound by instruction issue; 6 CTAs a SM (80
+// registers) 37.7 ms, 5 37.8, 7 37.5, 8 38.4.
 template <class S>
 __global__ void __launch_bounds__(128, 6) k_light_gt(const __grid_constant__ GtArgs g,
                                                         const __grid_constant__ FrameArgs f,
@@ -52,6 +53,14 @@ cudaError_t launch_light_gt(const FrameArgs& f, const GtArgs& g, const Deferred&
   return with_sampler(f.vol, [&](auto* s) {
     using S = std::remove_pointer_t<decltype(s)>;
     return launch_persistent(k_light_gt<S>, GtStage::bytes(f.tf_n, g), st, g, f, d);
+  });
+}
+
+cudaError_t load_light_gt(const FrameArgs& f) {
+  return with_sampler(f.vol, [&](auto* s) {
+    using S = std::remove_pointer_t<decltype(s)>;
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, k_light_gt<S>);
   });
 }
 

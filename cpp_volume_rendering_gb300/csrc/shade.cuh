@@ -742,57 +742,84 @@ struct GtShadeT {
   // The samples' positions do not depend on the transmittance, only the ray's
   // end does, so kAhead samples are fetched together and then taken one by
   // one until the ray ends: kAhead loads in flight instead of one, for at
-  // most kAhead - 1 samples fetched past the end of a ray.
+  // most kAhead - 1 samples fetched past the end of a ray.  The steps' optical
+  // depths are summed and exponentiated once, at the end of the ray: where
+  // kAhead whole steps remain, all inside, they take one test for the ray's
+  // end between them (256^3 -> 512^2: 45.8 -> 37.7 ms against an exponential and
+  // three tests a step).
   static constexpr int kAhead = 4;
+  static constexpr float kOpaque = 4.60517f;  // -ln(0.01): 1 - transmittance > 0.99
   __device__ float light_ray(float3 tx, float3 w, float dist, const FrameArgs& f, unsigned& aux) const {
-    float vt = 1.0f;
+    float tau = 0.0f;
     ++aux;
     float s = g->gap;
     const float3 B = f.vol.grid;
     float st0 = alpha(sample(tx + w * s));
     float ta = 0.0f, tb = -1.0f;  // the samples that need no box test and no clamp
     if constexpr (S::kInside) inside_part(f.vol, tx, w, ta, tb);
+    const float step = g->lstep, half = 0.5f * step;
+    const float whole = dist - (kAhead + 0.5f) * step;  // kAhead whole steps remain up to here
     for (int guard = 0; guard < kMaxLightSteps && s < dist; guard += kAhead) {
-      float h[kAhead], at[kAhead], st[kAhead];
+      float at[kAhead], st[kAhead];
+      if (S::kInside && s < whole) {
+        float sj = s;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) at[j] = sj = sj + step;
+        if (at[0] >= ta && sj <= tb) {
+#pragma unroll
+          for (int j = 0; j < kAhead; j += 2) {
+            const float2 a = un2(alpha.two(sample.two_inside(along2(tx, w, mk2(at[j], at[j + 1])))));
+            st[j] = a.x;
+            st[j + 1] = a.y;
+          }
+          float t[kAhead];
+#pragma unroll
+          for (int j = 0; j < kAhead; ++j) {
+            tau = fmaf(st0 + st[j], half, tau);
+            t[j] = tau;
+            st0 = st[j];
+          }
+          if (fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3])) > kOpaque) {
+            const int n = t[0] > kOpaque ? 0 : (t[1] > kOpaque ? 1 : (t[2] > kOpaque ? 2 : 3));
+            aux += n + 1;
+            return expf(-(n == 0 ? t[0] : (n == 1 ? t[1] : (n == 2 ? t[2] : t[3]))));
+          }
+          aux += kAhead;
+          s = sj;
+          continue;
+        }
+      }
+      float h[kAhead];
       bool in[kAhead];
       float sj = s;
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
-        h[j] = fminf(g->lstep, dist - sj);
+        h[j] = fminf(step, dist - sj);
         in[j] = sj < dist;
         sj = sj + h[j];
         at[j] = sj;
       }
-      if (S::kInside && at[0] >= ta && at[kAhead - 1] <= tb) {
 #pragma unroll
-        for (int j = 0; j < kAhead; j += 2) {
-          const float2 a = un2(alpha.two(sample.two_inside(along2(tx, w, mk2(at[j], at[j + 1])))));
-          st[j] = a.x;
-          st[j + 1] = a.y;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < kAhead; j += 2) {
-          const pos2 p = along2(tx, w, mk2(at[j], at[j + 1]));
-          const float2 x = un2(p.x), y = un2(p.y), z = un2(p.z);
-          in[j] = in[j] && !(x.x < 0.0f || x.x > B.x || y.x < 0.0f || y.x > B.y || z.x < 0.0f || z.x > B.z);
-          in[j + 1] = in[j + 1] && !(x.y < 0.0f || x.y > B.x || y.y < 0.0f || y.y > B.y || z.y < 0.0f || z.y > B.z);
-          const float2 a = un2(alpha.two(sample.two(p)));
-          st[j] = a.x;
-          st[j + 1] = a.y;
-        }
+      for (int j = 0; j < kAhead; j += 2) {
+        const pos2 p = along2(tx, w, mk2(at[j], at[j + 1]));
+        const float2 x = un2(p.x), y = un2(p.y), z = un2(p.z);
+        in[j] = in[j] && !(x.x < 0.0f || x.x > B.x || y.x < 0.0f || y.x > B.y || z.x < 0.0f || z.x > B.z);
+        in[j + 1] = in[j + 1] && !(x.y < 0.0f || x.y > B.x || y.y < 0.0f || y.y > B.y || z.y < 0.0f || z.y > B.z);
+        const float2 a = un2(alpha.two(sample.two(p)));
+        st[j] = a.x;
+        st[j + 1] = a.y;
       }
 #pragma unroll
       for (int j = 0; j < kAhead; ++j) {
-        if (!in[j]) return vt;
+        if (!in[j]) return expf(-tau);
         ++aux;
-        vt *= expf(-((st0 + st[j]) * 0.5f) * h[j]);
-        if ((1.0f - vt) > 0.99f) return vt;
+        tau = fmaf((st0 + st[j]) * 0.5f, h[j], tau);
+        if (tau > kOpaque) return expf(-tau);
         st0 = st[j];
       }
       s = sj;
     }
-    return vt;
+    return expf(-tau);
   }
 
   // ConeOcclusionEvaluationRayCasting (gt_ray_marching.comp:109-169).

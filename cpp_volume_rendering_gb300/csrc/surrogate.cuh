@@ -217,6 +217,7 @@ SurSpiral sur_spiral(const FrameArgs& f);
 
 struct Deferred;
 // The light terms of a frame's collected samples (deferred.cuh).
+cudaError_t load_light_sur(bool tex);  // as load_deferred
 cudaError_t launch_light_sur(const FrameArgs& f, const SurArgs& a, bool tex, const Deferred& d, int* err,
                              cudaStream_t st);
 
