@@ -32,6 +32,7 @@ struct cvr_batch {
   unsigned long long* d_stats = nullptr;  // 3 per job, in the caller's job order
   bool ext_compact = false;
   bool ext_aligned = false;  // every job: an aligned shadow table and aligned AO boxes (or AO off)
+  std::vector<std::shared_ptr<VolCopy>> copies;  // the volume copies its jobs read
   std::vector<uint4*> sat32;              // the batch's own compact SATs, one per volume slot used
   std::vector<uint4*> walks;              // their walk tables, one per (slot, walk axis, depth) in use
   std::vector<long long> walk_keys;
@@ -151,6 +152,8 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     FrameArgs f;
     st = frame_args(c, &j.camera, j.params, j.out_rgba_dev, j.width, j.height, &f);
     if (st != CVR_OK) break;
+    if (f.vol.voxels != c->d_vol && std::find(b->copies.begin(), b->copies.end(), c->vcopy) == b->copies.end())
+      b->copies.push_back(c->vcopy);
     st = grad_args(c, j.method, &j.light, &f);
     if (st != CVR_OK) break;
     f.stats = b->d_stats + 3 * (size_t)i;

@@ -132,6 +132,13 @@ static bool quads_pay(cvr_ctx* c, double pixels) {
   return 2.0 * c->quad_seen * std::max(c->nx, std::max(c->ny, c->nz)) >= voxels;
 }
 
+// Room for the volume's copy in another layout; a copy that a batch reads stays
+// the batch's.
+static cudaError_t copy_room(cvr_ctx* c, size_t bytes) {
+  if (!c->vcopy || c->vcopy.use_count() > 1) c->vcopy = std::make_shared<VolCopy>();
+  return ensure(c->vcopy->data, c->vcopy->cap, bytes);
+}
+
 cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, double pixels) {
   VolumeView v = volume_view(c);
   // the quad copy is indexed with 32-bit cell numbers
@@ -143,28 +150,28 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, doubl
     v.qrow = (unsigned)qrow;
     v.qplane = (unsigned)qplane;
     if (c->vbrick_bs != kQuadCopy) {
-      cudaError_t qe = ensure(c->d_vbrick, c->vbrick_cap, qplane * c->nz * qbytes);
+      cudaError_t qe = copy_room(c, qplane * c->nz * qbytes);
       if (qe == cudaErrorMemoryAllocation && !c->quads) {  // not asked for: the plain array serves
         cudaGetLastError();
         *out = volume_view(c);
         return CVR_OK;
       }
       CK(c, qe);
-      CK(c, launch_quad_volume(c->d_vol, c->d_vbrick, c->dtype, c->nx, c->ny, c->nz, v.qrow, v.qplane, c->stream));
+      CK(c, launch_quad_volume(c->d_vol, c->vcopy->data, c->dtype, c->nx, c->ny, c->nz, v.qrow, v.qplane, c->stream));
       c->vbrick_bs = kQuadCopy;
     }
-    v.voxels = c->d_vbrick;
+    v.voxels = c->vcopy->data;
     v.quad = 1;
   } else if (c->brick_bs > 0) {
     if (c->vbrick_bs != c->brick_bs) {
       const long long n = brick_elements(c->nx, c->ny, c->nz, c->brick_bs);
-      CK(c, ensure(c->d_vbrick, c->vbrick_cap, (size_t)n * (c->dtype == CVR_U8 ? 1 : 2)));
-      CK(c, launch_brick_volume(c->d_vol, c->d_vbrick, c->dtype, c->nx, c->ny, c->nz, c->brick_bs, c->stream));
+      CK(c, copy_room(c, (size_t)n * (c->dtype == CVR_U8 ? 1 : 2)));
+      CK(c, launch_brick_volume(c->d_vol, c->vcopy->data, c->dtype, c->nx, c->ny, c->nz, c->brick_bs, c->stream));
       c->vbrick_bs = c->brick_bs;
     }
     const int B = 1 << c->brick_bs;
     const long long bx = (c->nx + B - 1) / B, by = (c->ny + B - 1) / B;
-    v.voxels = c->d_vbrick;
+    v.voxels = c->vcopy->data;
     v.bs = c->brick_bs;
     v.stride[0] = (long long)B * B * B;
     v.stride[1] = bx * v.stride[0];
@@ -656,7 +663,7 @@ void cvr_destroy(cvr_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_vol, c->d_rgbt, c->d_rgba, c->d_sat, c->d_lut, c->d_pyr, c->d_occ_sec, c->d_sdw_sec,
-                  c->d_occ_vec, c->d_sdw_vec, c->d_stats, c->d_out, c->d_flush, c->d_probe, c->d_vbrick, c->d_lcache, c->d_grad, c->d_ms, c->d_msf,
+                  c->d_occ_vec, c->d_sdw_vec, c->d_stats, c->d_out, c->d_flush, c->d_probe, c->d_lcache, c->d_grad, c->d_ms, c->d_msf,
                   c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc, c->d_defer};
   for (void* p : bufs)
     if (p) cudaFree(p);

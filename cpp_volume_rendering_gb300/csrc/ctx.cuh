@@ -134,6 +134,16 @@ struct BoxTables {
 // Largest quad copy made without cvr_set_volume_layout asking for the quads.
 constexpr size_t kAutoCopyBytes = (size_t)2 << 30;
 
+// A copy of a volume in another layout.  Batches hold the copies that their
+// jobs read, so a layout set afterwards makes its own (copy_room).
+struct VolCopy {
+  void* data = nullptr;
+  size_t cap = 0;  // bytes
+  ~VolCopy() {
+    if (data) cudaFree(data);
+  }
+};
+
 // A resident volume that is not the current one (cvr_select_volume): the
 // volume, its SAT, pyramid and texture copies.  The current volume lives in
 // the cvr_ctx fields of the same names.
@@ -168,8 +178,7 @@ struct VolSlot {
   size_t pyrq_cap = 0;
   bool pyrq_ready = false;
   TexState tex;
-  void* d_vbrick = nullptr;
-  size_t vbrick_cap = 0;
+  std::shared_ptr<VolCopy> vcopy;
   int vbrick_bs = -1;
   double quad_seen = 0.0;
   uint2* d_grad = nullptr;
@@ -177,7 +186,7 @@ struct VolSlot {
   bool grad_ready = false;
   cvr_gradient_params grad_params{CVR_GRADIENT_NONE, 1, 0, 1};
   ~VolSlot() {
-    void* bufs[] = {d_vol, d_sat, d_lut, d_pyr, d_vbrick, d_grad, d_sat32, d_lut32, d_pyrq};
+    void* bufs[] = {d_vol, d_sat, d_lut, d_pyr, d_grad, d_sat32, d_lut32, d_pyrq};
     for (void* p : bufs)
       if (p) cudaFree(p);
   }
@@ -305,10 +314,9 @@ struct cvr_ctx {
   // (cvr_set_brick_size, cvr_set_volume_layout)
   int brick_bs = 0;                          // tuning: 0 plain layout, else log2 of the brick edge
   bool quads = false;                        // tuning: the x-y quad layout (takes precedence)
-  void* d_vbrick = nullptr;
-  size_t vbrick_cap = 0;
+  std::shared_ptr<VolCopy> vcopy;
   double quad_seen = 0.0;                    // pixels of the volume's frames without a quad copy (quads_pay)
-  int vbrick_bs = -1;                        // layout of d_vbrick's contents (-1: stale, kQuadCopy: quads)
+  int vbrick_bs = -1;                        // layout of the copy's contents (-1: stale, kQuadCopy: quads)
   // object-space light cache (cvr_set_light_cache): 0 = off
   int lc_dims[3] = {0, 0, 0};
   bool deferred_frame = false;  // the last frame was shaded in a pass of its own
@@ -365,8 +373,7 @@ inline void swap_volume(cvr_ctx* c, VolSlot& s) {
   std::swap(c->pyrq_cap, s.pyrq_cap);
   std::swap(c->pyrq_ready, s.pyrq_ready);
   swap_tex(c->tex, s.tex);
-  std::swap(c->d_vbrick, s.d_vbrick);
-  std::swap(c->vbrick_cap, s.vbrick_cap);
+  std::swap(c->vcopy, s.vcopy);
   std::swap(c->vbrick_bs, s.vbrick_bs);
   std::swap(c->quad_seen, s.quad_seen);
   std::swap(c->d_grad, s.d_grad);

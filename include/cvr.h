@@ -505,8 +505,8 @@ cvr_status cvr_get_blinn_phong(cvr_ctx* ctx, cvr_blinn_phong* out);
  * first; CVR_METHOD_SURROGATE: each job's passes on one of three lanes beside
  * them; other methods are rejected).  The launches, with the resets of their
  * counters, are captured in one CUDA graph at creation; cvr_batch_run replays
- * it.  A batch holds its jobs' tables and at most 4.5 GiB of sample lists a
- * lane.  Every image equals the image
+ * it.  A batch holds its jobs' tables and volume copies (a layout set later
+ * does not touch them) and at most 4.5 GiB of sample lists a lane.  Every image equals the image
  * of the same job rendered alone by cvr_render with the context's tuning at
  * creation.  Jobs keep pointers to their output buffers; the volumes, tables
  * and network they use must not change while the batch exists (re-create it). */
