@@ -64,8 +64,8 @@ __device__ __forceinline__ f2 trilinear2(f2 c000, f2 c100, f2 c010, f2 c110, f2 
 // The part [ta, tb] of the line o + d t whose positions are at least 0.51
 // voxels inside the box on every axis: there a sample's cell needs no clamp
 // and both its planes exist (0.01 voxels are far more than the roundings of
-// t and of the position, for axes of up to 8192 voxels; larger ones, and
-// lines with a NaN, get an empty part).
+// t and of the position, for axes of up to 8192 voxels; larger ones, axes of
+// one voxel, which have no second plane, and lines with a NaN get an empty part).
 __device__ __forceinline__ void inside_part(const VolumeView& v, float3 o, float3 d, float& ta, float& tb) {
   const float3 m = v.spacing * 0.51f;
   const float3 inv = f3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
@@ -74,7 +74,7 @@ __device__ __forceinline__ void inside_part(const VolumeView& v, float3 o, float
   ta = fmaxf(fmaxf(lo.x, lo.y), lo.z);
   tb = fminf(fminf(hi.x, hi.y), hi.z);
   const float sum = d.x + d.y + d.z + o.x + o.y + o.z;
-  if (!(sum - sum == 0.0f) || v.nx > 8192 || v.ny > 8192 || v.nz > 8192) tb = -1.0f, ta = 0.0f;
+  if (!(sum - sum == 0.0f) || min(min(v.nx, v.ny), v.nz) < 2 || max(max(v.nx, v.ny), v.nz) > 8192) tb = -1.0f, ta = 0.0f;
 }
 
 // Voxel values as FP32 plus 2^23: the integer below 2^16 placed in the
