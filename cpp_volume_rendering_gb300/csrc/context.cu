@@ -132,9 +132,10 @@ static bool quads_pay(cvr_ctx* c, double pixels) {
   return 2.0 * c->quad_seen * std::max(c->nx, std::max(c->ny, c->nz)) >= voxels;
 }
 
-// Room for the volume's copy in another layout; a copy that a batch reads stays
-// the batch's.
+// Room for the volume's copy in another layout, whose contents are gone; a
+// copy that a batch reads stays the batch's.
 static cudaError_t copy_room(cvr_ctx* c, size_t bytes) {
+  c->vbrick_bs = -1;
   if (!c->vcopy || c->vcopy.use_count() > 1) c->vcopy = std::make_shared<VolCopy>();
   return ensure(c->vcopy->data, c->vcopy->cap, bytes);
 }
@@ -153,6 +154,7 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, doubl
       cudaError_t qe = copy_room(c, qplane * c->nz * qbytes);
       if (qe == cudaErrorMemoryAllocation && !c->quads) {  // not asked for: the plain array serves
         cudaGetLastError();
+        c->quad_seen = -HUGE_VAL;  // nor tried again for this volume
         *out = volume_view(c);
         return CVR_OK;
       }
