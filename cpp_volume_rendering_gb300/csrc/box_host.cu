@@ -30,7 +30,8 @@ int texel_width(const ShadowBoxTable& t, int k, int axis) {
 
 // Grid of a table along SAT axes ax (fastest first) with pads; one cell per
 // low corner -pad ... n-1, and one plane more, the successor of the last.
-BoxTableDesc table_desc(const int n[3], const int ax[3], const int w[3], const int pad[3]) {
+// False: beyond 32-bit plane pitches or the build's launches.
+bool table_desc(const int n[3], const int ax[3], const int w[3], const int pad[3], BoxTableDesc* out) {
   BoxTableDesc d{};
   for (int i = 0; i < 3; ++i) {
     d.axis[i] = ax[i];
@@ -41,8 +42,10 @@ BoxTableDesc table_desc(const int n[3], const int ax[3], const int w[3], const i
   d.g.nb = n[ax[1]] + pad[1] + 1;
   d.g.nc = n[ax[2]] + pad[2] + 1;
   d.g.row = (int)padded_row((unsigned)d.g.na, (int)kCellBytes);
+  if ((size_t)d.g.row * (size_t)d.g.nb > kBoxPoolBytes / kCellBytes || !box_table_builds(d.g)) return false;
   d.g.nab = padded_plane((unsigned)d.g.row * (unsigned)d.g.nb, (int)kCellBytes);
-  return d;
+  *out = d;
+  return true;
 }
 size_t cells_of(const BoxGrid& g) { return (size_t)g.nab * (size_t)g.nc; }
 // The grid a lookup clamps to: without the successor row and plane.
@@ -79,7 +82,8 @@ bool shadow_plan(BoxTables& B, unsigned long long gen, const int n[3], const Sha
   }
   const bool same = kin && pool.key[2] == pad[0] && pool.key[3] == pad[1];
   const int none[3] = {0, 0, 0};
-  const BoxTableDesc grid = table_desc(n, ax, none, pad);
+  BoxTableDesc grid;
+  if (!table_desc(n, ax, none, pad, &grid)) return false;
   const size_t cells = cells_of(grid.g);
   P->shadow = true;
   P->sdw_key = {axis, ww, pad[0], pad[1]};
@@ -99,7 +103,8 @@ bool shadow_plan(BoxTables& B, unsigned long long gen, const int n[3], const Sha
   P->sdw_bytes = P->sdw_new ? std::max(room, P->have.size()) * cells * kCellBytes : pool.cap;
   for (size_t i = P->sdw_new ? 0 : had; i < P->have.size(); ++i) {
     const int w[3] = {P->have[i] & 1023, P->have[i] >> 10, ww};
-    BoxTableDesc d = table_desc(n, ax, w, pad);
+    BoxTableDesc d;
+    if (!table_desc(n, ax, w, pad, &d)) return false;
     d.cell = (unsigned)(i * cells);
     P->sdw.t[P->sdw.n++] = d;
     P->missing += cells;
@@ -140,7 +145,8 @@ bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const Shadow
     for (int i = 0; i < e->n_shells; ++i) {
       const int w = (int)std::nearbyint(2.0f * e->radii[i]);
       const int ww[3] = {w, w, w}, pad[3] = {w + 1, w + 1, w + 1};
-      BoxTableDesc d = table_desc(n, xyz, ww, pad);
+      BoxTableDesc d;
+      if (!table_desc(n, xyz, ww, pad, &d)) return false;
       d.cell = (unsigned)cell;
       cell += cells_of(d.g);
       if (cell * kCellBytes > kBoxPoolBytes) return false;

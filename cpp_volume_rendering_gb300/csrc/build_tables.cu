@@ -436,7 +436,7 @@ cudaError_t launch_sat_quads(const unsigned* sat, uint4* out, int sx, int sy, in
 }
 
 // ------------------------------------------------------------- box tables
-// All tables of a set in one launch: a warp per row segment of 31 cells (lane
+// All tables of a set in one launch (as many as its grid holds): a warp per row segment of 31 cells (lane
 // 31 only supplies the last cell's successor), 8 rows per CTA, kBoxPlanes
 // planes per thread, the sums of the box's rectangle in the planes at its two
 // ends.  Along a walk of interval 2 (the default) a plane's rectangle is the
@@ -449,8 +449,8 @@ constexpr int kBoxRow = 31, kBoxRows = 8, kBoxPlanes = 16;
 // 546 with 64-bit numbers, bound by issue).
 template <class W, class I>
 __global__ void __launch_bounds__(32 * kBoxRows) k_box_tables(BoxSource src, const __grid_constant__ BoxTableSet set,
-                                                               float* __restrict__ out) {
-  const int ti = blockIdx.z % set.n, c0 = (blockIdx.z / set.n) * kBoxPlanes;
+                                                               int first, int count, float* __restrict__ out) {
+  const int ti = first + blockIdx.z % count, c0 = (blockIdx.z / count) * kBoxPlanes;
   const BoxTableDesc& d = set.t[ti];
   const int lane = threadIdx.x & 31;
   const int a = blockIdx.x * kBoxRow + lane, b = blockIdx.y * kBoxRows + (threadIdx.x >> 5);
@@ -511,19 +511,24 @@ cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, floa
   for (int i = 0; i < set.n; ++i) {
     na = std::max(na, set.t[i].g.na); nb = std::max(nb, set.t[i].g.nb); nc = std::max(nc, set.t[i].g.nc);
   }
-  const dim3 grid((na + kBoxRow - 1) / kBoxRow, (nb + kBoxRows - 1) / kBoxRows,
-                  ((nc + kBoxPlanes - 1) / kBoxPlanes) * set.n);
-  if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
+  const int chunks = (nc + kBoxPlanes - 1) / kBoxPlanes;
   const size_t cells = (size_t)src.n[0] * src.n[1] * src.n[2];
   const bool small = cells * (src.s32 ? src.stride : 1) < ((size_t)1 << 32);
-  if (src.s32) {
-    if (small) k_box_tables<unsigned, unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
-    else k_box_tables<unsigned, size_t><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
-  } else {
-    if (small) k_box_tables<unsigned long long, unsigned><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
-    else k_box_tables<unsigned long long, size_t><<<grid, 32 * kBoxRows, 0, st>>>(src, set, out);
+  auto kern = src.s32 ? (small ? k_box_tables<unsigned, unsigned> : k_box_tables<unsigned, size_t>)
+                      : (small ? k_box_tables<unsigned long long, unsigned> : k_box_tables<unsigned long long, size_t>);
+  const int most = std::max(65535 / chunks, 1);  // tables a launch: a grid has at most 65535 along z
+  for (int first = 0; first < set.n; first += most) {
+    const int count = std::min(most, set.n - first);
+    const dim3 grid((na + kBoxRow - 1) / kBoxRow, (nb + kBoxRows - 1) / kBoxRows, chunks * count);
+    kern<<<grid, 32 * kBoxRows, 0, st>>>(src, set, first, count, out);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
-  return cudaGetLastError();
+  return cudaSuccess;
+}
+
+bool box_table_builds(const BoxGrid& g) {
+  return (g.nb + kBoxRows - 1) / kBoxRows <= 65535 && (g.nc + kBoxPlanes - 1) / kBoxPlanes <= 65535;
 }
 
 // --------------------------------------------------------------- pyramid

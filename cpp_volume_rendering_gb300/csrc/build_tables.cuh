@@ -47,6 +47,8 @@ struct BoxSource {
   float scale;
   int n[3];  // SAT extents
 };
+// Whether a table of this grid fits the build's launches.
+bool box_table_builds(const BoxGrid& g);
 cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, float* out, cudaStream_t st);
 
 // Builds every level of P (dims/offsets/grid filled by the caller) into data,
