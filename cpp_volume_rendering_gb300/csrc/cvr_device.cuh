@@ -97,7 +97,10 @@ __device__ __forceinline__ float3 primary_dir(const CameraView& c, int px, int p
   float vy = ((float(py) + 0.5f) / float(H)) * 2.0f - 1.0f;
   float a = vx * c.tan_half_fovy * c.aspect;
   float b = vy * c.tan_half_fovy;
-  return normalize3(c.s * a + c.u * b + c.f);
+  // roundings spelled out: several kernels of a frame work out the same ray
+  auto sum = [&](float s, float u, float w) { return __fadd_rn(fmaf(s, a, __fmul_rn(u, b)), w); };
+  const float3 d = f3(sum(c.s.x, c.u.x, c.f.x), sum(c.s.y, c.u.y, c.f.y), sum(c.s.z, c.u.z, c.f.z));
+  return d * rsqrtf(fmaf(d.z, d.z, fmaf(d.x, d.x, __fmul_rn(d.y, d.y))));
 }
 
 // ray_bbox_intersection.comp:18-52 (IntersectBox + RayAABBIntersection):

@@ -86,13 +86,11 @@ __global__ void __launch_bounds__(NT) k_collect(const __grid_constant__ FrameArg
     for (int j = 0; j < kAhead; ++j) {
       bool shaded = false;
       if (live) {
-        float a = tf(st.density[j]);
+        const float a = tf(st.density[j]);
         ++n;
         if (a > 0.0f) {
           shaded = true;
-          a = 1.0f - expf(-a * st.h[j]);
-          const float left = 1.0f - opacity;
-          opacity += left * a;
+          opacity = over(opacity, __fsub_rn(1.0f, opacity), step_opacity(a, st.h[j]));
           if (opacity > 0.99f) live = false;
         }
         s = st.end[j];
@@ -162,10 +160,7 @@ __global__ void __launch_bounds__(NT) k_resolve(const __grid_constant__ FrameArg
         const unsigned i = filled + (unsigned)__popc(m & ((1u << lane) - 1u));
         const float2 l = d.light[chunk[i / kRecChunk] + i % kRecChunk];
         src = ext ? t.apply<true>(f, src, st.at(j), l) : t.apply<false>(f, src, st.at(j), l);
-        src.w = 1.0f - expf(-src.w * st.h[j]);
-        src.x *= src.w; src.y *= src.w; src.z *= src.w;
-        const float left = 1.0f - dst.w;
-        dst.x += left * src.x; dst.y += left * src.y; dst.z += left * src.z; dst.w += left * src.w;
+        composite(dst, src, st.h[j]);
         if (dst.w > 0.99f) live = false;
       }
       filled += (unsigned)__popc(m);

@@ -901,6 +901,22 @@ __device__ __forceinline__ void add_stats(const FrameArgs& f, unsigned int n, un
   }
 }
 
+// One step's opacity, and its colour composited front to back.  Which samples a
+// ray shades and where it ends follow from these and the primary ray alone; the
+// passes of a deferred frame (deferred.cuh) and its methods' direct marchers work
+// them out in different kernels, so every rounding is spelled out.
+__device__ __forceinline__ float step_opacity(float sigma, float h) {
+  return __fsub_rn(1.0f, expf(__fmul_rn(-sigma, h)));
+}
+__device__ __forceinline__ float over(float dst, float left, float src) { return fmaf(left, src, dst); }
+__device__ __forceinline__ void composite(float4& dst, float4 src, float h) {
+  const float a = step_opacity(src.w, h), left = __fsub_rn(1.0f, dst.w);
+  dst.x = over(dst.x, left, __fmul_rn(src.x, a));
+  dst.y = over(dst.y, left, __fmul_rn(src.y, a));
+  dst.z = over(dst.z, left, __fmul_rn(src.z, a));
+  dst.w = over(dst.w, left, a);
+}
+
 // The a5 loop (ray_marching_1p.comp:170-247): h = min(StepSize, D - s),
 // sample at s + h/2, skip transparent samples, alpha = 1 - exp(-sigma h),
 // front-to-back composite, stop once alpha > 0.99.
@@ -929,10 +945,7 @@ __device__ __forceinline__ void march_ray_with(const FrameArgs& f, const S& samp
         if (src.w > 0.0f) {
           ++shaded;
           src = sh.shade(src, p, ray, f, aux);
-          src.w = 1.0f - expf(-src.w * h);
-          src.x *= src.w; src.y *= src.w; src.z *= src.w;
-          float r = 1.0f - dst.w;
-          dst.x += r * src.x; dst.y += r * src.y; dst.z += r * src.z; dst.w += r * src.w;
+          composite(dst, src, h);
           if (dst.w > 0.99f) break;
         }
         s = s + h;
@@ -1131,10 +1144,7 @@ __device__ __forceinline__ void march_refill(const FrameArgs& f, const float4* t
     if (pending) {
       ++shaded;
       src = sh.shade(src, p, ray, f, aux);
-      src.w = 1.0f - expf(-src.w * h);
-      src.x *= src.w; src.y *= src.w; src.z *= src.w;
-      const float r = 1.0f - dst.w;
-      dst.x += r * src.x; dst.y += r * src.y; dst.z += r * src.z; dst.w += r * src.w;
+      composite(dst, src, h);
       s = s + h;
       if (dst.w > 0.99f) finish();
     }

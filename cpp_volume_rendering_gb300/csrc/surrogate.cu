@@ -49,9 +49,7 @@ __global__ void __launch_bounds__(128) k_sur_collect(FrameArgs f, float rate, un
           pts[2 * (size_t)idx + 1] = make_float4(dir.x, dir.y, dir.z, 0.0f);
         }
       }
-      float a = 1.0f - expf(-src.w * h);
-      float r = 1.0f - dw;
-      dw += r * a;
+      dw = over(dw, __fsub_rn(1.0f, dw), step_opacity(src.w, h));
       if (dw > 0.99f) break;
     }
     s = s + h;
@@ -261,10 +259,7 @@ __global__ void __launch_bounds__(128, MINB) k_march_surrogate(const __grid_cons
       ++shaded;
       pending = false;
       src = f.grad.g ? sur_phong(a, f, src, p, y[0], y[1]) : sur_shade(a, src, y[0], y[1]);
-      src.w = 1.0f - expf(-src.w * h);
-      src.x *= src.w; src.y *= src.w; src.z *= src.w;
-      float r = 1.0f - ray.dst.w;
-      ray.dst.x += r * src.x; ray.dst.y += r * src.y; ray.dst.z += r * src.z; ray.dst.w += r * src.w;
+      composite(ray.dst, src, h);
       if (ray.dst.w > 0.99f) {
         sur_finish(f, ray);
         n += ray.n;
