@@ -640,9 +640,13 @@ __global__ void k_pyr_backtotau(float* data, long long n) {
 //    axis and lie in an 8^3 window of voxels, interpolated axis by axis
 //    (k_pyr_base_window); with half as many cells as voxels on every axis (the
 //    reference's 128^3 base of a 256^3 volume) the taps of all cells are one
-//    lattice, whose points are taken once (k_pyr_base_half).
-// Other tap spacings, and windows that shared memory cannot hold, take the
-// direct kernels above.
+//    lattice, whose points are taken once (k_pyr_base_half);
+//  - where cells and taps are whole numbers of texels apart on every axis, a
+//    lattice of any such ratio in memory and a 7-tap pass along each axis
+//    (k_pyr_lattice_base, k_pyr_lattice_level, k_pyr_pass): other bases that
+//    have few lattice points per cell (a base of the volume's own size, taps of
+//    several voxels), and levels whose windows shared memory cannot hold.
+// Everything else takes the direct kernels above.
 struct PyrWeights { float w[7]; };
 
 // The centre of cell i in texels of the input, exact before the one rounding
@@ -821,6 +825,76 @@ __global__ void __launch_bounds__(128, 3) k_pyr_base_window(const T* __restrict_
   out.put(idx, sum);
 }
 
+// ---- lattices: cell i, tap k of a level reads lattice point i m + (k + 3) t, at
+// texel coordinate j0 + q + f.  One pass takes every lattice point once (0
+// outside the box, as in_grid), three more apply the 7 weights of each axis.
+// Bound by the traffic of the points (9 ps each with their passes).
+struct PyrAxis {
+  int m, t;   // texels per cell, per tap step
+  int j0, g;  // lattice start (integer part) and size
+  int n_out;  // cells
+  float f;    // the constant fraction
+};
+struct PyrAxes { PyrAxis a[3]; };
+
+// Lattice point (qx, qy, qz) in texels; whether it lies inside the box: texel
+// coordinates in [-0.5, n - 0.5].
+__device__ __forceinline__ bool pyr_lattice_point(const PyrAxis* A, const int* n_in, int qx, int qy, int qz, float3& u) {
+  u = f3((float)(A[0].j0 + qx) + A[0].f, (float)(A[1].j0 + qy) + A[1].f, (float)(A[2].j0 + qz) + A[2].f);
+  return u.x >= -0.5f && u.y >= -0.5f && u.z >= -0.5f && u.x <= (float)n_in[0] - 0.5f &&
+         u.y <= (float)n_in[1] - 0.5f && u.z <= (float)n_in[2] - 0.5f;
+}
+
+// Grids of (x blocks, y, z): no division of a flat index per point.
+template <class S>
+__global__ void k_pyr_lattice_base(const __grid_constant__ VolumeView vol, const float4* __restrict__ tf_rgba, int tf_n,
+                                   PyrAxes A, float* __restrict__ G) {
+  extern __shared__ float2 sm_alpha[];
+  stage_tf_alpha(tf_rgba, tf_n, sm_alpha);
+  __syncthreads();
+  const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y, qz = blockIdx.z;
+  if (qx >= A.a[0].g) return;
+  const int n_in[3] = {vol.nx, vol.ny, vol.nz};
+  float3 u;
+  const bool inside = pyr_lattice_point(A.a, n_in, qx, qy, qz, u);
+  const float3 p = f3((u.x + 0.5f) * vol.spacing.x, (u.y + 0.5f) * vol.spacing.y, (u.z + 0.5f) * vol.spacing.z);
+  G[((size_t)qz * A.a[1].g + qy) * A.a[0].g + qx] = inside ? TfAlpha{sm_alpha, tf_n}(S(vol)(p)) : 0.0f;
+}
+
+__global__ void k_pyr_lattice_level(PyramidView P, int l_in, PyrAxes A, float* __restrict__ G) {
+  const int qx = blockIdx.x * blockDim.x + threadIdx.x, qy = blockIdx.y, qz = blockIdx.z;
+  if (qx >= A.a[0].g) return;
+  const int* n_in = P.dims[l_in];
+  float3 u;
+  const bool inside = pyr_lattice_point(A.a, n_in, qx, qy, qz, u);
+  const float3 p = f3((u.x + 0.5f) * (P.grid.x / (float)n_in[0]), (u.y + 0.5f) * (P.grid.y / (float)n_in[1]),
+                      (u.z + 0.5f) * (P.grid.z / (float)n_in[2]));
+  G[((size_t)qz * A.a[1].g + qy) * A.a[0].g + qx] = inside ? pyr_sample_level(P, l_in, p) : 0.0f;
+}
+
+// One 7-tap pass along axis ax of an (nx, ny, nz) array: out has n_out cells
+// along that axis, out[i] = sum_k w[k] in[i m + (k + 3) t]; the last pass is
+// the level.
+template <class Out>
+__global__ void k_pyr_pass(const float* __restrict__ in, int nx, int ny, int nz, int ax, PyrAxis a, PyrWeights w,
+                           Out out) {
+  const int ox = ax == 0 ? a.n_out : nx, oy = ax == 1 ? a.n_out : ny;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+  if (x >= ox) return;
+  const size_t idx = ((size_t)z * oy + y) * ox + x;
+  const int i = ax == 0 ? x : (ax == 1 ? y : z);
+  const long long stride = ax == 0 ? 1 : (ax == 1 ? (long long)nx : (long long)nx * ny);
+  const long long base = (ax == 0 ? 0 : x) + (ax == 1 ? 0 : (long long)y * nx) + (ax == 2 ? 0 : (long long)z * nx * ny);
+  float acc = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) acc = fmaf(w.w[k], __ldg(in + base + (long long)(i * a.m + k * a.t) * stride), acc);
+  out.put(idx, acc);
+}
+struct PassOut {
+  float* p;
+  __device__ __forceinline__ void put(size_t i, float v) const { p[i] = v; }
+};
+
 // A level from the one below, all three passes in one CTA of T^3 cells: the
 // window of the input in shared memory, then along each axis a dense dot
 // product per cell, whose weights (7 taps of two texels each, folded to the
@@ -943,6 +1017,106 @@ static size_t pyr_level_plan(const VolumeView& vol, const PyramidView& P, int l,
                           (size_t)tile * (L->a[0].span + L->a[1].span + L->a[2].span));
 }
 
+// The lattice of level l (0: from the volume): false when cells or taps are not
+// whole numbers of texels apart.
+static bool pyr_lattice(const VolumeView& vol, const PyramidView& P, int l, float s0, PyrAxes* L) {
+  const int in[3] = {l == 0 ? vol.nx : P.dims[l - 1][0], l == 0 ? vol.ny : P.dims[l - 1][1],
+                     l == 0 ? vol.nz : P.dims[l - 1][2]};
+  for (int a = 0; a < 3; ++a) {
+    PyrAxis& A = L->a[a];
+    const double step = pyr_tap_step(vol, P, l, s0, a), t = std::nearbyint(step);
+    A.n_out = P.dims[l][a];
+    if (in[a] % A.n_out || !(t >= 1.0 && t < 65536.0) || std::fabs(step - t) > 1e-9 * t) return false;
+    A.m = in[a] / A.n_out;
+    A.t = (int)t;
+    const double c0 = 0.5 * A.m - 0.5;  // texel coordinate of cell 0, tap 0
+    A.f = (float)(c0 - std::floor(c0));
+    A.j0 = (int)std::floor(c0) - 3 * A.t;
+    const long long g = (long long)(A.n_out - 1) * A.m + 6LL * A.t + 1;
+    if (g > 65535) return false;  // a grid dimension of the launches
+    A.g = (int)g;
+  }
+  return true;
+}
+static long long pyr_lattice_points(const PyrAxes& L) { return (long long)L.a[0].g * L.a[1].g * L.a[2].g; }
+// Floats of the lattice and of the first two passes' results.
+static long long pyr_lattice_floats(const PyrAxes& L) {
+  return pyr_lattice_points(L) + (long long)L.a[0].n_out * L.a[1].g * L.a[2].g +
+         (long long)L.a[0].n_out * L.a[1].n_out * L.a[2].g;
+}
+
+// Which form the base takes (see above).  A window costs as much as 55 lattice
+// points a cell (384^3 -> 128^3, 28 points a cell, 1.09 ms; as a lattice 0.61;
+// 128^3 -> 128^3, 1.2 points, 1.09 against 0.17), a direct cell as much as 200
+// (256^3 -> 128^3 with taps of two voxels, 9 points, 3.67 ms against 0.33).
+enum class PyrBase { kHalf, kWindow, kLattice, kDirect };
+static PyrBase pyr_base_form(const VolumeView& plain, const PyramidView& P, float s0, bool lattices, PyrAxes* L) {
+  const int* d = P.dims[0];
+  // a step of one voxel to FP32 accuracy: the taps of a cell share their fractions
+  bool window = (size_t)plain.nx * plain.ny < ((size_t)1 << 31);
+  for (int a = 0; a < 3; ++a) window = window && std::fabs(pyr_tap_step(plain, P, 0, s0, a) - 1.0) <= 1e-6;
+  if (window && plain.nx == 2 * d[0] && plain.ny == 2 * d[1] && plain.nz == 2 * d[2]) return PyrBase::kHalf;
+  if (lattices && pyr_lattice(plain, P, 0, s0, L) &&
+      pyr_lattice_points(*L) <= (window ? 55LL : 200LL) * d[0] * d[1] * d[2])
+    return PyrBase::kLattice;
+  return window ? PyrBase::kWindow : PyrBase::kDirect;
+}
+
+// Cells per edge of level l's tiles.  8^3 cells read 2.6 times their texels,
+// 4^3 cells 5.4 times: the smaller tile where the larger leaves SMs idle
+// (32^3: 21 -> 12 us as 512 CTAs; 64^3 would take 52 instead of 41).
+static int pyr_level_tile(const PyramidView& P, int l) {
+  auto tiles = [&](int a) { return (long long)(P.dims[l][a] + 7) / 8; };
+  return tiles(0) * tiles(1) * tiles(2) < 152 ? 4 : 8;
+}
+// windows of up to 160 KB: taps of up to three texels apart
+constexpr size_t kLevelSmem = 160 * 1024;
+
+// Which form level l >= 1 takes.  Tiles read windows that grow with the cube of
+// the tap step: with steps beyond a texel (2 with a base of the volume's own
+// size) levels from 30^3 cells on are lattices where they can be (the pyramid of
+// 256^3 -> 256^3: 751 us, 1298 with tiles; 128^3 178 against 218, 100 x 90 x 80
+// 118 against 136; levels of 32^3 and below the same).
+constexpr long long kLatticeLevel = 27000;
+enum class PyrLevel { kTile, kLattice, kDirect };
+static PyrLevel pyr_level_form(const VolumeView& vol, const PyramidView& P, int l, float s0, bool lattices, int* tile,
+                               size_t* smem, LevelAxes* L, PyrAxes* A) {
+  *tile = pyr_level_tile(P, l);
+  *smem = pyr_level_plan(vol, P, l, s0, *tile, L);
+  const int* d = P.dims[l];
+  const bool fits = *smem > 0 && *smem <= kLevelSmem;
+  const bool wide = std::max(L->a[0].t, std::max(L->a[1].t, L->a[2].t)) > 1.5f &&
+                    (long long)d[0] * d[1] * d[2] >= kLatticeLevel;
+  if (fits && !wide) return PyrLevel::kTile;
+  if (lattices && pyr_lattice(vol, P, l, s0, A)) return PyrLevel::kLattice;
+  return fits ? PyrLevel::kTile : PyrLevel::kDirect;
+}
+
+long long pyramid_lattice_floats(const VolumeView& plain, const PyramidView& P, float s0) {
+  PyrAxes A;
+  long long need = pyr_base_form(plain, P, s0, true, &A) == PyrBase::kLattice ? pyr_lattice_floats(A) : 0;
+  for (int l = 1; l < P.n_levels; ++l) {
+    LevelAxes L;
+    int tile;
+    size_t sm;
+    if (pyr_level_form(plain, P, l, s0, true, &tile, &sm, &L, &A) == PyrLevel::kLattice)
+      need = std::max(need, pyr_lattice_floats(A));
+  }
+  return need;
+}
+
+// The three passes of a lattice G (followed by room for two of their results).
+static cudaError_t launch_pyr_passes(const PyrAxes& L, float* G, const PyrWeights& w, const PyrOut& out, cudaStream_t st) {
+  const PyrAxis* A = L.a;
+  float* T1 = G + pyr_lattice_points(L);
+  float* T2 = T1 + (long long)A[0].n_out * A[1].g * A[2].g;
+  const unsigned bx = (unsigned)(A[0].n_out + 127) / 128;  // every pass's output has n_out along x
+  k_pyr_pass<<<dim3(bx, A[1].g, A[2].g), 128, 0, st>>>(G, A[0].g, A[1].g, A[2].g, 0, A[0], w, PassOut{T1});
+  k_pyr_pass<<<dim3(bx, A[1].n_out, A[2].g), 128, 0, st>>>(T1, A[0].n_out, A[1].g, A[2].g, 1, A[1], w, PassOut{T2});
+  k_pyr_pass<<<dim3(bx, A[1].n_out, A[2].n_out), 128, 0, st>>>(T2, A[0].n_out, A[1].n_out, A[2].g, 2, A[2], w, out);
+  return cudaGetLastError();
+}
+
 template <class T>
 static cudaError_t launch_pyr_base(const VolumeView& v, const float4* tf_rgba, int tf_n, const int* d, bool half,
                                    const PyrWeights& w, const PyrOut& out, cudaStream_t st) {
@@ -967,7 +1141,8 @@ static cudaError_t launch_pyr_base(const VolumeView& v, const float4* tf_rgba, i
 }
 
 cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain, const float4* tf_rgba, int tf_n,
-                                 float s0, PyramidView& P, float* data, float* opacity, cudaStream_t st) {
+                                 float s0, PyramidView& P, float* data, float* opacity, float* lattice,
+                                 cudaStream_t st) {
   const int threads = 128;
   const int* d0 = P.dims[0];
   float* op = opacity ? opacity : data;
@@ -977,14 +1152,24 @@ cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain,
   for (int k = -3; k <= 3; ++k) sum += std::exp(-0.5 * k * k);
   for (int k = -3; k <= 3; ++k) w.w[k + 3] = (float)(std::exp(-0.5 * k * k) / sum);
 
-  // a step of one voxel to FP32 accuracy: the taps of a cell share their fractions
-  bool window = (size_t)plain.nx * plain.ny < ((size_t)1 << 31);
-  for (int a = 0; a < 3; ++a) window = window && std::fabs(pyr_tap_step(plain, P, 0, s0, a) - 1.0) <= 1e-6;
   cudaError_t e = cudaSuccess;
-  if (window) {
-    const bool half = plain.nx == 2 * d0[0] && plain.ny == 2 * d0[1] && plain.nz == 2 * d0[2];
+  PyrAxes A;
+  const PyrBase form = pyr_base_form(plain, P, s0, lattice != nullptr, &A);
+  if (form == PyrBase::kHalf || form == PyrBase::kWindow) {
+    const bool half = form == PyrBase::kHalf;
     e = plain.dtype == 1 ? launch_pyr_base<uint8_t>(plain, tf_rgba, tf_n, d0, half, w, out(0), st)
                          : launch_pyr_base<uint16_t>(plain, tf_rgba, tf_n, d0, half, w, out(0), st);
+  } else if (form == PyrBase::kLattice) {
+    const size_t sm = sizeof(float2) * ((size_t)tf_n + 1);
+    e = with_sampler(vol, [&](auto* smp) {
+      auto kern = k_pyr_lattice_base<std::remove_pointer_t<decltype(smp)>>;
+      cudaError_t err = cudaSuccess;
+      if (sm > 48 * 1024) err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+      if (err != cudaSuccess) return err;
+      kern<<<dim3((A.a[0].g + 127) / 128, A.a[1].g, A.a[2].g), 128, sm, st>>>(vol, tf_rgba, tf_n, A, lattice);
+      return cudaGetLastError();
+    });
+    if (e == cudaSuccess) e = launch_pyr_passes(A, lattice, w, out(0), st);
   } else {
     const size_t sm = sizeof(float4) * tf_n;
     if (sm > 48 * 1024) e = cudaFuncSetAttribute(k_pyr_base, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -996,8 +1181,6 @@ cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain,
   }
   if (e != cudaSuccess) return e;
   P.data = op;
-  // windows of up to 160 KB: taps of up to three texels apart
-  constexpr size_t kLevelSmem = 160 * 1024;
   e = cudaFuncSetAttribute(k_pyr_level_tile<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_pyr_level_tile<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmem);
@@ -1005,17 +1188,17 @@ cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain,
   for (int l = 1; l < P.n_levels; ++l) {
     LevelAxes L;
     const int* d = P.dims[l];
-    // 8^3 cells read 2.6 times their texels, 4^3 cells 5.4 times: the smaller
-    // tile where the larger leaves SMs idle (32^3: 21 -> 12 us
-    // as 512 CTAs; 64^3 would take 52 instead of 41)
-    auto tiles = [&](int t) { return dim3((d[0] + t - 1) / t, (d[1] + t - 1) / t, (d[2] + t - 1) / t); };
-    const dim3 g8 = tiles(8);
-    const int tile = (long long)g8.x * g8.y * g8.z < 152 ? 4 : 8;
-    const size_t sm = pyr_level_plan(vol, P, l, s0, tile, &L);
-    if (sm > 0 && sm <= kLevelSmem) {
+    int tile;
+    size_t sm;
+    const PyrLevel form = pyr_level_form(plain, P, l, s0, lattice != nullptr, &tile, &sm, &L, &A);
+    if (form == PyrLevel::kTile) {
       const float* below = op + P.offset[l - 1];
-      if (tile == 8) k_pyr_level_tile<8><<<g8, 512, sm, st>>>(below, L, w, out(l));
-      else k_pyr_level_tile<4><<<tiles(4), 256, sm, st>>>(below, L, w, out(l));
+      const dim3 grid((d[0] + tile - 1) / tile, (d[1] + tile - 1) / tile, (d[2] + tile - 1) / tile);
+      if (tile == 8) k_pyr_level_tile<8><<<grid, 512, sm, st>>>(below, L, w, out(l));
+      else k_pyr_level_tile<4><<<grid, 256, sm, st>>>(below, L, w, out(l));
+    } else if (form == PyrLevel::kLattice) {
+      k_pyr_lattice_level<<<dim3((A.a[0].g + 127) / 128, A.a[1].g, A.a[2].g), 128, 0, st>>>(P, l - 1, A, lattice);
+      if ((e = launch_pyr_passes(A, lattice, w, out(l), st)) != cudaSuccess) return e;
     } else {
       const long long nl = (long long)d[0] * d[1] * d[2];
       const float si = s0 * powf(2.0f, float(l));

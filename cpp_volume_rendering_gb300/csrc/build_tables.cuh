@@ -54,9 +54,13 @@ cudaError_t launch_box_tables(const BoxSource& src, const BoxTableSet& set, floa
 // Builds every level of P (dims/offsets/grid filled by the caller) into data,
 // their opacities into opacity (as many floats; nullptr: none to spare, and the
 // extinctions are converted in place at the end).  vol: the marchers' storage
-// of the volume, plain: the x-fastest array.
+// of the volume, plain: the x-fastest array.  lattice: room for
+// pyramid_lattice_floats, or nullptr (the levels that would use it take slower
+// forms).
 cudaError_t launch_pyramid_build(const VolumeView& vol, const VolumeView& plain, const float4* tf_rgba, int tf_n,
-                                 float s0, PyramidView& P, float* data, float* opacity, cudaStream_t st);
+                                 float s0, PyramidView& P, float* data, float* opacity, float* lattice,
+                                 cudaStream_t st);
+long long pyramid_lattice_floats(const VolumeView& plain, const PyramidView& P, float s0);
 
 // Grid-stride fill of a device buffer (used to flush L2 between timed frames).
 cudaError_t launch_fill(void* p, size_t bytes, unsigned int v, cudaStream_t st);

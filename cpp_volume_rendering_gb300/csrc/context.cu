@@ -858,14 +858,24 @@ cvr_status cvr_build_ext_pyramid(cvr_ctx* c, const cvr_pyramid_params* p) {
   P.grid = v.grid;
   P.inv_grid = f3(1.0f / v.grid.x, 1.0f / v.grid.y, 1.0f / v.grid.z);
   CK(c, ensure(c->d_pyr, c->pyr_cap, (size_t)off * sizeof(float)));
-  // the opacities that levels are built from, beside the extinctions; without
-  // room for them the levels are built in place and converted at the end
-  float* opacity = nullptr;
-  cudaError_t e = ensure(c->d_pyrs, c->pyrs_cap, (size_t)off * sizeof(float));
-  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
-  else if (e != cudaSuccess) return cuda_fail(c, e, "pyramid scratch");
-  else opacity = c->d_pyrs;
-  CK(c, launch_pyramid_build(v, volume_view(c), c->d_rgba, c->tf_n, p->sigma0, P, c->d_pyr, opacity, c->stream));
+  // the opacities that levels are built from, beside the extinctions, and the
+  // lattice that some of them take; without room for both the levels take other
+  // forms, without any they are built in place and converted at the end
+  const VolumeView plain = volume_view(c);
+  const size_t beside = ((size_t)off + 3) / 4 * 4, points = (size_t)pyramid_lattice_floats(plain, P, p->sigma0);
+  float *opacity = nullptr, *lattice = nullptr;
+  for (const size_t floats : {beside + points, beside}) {
+    const cudaError_t e = ensure(c->d_pyrs, c->pyrs_cap, floats * sizeof(float));
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      continue;
+    }
+    if (e != cudaSuccess) return cuda_fail(c, e, "pyramid scratch");
+    opacity = c->d_pyrs;
+    if (points > 0 && floats > beside) lattice = opacity + beside;
+    break;
+  }
+  CK(c, launch_pyramid_build(v, plain, c->d_rgba, c->tf_n, p->sigma0, P, c->d_pyr, opacity, lattice, c->stream));
   c->pyr = P;
   c->pyr_ready = true;
   c->pyrq_ready = false;
