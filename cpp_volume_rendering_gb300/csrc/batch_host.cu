@@ -128,7 +128,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     if (jobs[x].method != jobs[y].method) return jobs[x].method < jobs[y].method;
     return job_walk_axis(jobs[x]) < job_walk_axis(jobs[y]);
   });
-  CK(c, cudaMalloc((void**)&b->d_stats, sizeof(unsigned long long) * 3 * n_jobs));
+  NEED(c, cudaMalloc((void**)&b->d_stats, sizeof(unsigned long long) * 3 * n_jobs));
   std::vector<BatchExtJob> ext;
   std::vector<int> ext_slot;
   double slot_vmax[CVR_MAX_VOLUMES] = {};
@@ -203,7 +203,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       const size_t cells = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
       if (cells >= kCompactMaxCells) { all_compact = false; break; }
       uint4* d = nullptr;
-      cudaError_t e = cudaMalloc((void**)&d, cells * sizeof(uint4));
+      cudaError_t e = need(c, [&] { return cudaMalloc((void**)&d, cells * sizeof(uint4)); });
       if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); all_compact = false; break; }  // int64 tables
       if (e != cudaSuccess) { st = cuda_fail(c, e, "cvr_batch_create: compact SAT"); break; }
       b->sat32.push_back(d);
@@ -283,7 +283,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
         if (!d) {
           select_slot(c, slot);
           const int sx = c->nx + 2, sy = c->ny + 2, sz = c->nz + 2;
-          cudaError_t e = cudaMalloc((void**)&d, (size_t)sx * sy * sz * 2 * sizeof(uint4));
+          cudaError_t e = need(c, [&] { return cudaMalloc((void**)&d, (size_t)sx * sy * sz * 2 * sizeof(uint4)); });
           if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); continue; }  // this job reads the quads
           if (e != cudaSuccess) { st = cuda_fail(c, e, "cvr_batch_create: walk table"); break; }
           b->walks.push_back(d);
@@ -332,11 +332,11 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       (group ? b->box_blocks : b->ext_blocks) = blocks;
     }
     if (!table_dev.empty()) {
-      CK(c, cudaMalloc((void**)&b->d_tables, sizeof(float4) * table_dev.size()));
+      NEED(c, cudaMalloc((void**)&b->d_tables, sizeof(float4) * table_dev.size()));
       CK(c, cudaMemcpy(b->d_tables, table_dev.data(), sizeof(float4) * table_dev.size(), cudaMemcpyHostToDevice));
     }
     if (!cuts.empty()) {
-      CK(c, cudaMalloc((void**)&b->d_cuts, sizeof(float) * cuts.size()));
+      NEED(c, cudaMalloc((void**)&b->d_cuts, sizeof(float) * cuts.size()));
       CK(c, cudaMemcpy(b->d_cuts, cuts.data(), sizeof(float) * cuts.size(), cudaMemcpyHostToDevice));
     }
     for (size_t k = 0; k < jobs_dev.size(); ++k) {
@@ -352,7 +352,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
         J.ttx = next - table_at[k] == 3 * (size_t)J.tn ? base + 2 * J.tn : nullptr;
       }
     }
-    CK(c, cudaMalloc((void**)&b->d_ext, sizeof(BatchExtJob) * jobs_dev.size()));
+    NEED(c, cudaMalloc((void**)&b->d_ext, sizeof(BatchExtJob) * jobs_dev.size()));
     CK(c, cudaMemcpy(b->d_ext, jobs_dev.data(), sizeof(BatchExtJob) * jobs_dev.size(), cudaMemcpyHostToDevice));
     // the compact SATs were the box tables' source: they go when no job reads them
     if (b->n_ext == 0) {
@@ -362,7 +362,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     }
   }
   const size_t n_counters = 2 + sur.size();
-  CK(c, cudaMalloc((void**)&b->d_counters, sizeof(unsigned int) * n_counters));
+  NEED(c, cudaMalloc((void**)&b->d_counters, sizeof(unsigned int) * n_counters));
   // the lanes' lists, each as large as its largest job needs (a lane without
   // room leaves its jobs to the direct marcher)
   const int lanes = (int)std::min<size_t>(sur.size(), kSurLanes);
@@ -370,7 +370,8 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     size_t bytes = 0;
     for (size_t k = l; k < sur.size(); k += lanes) bytes = std::max(bytes, sur[k].bytes);
     if (bytes == 0) continue;
-    const cudaError_t me = cudaMalloc(&b->lists[l], bytes);
+    cudaError_t me = spare_room(bytes, 0);
+    if (me == cudaSuccess) me = cudaMalloc(&b->lists[l], bytes);
     if (me == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       for (size_t k = l; k < sur.size(); k += lanes) sur[k].bytes = 0;

@@ -176,20 +176,10 @@ bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const Shadow
 cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned long long gen, const BoxPlan& P,
                      ExtArgs* e, bool* used) {
   *used = false;
-  auto grow = [&](BoxPool& pool, size_t bytes) -> cudaError_t {
-    if (pool.cap >= bytes && pool.data) return cudaSuccess;
-    pool.release();
-    // at most half of what is free: the rest stays for the caller's buffers
-    size_t free_b = 0, total_b = 0;
-    cudaError_t err = cudaMemGetInfo(&free_b, &total_b);
-    if (err != cudaSuccess) return err;
-    if (bytes > free_b / 2) return cudaErrorMemoryAllocation;
-    return ensure(pool.data, pool.cap, bytes);
-  };
   auto build = [&](BoxPool& pool, bool fresh, size_t bytes, const BoxTableSet& set) -> cudaError_t {
     if (fresh) {
       pool.gen = 0;
-      cudaError_t err = grow(pool, bytes);
+      cudaError_t err = ensure_spare(pool.data, pool.cap, bytes);
       if (err != cudaSuccess) return err;
     }
     return launch_box_tables(src, set, pool.data, c->stream);

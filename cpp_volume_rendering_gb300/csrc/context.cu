@@ -151,7 +151,10 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, doubl
     v.qrow = (unsigned)qrow;
     v.qplane = (unsigned)qplane;
     if (c->vbrick_bs != kQuadCopy) {
-      cudaError_t qe = copy_room(c, qplane * c->nz * qbytes);
+      const size_t bytes = qplane * c->nz * qbytes;
+      cudaError_t qe = c->quads ? need(c, [&] { return copy_room(c, bytes); })
+                                : spare_room(bytes, c->vcopy && c->vcopy.use_count() == 1 ? c->vcopy->cap : 0);
+      if (qe == cudaSuccess && !c->quads) qe = copy_room(c, bytes);
       if (qe == cudaErrorMemoryAllocation && !c->quads) {  // not asked for: the plain array serves
         cudaGetLastError();
         c->quad_seen = -HUGE_VAL;  // nor tried again for this volume
@@ -167,7 +170,7 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, doubl
   } else if (c->brick_bs > 0) {
     if (c->vbrick_bs != c->brick_bs) {
       const long long n = brick_elements(c->nx, c->ny, c->nz, c->brick_bs);
-      CK(c, copy_room(c, (size_t)n * (c->dtype == CVR_U8 ? 1 : 2)));
+      NEED(c, copy_room(c, (size_t)n * (c->dtype == CVR_U8 ? 1 : 2)));
       CK(c, launch_brick_volume(c->d_vol, c->vcopy->data, c->dtype, c->nx, c->ny, c->nz, c->brick_bs, c->stream));
       c->vbrick_bs = c->brick_bs;
     }
@@ -241,7 +244,7 @@ static cvr_status frame_boxes(cvr_ctx* c, double vmax, const FrameArgs& f, const
   if (plan.missing > 0 && compact) {
     if (c->boxsrc_gen != gen) {
       c->boxsrc_gen = 0;
-      cudaError_t e = ensure(c->d_boxsrc, c->boxsrc_cap, cells * sizeof(unsigned));
+      cudaError_t e = ensure_spare(c->d_boxsrc, c->boxsrc_cap, cells * sizeof(unsigned));
       if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         return CVR_OK;
@@ -423,7 +426,7 @@ cvr_status ensure_walk_table(cvr_ctx* c, int axis, int w, WalkView* out) {
     const int sx = c->nx + 2, sy = c->ny + 2, sz = c->nz + 2;
     const size_t cells = (size_t)sx * sy * sz;
     c->walk_gen = 0;
-    cudaError_t e = ensure(c->d_walk, c->walk_cap, cells * 2 * sizeof(uint4));
+    cudaError_t e = need(c, [&] { return ensure(c->d_walk, c->walk_cap, cells * 2 * sizeof(uint4)); });
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       return CVR_OK;
@@ -484,7 +487,7 @@ bool compact_fixed_point(cvr_ctx* c, double vmax, int* F) {
 // Uploads a fixed-point table through the pinned staging region 1 (q may go
 // when the call returns).
 static cvr_status upload_lut32(cvr_ctx* c, const std::vector<unsigned>& q) {
-  CK(c, ensure(c->d_lut32, c->lut32_cap, sizeof(unsigned) * q.size()));
+  CK(c, ensure(c->d_lut32, c->lut32_cap, sizeof(unsigned) * q.size()));  // no give_back: a box source is being made
   void* stage = nullptr;
   cvr_status st = stage_region(c, 1, &stage);
   if (st != CVR_OK) return st;
@@ -501,7 +504,7 @@ cvr_status build_compact_sat(cvr_ctx* c, const std::vector<unsigned>& q, uint4* 
   const size_t cells = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
   cvr_status st = upload_lut32(c, q);
   if (st != CVR_OK) return st;
-  CK(c, ensure(c->d_satp, c->satp_cap, sizeof(unsigned) * cells));
+  NEED(c, ensure(c->d_satp, c->satp_cap, sizeof(unsigned) * cells));
   cudaError_t e = launch_sat_build_quads(c->d_vol, c->dtype, c->nx, c->ny, c->nz, c->d_lut32, c->d_satp, dst,
                                          c->stream);
   if (e != cudaSuccess) return cuda_fail(c, e, "compact SAT build");
@@ -527,7 +530,7 @@ cvr_status ensure_compact_sat(cvr_ctx* c, double vmax, float* inv_scale) {
     c->sat32_F = kNoCompactSat;
     // the quad table is twice the int64 one: without room for it the frame
     // keeps the int64 table
-    cudaError_t e = ensure(c->d_sat32, c->sat32_cap, cells * sizeof(uint4));
+    cudaError_t e = need(c, [&] { return ensure(c->d_sat32, c->sat32_cap, cells * sizeof(uint4)); });
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       return CVR_OK;
@@ -564,7 +567,8 @@ cvr_status pyramid_view(cvr_ctx* c, PyramidView* out) {
   }
   if (!c->pyrq_ready) {
     // without room for the copy the taps read the plain levels
-    cudaError_t e = ensure(c->d_pyrq, c->pyrq_cap, n * sizeof(float4));
+    cudaError_t e = c->quads ? need(c, [&] { return ensure(c->d_pyrq, c->pyrq_cap, n * sizeof(float4)); })
+                             : ensure_spare(c->d_pyrq, c->pyrq_cap, n * sizeof(float4));
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       *out = P;
@@ -607,11 +611,25 @@ cvr_status stage_upload(cvr_ctx* c, int r, void* dev, size_t n) {
   return CVR_OK;
 }
 
+bool give_back(cvr_ctx* c) {
+  if (!c->box.ao.data && !c->box.sdw.data && !c->d_boxsrc && !c->d_defer) return false;
+  cudaStreamSynchronize(c->stream);  // launches that read them
+  c->box.ao.release();
+  c->box.sdw.release();
+  if (c->d_boxsrc) cudaFree(c->d_boxsrc);
+  if (c->d_defer) cudaFree(c->d_defer);
+  c->d_boxsrc = nullptr;
+  c->d_defer = nullptr;
+  c->boxsrc_cap = c->defer_cap = 0;
+  c->boxsrc_gen = 0;
+  return true;
+}
+
 cvr_status ensure_sat(cvr_ctx* c) {
   if (!c->sat_ready || !c->sat_pending) return CVR_OK;
   CK(c, cudaSetDevice(c->device));
   size_t cells = (size_t)(c->nx + 2) * (c->ny + 2) * (c->nz + 2);
-  CK(c, ensure(c->d_sat, c->sat_cap, cells * sizeof(long long)));
+  NEED(c, ensure(c->d_sat, c->sat_cap, cells * sizeof(long long)));
   CK(c, launch_sat_build(c->d_vol, c->dtype, c->nx, c->ny, c->nz, c->d_lut, c->d_sat, c->stream));
   c->sat_pending = false;
   return CVR_OK;
@@ -695,7 +713,7 @@ static cvr_status set_volume_common(cvr_ctx* c, const void* src, bool src_device
   if ((long long)w * h * d > (1ll << 34)) return fail(c, CVR_ERR_INVALID_ARG, "cvr_set_volume: volume too large");
   CK(c, cudaSetDevice(c->device));
   size_t bytes = (size_t)w * h * d * (dtype == CVR_U8 ? 1 : 2);
-  CK(c, ensure(c->d_vol, c->vol_cap, bytes));
+  NEED(c, ensure(c->d_vol, c->vol_cap, bytes));
   if (c->nx != w || c->ny != h || c->nz != d) {  // the pools of another size go back
     c->box.ao.release();
     c->box.sdw.release();
@@ -743,8 +761,8 @@ cvr_status cvr_set_transfer_function(cvr_ctx* c, const float* rgbt, const float*
     if (c->d_rgba) cudaFree(c->d_rgba);
     c->d_rgbt = c->d_rgba = nullptr;
     c->tf_cap = 0;
-    CK(c, cudaMalloc((void**)&c->d_rgbt, sizeof(float4) * n));
-    CK(c, cudaMalloc((void**)&c->d_rgba, sizeof(float4) * n));
+    NEED(c, cudaMalloc((void**)&c->d_rgbt, sizeof(float4) * n));
+    NEED(c, cudaMalloc((void**)&c->d_rgba, sizeof(float4) * n));
     c->tf_cap = n;
   }
   CK(c, cudaMemcpyAsync(c->d_rgbt, rgbt, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
@@ -760,8 +778,7 @@ cvr_status cvr_set_transfer_function(cvr_ctx* c, const float* rgbt, const float*
 cvr_status cvr_build_sat(cvr_ctx* c, const double* ext, int n_values) {
   if (!c || !ext) return fail(c, CVR_ERR_INVALID_ARG, "cvr_build_sat: bad arguments");
   if (!c->has_volume) return fail(c, CVR_ERR_NO_VOLUME, "cvr_build_sat: no volume");
-  int need = c->dtype == CVR_U8 ? 256 : 65536;
-  if (n_values != need) return fail(c, CVR_ERR_INVALID_ARG, "cvr_build_sat: n_values must be 256 (u8) or 65536 (u16)");
+  if (n_values != (c->dtype == CVR_U8 ? 256 : 65536)) return fail(c, CVR_ERR_INVALID_ARG, "cvr_build_sat: n_values must be 256 (u8) or 65536 (u16)");
   double maxv = 0.0;
   for (int i = 0; i < n_values; ++i) {
     if (!(ext[i] >= 0.0) || !std::isfinite(ext[i]))
@@ -787,7 +804,7 @@ cvr_status cvr_build_sat(cvr_ctx* c, const double* ext, int n_values) {
     q[i] = v < 4503599627370496.0 ? (long long)(v + 0.5) : (long long)v;
   }
   // the table of every possible voxel value (65536 entries covers u8 and u16)
-  if (!c->d_lut) CK(c, cudaMalloc((void**)&c->d_lut, sizeof(long long) * 65536));
+  if (!c->d_lut) NEED(c, cudaMalloc((void**)&c->d_lut, sizeof(long long) * 65536));
   st = stage_upload(c, 0, c->d_lut, sizeof(long long) * n_values);
   if (st != CVR_OK) return st;
   c->sat_frac_bits = F;
@@ -857,7 +874,7 @@ cvr_status cvr_build_ext_pyramid(cvr_ctx* c, const cvr_pyramid_params* p) {
   if (vs != CVR_OK) return vs;
   P.grid = v.grid;
   P.inv_grid = f3(1.0f / v.grid.x, 1.0f / v.grid.y, 1.0f / v.grid.z);
-  CK(c, ensure(c->d_pyr, c->pyr_cap, (size_t)off * sizeof(float)));
+  NEED(c, ensure(c->d_pyr, c->pyr_cap, (size_t)off * sizeof(float)));
   // the opacities that levels are built from, beside the extinctions, and the
   // lattice that some of them take; without room for both the levels take other
   // forms, without any they are built in place and converted at the end
@@ -865,7 +882,7 @@ cvr_status cvr_build_ext_pyramid(cvr_ctx* c, const cvr_pyramid_params* p) {
   const size_t beside = ((size_t)off + 3) / 4 * 4, points = (size_t)pyramid_lattice_floats(plain, P, p->sigma0);
   float *opacity = nullptr, *lattice = nullptr;
   for (const size_t floats : {beside + points, beside}) {
-    const cudaError_t e = ensure(c->d_pyrs, c->pyrs_cap, floats * sizeof(float));
+    const cudaError_t e = need(c, [&] { return ensure(c->d_pyrs, c->pyrs_cap, floats * sizeof(float)); });
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       continue;
@@ -912,7 +929,7 @@ static cvr_status upload_cone(cvr_ctx* c, const cvr_cone_table* t, float4** d, C
     return fail(c, CVR_ERR_INVALID_ARG, "cone table: integration counts exceed the section count");
   if (*d) { cudaFree(*d); *d = nullptr; }
   size_t bytes = sizeof(float4) * std::max(1, t->n_sections);
-  CK(c, cudaMalloc((void**)d, bytes));
+  NEED(c, cudaMalloc((void**)d, bytes));
   if (t->n_sections) CK(c, cudaMemcpy(*d, t->sections, sizeof(float4) * t->n_sections, cudaMemcpyHostToDevice));
   host->resize(t->n_sections);
   std::memcpy(host->data(), t->sections, sizeof(float4) * t->n_sections);
@@ -943,8 +960,8 @@ cvr_status cvr_set_gt_kernels(cvr_ctx* c, const float* occ, int n_occ, const flo
   CK(c, cudaSetDevice(c->device));
   if (c->d_occ_vec) { cudaFree(c->d_occ_vec); c->d_occ_vec = nullptr; }
   if (c->d_sdw_vec) { cudaFree(c->d_sdw_vec); c->d_sdw_vec = nullptr; }
-  CK(c, cudaMalloc((void**)&c->d_occ_vec, sizeof(float3) * std::max(1, n_occ)));
-  CK(c, cudaMalloc((void**)&c->d_sdw_vec, sizeof(float3) * std::max(1, n_sdw)));
+  NEED(c, cudaMalloc((void**)&c->d_occ_vec, sizeof(float3) * std::max(1, n_occ)));
+  NEED(c, cudaMalloc((void**)&c->d_sdw_vec, sizeof(float3) * std::max(1, n_sdw)));
   if (n_occ) CK(c, cudaMemcpy(c->d_occ_vec, occ, sizeof(float3) * n_occ, cudaMemcpyHostToDevice));
   if (n_sdw) CK(c, cudaMemcpy(c->d_sdw_vec, sdw, sizeof(float3) * n_sdw, cudaMemcpyHostToDevice));
   c->n_occ = n_occ;
@@ -972,9 +989,9 @@ static cvr_status render_impl(cvr_ctx* c, int method, const cvr_camera* cam, con
   if (gw < 1 || gh < 1 || gw > 32768 || gh > 32768)
     return fail(c, CVR_ERR_INVALID_ARG, "cvr_render: multiscaled frame size out of range");
   CK(c, cudaSetDevice(c->device));
-  CK(c, ensure(c->d_ms, c->ms_cap, (size_t)gw * gh * sizeof(float4)));
+  NEED(c, ensure(c->d_ms, c->ms_cap, (size_t)gw * gh * sizeof(float4)));
   if (const size_t sb = multiscale_scratch(c->ms_mode, c->ms_kernel, gw, gh, w, h))
-    CK(c, ensure(c->d_msf, c->msf_cap, sb));
+    NEED(c, ensure(c->d_msf, c->msf_cap, sb));
   // the camera keeps the output's aspect (u_CameraAspectRatio is the screen's)
   cvr_camera cm = cam ? *cam : cvr_camera{};
   if (cam && !(cm.aspect > 0.0f)) cm.aspect = (float)w / (float)h;
@@ -1022,7 +1039,7 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
     f.step = step;
     DeferredPlan plan;
     if (const size_t bytes = deferred_bytes(f, &plan)) {
-      e = ensure(c->d_defer, c->defer_cap, bytes);
+      e = ensure_spare(c->d_defer, c->defer_cap, bytes);
       if (e == cudaErrorMemoryAllocation) {  // the direct marcher needs none
         cudaGetLastError();
         e = cudaSuccess;
@@ -1059,7 +1076,7 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       if (cached) {  // object-space light cache, then the object-space marcher
         if (!c->sdw_table) c->sdw_table.reset(new ShadowBoxTable());
         const size_t cells = (size_t)c->lc_dims[0] * c->lc_dims[1] * c->lc_dims[2];
-        CK(c, ensure(c->d_lcache, c->lcache_cap, cells * sizeof(float2)));
+        NEED(c, ensure(c->d_lcache, c->lcache_cap, cells * sizeof(float2)));
         e = launch_cache_extinction(f, a, table, *c->sdw_table, c->lc_dims, c->d_lcache, c->stream);
         if (e == cudaSuccess)
           e = launch_march_cached(f, c->d_lcache, c->lc_dims, p->apply_occlusion, p->apply_shadow, p->ka, p->kd,
@@ -1101,7 +1118,7 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       a.ka = p->ka; a.kd = p->kd;
       if (c->lc_dims[0] > 0) {  // object-space light cache, then the object-space marcher
         const size_t cells = (size_t)c->lc_dims[0] * c->lc_dims[1] * c->lc_dims[2];
-        CK(c, ensure(c->d_lcache, c->lcache_cap, cells * sizeof(float2)));
+        NEED(c, ensure(c->d_lcache, c->lcache_cap, cells * sizeof(float2)));
         e = launch_cache_dos(f, a, c->lc_dims, c->d_lcache, c->stream);
         if (e == cudaSuccess)
           e = launch_march_cached(f, c->d_lcache, c->lc_dims, p->apply_occlusion, p->apply_shadow, p->ka, p->kd,
@@ -1196,7 +1213,7 @@ cvr_status cvr_render_host(cvr_ctx* c, int method, const cvr_camera* cam, const 
   if (!c || !out_host || w <= 0 || h <= 0) return fail(c, CVR_ERR_INVALID_ARG, "cvr_render_host: bad arguments");
   CK(c, cudaSetDevice(c->device));
   size_t bytes = (size_t)w * h * sizeof(float4);
-  CK(c, ensure(c->d_out, c->out_cap, bytes));
+  NEED(c, ensure(c->d_out, c->out_cap, bytes));
   cvr_status s = render_impl(c, method, cam, light, params, params_size, reinterpret_cast<float*>(c->d_out), w, h,
                              nullptr, stats);
   if (s != CVR_OK) return s;
@@ -1494,7 +1511,7 @@ cvr_status cvr_get_frame_buffer(cvr_ctx* c, int w, int h, float** dev_out) {
   if (!c || !dev_out || w <= 0 || h <= 0 || w > 32768 || h > 32768)
     return fail(c, CVR_ERR_INVALID_ARG, "cvr_get_frame_buffer: bad arguments");
   CK(c, cudaSetDevice(c->device));
-  CK(c, ensure(c->d_out, c->out_cap, (size_t)w * h * sizeof(float4)));
+  NEED(c, ensure(c->d_out, c->out_cap, (size_t)w * h * sizeof(float4)));
   *dev_out = reinterpret_cast<float*>(c->d_out);
   return CVR_OK;
 }
@@ -1528,7 +1545,7 @@ cvr_status cvr_flush_l2(cvr_ctx* c) {
     int l2 = 0;
     CK(c, cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->device));
     size_t bytes = std::max<size_t>((size_t)l2 * 2, 256u << 20);
-    CK(c, cudaMalloc(&c->d_flush, bytes));
+    NEED(c, cudaMalloc(&c->d_flush, bytes));
     c->flush_bytes = bytes;
   }
   CK(c, launch_fill(c->d_flush, c->flush_bytes, 0x5a5a5a5au, c->stream));

@@ -430,6 +430,38 @@ cudaError_t ensure(T*& p, size_t& cap, size_t bytes) {
   return e;
 }
 
+// Buffers that only make frames faster (box tables and their source, sample
+// lists, copies nobody asked for) leave half of what is free to the rest of the
+// program: cudaErrorMemoryAllocation, with p as it was, when they would not.
+// Small ones take what there is: asking costs 28 us, as much as a small frame.
+inline cudaError_t spare_room(size_t bytes, size_t held) {
+  if (bytes <= (size_t)64 << 20) return cudaSuccess;
+  size_t free_b = 0, total_b = 0;
+  const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+  if (e != cudaSuccess) return e;
+  return bytes > (free_b + held) / 2 ? cudaErrorMemoryAllocation : cudaSuccess;
+}
+template <class T>
+cudaError_t ensure_spare(T*& p, size_t& cap, size_t bytes) {
+  if (cap >= bytes && p) return cudaSuccess;
+  const cudaError_t e = spare_room(bytes, cap);
+  return e == cudaSuccess ? ensure(p, cap, bytes) : e;
+}
+// Frees the context's table pools, their source and the sample lists (frames
+// make them again); false: there was nothing to free.  A frame takes their
+// addresses after its last allocation that may come here (a box plan's source is
+// only allocated for sums that no pool holds yet).
+bool give_back(cvr_ctx* c);
+// An allocation that a call cannot do without: tried again once they are gone.
+template <class F>
+cudaError_t need(cvr_ctx* c, F allocate) {
+  cudaError_t e = allocate();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  return give_back(c) ? allocate() : e;
+}
+#define NEED(ctx, call) CK(ctx, need(ctx, [&] { return (call); }))
+
 // Deferred shading of one frame: its bands and the lists they need.
 // deferred_bytes: 0 leaves the frame to the direct marcher (the ray-refill
 // variant, a ray with more steps than the lists hold, or a camera so far away
@@ -471,7 +503,7 @@ cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t,
   DeferredPlan p;
   const size_t bytes = deferred_bytes(f, &p);
   if (bytes == 0) return cudaSuccess;
-  cudaError_t e = ensure(c->d_defer, c->defer_cap, bytes);
+  cudaError_t e = ensure_spare(c->d_defer, c->defer_cap, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return cudaSuccess;

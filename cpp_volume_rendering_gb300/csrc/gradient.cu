@@ -408,7 +408,7 @@ cvr_status check_gradient_params(cvr_ctx* c, const cvr_gradient_params& p) {
 cvr_status build_gradient(cvr_ctx* c) {
   const cvr_gradient_params& p = c->grad_params;
   const size_t n = (size_t)c->nx * c->ny * c->nz;
-  CK(c, ensure(c->d_grad, c->grad_cap, n * sizeof(uint2)));
+  NEED(c, ensure(c->d_grad, c->grad_cap, n * sizeof(uint2)));
   GradBuild b{p.model, p.sample_size, p.filter_nxnxn, p.normalized, c->dtype == CVR_U8 ? 1.0f / 255.0f : 1.0f / 65535.0f};
   const bool u8 = c->dtype == CVR_U8;
   const bool stencil = p.model != CVR_GRADIENT_FINITE_DIFFERENCES || p.sample_size == 1;
@@ -529,7 +529,7 @@ cvr_status cvr_download_gradient(cvr_ctx* c, float* host, size_t n_floats) {
   cvr_status ks = check_kernel_flag(c, "gradient build: a plane copy did not complete");
   if (ks != CVR_OK) return ks;
   float* tmp = nullptr;
-  CK(c, cudaMalloc((void**)&tmp, sizeof(float) * 3 * (size_t)n));
+  NEED(c, cudaMalloc((void**)&tmp, sizeof(float) * 3 * (size_t)n));
   k_gradient_to_float<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->d_grad, tmp, n);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(host, tmp, sizeof(float) * 3 * (size_t)n, cudaMemcpyDeviceToHost, c->stream);

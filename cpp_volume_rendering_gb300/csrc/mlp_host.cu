@@ -26,14 +26,14 @@ cvr_status alloc_mlp(cvr_ctx* c) {
   c->mlp.reset(new MlpState());
   MlpState& s = *c->mlp;
   CK(c, cudaSetDevice(c->device));
-  CK(c, cudaMalloc((void**)&s.params, sizeof(float) * kMlpParams));
-  CK(c, cudaMalloc((void**)&s.m, sizeof(float) * kMlpParams));
-  CK(c, cudaMalloc((void**)&s.v, sizeof(float) * kMlpParams));
-  CK(c, cudaMalloc((void**)&s.packed, kPkBytes));
-  CK(c, cudaMalloc((void**)&s.grad, sizeof(float) * (kMlpParams + 1)));
-  CK(c, cudaMalloc((void**)&s.loss_acc, sizeof(float)));
-  CK(c, cudaMalloc((void**)&s.err, sizeof(int)));
-  CK(c, cudaMalloc((void**)&s.step, sizeof(int)));
+  NEED(c, cudaMalloc((void**)&s.params, sizeof(float) * kMlpParams));
+  NEED(c, cudaMalloc((void**)&s.m, sizeof(float) * kMlpParams));
+  NEED(c, cudaMalloc((void**)&s.v, sizeof(float) * kMlpParams));
+  NEED(c, cudaMalloc((void**)&s.packed, kPkBytes));
+  NEED(c, cudaMalloc((void**)&s.grad, sizeof(float) * (kMlpParams + 1)));
+  NEED(c, cudaMalloc((void**)&s.loss_acc, sizeof(float)));
+  NEED(c, cudaMalloc((void**)&s.err, sizeof(int)));
+  NEED(c, cudaMalloc((void**)&s.step, sizeof(int)));
   CK(c, cudaMemsetAsync(s.packed, 0, kPkBytes, c->stream));  // padding of the BF16 tiles stays zero
   CK(c, cudaMemsetAsync(s.err, 0, sizeof(int), c->stream));
   return CVR_OK;
@@ -152,8 +152,8 @@ cvr_status cvr_mlp_forward(cvr_ctx* c, const float* x, int n, float* y) {
     if (s.io_y) cudaFree(s.io_y);
     s.io_x = s.io_y = nullptr;
     s.io_cap = 0;
-    CK(c, cudaMalloc((void**)&s.io_x, sizeof(float) * 48 * (size_t)n));
-    CK(c, cudaMalloc((void**)&s.io_y, sizeof(float) * 2 * (size_t)n));
+    NEED(c, cudaMalloc((void**)&s.io_x, sizeof(float) * 48 * (size_t)n));
+    NEED(c, cudaMalloc((void**)&s.io_y, sizeof(float) * 2 * (size_t)n));
     s.io_cap = (size_t)n;
   }
   CK(c, cudaMemcpyAsync(s.io_x, x, sizeof(float) * 48 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
@@ -221,8 +221,8 @@ cvr_status cvr_mlp_set_training_data(cvr_ctx* c, const float* x, const float* t,
     if (s.t) cudaFree(s.t);
     s.x = s.t = nullptr;
     s.data_cap = 0;
-    CK(c, cudaMalloc((void**)&s.x, sizeof(float) * 48 * (size_t)n));
-    CK(c, cudaMalloc((void**)&s.t, sizeof(float) * 2 * (size_t)n));
+    NEED(c, cudaMalloc((void**)&s.x, sizeof(float) * 48 * (size_t)n));
+    NEED(c, cudaMalloc((void**)&s.t, sizeof(float) * 2 * (size_t)n));
     s.data_cap = (size_t)n;
   }
   CK(c, cudaMemcpyAsync(s.x, x, sizeof(float) * 48 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
@@ -258,8 +258,8 @@ cvr_status cvr_mlp_train(cvr_ctx* c, int epochs, int batch, float lr, uint64_t s
   CK(c, cudaSetDevice(c->device));
   const int n = s.n;
   const int n_batches = (n + batch - 1) / batch;
-  CK(c, grow(s.idx, s.idx_cap, (size_t)n));
-  CK(c, grow(s.partials, s.partials_cap, (size_t)(batch / 128) * kMlpPitch));
+  NEED(c, grow(s.idx, s.idx_cap, (size_t)n));
+  NEED(c, grow(s.partials, s.partials_cap, (size_t)(batch / 128) * kMlpPitch));
   // (Re)capture the epoch when the batch structure or the rate changed.
   if (!s.epoch_graph || s.graph_batch != batch || s.graph_n != n || s.graph_lr != lr) {
     if (s.epoch_graph) {

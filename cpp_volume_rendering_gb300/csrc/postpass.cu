@@ -310,9 +310,9 @@ cvr_status cvr_rescale_frame(cvr_ctx* c, int mode, int kernel, const float* src_
     return fail(c, CVR_ERR_INVALID_ARG, "cvr_rescale_frame: bad arguments");
   CK(c, cudaSetDevice(c->device));
   const size_t bytes = (size_t)sw * sh * sizeof(float4);
-  CK(c, ensure(c->d_ms, c->ms_cap, bytes));
+  NEED(c, ensure(c->d_ms, c->ms_cap, bytes));
   if (const size_t sb = multiscale_scratch(mode, kernel, sw, sh, w, h))
-    CK(c, ensure(c->d_msf, c->msf_cap, sb));
+    NEED(c, ensure(c->d_msf, c->msf_cap, sb));
   CK(c, cudaMemcpyAsync(c->d_ms, src_dev, bytes, cudaMemcpyDeviceToDevice, c->stream));
   CK(c, launch_multiscale(mode, kernel, c->d_ms, sw, sh, reinterpret_cast<float4*>(dst_dev), w, h, c->d_msf,
                           c->stream));

@@ -44,7 +44,7 @@ extern "C" cvr_status cvr_measure_l1_bandwidth(cvr_ctx* c, float* gbs) {
   int sms = 0;
   CK(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
   uint4* buf = nullptr;
-  CK(c, ensure(c->d_probe, c->probe_cap, kProbeEntries * sizeof(uint4) + 256));
+  NEED(c, ensure(c->d_probe, c->probe_cap, kProbeEntries * sizeof(uint4) + 256));
   buf = reinterpret_cast<uint4*>(c->d_probe);
   CK(c, launch_fill(buf, kProbeEntries * sizeof(uint4), 0x01234567u, c->stream));
   unsigned* sink = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(c->d_probe) + kProbeEntries * sizeof(uint4));

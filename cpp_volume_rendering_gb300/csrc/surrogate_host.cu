@@ -19,8 +19,8 @@ cvr_status need_sur(cvr_ctx* c) {
   CK(c, cudaSetDevice(c->device));
   if (!c->sur) c->sur.reset(new SurState());
   SurState& s = *c->sur;
-  if (!s.counter) CK(c, cudaMalloc((void**)&s.counter, sizeof(unsigned int)));
-  if (!s.acc) CK(c, cudaMalloc((void**)&s.acc, sizeof(double) * 8));
+  if (!s.counter) NEED(c, cudaMalloc((void**)&s.counter, sizeof(unsigned int)));
+  if (!s.acc) NEED(c, cudaMalloc((void**)&s.acc, sizeof(double) * 8));
   return CVR_OK;
 }
 
@@ -28,7 +28,7 @@ cvr_status grow_points(cvr_ctx* c, size_t cap) {
   SurState& s = *c->sur;
   if (s.pts_cap >= cap && s.pts) return CVR_OK;
   float4* np = nullptr;
-  CK(c, cudaMalloc((void**)&np, sizeof(float4) * 2 * cap));
+  NEED(c, cudaMalloc((void**)&np, sizeof(float4) * 2 * cap));
   if (s.n_pts > 0) {
     cudaError_t e = cudaMemcpyAsync(np, s.pts, sizeof(float4) * 2 * (size_t)s.n_pts, cudaMemcpyDeviceToDevice, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -46,10 +46,10 @@ cvr_status grow_points(cvr_ctx* c, size_t cap) {
 cvr_status grow_chunk(cvr_ctx* c) {
   SurState& s = *c->sur;
   if (s.chunk_cap >= kChunk) return CVR_OK;
-  CK(c, cudaMalloc((void**)&s.cx, sizeof(float) * kMlpIn * kChunk));
-  CK(c, cudaMalloc((void**)&s.ct, sizeof(float) * 2 * kChunk));
-  CK(c, cudaMalloc((void**)&s.cy, sizeof(float) * 2 * kChunk));
-  CK(c, cudaMalloc((void**)&s.cd, sizeof(float) * 2 * kChunk));
+  NEED(c, cudaMalloc((void**)&s.cx, sizeof(float) * kMlpIn * kChunk));
+  NEED(c, cudaMalloc((void**)&s.ct, sizeof(float) * 2 * kChunk));
+  NEED(c, cudaMalloc((void**)&s.cy, sizeof(float) * 2 * kChunk));
+  NEED(c, cudaMalloc((void**)&s.cd, sizeof(float) * 2 * kChunk));
   s.chunk_cap = kChunk;
   return CVR_OK;
 }

@@ -26,7 +26,7 @@ cudaError_t make_texture(cvr_ctx* c, TexImage& t, const void* src, size_t elem, 
                          int h, int d, cudaTextureReadMode mode) {
   t.release();
   cudaExtent ext = make_cudaExtent((size_t)w, (size_t)h, (size_t)d);
-  cudaError_t e = cudaMalloc3DArray(&t.arr, &desc, ext);
+  cudaError_t e = need(c, [&] { return cudaMalloc3DArray(&t.arr, &desc, ext); });
   if (e != cudaSuccess) return e;
   cudaMemcpy3DParms cp{};
   cp.srcPtr = make_cudaPitchedPtr(const_cast<void*>(src), (size_t)w * elem, (size_t)w, (size_t)h);
@@ -76,7 +76,7 @@ cvr_status ensure_pyramid_textures(cvr_ctx* c) {
   for (int l = 0; l < c->pyr.n_levels; ++l)
     total = std::max(total, (long long)c->pyr.dims[l][0] * c->pyr.dims[l][1] * c->pyr.dims[l][2]);
   __half* tmp = nullptr;
-  CK(c, cudaMalloc((void**)&tmp, sizeof(__half) * (size_t)total));
+  NEED(c, cudaMalloc((void**)&tmp, sizeof(__half) * (size_t)total));
   cudaError_t e = cudaSuccess;
   for (int l = 0; l < c->pyr.n_levels && e == cudaSuccess; ++l) {
     const int* d = c->pyr.dims[l];

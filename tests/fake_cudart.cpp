@@ -11,7 +11,7 @@
 #include <string>
 
 namespace {
-size_t capacity = (size_t)280 << 30, used = 0;
+size_t capacity = (size_t)280 << 30, used = 0, largest = ~(size_t)0;
 std::map<void*, size_t> blocks;
 std::map<const void*, std::string> names;
 std::map<const void*, int> raised;  // dynamic shared memory a kernel was given leave for
@@ -38,8 +38,10 @@ int encode_tiled(...) { return 0; }
 }  // namespace
 
 extern "C" {
-void fake_reset(size_t bytes) {
+// Capacity, and the largest block that is free in one piece.
+void fake_reset(size_t bytes, size_t block) {
   capacity = bytes;
+  largest = block;
   launches.clear();
   refused = 0;
 }
@@ -88,7 +90,7 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void
 cudaError_t cudaMalloc(void** p, size_t n) {
   *p = nullptr;
   if (n == 0) n = 1;
-  if (used + n > capacity) {
+  if (used + n > capacity || n > largest) {
     ++refused;
     return put(cudaErrorMemoryAllocation);
   }

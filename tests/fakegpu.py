@@ -21,7 +21,7 @@ def load():
         build._run([build.CXX, "-O1", "-fPIC", "-std=c++17", "-shared", f"-I{CUDA / 'include'}", str(src)] +
                    [str(o) for o in objs] + ["-fopenmp", "-Wl,-Bsymbolic", "-o", str(out)])
     fake = abi.load(out)
-    fake.fake_reset.argtypes, fake.fake_reset.restype = [C.c_size_t], None
+    fake.fake_reset.argtypes, fake.fake_reset.restype = [C.c_size_t, C.c_size_t], None
     fake.fake_used.argtypes, fake.fake_used.restype = [], C.c_size_t
     fake.fake_refused.argtypes, fake.fake_refused.restype = [], C.c_int
     fake.fake_launches.argtypes, fake.fake_launches.restype = [C.c_char_p], C.c_int
@@ -32,15 +32,16 @@ class Context(scene.Context):
     """A context on a device of `capacity` bytes."""
 
     def __init__(self, lib, capacity=280 << 30):
-        lib.fake_reset(capacity)
+        lib.fake_reset(capacity, 1 << 62)
         self.lib = lib
         self.h = C.c_void_p()
         assert lib.cvr_create(C.byref(self.h), 0) == abi.CVR_OK
         self.dims = self.dtype = self.spacing = None
 
-    def resize(self, capacity):
-        """Another capacity; the counts of launches and refusals start over."""
-        self.lib.fake_reset(capacity)
+    def resize(self, capacity, largest=1 << 62):
+        """Another capacity and largest free block; the counts of launches and
+        refusals start over."""
+        self.lib.fake_reset(capacity, largest)
 
     def launches(self, part):
         return self.lib.fake_launches(part.encode())

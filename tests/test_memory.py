@@ -29,7 +29,7 @@ def test_no_room_for_the_automatic_quad_copy(fake):
         frame()
         assert ctx.launches("k_brick") == 1
         abi.check(fake.cvr_set_brick_size(ctx.h, 0), ctx.h)
-        ctx.resize(fake.fake_used() + (1 << 18))  # the quads take 1.2 MB
+        ctx.resize(280 << 30, 1 << 20)  # no 1.2 MB for the quads in one piece
         for _ in range(3):
             frame()
         assert ctx.launches("k_quad_volume") == 0 and ctx.launches("k_march_plain") == 3
@@ -43,5 +43,52 @@ def test_no_room_for_the_automatic_quad_copy(fake):
         frame = plain(ctx)
         frame()
         assert ctx.launches("k_quad_volume") == 1
+    finally:
+        ctx.close()
+
+
+def extinction(ctx, n=128, image=256, light=abi.LIGHT_DIRECTIONAL):
+    wl = scene.workload("extinction", n=n, image=image)
+    scene.prepare(ctx, wl)
+    return lambda: ctx.render(wl.method, wl.cam, wl.light, wl.params, image, image)
+
+
+def test_tables_and_lists_are_given_back(fake):
+    """A volume that has no room beside the box tables and sample lists of the
+    one before gets theirs; the next frame makes its own again."""
+    ctx = fakegpu.Context(fake, 4 << 30)
+    try:
+        frame = extinction(ctx)
+        frame()
+        assert ctx.launches("k_box_tables") and ctx.launches("k_collect")
+        held = fake.fake_used()
+        assert held > 600 << 20
+        ctx.resize(held + (200 << 20))
+        ctx.set_volume(np.zeros((480, 1024, 1024), np.uint8))  # 480 MB
+        assert fake.fake_used() < held
+        ctx.resize(4 << 30)
+        frame = extinction(ctx)
+        frame()
+        assert ctx.launches("k_box_tables") and ctx.launches("k_collect")
+    finally:
+        ctx.close()
+
+
+def test_spare_buffers_leave_half(fake):
+    """Lists and copies that would take more than half of what is free are not
+    made: the direct marchers on the plain array."""
+    ctx = fakegpu.Context(fake)
+    try:
+        wl = scene.workload("ground_truth", n=64, image=256)
+        scene.prepare(ctx, wl)
+        lists = 24 * 8192 * 256 * 8  # more than 300 MB
+        ctx.resize(fake.fake_used() + lists)
+        ctx.render(wl.method, wl.cam, wl.light, wl.params, 256, 256)
+        assert ctx.launches("k_collect") == 0 and ctx.launches("k_march_gt") == 1
+        assert ctx.launches("k_quad_volume") == 1  # 1.2 MB
+        assert fake.fake_refused() == 0
+        ctx.resize(fake.fake_used() + 4 * lists)
+        ctx.render(wl.method, wl.cam, wl.light, wl.params, 256, 256)
+        assert ctx.launches("k_collect") == 1
     finally:
         ctx.close()
