@@ -208,6 +208,8 @@ SIGNATURES = {
     "cvr_get_brick_staging": (_I, [_P]),
     "cvr_set_walk_tables": (_I, [_P, _I]),
     "cvr_get_walk_tables": (_I, [_P]),
+    "cvr_set_cache_limit": (_I, [_P, C.c_size_t]),
+    "cvr_get_cache_limit": (C.c_size_t, [_P]),
     "cvr_set_volume_layout": (_I, [_P, _I]),
     "cvr_get_volume_layout": (_I, [_P]),
     "cvr_set_compact_sat": (_I, [_P, _I]),

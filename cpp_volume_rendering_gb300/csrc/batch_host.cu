@@ -32,7 +32,7 @@ struct cvr_batch {
   unsigned long long* d_stats = nullptr;  // 3 per job, in the caller's job order
   bool ext_compact = false;
   bool ext_aligned = false;  // every job: an aligned shadow table and aligned AO boxes (or AO off)
-  std::vector<std::shared_ptr<VolCopy>> copies;  // the volume copies its jobs read
+  std::vector<std::shared_ptr<DevCopy>> copies;  // the volume and pyramid copies its jobs read
   std::vector<uint4*> sat32;              // the batch's own compact SATs, one per volume slot used
   std::vector<uint4*> walks;              // their walk tables, one per (slot, walk axis, depth) in use
   std::vector<long long> walk_keys;
@@ -152,8 +152,10 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     FrameArgs f;
     st = frame_args(c, &j.camera, j.params, j.out_rgba_dev, j.width, j.height, &f);
     if (st != CVR_OK) break;
-    if (f.vol.voxels != c->d_vol && std::find(b->copies.begin(), b->copies.end(), c->vcopy) == b->copies.end())
-      b->copies.push_back(c->vcopy);
+    auto hold = [&](const std::shared_ptr<DevCopy>& p) {
+      if (std::find(b->copies.begin(), b->copies.end(), p) == b->copies.end()) b->copies.push_back(p);
+    };
+    if (f.vol.voxels != c->d_vol) hold(c->vcopy);
     st = grad_args(c, j.method, &j.light, &f);
     if (st != CVR_OK) break;
     f.stats = b->d_stats + 3 * (size_t)i;
@@ -185,7 +187,8 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       st = sur_job_args(c, static_cast<const cvr_gt_params*>(j.params), &j.light, &J.a, &J.tex);
       if (st != CVR_OK) break;
       J.f = f;
-      J.bytes = deferred_bytes(f, &J.plan);
+      if (J.a.pyr.quads) hold(c->pyrq);
+      J.bytes = deferred_bytes(c, f, &J.plan);
       sur.push_back(J);
     }
   }
@@ -242,6 +245,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
       if (at == b->box_keys.size()) {
         b->box_keys.push_back(key);
         b->boxes.emplace_back(new BoxTables());
+        b->boxes.back()->limit = std::min(kBoxPoolBytes, c->cache_limit);
       }
       select_slot(c, ext_slot[k]);
       const int n[3] = {c->nx + 2, c->ny + 2, c->nz + 2};
@@ -370,7 +374,7 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
     size_t bytes = 0;
     for (size_t k = l; k < sur.size(); k += lanes) bytes = std::max(bytes, sur[k].bytes);
     if (bytes == 0) continue;
-    cudaError_t me = spare_room(bytes, 0);
+    cudaError_t me = spare_room(c, bytes, 0);
     if (me == cudaSuccess) me = cudaMalloc(&b->lists[l], bytes);
     if (me == cudaErrorMemoryAllocation) {
       cudaGetLastError();

@@ -91,7 +91,7 @@ bool shadow_plan(BoxTables& B, unsigned long long gen, const int n[3], const Sha
   const size_t had = P->have.size();
   for (int p : need)
     if (std::find(P->have.begin(), P->have.end(), p) == P->have.end()) P->have.push_back(p);
-  auto fits = [&]() { return P->have.size() <= (size_t)kMaxBoxTables && P->have.size() * cells * kCellBytes <= kBoxPoolBytes; };
+  auto fits = [&]() { return P->have.size() <= (size_t)kMaxBoxTables && P->have.size() * cells * kCellBytes <= B.limit; };
   P->sdw_new = !same;
   if (!fits() || P->have.size() * cells * kCellBytes > pool.cap) {
     P->sdw_new = true;          // the pool grows: its tables are built again
@@ -99,7 +99,7 @@ bool shadow_plan(BoxTables& B, unsigned long long gen, const int n[3], const Sha
     if (!fits()) return false;
   }
   // room for a few more widths (a moving light's), as far as the bound goes
-  const size_t room = std::min((P->have.size() + 3) / 4 * 4, kBoxPoolBytes / (cells * kCellBytes));
+  const size_t room = std::min((P->have.size() + 3) / 4 * 4, B.limit / (cells * kCellBytes));
   P->sdw_bytes = P->sdw_new ? std::max(room, P->have.size()) * cells * kCellBytes : pool.cap;
   for (size_t i = P->sdw_new ? 0 : had; i < P->have.size(); ++i) {
     const int w[3] = {P->have[i] & 1023, P->have[i] >> 10, ww};
@@ -149,7 +149,7 @@ bool box_plan(BoxTables& B, unsigned long long gen, const int n[3], const Shadow
       if (!table_desc(n, xyz, ww, pad, &d)) return false;
       d.cell = (unsigned)cell;
       cell += cells_of(d.g);
-      if (cell * kCellBytes > kBoxPoolBytes) return false;
+      if (cell * kCellBytes > B.limit) return false;
       e->box.ao_cell[i] = d.cell;
       e->box.ao_grid[i] = lookup_grid(d.g);
       P->ao.t[P->ao.n++] = d;
@@ -179,7 +179,7 @@ cvr_status box_build(cvr_ctx* c, BoxTables& B, const BoxSource& src, unsigned lo
   auto build = [&](BoxPool& pool, bool fresh, size_t bytes, const BoxTableSet& set) -> cudaError_t {
     if (fresh) {
       pool.gen = 0;
-      cudaError_t err = ensure_spare(pool.data, pool.cap, bytes);
+      cudaError_t err = ensure_spare(c, pool.data, pool.cap, bytes);
       if (err != cudaSuccess) return err;
     }
     return launch_box_tables(src, set, pool.data, c->stream);

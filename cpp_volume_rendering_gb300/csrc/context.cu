@@ -126,7 +126,7 @@ namespace ctxutil {
 static bool quads_pay(cvr_ctx* c, double pixels) {
   if (c->brick_bs > 0 || c->staging) return false;
   const double voxels = (double)c->nx * c->ny * c->nz;
-  if (voxels * 4.0 * (c->dtype == CVR_U8 ? 1 : 2) > (double)kAutoCopyBytes) return false;
+  if (voxels * 4.0 * (c->dtype == CVR_U8 ? 1 : 2) > (double)std::min(kAutoCopyBytes, c->cache_limit)) return false;
   if (c->vbrick_bs == kQuadCopy) return true;
   c->quad_seen += pixels;
   return 2.0 * c->quad_seen * std::max(c->nx, std::max(c->ny, c->nz)) >= voxels;
@@ -136,7 +136,7 @@ static bool quads_pay(cvr_ctx* c, double pixels) {
 // copy that a batch reads stays the batch's.
 static cudaError_t copy_room(cvr_ctx* c, size_t bytes) {
   c->vbrick_bs = -1;
-  if (!c->vcopy || c->vcopy.use_count() > 1) c->vcopy = std::make_shared<VolCopy>();
+  if (!c->vcopy || c->vcopy.use_count() > 1) c->vcopy = std::make_shared<DevCopy>();
   return ensure(c->vcopy->data, c->vcopy->cap, bytes);
 }
 
@@ -153,7 +153,7 @@ cvr_status render_volume_view(cvr_ctx* c, VolumeView* out, bool allow_tex, doubl
     if (c->vbrick_bs != kQuadCopy) {
       const size_t bytes = qplane * c->nz * qbytes;
       cudaError_t qe = c->quads ? need(c, [&] { return copy_room(c, bytes); })
-                                : spare_room(bytes, c->vcopy && c->vcopy.use_count() == 1 ? c->vcopy->cap : 0);
+                                : spare_room(c, bytes, c->vcopy && c->vcopy.use_count() == 1 ? c->vcopy->cap : 0);
       if (qe == cudaSuccess && !c->quads) qe = copy_room(c, bytes);
       if (qe == cudaErrorMemoryAllocation && !c->quads) {  // not asked for: the plain array serves
         cudaGetLastError();
@@ -244,7 +244,7 @@ static cvr_status frame_boxes(cvr_ctx* c, double vmax, const FrameArgs& f, const
   if (plan.missing > 0 && compact) {
     if (c->boxsrc_gen != gen) {
       c->boxsrc_gen = 0;
-      cudaError_t e = ensure_spare(c->d_boxsrc, c->boxsrc_cap, cells * sizeof(unsigned));
+      cudaError_t e = ensure_spare(c, c->d_boxsrc, c->boxsrc_cap, cells * sizeof(unsigned));
       if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         return CVR_OK;
@@ -560,25 +560,27 @@ cvr_status pyramid_view(cvr_ctx* c, PyramidView* out) {
     n += (size_t)P.quad_plane(l) * (P.dims[l][2] + 2);  // dims <= 4096: a plane is below 2^25 cells
     // 32-bit cell numbers, and without the quad layout a copy of at most
     // kAutoCopyBytes: else the plain levels
-    if (n >= kCompactMaxCells || (!c->quads && n * sizeof(float4) > kAutoCopyBytes)) {
+    if (n >= kCompactMaxCells || (!c->quads && n * sizeof(float4) > std::min(kAutoCopyBytes, c->cache_limit))) {
       *out = P;
       return CVR_OK;
     }
   }
   if (!c->pyrq_ready) {
     // without room for the copy the taps read the plain levels
-    cudaError_t e = c->quads ? need(c, [&] { return ensure(c->d_pyrq, c->pyrq_cap, n * sizeof(float4)); })
-                             : ensure_spare(c->d_pyrq, c->pyrq_cap, n * sizeof(float4));
+    if (!c->pyrq || c->pyrq.use_count() > 1) c->pyrq = std::make_shared<DevCopy>();
+    DevCopy& q = *c->pyrq;
+    cudaError_t e = c->quads ? need(c, [&] { return ensure(q.data, q.cap, n * sizeof(float4)); })
+                             : ensure_spare(c, q.data, q.cap, n * sizeof(float4));
     if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
       *out = P;
       return CVR_OK;
     }
     if (e != cudaSuccess) return cuda_fail(c, e, "pyramid quads");
-    CK(c, launch_pyramid_quads(P, c->d_pyr, c->d_pyrq, c->stream));
+    CK(c, launch_pyramid_quads(P, c->d_pyr, static_cast<float4*>(q.data), c->stream));
     c->pyrq_ready = true;
   }
-  P.quads = c->d_pyrq;
+  P.quads = static_cast<const float4*>(c->pyrq->data);
   *out = P;
   return CVR_OK;
 }
@@ -684,7 +686,7 @@ void cvr_destroy(cvr_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_vol, c->d_rgbt, c->d_rgba, c->d_sat, c->d_lut, c->d_pyr, c->d_occ_sec, c->d_sdw_sec,
                   c->d_occ_vec, c->d_sdw_vec, c->d_stats, c->d_out, c->d_flush, c->d_probe, c->d_lcache, c->d_grad, c->d_ms, c->d_msf,
-                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_pyrq, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc, c->d_defer};
+                  c->d_sat32, c->d_lut32, c->d_kerr, c->d_satp, c->d_walk, c->d_pyrs, c->d_boxsrc, c->d_defer};
   for (void* p : bufs)
     if (p) cudaFree(p);
   for (int i = 0; i < 4; ++i)
@@ -1038,8 +1040,8 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
   if (step > 0.0f) {
     f.step = step;
     DeferredPlan plan;
-    if (const size_t bytes = deferred_bytes(f, &plan)) {
-      e = ensure_spare(c->d_defer, c->defer_cap, bytes);
+    if (const size_t bytes = deferred_bytes(c, f, &plan)) {
+      e = ensure_spare(c, c->d_defer, c->defer_cap, bytes);
       if (e == cudaErrorMemoryAllocation) {  // the direct marcher needs none
         cudaGetLastError();
         e = cudaSuccess;
@@ -1088,7 +1090,7 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
         // box-table samples are cheap: passes of their own pay while the frame
         // needs few bands (512^2: 4.2 -> 2.2 ms; 1024^2: 4.2 -> 6.8 ms in 15)
         DeferredPlan plan;
-        if (!walk || (deferred_bytes(f, &plan) && plan.bands <= kBoxBands))
+        if (!walk || (deferred_bytes(c, f, &plan) && plan.bands <= kBoxBands))
           e = render_deferred(c, f, terms, true, 0u, [&](const Deferred& d) {
             return walk ? launch_light_box(f, a, *walk, d, c->stream)
                         : launch_light_ext(f, a, table, *c->sdw_table, d, c->stream);
@@ -1235,6 +1237,43 @@ cvr_status cvr_set_walk_tables(cvr_ctx* c, int on) {
 }
 
 int cvr_get_walk_tables(const cvr_ctx* c) { return c && c->walk_tables ? 1 : 0; }
+
+cvr_status cvr_set_cache_limit(cvr_ctx* c, size_t bytes) {
+  if (!c) return CVR_ERR_INVALID_ARG;
+  CK(c, cudaSetDevice(c->device));
+  CK(c, cudaStreamSynchronize(c->stream));  // launches that read what goes
+  c->cache_limit = bytes;
+  c->box.limit = std::min(kBoxPoolBytes, bytes);
+  if (c->box.ao.cap > bytes) c->box.ao.release();
+  if (c->box.sdw.cap > bytes) c->box.sdw.release();
+  auto drop = [&](auto*& p, size_t& cap) {
+    if (cap <= bytes) return false;
+    cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    return true;
+  };
+  drop(c->d_defer, c->defer_cap);
+  if (drop(c->d_boxsrc, c->boxsrc_cap)) c->boxsrc_gen = 0;
+  if (c->quads) return CVR_OK;  // the copies were asked for
+  const int keep = c->cur_slot;
+  for (int s = 0; s < CVR_MAX_VOLUMES; ++s) {
+    cvr_select_volume(c, s);
+    if (c->vbrick_bs == kQuadCopy && c->vcopy->cap > bytes) {
+      c->vcopy.reset();
+      c->vbrick_bs = -1;
+    }
+    c->quad_seen = 0.0;  // a copy that found no room may have it now
+    if (c->pyrq && c->pyrq->cap > bytes) {
+      c->pyrq.reset();
+      c->pyrq_ready = false;
+    }
+  }
+  cvr_select_volume(c, keep);
+  return CVR_OK;
+}
+
+size_t cvr_get_cache_limit(const cvr_ctx* c) { return c ? c->cache_limit : 0; }
 
 cvr_status cvr_set_brick_staging(cvr_ctx* c, int on) {
   if (!c) return CVR_ERR_INVALID_ARG;

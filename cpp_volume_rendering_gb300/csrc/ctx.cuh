@@ -127,6 +127,7 @@ struct BoxPool {
 };
 struct BoxTables {
   BoxPool ao, sdw;
+  size_t limit = kBoxPoolBytes;  // of each pool
   double seen = 0.0;             // pixels rendered without the tables they miss (box_tables)
   unsigned long long seen_gen = 0;
 };
@@ -134,12 +135,12 @@ struct BoxTables {
 // Largest quad copy made without cvr_set_volume_layout asking for the quads.
 constexpr size_t kAutoCopyBytes = (size_t)2 << 30;
 
-// A copy of a volume in another layout.  Batches hold the copies that their
-// jobs read, so a layout set afterwards makes its own (copy_room).
-struct VolCopy {
+// A copy of a volume or pyramid in another layout.  Batches hold the copies that
+// their jobs read, so a layout set afterwards makes its own (copy_room).
+struct DevCopy {
   void* data = nullptr;
   size_t cap = 0;  // bytes
-  ~VolCopy() {
+  ~DevCopy() {
     if (data) cudaFree(data);
   }
 };
@@ -174,11 +175,10 @@ struct VolSlot {
   size_t pyr_cap = 0;
   PyramidView pyr{};
   bool pyr_ready = false;
-  float4* d_pyrq = nullptr;
-  size_t pyrq_cap = 0;
+  std::shared_ptr<DevCopy> pyrq;
   bool pyrq_ready = false;
   TexState tex;
-  std::shared_ptr<VolCopy> vcopy;
+  std::shared_ptr<DevCopy> vcopy;
   int vbrick_bs = -1;
   double quad_seen = 0.0;
   uint2* d_grad = nullptr;
@@ -186,7 +186,7 @@ struct VolSlot {
   bool grad_ready = false;
   cvr_gradient_params grad_params{CVR_GRADIENT_NONE, 1, 0, 1};
   ~VolSlot() {
-    void* bufs[] = {d_vol, d_sat, d_lut, d_pyr, d_grad, d_sat32, d_lut32, d_pyrq};
+    void* bufs[] = {d_vol, d_sat, d_lut, d_pyr, d_grad, d_sat32, d_lut32};
     for (void* p : bufs)
       if (p) cudaFree(p);
   }
@@ -247,6 +247,7 @@ struct cvr_ctx {
   unsigned long long sat32_gen = 0;          // which build of the compact table (walk tables follow it)
   bool compact_sat = true;                   // cvr_set_compact_sat
   bool walk_tables = true;                   // cvr_set_walk_tables
+  size_t cache_limit = SIZE_MAX;             // cvr_set_cache_limit
   unsigned* d_satp = nullptr;                // compact builds' plane-prefix scratch (any volume slot)
   size_t satp_cap = 0;
   float* d_pyrs = nullptr;                   // opacities of a pyramid build (any volume slot)
@@ -271,8 +272,7 @@ struct cvr_ctx {
   size_t pyr_cap = 0;
   PyramidView pyr{};
   bool pyr_ready = false;
-  float4* d_pyrq = nullptr;
-  size_t pyrq_cap = 0;
+  std::shared_ptr<DevCopy> pyrq;
   bool pyrq_ready = false;
   // cone tables
   float4* d_occ_sec = nullptr;
@@ -314,7 +314,7 @@ struct cvr_ctx {
   // (cvr_set_brick_size, cvr_set_volume_layout)
   int brick_bs = 0;                          // tuning: 0 plain layout, else log2 of the brick edge
   bool quads = false;                        // tuning: the x-y quad layout (takes precedence)
-  std::shared_ptr<VolCopy> vcopy;
+  std::shared_ptr<DevCopy> vcopy;
   double quad_seen = 0.0;                    // pixels of the volume's frames without a quad copy (quads_pay)
   int vbrick_bs = -1;                        // layout of the copy's contents (-1: stale, kQuadCopy: quads)
   // object-space light cache (cvr_set_light_cache): 0 = off
@@ -369,8 +369,7 @@ inline void swap_volume(cvr_ctx* c, VolSlot& s) {
   std::swap(c->pyr_cap, s.pyr_cap);
   std::swap(c->pyr, s.pyr);
   std::swap(c->pyr_ready, s.pyr_ready);
-  std::swap(c->d_pyrq, s.d_pyrq);
-  std::swap(c->pyrq_cap, s.pyrq_cap);
+  std::swap(c->pyrq, s.pyrq);
   std::swap(c->pyrq_ready, s.pyrq_ready);
   swap_tex(c->tex, s.tex);
   std::swap(c->vcopy, s.vcopy);
@@ -432,9 +431,11 @@ cudaError_t ensure(T*& p, size_t& cap, size_t bytes) {
 
 // Buffers that only make frames faster (box tables and their source, sample
 // lists, copies nobody asked for) leave half of what is free to the rest of the
-// program: cudaErrorMemoryAllocation, with p as it was, when they would not.
+// program and keep to cvr_set_cache_limit: cudaErrorMemoryAllocation, with p as
+// it was, when they would not.
 // Small ones take what there is: asking costs 28 us, as much as a small frame.
-inline cudaError_t spare_room(size_t bytes, size_t held) {
+inline cudaError_t spare_room(const cvr_ctx* c, size_t bytes, size_t held) {
+  if (bytes > c->cache_limit) return cudaErrorMemoryAllocation;
   if (bytes <= (size_t)64 << 20) return cudaSuccess;
   size_t free_b = 0, total_b = 0;
   const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
@@ -442,9 +443,9 @@ inline cudaError_t spare_room(size_t bytes, size_t held) {
   return bytes > (free_b + held) / 2 ? cudaErrorMemoryAllocation : cudaSuccess;
 }
 template <class T>
-cudaError_t ensure_spare(T*& p, size_t& cap, size_t bytes) {
+cudaError_t ensure_spare(const cvr_ctx* c, T*& p, size_t& cap, size_t bytes) {
   if (cap >= bytes && p) return cudaSuccess;
-  const cudaError_t e = spare_room(bytes, cap);
+  const cudaError_t e = spare_room(c, bytes, cap);
   return e == cudaSuccess ? ensure(p, cap, bytes) : e;
 }
 // Frees the context's table pools, their source and the sample lists (frames
@@ -466,10 +467,10 @@ cudaError_t need(cvr_ctx* c, F allocate) {
 // deferred_bytes: 0 leaves the frame to the direct marcher (the ray-refill
 // variant, a ray with more steps than the lists hold, or a camera so far away
 // that a ray's length is mostly rounding).
-inline size_t deferred_bytes(const FrameArgs& f, DeferredPlan* p) {
+inline size_t deferred_bytes(const cvr_ctx* c, const FrameArgs& f, DeferredPlan* p) {
   const double diag2 = (double)dot3(f.vol.grid, f.vol.grid), eye2 = (double)dot3(f.cam.eye, f.cam.eye);
-  if (f.work || !(eye2 <= 1.0e4 * diag2) || !deferred_plan(f, p)) return 0;
-  return 256 + (p->warps * p->chunks * sizeof(unsigned) + 255) / 256 * 256 + p->records * (sizeof(float4) + sizeof(float2));
+  if (f.work || !(eye2 <= 1.0e4 * diag2) || !deferred_plan(f, c->cache_limit, p)) return 0;
+  return p->bytes;
 }
 // The launches of a frame over lists in mem (deferred_bytes of it): light(d)
 // launches the light pass over a band's records; taps: secondary lookups it
@@ -481,7 +482,7 @@ cudaError_t launch_deferred(void* mem, const DeferredPlan& p, const FrameArgs& f
   Deferred d;
   d.counter = reinterpret_cast<unsigned*>(base);
   d.chunk = reinterpret_cast<unsigned*>(base + 256);
-  d.rec = reinterpret_cast<float4*>(base + 256 + (p.warps * p.chunks * sizeof(unsigned) + 255) / 256 * 256);
+  d.rec = reinterpret_cast<float4*>(base + p.bytes - p.records * (sizeof(float4) + sizeof(float2)));
   d.light = reinterpret_cast<float2*>(d.rec + p.records);
   d.chunks = p.chunks;
   cudaError_t e = cudaSuccess;
@@ -501,9 +502,9 @@ cudaError_t render_deferred(cvr_ctx* c, const FrameArgs& f, const LightTerms& t,
                             bool* done) {
   *done = c->deferred_frame = false;
   DeferredPlan p;
-  const size_t bytes = deferred_bytes(f, &p);
+  const size_t bytes = deferred_bytes(c, f, &p);
   if (bytes == 0) return cudaSuccess;
-  cudaError_t e = ensure_spare(c->d_defer, c->defer_cap, bytes);
+  cudaError_t e = ensure_spare(c, c->d_defer, c->defer_cap, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return cudaSuccess;

@@ -194,7 +194,7 @@ cudaError_t with_threads(const FrameArgs& f, F fn) {
 
 }  // namespace
 
-bool deferred_plan(const FrameArgs& f, DeferredPlan* p) {
+bool deferred_plan(const FrameArgs& f, size_t limit, DeferredPlan* p) {
   // steps of the longest ray of any camera: the diagonal, and the four the
   // marchers' own bound allows past it
   const double diag = std::sqrt((double)dot3(f.vol.grid, f.vol.grid));
@@ -206,10 +206,15 @@ bool deferred_plan(const FrameArgs& f, DeferredPlan* p) {
   if ((size_t)f.W * f.H > 0x7fffffff) return false;
   p->chunks = (unsigned)chunks;
   const size_t row = row_warps * p->chunks * kRecChunk;
-  p->rows = (unsigned)std::min(all, kDeferredRecords / row);
+  // a row's records (24 bytes each) and its warps' chunk numbers
+  const size_t row_bytes = row * (sizeof(float4) + sizeof(float2)) + row_warps * p->chunks * sizeof(unsigned);
+  const size_t fit = limit > 512 ? (limit - 512) / row_bytes : 0;
+  if (fit == 0) return false;
+  p->rows = (unsigned)std::min(std::min(all, kDeferredRecords / row), fit);
   p->bands = (unsigned)((all + p->rows - 1) / p->rows);
   p->records = row * p->rows;
-  p->warps = row_warps * p->rows;
+  p->bytes = 256 + (p->rows * row_warps * p->chunks * sizeof(unsigned) + 255) / 256 * 256 +
+             p->records * (sizeof(float4) + sizeof(float2));
   return p->bands <= kMaxBands;
 }
 

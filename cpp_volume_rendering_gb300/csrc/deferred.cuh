@@ -73,13 +73,14 @@ __device__ __forceinline__ void light_samples(const FrameArgs& f, const Deferred
   }
 }
 
-// Tile rows of a frame one band may hold with 'cap' records, and the chunks a
-// warp may need (0: a ray has too many steps to defer).
+// A frame's bands (of 'rows' tile rows), the chunks a warp may need, and the
+// lists of a band: 'bytes' of memory, at most limit, its records at the end.
+// false: not one row fits (its rays have too many steps).
 struct DeferredPlan {
   unsigned chunks, rows, bands;
-  size_t records, warps;
+  size_t records, bytes;
 };
-bool deferred_plan(const FrameArgs& f, DeferredPlan* p);
+bool deferred_plan(const FrameArgs& f, size_t limit, DeferredPlan* p);
 cudaError_t launch_collect(const FrameArgs& f, const Deferred& d, unsigned rows, cudaStream_t st);
 // A kernel's code is loaded at its first use (0.1 to 0.4 ms each): loaded ahead
 // of a frame that is timed.

@@ -364,6 +364,18 @@ int cvr_get_compact_sat(cvr_ctx* ctx);
  * disables the walk table. */
 cvr_status cvr_set_walk_tables(cvr_ctx* ctx, int enable);
 int cvr_get_walk_tables(const cvr_ctx* ctx);
+/* Device memory that a context takes only to render faster (no reference
+ * counterpart): the box tables of shadow and of occlusion (at most 24 GiB each)
+ * and the 32-bit table that they are made from, the sample lists of deferred
+ * frames (4.5 GiB), and the quad copies of volumes and pyramids that no layout
+ * asks for (2 GiB each).  One above 64 MiB is made only when it leaves half of
+ * the free memory; tables, their source and lists go when another allocation of
+ * the context finds no room.  This bounds each of them to 'bytes' as well, in
+ * the context and the batches created afterwards, and frees those above it at
+ * once; 0 keeps none, so that frames come from the SAT, the direct marchers and,
+ * with CVR_LAYOUT_PLAIN, the plain arrays.  Same images.  Default: SIZE_MAX. */
+cvr_status cvr_set_cache_limit(cvr_ctx* ctx, size_t bytes);
+size_t cvr_get_cache_limit(const cvr_ctx* ctx);
 
 /* Object-space light cache (PreIlluminationStructuredVolume,
  * cppvolrend/utils/preillumination.h:15-47; reference default 32^3, off):
