@@ -188,14 +188,18 @@ def algorithmic_bytes(wl, st, abi):
 
 
 def l1_request_bytes(wl, st, abi, tables):
-    """Bytes the extinction marcher's loads request from L1 per frame: the
-    volume's trilinear footprint per primary step, per AO and shadow box 4
-    eight-byte pairs of its box table or, without tables, 16 sixteen-byte
-    quads, and the image.  Other methods: their algorithmic bytes."""
+    """Bytes the extinction frame's loads request from L1: the volume's
+    trilinear footprint per primary step, per shadow and per occlusion box the
+    loads of the tables that the frame reads (cvr_get_frame_tables), and the
+    image.  Other methods: their algorithmic bytes."""
     if wl.method != abi.EXTINCTION:
         return algorithmic_bytes(wl, st, abi)
     bvox = 1 if wl.dtype == abi.CVR_U8 else 2
-    return st.samples * 8 * bvox + st.aux_fetches * (32 if tables else 256) + wl.width * wl.height * 16
+    per_box = {abi.TABLES_NONE: 0, abi.TABLES_SAT: 512, abi.TABLES_COMPACT: 256, abi.TABLES_WALK: 128,
+               abi.TABLES_BOX: 32}
+    ao = st.shaded_samples * wl.params.ao_n_shells if wl.params.apply_occlusion else 0
+    boxes = (st.aux_fetches - ao) * per_box[tables[0]] + ao * per_box[tables[1]]
+    return st.samples * 8 * bvox + boxes + wl.width * wl.height * 16
 
 
 def cpu_baseline(wl, target_s=12.0, threads=None):
@@ -881,10 +885,13 @@ def run_ours(args):
     samples_all, = barrier_sum([float(st.samples * args.steps)], ws)
     value = samples_all / (total_ms / 1000.0) / 1e6
     ms_per_step = total_ms / args.steps
-    # roofline of the dominant kernel (the marcher is the only launch per frame)
+    # roofline of the frame (its marcher, or the passes of a deferred frame)
     alg = algorithmic_bytes(wl, st, abi)
     walk = bool(lib.cvr_get_walk_tables(ctx.h)) and wl.method == abi.EXTINCTION and wl.params.shadow_type == 1
-    req = l1_request_bytes(wl, st, abi, wl.method == abi.EXTINCTION and wl.params.shadow_type == 1)
+    sdw_tables, occ_tables = C.c_int(), C.c_int()
+    abi.check(lib.cvr_get_frame_tables(ctx.h, C.byref(sdw_tables), C.byref(occ_tables)), ctx.h)
+    tables = (sdw_tables.value, occ_tables.value)
+    req = l1_request_bytes(wl, st, abi, tables)
     med_ms = statistics.median(times)
     achieved = req / (med_ms / 1000.0) / 1e9
     peak_hbm, peak_src = measured_peak_hbm()
@@ -894,9 +901,11 @@ def run_ours(args):
                 "peak_source": "measured in this run: cvr_measure_l1_bandwidth (coalesced 16-byte L1 hits)",
                 "bytes_per_launch": req, "kernel_ms": round(med_ms, 4),
                 "effective_gather_gbs": round(alg / (med_ms / 1000.0) / 1e9, 1),
-                "note": "achieved = bytes the marcher's loads request from L1 per launch (box tables: 4 x 8 B per "
-                        "box) / CUDA-event time; effective_gather_gbs counts the reference's 64 SAT texels "
-                        "of 4 B per box query"}
+                "tables": dict(zip(("shadow", "occlusion"), ({0: "none", 1: "int64 SAT", 2: "compact SAT",
+                                                               3: "walk table", 4: "box tables"}[t] for t in tables))),
+                "note": "achieved = bytes the marcher's loads request from L1 per frame (a box: 32 B from box "
+                        "tables, 128 from a walk table, 256 from the compact SAT, 512 from the int64 SAT) / CUDA-event "
+                        "time; effective_gather_gbs counts the reference's 64 SAT texels of 4 B per box query"}
     if traffic:
         roofline["hbm"] = {"achieved": round(traffic / (med_ms / 1000.0) / 1e9, 2), "peak": peak_hbm,
                            "frac": round(traffic / (med_ms / 1000.0) / 1e9 / peak_hbm, 5),

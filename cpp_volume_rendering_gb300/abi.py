@@ -43,6 +43,8 @@ GRADIENT_KERNEL_AUTO = 0
 GRADIENT_KERNEL_TILED = 1
 GRADIENT_KERNEL_GENERIC = 2
 GRADIENT_KERNEL_TMA = 3
+# cvr_get_frame_tables
+TABLES_NONE, TABLES_SAT, TABLES_COMPACT, TABLES_WALK, TABLES_BOX = range(5)
 # cvr_set_volume_layout
 LAYOUT_PLAIN = 0
 LAYOUT_QUADS = 1
@@ -210,6 +212,7 @@ SIGNATURES = {
     "cvr_get_walk_tables": (_I, [_P]),
     "cvr_set_cache_limit": (_I, [_P, C.c_size_t]),
     "cvr_get_cache_limit": (C.c_size_t, [_P]),
+    "cvr_get_frame_tables": (_I, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "cvr_set_volume_layout": (_I, [_P, _I]),
     "cvr_get_volume_layout": (_I, [_P]),
     "cvr_set_compact_sat": (_I, [_P, _I]),

@@ -1075,6 +1075,10 @@ static cvr_status render_frame(cvr_ctx* c, int method, const cvr_camera* cam, co
       const BoxWalk* walk = nullptr;
       cvr_status es = ext_args(c, p, light, f, &a, &table, cached ? &no_compact : nullptr, cached ? nullptr : &walk);
       if (es != CVR_OK) return es;
+      const int sat = a.sat.sat32 ? CVR_TABLES_COMPACT : CVR_TABLES_SAT;
+      c->shadow_tables = !a.apply_sdw ? CVR_TABLES_NONE : walk ? CVR_TABLES_BOX
+                         : a.walk.oct && (a.ao_aligned || !a.apply_occ) ? CVR_TABLES_WALK : sat;
+      c->occlusion_tables = !a.apply_occ ? CVR_TABLES_NONE : a.box.ao ? CVR_TABLES_BOX : sat;
       if (cached) {  // object-space light cache, then the object-space marcher
         if (!c->sdw_table) c->sdw_table.reset(new ShadowBoxTable());
         const size_t cells = (size_t)c->lc_dims[0] * c->lc_dims[1] * c->lc_dims[2];
@@ -1274,6 +1278,13 @@ cvr_status cvr_set_cache_limit(cvr_ctx* c, size_t bytes) {
 }
 
 size_t cvr_get_cache_limit(const cvr_ctx* c) { return c ? c->cache_limit : 0; }
+
+cvr_status cvr_get_frame_tables(const cvr_ctx* c, int* shadow, int* occlusion) {
+  if (!c || !shadow || !occlusion) return CVR_ERR_INVALID_ARG;
+  *shadow = c->shadow_tables;
+  *occlusion = c->occlusion_tables;
+  return CVR_OK;
+}
 
 cvr_status cvr_set_brick_staging(cvr_ctx* c, int on) {
   if (!c) return CVR_ERR_INVALID_ARG;

@@ -320,6 +320,7 @@ struct cvr_ctx {
   // object-space light cache (cvr_set_light_cache): 0 = off
   int lc_dims[3] = {0, 0, 0};
   bool deferred_frame = false;  // the last frame was shaded in a pass of its own
+  int shadow_tables = CVR_TABLES_NONE, occlusion_tables = CVR_TABLES_NONE;  // cvr_get_frame_tables
   float2* d_lcache = nullptr;
   size_t lcache_cap = 0;
   // per-voxel gradient of the current volume (cvr_build_gradient) and the

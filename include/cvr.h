@@ -376,6 +376,16 @@ int cvr_get_walk_tables(const cvr_ctx* ctx);
  * with CVR_LAYOUT_PLAIN, the plain arrays.  Same images.  Default: SIZE_MAX. */
 cvr_status cvr_set_cache_limit(cvr_ctx* ctx, size_t bytes);
 size_t cvr_get_cache_limit(const cvr_ctx* ctx);
+/* What the last CVR_METHOD_EXTINCTION frame of cvr_render read its shadow and
+ * its occlusion boxes from (frames from a light cache: its cells did). */
+enum {
+  CVR_TABLES_NONE = 0,    /* the term is off, or no such frame yet */
+  CVR_TABLES_SAT = 1,     /* the int64 SAT: 64 8-byte loads a box */
+  CVR_TABLES_COMPACT = 2, /* the compact SAT: 16 16-byte loads */
+  CVR_TABLES_WALK = 3,    /* the walk table: 4 32-byte loads */
+  CVR_TABLES_BOX = 4      /* box tables: 4 8-byte loads */
+};
+cvr_status cvr_get_frame_tables(const cvr_ctx* ctx, int* shadow, int* occlusion);
 
 /* Object-space light cache (PreIlluminationStructuredVolume,
  * cppvolrend/utils/preillumination.h:15-47; reference default 32^3, off):

@@ -108,6 +108,48 @@ def test_small_frames_come_to_read_box_tables(fake, direction, radii, angle, int
     assert boxes() == seen
 
 
+def test_frames_say_what_they_read(fake):
+    """cvr_get_frame_tables, and with it the bytes that the benchmark's roofline counts."""
+    import ctypes as C
+
+    import bench
+
+    def tables():
+        a, b = C.c_int(-1), C.c_int(-1)
+        abi.check(fake.lib.cvr_get_frame_tables(fake.h, C.byref(a), C.byref(b)), fake.h)
+        return a.value, b.value
+
+    ck = abi.check
+    assert tables() == (abi.TABLES_NONE, abi.TABLES_NONE)
+    wl = scene.workload("extinction", n=64, image=160)  # a directional light, three AO boxes of whole widths
+    scene.prepare(fake, wl)
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_BOX, abi.TABLES_BOX)
+    ck(fake.lib.cvr_set_ray_refill(fake.h, 1), fake.h)
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_WALK, abi.TABLES_COMPACT)
+    ck(fake.lib.cvr_set_walk_tables(fake.h, 0), fake.h)
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_COMPACT, abi.TABLES_COMPACT)
+    ck(fake.lib.cvr_set_compact_sat(fake.h, 0), fake.h)
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_SAT, abi.TABLES_SAT)
+    ck(fake.lib.cvr_set_ray_refill(fake.h, 0), fake.h)
+    wl.params.shadow_type = 0  # a point light: occlusion alone has box tables
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_SAT, abi.TABLES_BOX)
+    wl.params.apply_occlusion = 0
+    frame(fake, wl)
+    assert tables() == (abi.TABLES_SAT, abi.TABLES_NONE)
+
+    st = abi.FrameStats(1000, 100, 100 * 53, 1.0)
+    wl.params.apply_occlusion, wl.params.ao_n_shells = 1, 3
+    rest = 1000 * 8 * 2 + 160 * 160 * 16
+    assert bench.l1_request_bytes(wl, st, abi, (abi.TABLES_BOX, abi.TABLES_BOX)) == rest + 5300 * 32
+    assert bench.l1_request_bytes(wl, st, abi, (abi.TABLES_WALK, abi.TABLES_COMPACT)) == rest + 5000 * 128 + 300 * 256
+    assert bench.l1_request_bytes(wl, st, abi, (abi.TABLES_SAT, abi.TABLES_BOX)) == rest + 5000 * 512 + 300 * 32
+
+
 def test_limit_frees_and_bounds(fake):
     """Limit 0: no tables, lists or copies are held or made, in slots and batches."""
     wl = scene.workload("extinction", n=64, image=128)
