@@ -230,7 +230,8 @@ cvr_status cvr_batch_create(cvr_ctx* c, const cvr_job* jobs, int n_jobs, cvr_bat
   std::vector<std::unique_ptr<BoxWalk>> walks(ext.size());
   size_t box_budget = 0, mem_free = 0;
   if (st == CVR_OK && !ext.empty()) {
-    CK(c, cudaMemGetInfo(&mem_free, &box_budget));
+    const cudaError_t e = cudaMemGetInfo(&mem_free, &box_budget);
+    if (e != cudaSuccess) st = cuda_fail(c, e, "cvr_batch_create: free memory");  // the current volume is set back below
     box_budget /= 4;
   }
   for (int pass = 0; pass < 2 && st == CVR_OK; ++pass) {

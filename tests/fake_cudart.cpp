@@ -17,6 +17,7 @@ std::map<const void*, std::string> names;
 std::map<const void*, int> raised;  // dynamic shared memory a kernel was given leave for
 std::map<std::string, int> launches;
 int refused = 0;
+bool mute = false;
 cudaError_t last = cudaSuccess;
 
 cudaError_t put(cudaError_t e) {
@@ -46,6 +47,8 @@ void fake_reset(size_t bytes, size_t block) {
   refused = 0;
 }
 size_t fake_used() { return used; }
+// Whether cudaMemGetInfo fails.
+void fake_mute(int on) { mute = on != 0; }
 // Allocations that found no room since the reset.
 int fake_refused() { return refused; }
 // Launches of the kernels whose name holds part.
@@ -111,6 +114,7 @@ cudaError_t cudaFree(void* p) {
   return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
+  if (mute) return put(cudaErrorUnknown);
   *f = capacity > used ? capacity - used : 0;
   *t = capacity;
   return cudaSuccess;

@@ -1,6 +1,8 @@
 """What the context does when the device has no room, on a fake CUDA runtime
 (no GPU): optional tables and copies are done without, and nothing is read
 that was not made."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -90,5 +92,23 @@ def test_spare_buffers_leave_half(fake):
         ctx.resize(fake.fake_used() + 4 * lists)
         ctx.render(wl.method, wl.cam, wl.light, wl.params, 256, 256)
         assert ctx.launches("k_collect") == 1
+    finally:
+        ctx.close()
+
+
+def test_failed_batch_keeps_the_current_volume(fake):
+    ctx = fakegpu.Context(fake)
+    try:
+        vols = [scene.synth_blobs(24, 24, 24, abi.CVR_U8, 8, seed=7 + k) for k in range(2)]
+        scene.prepare_batch_volumes(ctx, vols, pyramid=False)
+        b = scene.batch_jobs(vols, n_views=1, lights=scene.BATCH_LIGHTS[:1], image=32, methods=(abi.EXTINCTION,),
+                             out_ptrs=[1 << 20] * 2)
+        bh = C.c_void_p()
+        fake.fake_mute(1)
+        try:
+            assert fake.cvr_batch_create(ctx.h, (abi.Job * 2)(*b.jobs), 2, C.byref(bh)) == abi.CVR_ERR_CUDA
+        finally:
+            fake.fake_mute(0)
+        assert fake.cvr_current_volume(ctx.h) == 0 and not bh
     finally:
         ctx.close()
