@@ -434,10 +434,11 @@ cudaError_t ensure(T*& p, size_t& cap, size_t bytes) {
 // lists, copies nobody asked for) leave half of what is free to the rest of the
 // program and keep to cvr_set_cache_limit: cudaErrorMemoryAllocation, with p as
 // it was, when they would not.
-// Small ones take what there is: asking costs 28 us, as much as a small frame.
+// Those of up to 1 GiB take what there is: asking costs 28 us, as much as a
+// small frame.
 inline cudaError_t spare_room(const cvr_ctx* c, size_t bytes, size_t held) {
   if (bytes > c->cache_limit) return cudaErrorMemoryAllocation;
-  if (bytes <= (size_t)64 << 20) return cudaSuccess;
+  if (bytes <= (size_t)1 << 30) return cudaSuccess;
   size_t free_b = 0, total_b = 0;
   const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
   if (e != cudaSuccess) return e;

@@ -81,16 +81,16 @@ def test_spare_buffers_leave_half(fake):
     made: the direct marchers on the plain array."""
     ctx = fakegpu.Context(fake)
     try:
-        wl = scene.workload("ground_truth", n=64, image=256)
+        wl = scene.workload("ground_truth", n=64, image=512)
         scene.prepare(ctx, wl)
-        lists = 24 * 8192 * 256 * 8  # more than 300 MB
-        ctx.resize(fake.fake_used() + lists)
-        ctx.render(wl.method, wl.cam, wl.light, wl.params, 256, 256)
+        lists = 24 * 8192 * 256 * 31  # 8192 warps of 30 chunks of records, and the chunks' numbers
+        ctx.resize(fake.fake_used() + 2 * lists - (200 << 20))
+        ctx.render(wl.method, wl.cam, wl.light, wl.params, 512, 512)
         assert ctx.launches("k_collect") == 0 and ctx.launches("k_march_gt") == 1
         assert ctx.launches("k_quad_volume") == 1  # 1.2 MB
         assert fake.fake_refused() == 0
         ctx.resize(fake.fake_used() + 4 * lists)
-        ctx.render(wl.method, wl.cam, wl.light, wl.params, 256, 256)
+        ctx.render(wl.method, wl.cam, wl.light, wl.params, 512, 512)
         assert ctx.launches("k_collect") == 1
     finally:
         ctx.close()
