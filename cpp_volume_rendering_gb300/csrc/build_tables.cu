@@ -1067,7 +1067,7 @@ static PyrBase pyr_base_form(const VolumeView& plain, const PyramidView& P, floa
 // (32^3: 21 -> 12 us as 512 CTAs; 64^3 would take 52 instead of 41).
 static int pyr_level_tile(const PyramidView& P, int l) {
   auto tiles = [&](int a) { return (long long)(P.dims[l][a] + 7) / 8; };
-  return tiles(0) * tiles(1) * tiles(2) < 152 ? 4 : 8;
+  return tiles(0) * tiles(1) * tiles(2) < kSms ? 4 : 8;
 }
 // windows of up to 160 KB: taps of up to three texels apart
 constexpr size_t kLevelSmem = 160 * 1024;

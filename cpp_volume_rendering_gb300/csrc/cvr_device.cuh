@@ -13,6 +13,9 @@
 
 namespace cvr {
 
+// SMs of the GB300, where a rule weighs a launch against the chip it fills.
+constexpr int kSms = 152;
+
 // ---------------------------------------------------------------- float3 math
 __host__ __device__ __forceinline__ float3 f3(float x, float y, float z) { return make_float3(x, y, z); }
 __host__ __device__ __forceinline__ float3 operator+(float3 a, float3 b) { return f3(a.x + b.x, a.y + b.y, a.z + b.z); }

@@ -206,10 +206,11 @@ struct DosConstShade {
   }
 };
 
-// 256^3, base 128^3, 156 taps a sample -> 512^2: 14.6 ms a frame, 36 with the
-// taps along each ray, 20.4 with the taps' constants in shared memory.  Bound
-// by instruction issue (74 %; 74 instructions a tap, 107 without the runs)
-// beside the L1 data pipe; 8 CTAs a SM (64 registers) 15.0 ms, 6 15.6, 5 16.7.
+// 256^3, base 128^3, 156 taps a sample -> 512^2: 13.2 ms a frame, 37.1 with the
+// taps along each ray (20.4 with the taps' constants in shared memory where this
+// took 14.6).  Bound by instruction issue (78 %; 74 instructions a tap, 107
+// without the runs) beside the L1 data pipe; 8 CTAs a SM (64 registers) 13.2 ms,
+// 7 13.5, 6 14.2, 5 15.0.
 __global__ void __launch_bounds__(128, 8) k_light_dos(const __grid_constant__ DosArgs a,
                                                                  const __grid_constant__ FrameArgs f,
                                                                  const __grid_constant__ Deferred d,

@@ -13,9 +13,9 @@ namespace cvr {
 // another's layers do.  The groups share one copy of the weights (19 KB), so
 // the SM keeps more L1 for the pyramid's texels than with a CTA per tile.
 // Bound by the texture pipe (67 trilinear 3D fetches a sample).  8 groups (64
-// registers, all 512 TMEM columns): 320^3 -> 720^2 12.4 ms through the texture
-// unit, 18.7 with FP32 taps; 6 groups 12.7 and 21.7, 4 groups 14.0 and 29.4;
-// the direct marcher 14.0 and 34.3 (128^3 -> 256^2: 0.68 against 1.68 ms).
+// registers, all 512 TMEM columns): 320^3 -> 720^2 10.1 ms through the texture
+// unit, 17.1 with FP32 taps; 6 groups 10.5 and 19.7, 4 groups 11.8 and 27.3;
+// the direct marcher 14.0 and 35.2 (128^3 -> 256^2: 0.68 against 1.60 ms).
 constexpr int kSurGroups = 8;
 template <bool TEX, int NG>
 __global__ void __launch_bounds__(128 * NG, 1) k_light_sur(const __grid_constant__ FrameArgs f,

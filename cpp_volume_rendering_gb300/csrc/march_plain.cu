@@ -37,7 +37,7 @@ static cudaError_t launch_plain_nt(const FrameArgs& f, cudaStream_t st) {
 
 template <int NT>
 static cudaError_t launch_plain_size(const FrameArgs& f, cudaStream_t st) {
-  const size_t full = (size_t)152 * 1024;  // threads at 64 registers
+  const size_t full = (size_t)kSms * 1024;  // threads at 64 registers
   return (size_t)f.W * f.H > full ? launch_plain_nt<NT, 1024 / NT>(f, st) : launch_plain_nt<NT, 1>(f, st);
 }
 

@@ -98,6 +98,8 @@ __global__ void __launch_bounds__(128) k_sur_label(const float4* __restrict__ pt
   }
   unsigned aux = 0;
   if (want_gt) {
+    // the clamped general sampler, a test for the box at every step
+    static_assert(!SampleAny::kInside, "whole groups of steps are not for arbitrary training points");
     GtShadeT<SampleAny> sh{&g, SampleAny(f.vol), TfAlpha{gs.alpha, f.tf_n}, gs.occ, gs.sdw};
     GtShadeT<SampleAny>::Ray r;
     sh.begin(r, dir);

@@ -187,7 +187,10 @@ typedef struct cvr_frame_stats {
   uint64_t aux_fetches;     /* secondary lookups: SAT box queries (extinction), pyramid
                                taps (cone; the surrogate: 67 per shaded sample),
                                light-ray volume samples (ground truth) */
-  float kernel_ms;          /* device time of the render kernel (CUDA events) */
+  float kernel_ms;          /* device time of the frame's kernels and of the tables that
+                               they were first to need (CUDA events); a cone, ground-truth
+                               or surrogate frame's sample lists are allocated, and its
+                               passes' code loaded, before it starts */
 } cvr_frame_stats;
 
 /* ---- context ------------------------------------------------------------ */
@@ -368,7 +371,7 @@ int cvr_get_walk_tables(const cvr_ctx* ctx);
  * counterpart): the box tables of shadow and of occlusion (at most 24 GiB each)
  * and the 32-bit table that they are made from, the sample lists of deferred
  * frames (4.5 GiB), and the quad copies of volumes and pyramids that no layout
- * asks for (2 GiB each).  One above 64 MiB is made only when it leaves half of
+ * asks for (2 GiB each).  One above 1 GiB is made only when it leaves half of
  * the free memory; tables, their source and lists go when another allocation of
  * the context finds no room.  This bounds each of them to 'bytes' as well, in
  * the context and the batches created afterwards, and frees those above it at
